@@ -431,6 +431,9 @@ long long out_floats(long long rows) {
   return (long long)s.conv_shape[0] * C * Ho * Wo;
 }
 
+// row pitch of the feature-major activation buffers: every feature starts on a 16-byte boundary
+long long act_ld(long long rows) { return (rows + 3) / 4 * 4; }
+
 void ensure_buffers(long long rows) {
   Session& s = S();
   if (rows <= s.buf_rows && s.din) return;
@@ -442,8 +445,8 @@ void ensure_buffers(long long rows) {
   s.dout = (float*)pool_alloc(out_floats(rows) * 4);
   (void)nout;
   const bool need_act = s.model.is_mlp() && s.model.layers.size() > 1;
-  s.act0 = need_act ? (float*)pool_alloc(rows * wmax * 4) : nullptr;
-  s.act1 = need_act && s.model.layers.size() > 2 ? (float*)pool_alloc(rows * wmax * 4) : nullptr;
+  s.act0 = need_act ? (float*)pool_alloc(act_ld(rows) * wmax * 4) : nullptr;
+  s.act1 = need_act && s.model.layers.size() > 2 ? (float*)pool_alloc(act_ld(rows) * wmax * 4) : nullptr;
   if (!s.din || !s.dout || (need_act && !s.act0)) throw std::runtime_error("out of device memory for the model buffers");
   s.buf_rows = rows;
   drop_graph();
@@ -617,7 +620,9 @@ void download_stores(PlanDev& P, const int* args, int nargs, bool multi_plane, c
 // ---------------------------------------------------------------------------------------------------------------
 // the step
 // ---------------------------------------------------------------------------------------------------------------
-constexpr long long kF32TcMinRows = 512;     // below this the per-layer FFMA kernels win on latency
+// fortis_gemm: from this batch on the weights are split once per address (constants of the caller); below it W is read as
+// it is on every call, by the FFMA kernel
+constexpr long long kGemmTcMinRows = 512;
 
 struct StepArgs {
   bool use_gather = false;      // model input comes from the gather plan (else din)
@@ -725,13 +730,15 @@ void run_step_kernels(const StepArgs& A) {
   const int nl = (int)s.model.layers.size();
   if (s.model.is_conv()) {
     std::string err;
-    if (!conv_forward(s.conv, s.din, s.dout, s.conv_shape[0], s.conv_shape[1], s.conv_shape[2], s.conv_shape[3], st, &err))
+    ensure_aux(1);
+    if (!conv_forward(s.conv, s.din, s.dout, s.conv_shape[0], s.conv_shape[1], s.conv_shape[2], s.conv_shape[3], s.d_status, st, &err))
       throw std::runtime_error(err);
     return;
   }
   if (s.model.is_opnet()) {
     std::string err;
-    if (!opnet_forward(s.opnet, s.din, s.dout, s.conv_shape[0], s.conv_shape[2], s.conv_shape[3], st, &err)) throw std::runtime_error(err);
+    ensure_aux(1);
+    if (!opnet_forward(s.opnet, s.din, s.dout, s.conv_shape[0], s.conv_shape[2], s.conv_shape[3], s.d_status, st, &err)) throw std::runtime_error(err);
     return;
   }
   const bool fuse = s.fuse && !A.unfused;
@@ -751,8 +758,9 @@ void run_step_kernels(const StepArgs& A) {
     if (fuse_out) { L.SP = s.S.hdr; L.stores = (const StoreTarget*)s.S.items; L.TS = A.TS; L.fast_out = 1;
                     L.store_by_slot = s.S.store_by_slot; std::memcpy(L.cout, s.S.cls, sizeof L.cout); }
     L.Y = fuse_out ? nullptr : s.dout;
+    L.act[0] = s.act0; L.act[1] = s.act1; L.act_ld = act_ld(s.buf_rows);
     L.g = g;
-    ensure_aux(tc_grid(s.tc, rows));
+    ensure_aux(std::max(tc_grid(s.tc, rows), f32tc_grid(rows)));
     L.partials = (fuse_out && s.want_checksum) ? s.d_partials : nullptr;
     L.sum = L.partials ? s.d_sum : nullptr; L.done = s.d_done;
     L.status = s.d_status;
@@ -796,7 +804,7 @@ void run_step_kernels(const StepArgs& A) {
     if (L.partials) launch_fold(s.d_partials, L.grid, s.d_sum, 1, st);
     return;
   }
-  if (s.f32 && rows >= kF32TcMinRows) {
+  if (s.f32) {
     // fp32 on the tensor cores: one split-TF32 kernel per layer, gather fused into the first layer's operand load and
     // scatter (+ checksum) into the last epilogue when the descriptors are table-driven, activations feature-major
     F32TcLaunch L{};
@@ -810,7 +818,7 @@ void run_step_kernels(const StepArgs& A) {
     if (fuse_out) { L.fast_out = 1; L.store_by_slot = s.S.store_by_slot; L.TS = A.TS; std::memcpy(L.cout, s.S.cls, sizeof L.cout); }
     else L.Y = s.dout;
     L.g = g;
-    L.act[0] = s.act0; L.act[1] = s.act1; L.act_ld = s.buf_rows;
+    L.act[0] = s.act0; L.act[1] = s.act1; L.act_ld = act_ld(s.buf_rows);
     ensure_aux(f32tc_grid(rows));
     if (fuse_out && s.want_checksum) { L.partials = s.d_partials; L.sum = s.d_sum; L.done = s.d_done; }
     L.status = s.d_status;
@@ -1695,7 +1703,7 @@ void fortis_gemm(float* Aa, float* A, long Ao, long As0, long As1, long At0, lon
                  B, K, At0, At1, N, K, Wt0, Wt1, B, N, Ct0, Ct1);
     return;
   }
-  if (B >= kF32TcMinRows) {
+  if (B >= kGemmTcMinRows) {
     // large batch: the tensor-core kernel (three TF32 MMAs per product, fp32-class accuracy)
     S();
     ensure_aux(1);
@@ -1733,7 +1741,9 @@ static void conv3d_entry(const char* who, float* x, long xo, float* w, long wo, 
   }
   const int K[3] = {(int)KD, (int)KH, (int)KW}, st[3] = {(int)sd, (int)sh, (int)sw}, pad[3] = {(int)pd, (int)ph, (int)pw};
   std::string err;
-  if (!conv3d_ncdhw(x + xo, w + wo, y + yo, (int)N, (int)C, (int)Din, (int)Hin, (int)Win, (int)F, K, st, pad, stream(), &err))
+  S();
+  ensure_aux(1);
+  if (!conv3d_ncdhw(x + xo, w + wo, y + yo, (int)N, (int)C, (int)Din, (int)Hin, (int)Win, (int)F, K, st, pad, S().d_status, stream(), &err))
     std::fprintf(stderr, "%s: %s\n", who, err.c_str());
 }
 

@@ -105,6 +105,7 @@ struct TcLaunch {
   RowGeom g;
   const float* X;                                    // (rows, n_in) when there is no gather plan
   float* Y;                                          // (rows, n_out) when there is no scatter plan (may be set with SP too)
+  float* act[2]; long long act_ld;                   // activation buffers of the layer-by-layer form, as F32TcLaunch
   double* partials;                                  // per-CTA checksum partials (size >= tc_grid())
   double* sum; unsigned int* done;                   // optional: fold the partials into *sum inside the kernel (done: zeroed counter)
   int* status;                                       // device word: 0 ok, else the code of the wait that gave up
@@ -130,6 +131,36 @@ struct F32TcLaunch {
 };
 int f32tc_grid(long long nrows);
 bool f32tc_forward(F32TcModel* m, const F32TcLaunch& L, cudaStream_t s, std::string* err);
+// Extents and element strides of one convolution layer (cross-correlation, zero padding)
+struct ConvGeom {
+  int N, D, H, W, C, F;
+  int KD, KH, KW, pd, ph, pw, sd, sh, sw;
+  int dd, dh, dw;                             // input dilation (1 = none): tap positions that fall between input samples read zero
+  int Do, Ho, Wo;
+  long long xs_n, xs_d, xs_h, xs_w, xs_c;     // element strides of x
+  long long ys_n, ys_d, ys_h, ys_w, ys_c;     // element strides of y
+  long long rs_n, rs_d, rs_h, rs_w, rs_c;     // element strides of the residual, where there is one
+};
+// the 16-bit forms of the same kernel: MLPs of few rows, layer by layer
+struct F16Layer {
+  const void* w;                                       // [N_pad][K_pad] 16-bit, zero padded
+  int K_pad, N_pad, k_real, n_real;
+  const float *bias, *scale;                           // [N_pad]; scale null without FP8 weights
+  float slope;                                         // act(v) = max(v, v * slope)
+};
+struct RowsMlp;
+RowsMlp* rows_mlp_create(const std::vector<F16Layer>& layers, bool f16, const float* in_div, const float* out_mul, const float* relu_mask,
+                         std::string* err);
+void rows_mlp_destroy(RowsMlp* m);
+bool rows_mlp_forward(RowsMlp* m, const F32TcLaunch& L, cudaStream_t s, std::string* err);
+// one fp32 convolution layer on the same kernel (rows = output voxels, reduction = taps x channels)
+struct F32ConvW;                                       // split weights of one layer
+bool f32tc_conv_supported(const ConvGeom& g);
+F32ConvW* f32tc_conv_pack(const float* w_dev, int F, int C, int taps, cudaStream_t s, std::string* err);
+void f32tc_conv_free(F32ConvW* w);
+// `early`: the launch may start (and read its weights) before the kernel in front of it in the stream has finished
+bool f32tc_conv(const F32ConvW* w, const float* x, const float* bias, const float* residual, float* y, const ConvGeom& g, int act,
+                float slope, int* status, cudaStream_t s, bool early, std::string* err);
 // C[M][N] = A[M][K] . W[N][K]^T, row-major device operands (the memref entry fortis_gemm)
 bool f32tc_gemm(const float* A, const float* W, float* C, long long M, int N, int K, int* status, cudaStream_t s, std::string* err);
 
@@ -140,16 +171,16 @@ void conv_model_destroy(ConvModel* m);
 int conv_model_status(ConvModel* m);
 void conv_model_clear_status(ConvModel* m);        // 0, or the code of a bounded wait that gave up in the tensor-core conv kernel
 // x (N,D,H,W,Cin) fp32 NDHWC on the device -> y (N,D,H,W,Cout)
-bool conv_forward(ConvModel* m, const float* x, float* y, int N, int D, int H, int W, cudaStream_t s, std::string* err);
+bool conv_forward(ConvModel* m, const float* x, float* y, int N, int D, int H, int W, int* status, cudaStream_t s, std::string* err);
 // single layer, NCDHW fp32 (the memref ABI of runtime/fortis_rt.c:128-131)
 // networks of 2-D operator layers (NCHW fp32)
 struct OpNet;
 OpNet* opnet_create(const ModelHost& M, std::string* err);
 void opnet_destroy(OpNet* m);
 bool opnet_shape(const ModelHost& M, int H, int W, int* C, int* Ho, int* Wo, long long* max_elems_per_image);
-bool opnet_forward(OpNet* m, const float* x, float* y, int N, int H, int W, cudaStream_t s, std::string* err);
+bool opnet_forward(OpNet* m, const float* x, float* y, int N, int H, int W, int* status, cudaStream_t s, std::string* err);
 bool conv3d_ncdhw(const float* x, const float* w, float* y, int N, int C, int D, int H, int W, int F, const int K[3],
-                  const int stride[3], const int pad[3], cudaStream_t s, std::string* err);
+                  const int stride[3], const int pad[3], int* status, cudaStream_t s, std::string* err);
 
 // tensor-core conv network (fortis_conv3d_tc.cu): bf16 activations in a zero-padded channels-last volume
 struct ConvTcModel;

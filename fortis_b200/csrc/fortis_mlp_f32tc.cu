@@ -1,31 +1,41 @@
-// fp32-class Linear layers on the tensor cores: C = act(A . W^T + b) with every product formed as three TF32 MMAs
+// fp32-class Linear layers and convolutions on the tensor cores: C = act(A . W^T + b) with every product formed as three
+// TF32 MMAs
 //     A . W  ~=  A_hi . W_hi + A_hi . W_lo + A_lo . W_hi        (x_hi = tf32(x), x_lo = x - x_hi, accumulation in fp32)
-// which keeps 21 significant bits per operand: 9e-7 relative L2 against fp64 on the 244 -> 768 x4 -> 128 column network,
-// the same as fp32 FFMA arithmetic, at six bf16-MMA-equivalents per multiply-add instead of one FFMA per MAC.
+// which keeps 21 significant bits per operand at six bf16-MMA-equivalents per multiply-add instead of one FFMA per MAC.
 //
 // Replaces, for the fp32 precision, the reference's large-batch lowering of a Linear layer: fortis_gemm = cuBLAS SGEMM on
 // pre-transposed weights plus a separate bias / activation kernel (runtime/fortis_rt.c:45-75, compiler/FortisFuse.cpp:616-624,
-// 687-760), with fortis_gather_k in front and fortis_scatter_k behind (driver/fortis_gather_emit.py:52-62, 75-83): the
-// gather is fused into the first layer's operand load, bias + activation into every epilogue, the scatter (and the fp64
-// checksum) into the last one.  Activations travel between layers in fp32, feature-major ([feature][row]: the memory
-// order of a Fortran (ncol, nlev) array), so both the epilogue's stores and the next layer's loads are coalesced with
-// one thread per row.
+// 687-760), with fortis_gather_k in front and fortis_scatter_k behind (driver/fortis_gather_emit.py:52-62, 75-83), and its
+// cuDNN convolutions (runtime/fortis_rt.c:108-156): the gather is fused into the first layer's operand load, bias +
+// residual + activation into every epilogue, the scatter (and the fp64 checksum) into the last one.  Activations travel
+// between layers in fp32, feature-major ([feature][row]: the memory order of a Fortran (ncol, nlev) array and of an NCDHW
+// volume), so both the epilogue's stores and the next layer's loads are coalesced with one thread per row.
 //
-// One persistent CTA per SM, output tiles of 128 rows x n_tile (<= 256) features, K in steps of 32:
-//   * warps 2-5 (thread = row) load the tile's activations (from the host arrays through the slot table, from a
-//     feature-major buffer, or from a row-major matrix), split them and write A_hi / A_lo into shared memory in the
-//     K-major 128-byte-swizzled layout the MMA reads;
-//   * warp 0 brings the matching W_hi / W_lo tiles (split once on the host or by a kernel) with two TMA loads;
-//   * warp 1 issues, per 8-wide k step, the three kind::tf32 MMAs (M = 128, N = n_tile) into a 256-column accumulator
-//     in tensor memory;
-//   * warps 6-9 (thread = row) read the accumulator, add the bias, apply the activation and store.
-// The tensor core adds into its fp32 accumulator with truncation, not rounding: measured on this kernel, a relative
-// bias of -6e-9 per unit of K (-4.7e-6 at K = 768, 2.2e-5 over the five layers of the column network).  So K is
-// accumulated in chunks of 128: after each chunk the epilogue warps add the chunk's accumulator into a running sum
-// held in the other 256 tensor-memory columns with IEEE additions (tcgen05.ld, FADD, tcgen05.st), which divides the
-// bias by the number of chunks; the last chunk's pass goes straight on to bias, activation and store.
-// Two stages of 96 KB (A_hi, A_lo 16 KB each; W_hi, W_lo up to 32 KB each).  Every barrier wait is bounded.
+// One persistent CTA per SM, output tiles of 128 rows x NT (32, 64 or 128) features, K in steps of 32:
+//   * fp32 activations arrive as tiles through the TMA (a feature-major buffer, or a row-major matrix whose rows start on
+//     16-byte boundaries), or are loaded by the threads (host arrays through the slot table, other matrices, a volume at
+//     the taps' offsets); two sets of four warps (thread = row; the sets take alternate k steps) split them and write
+//     A_hi / A_lo into TENSOR MEMORY (lane = row);
+//   * one warp brings the matching W_hi / W_lo tiles (split once) into shared memory with two TMA loads;
+//   * one warp issues, per 8-wide k step, the three kind::tf32 MMAs (M = 128, N = NT, A from tensor memory);
+//   * two sets of four warps (thread = row, half of the features) read the accumulator, add bias (and residual), apply the
+//     activation and store.
+// Operand traffic is why A sits in tensor memory: with A in shared memory (the form before this one) the three MMAs of a
+// k step read 12 KB per 128 clocks and the producers and the TMA write 96 KB per 1536, together 1.25 times what shared
+// memory moves; in this form only the weights (64 B/clk at any NT) and the fp32 tiles pass through it.
+// Measured, that form / this one: fortis_gemm 8192 x 768 x 768 756 / 59 us (a row-major operand was read by one dependent load
+// per row), column network 30,011 rows 994 / 769 us; convolutions against the FFMA kernel: 32 -> 64 channels 3x3x3 on 40^3
+// 297 / 70 us, 14-layer network 2 x 33^3 8.76 / 1.80 ms.
+//
+// The tensor core adds into its fp32 accumulator with truncation, not rounding, a bias per accumulation of half a unit in
+// the last place of the partial sum.  Two things keep it below fp32 rounding: the hi.hi products go into an accumulator
+// of their own that is taken over every 64 k (8 truncating additions) and summed by the epilogue warps in registers with
+// IEEE additions, and the two cross products go into a second accumulator (2^-11 of the result, so its truncation does not
+// count) that lives for the whole K.
+// Infinities: x_hi saturates at the largest finite TF32 value and x_lo = x - x_hi carries the infinity, so a product is
+// infinite, or NaN, where the fp32 product is.  Every barrier wait is bounded.
 #include <cuda.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -48,64 +58,196 @@ using namespace tc;
 
 constexpr int kM = 128;                    // rows per tile
 constexpr int kKt = 32;                    // k per stage: one 128-byte swizzle row of fp32
-constexpr int kNtMax = 256;                // widest output tile (the MMA's N)
-constexpr int kStagesF = 2;
-constexpr int kChunkKt = 4;                // k steps of 32 accumulated in the tensor core before the sum is taken over (K = 128)
-constexpr int kABytes = kM * kKt * 4;      // 16 KB per split half
-constexpr int kWBytes = kNtMax * kKt * 4;  // 32 KB per split half
-constexpr int kStageBytesF = 2 * kABytes + 2 * kWBytes;   // 96 KB
-constexpr int kBarF = 128;
+constexpr int kChunkKt = 2;                // k steps of 32 accumulated in the tensor core before the sum is taken over (K = 64)
+constexpr int kBarF = 384;
 constexpr int kTabIn = 768, kTabOut = 256;     // widest gathered input / scattered output the tables hold
-constexpr int kTabBytesF = kTabIn * 5 + kTabOut * 5 + 2 * kMaxArrays * 8 + 64;
-constexpr int kSmemF = kStagesF * kStageBytesF + kBarF + kTabBytesF + 64;
-constexpr int kThreadsF = 320;
-enum { FST_FULL = 21, FST_EMPTY = 22, FST_ACC_FULL = 23, FST_ACC_EMPTY = 24, FST_ALIGN = 25 };
-enum { A_FEATURE_MAJOR = 0, A_ROW_MAJOR = 1, A_GATHER = 2 };
-enum { C_FEATURE_MAJOR = 0, C_ROW_MAJOR = 1, C_SCATTER = 2 };
+constexpr int kTileScratch = 32 * 32 * 4;      // one warp's 32 x 32 transpose
+constexpr int kConvTabMax = 40 * 1024;         // widest table of taps a convolution may need
+// warps 0-7 produce A (two sets of four that take alternate k steps), 8-15 are the epilogue (two sets, half of the
+// features each), then the two TMA warps and the MMA warp.  (Three producer sets and one epilogue set for the
+// convolutions: 64 -> 64 channels 3 % slower.)
+constexpr int kPSets = 2, kPWarps = 8, kESets = 2, kEWarps = 8, kWarpW = 16, kWarpA = 17, kWarpMma = 18;
+constexpr int kThreadsF = 19 * 32;
+constexpr int kRawStages = 4;                  // fp32 activation tiles on their way to the producers, 16 KB each
+constexpr int kRawBytes = kM * kKt * 4;
+enum { FST_A_FULL = 21, FST_A_EMPTY = 22, FST_ACC_FULL = 23, FST_ACC_EMPTY = 24, FST_ALIGN = 25, FST_W_FULL = 26, FST_W_EMPTY = 27, FST_RAW_FULL = 28, FST_RAW_EMPTY = 29 };
+enum { A_TILE_T = 0, A_TILE_R = 1, A_ROW_MAJOR = 2, A_GATHER = 3, A_CONV8 = 4, A_CONV1 = 5 };   // the first two through the TMA
+enum { C_FEATURE_MAJOR = 0, C_ROW_MAJOR = 1, C_SCATTER = 2, C_CONV = 3 };
+
+template <int NT> struct TileCfg {
+  static constexpr int kAStages = NT == 128 ? 2 : 4;     // 64 tensor-memory columns each (32 hi, 32 lo)
+  static constexpr int kWStages = NT == 128 ? 3 : 6;
+  static constexpr int kWHalf = NT * kKt * 4, kWStage = 2 * kWHalf;
+  static constexpr int kWBytes = kWStages * kWStage;
+  static constexpr uint32_t kColCross = 2 * NT, kColA = 3 * NT;   // tensor-memory columns: hi.hi [0,NT) and [NT,2NT), cross, A
+  static_assert(kColA + 64 * kAStages <= 512, "tensor memory");
+};
 
 struct StrideClassF { long long si, sj, sk; };
 
 struct F32Params {
-  CUtensorMap map_hi, map_lo;            // W_hi / W_lo [N_pad][K_pad] fp32, box 32 x n_tile
-  int K_pad, N_pad, n_tile, K_real, N_real;
-  const float* bias;                     // [N_pad] or null
-  float slope;                           // act(v) = max(v, v * slope)
+  CUtensorMap map_hi, map_lo;            // W_hi / W_lo [N_pad][K_pad] fp32, box 32 x NT
+  int K_pad, K_real, N_real, ntn;        // ntn: output tiles along N (16-bit: K_pad counts pairs, a step is 64 inputs)
+  const float* scale;                    // 16-bit forms, FP8 weights: per feature
+  uint32_t* C16;                         // 16-bit forms, hidden layers: [feature / 2][row] pairs
+  const float* bias;                     // [N_real] or null
+  int act; float slope;
   const float* in_div;                   // first layer only, optional
   const float* out_mul;                  // last layer only, optional
   const float* relu_mask;                // last layer only, optional
-  int a_mode; const float* A; long long lda;
+  CUtensorMap map_a;                     // A_TILE_T: [K][rows], box 128 rows x 32; A_TILE_R: [rows][K], box 32 x 128, 128-byte swizzle
+  const float* A; long long lda;
   const Access* slots; ArrayTable TG; StrideClassF cin[2]; RowGeom g;
-  int c_mode; float* C; long long ldc;
+  ConvGeom cv; const float* residual;    // A_CONV*: x = A, y = C
+  int c_mode; float* C; long long ldc; int c_vec;
   const Access* store_by_slot; ArrayTable TS; StrideClassF cout[2];
   long long nrows;
   double* partials; double* sum; unsigned int* done;
   int* status;
 };
 
-// instruction descriptor of kind::tf32: D = f32, A = B = tf32 (format code 2), both K-major, M = 128, N at run time
-__device__ __forceinline__ uint32_t idesc_tf32(int n) {
+// instruction descriptor of kind::tf32: D = f32, A = B = tf32 (format code 2), both K-major, M = 128
+__host__ __device__ constexpr uint32_t idesc_tf32(int n) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kM >> 4) << 24);
 }
 
-__device__ __forceinline__ void mma_tf32_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// kind::f16: D = f32, A = B = bf16 (format code 1) or fp16 (0)
+__host__ __device__ constexpr uint32_t idesc_16(int n, bool f16) {
+  return (1u << 4) | (f16 ? 0u : (1u << 7) | (1u << 10)) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kM >> 4) << 24);
+}
+
+// D[tmem] (+)= A[tmem] . B[smem]^T
+template <uint32_t IDESC>
+__device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p, q;\n\telect.sync _|p, 0xffffffff;\n\tsetp.ne.b32 q, %4, 0;\n\t"
-      "@p tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, q;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+      "@p tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, q;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "n"(IDESC), "r"(accumulate) : "memory");
 }
 
-// x = hi + lo with hi the nearest TF32 value (10 explicit mantissa bits); lo is exact in fp32 and is truncated to TF32
-// by the MMA, which leaves 21 significant bits
-__device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
-  uint32_t h;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(x));
-  hi = __uint_as_float(h);
-  lo = x - hi;
+// x = hi + lo with hi the nearest finite TF32 value (10 explicit mantissa bits); lo is exact in fp32 and is truncated to
+// TF32 by the MMA, which leaves 21 significant bits
+__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
+  asm("cvt.rna.satfinite.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
+  lo = __float_as_uint(x - __uint_as_float(hi));
 }
 
-__device__ __forceinline__ float act_slope(float v, float slope) { return fmaxf(v, v * slope); }
+template <bool F16> __device__ __forceinline__ uint32_t pack_pair(float lo, float hi) {
+  if constexpr (F16) { const __half2 v = __floats2half2_rn(lo, hi); return *reinterpret_cast<const uint32_t*>(&v); }
+  else return pack_bf16(lo, hi);
+}
 
-__global__ void __launch_bounds__(kThreadsF, 1) linear_tf32x3_kernel(const __grid_constant__ F32Params P) {
+template <int N> __device__ __forceinline__ void act_f32(float (&v)[N], int act, float slope) {
+  if (act == ACT_RELU) {
+#pragma unroll
+    for (int j = 0; j < N; j++) v[j] = fmaxf(v[j], 0.f);
+  } else if (act == ACT_LEAKY) {
+#pragma unroll
+    for (int j = 0; j < N; j++) v[j] = v[j] > 0.f ? v[j] : v[j] * slope;
+  }
+}
+
+// a load that keeps its place in front of the wait that follows it; reads 0 where `ok` is 0
+__device__ __forceinline__ float ld_ahead_if(const float* p, bool ok) {
+  float v;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@p ld.global.nc.f32 %0, [%1];\n\t}"
+               : "=f"(v) : "l"(p), "r"((int)ok));
+  return v;
+}
+// One step's activations of a producer thread, and where the next step lies.  `t`, `kt`: tile and k step.
+template <int AMODE>
+struct ACursor {
+  long long t;
+  int kt;
+  const float* rowp;            // conv: the element tap 0 of this row reads (may lie outside the volume)
+  long long p0, p1;             // gather: byte positions of the two stride classes
+  uint32_t md, mh, mw;          // conv: taps per axis that fall inside the volume
+};
+
+template <int AMODE>
+__device__ __forceinline__ void cursor_tile(const F32Params& P, ACursor<AMODE>& c, int r) {
+  const long long m0 = (c.t / P.ntn) * kM;
+  // rows behind the last one read what the last one reads (in bounds); their results are not stored
+  const long long row = m0 + r < P.nrows ? m0 + r : P.nrows - 1;
+  if constexpr (AMODE == A_ROW_MAJOR) c.rowp = P.A + m0 * P.lda;
+  if constexpr (AMODE == A_GATHER) {
+    long long ci, cj, kk;
+    row_to_pos(P.g, row, &ci, &cj, &kk);
+    c.p0 = 4 * (ci * P.cin[0].si + cj * P.cin[0].sj + kk * P.cin[0].sk);
+    c.p1 = 4 * (ci * P.cin[1].si + cj * P.cin[1].sj + kk * P.cin[1].sk);
+  }
+  if constexpr (AMODE == A_CONV8 || AMODE == A_CONV1) {
+    const ConvGeom& g = P.cv;
+    unsigned q = (unsigned)row;
+    const int ow = (int)(q % (unsigned)g.Wo); q /= (unsigned)g.Wo;
+    const int oh = (int)(q % (unsigned)g.Ho); q /= (unsigned)g.Ho;
+    const int od = (int)(q % (unsigned)g.Do);
+    const int on = (int)(q / (unsigned)g.Do);
+    const int id = od * g.sd - g.pd, ih = oh * g.sh - g.ph, iw = ow * g.sw - g.pw;
+    c.rowp = P.A + ((long long)on * g.xs_n + (long long)id * g.xs_d + (long long)ih * g.xs_h + (long long)iw * g.xs_w);
+    auto inside = [](int first, int extent, int taps) {          // bit k: 0 <= first + k < extent
+      const int lo = first < 0 ? -first : 0, hi = extent - first < taps ? extent - first : taps;
+      const uint32_t upto = hi <= 0 ? 0u : (hi >= 32 ? 0xFFFFFFFFu : (1u << hi) - 1u);
+      return lo >= 32 ? 0u : (upto >> lo) << lo;
+    };
+    c.md = inside(id, g.D, g.KD); c.mh = inside(ih, g.H, g.KH); c.mw = inside(iw, g.W, g.KW);
+  }
+}
+
+template <int AMODE, int STEP>
+__device__ __forceinline__ void cursor_advance(const F32Params& P, ACursor<AMODE>& c, int nkt, long long ntiles, int r) {
+  c.kt += STEP;
+  if (c.kt < nkt) return;
+  while (c.kt >= nkt) { c.kt -= nkt; c.t += gridDim.x; }
+  if (c.t < ntiles) cursor_tile<AMODE>(P, c, r);
+}
+
+// `tab`: gather: 64-bit addresses (bit 0: stride class, 0: no such input); conv: {element offset, taps | channels << 24}
+template <int AMODE>
+__device__ __forceinline__ void cursor_load(const F32Params& P, const ACursor<AMODE>& c, const uint2* tab, int quad, int lane, int k0, float (&v)[kKt]) {
+  if constexpr (AMODE == A_ROW_MAJOR) {
+    // rows that do not start on 16-byte boundaries: one row per instruction, a whole line each; publish() turns the warp's
+    // 32 x 32 block so that a thread holds its row
+    const long long m0 = (c.t / P.ntn) * kM + quad * 32;
+    const float* base = c.rowp + (long long)(quad * 32) * P.lda + k0;
+#pragma unroll
+    for (int rr = 0; rr < 32; rr++) v[rr] = ld_ahead_if(base + (long long)rr * P.lda + lane, k0 + lane < P.K_real && m0 + rr < P.nrows);
+  } else if constexpr (AMODE == A_GATHER) {
+#pragma unroll
+    for (int j = 0; j < kKt; j++) {
+      const unsigned long long e = *reinterpret_cast<const unsigned long long*>(tab + k0 + j);
+      v[j] = ld_ahead_if(reinterpret_cast<const float*>((e & ~1ull) + (unsigned long long)((e & 1ull) ? c.p1 : c.p0)), e != 0ull);
+    }
+  } else if constexpr (AMODE == A_CONV8) {
+#pragma unroll
+    for (int gq = 0; gq < kKt / 8; gq++) {
+      const uint2 e = tab[k0 / 8 + gq];
+      const bool in = ((c.md >> (e.y & 0xFF)) & (c.mh >> ((e.y >> 8) & 0xFF)) & (c.mw >> ((e.y >> 16) & 0xFF)) & 1u) != 0u;
+      const float* p = c.rowp + (int)e.x;
+      const int n = (int)(e.y >> 24);
+      if (n == 8) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) { v[8 * gq + j] = ld_ahead_if(p, in); p += P.cv.xs_c; }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; j++) { v[8 * gq + j] = ld_ahead_if(p, in && j < n); p += P.cv.xs_c; }
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < kKt; j++) {
+      const uint2 e = tab[k0 + j];
+      const bool in = ((c.md >> (e.y & 0xFF)) & (c.mh >> ((e.y >> 8) & 0xFF)) & (c.mw >> ((e.y >> 16) & 0xFF)) & (e.y >> 24)) != 0u;
+      v[j] = ld_ahead_if(c.rowp + (int)e.x, in);
+    }
+  }
+}
+
+// P16: 0 = fp32 as three TF32 products, 1 = bf16, 2 = fp16 (one product, one accumulator for the whole K: the arithmetic
+// of the fused 16-bit kernel, whose results these forms reproduce bit for bit)
+template <int NT, int AMODE, int P16>
+__global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_constant__ F32Params P) {
+  using CF = TileCfg<NT>;
   extern __shared__ __align__(1024) uint8_t smem[];
   // Programmatic dependent launch: the next layer's CTAs may be scheduled as SMs free up; they set up, start streaming
   // their weights, and wait (griddepcontrol.wait in the warps that read or write activations) for this grid to finish.
@@ -115,59 +257,78 @@ __global__ void __launch_bounds__(kThreadsF, 1) linear_tf32x3_kernel(const __gri
     if (threadIdx.x == 0) atomicCAS(P.status, 0, FST_ALIGN);
     return;
   }
-  uint8_t* tail = smem + kStagesF * kStageBytesF;
-  const uint32_t bars = base + kStagesF * kStageBytesF;
-  // barrier block: full [2] | empty [2] | acc_full [2] | acc_empty [2]; tmem base 64, abort flag 68, checksum scratch [72,104)
-  const uint32_t bar_full = bars, bar_empty = bars + 16, bar_acc_full = bars + 32, bar_acc_empty = bars + 48;
-  uint32_t* tmem_slot = (uint32_t*)(tail + 64);
-  volatile int* abort_flag = (volatile int*)(tail + 68);
-  uint32_t* s_off = (uint32_t*)(tail + kBarF);
-  uint32_t* o_off = s_off + kTabIn;
-  uint8_t* s_code = (uint8_t*)(o_off + kTabOut);
-  uint8_t* o_code = s_code + kTabIn;
-  const float** s_base_in = (const float**)(((uintptr_t)(o_code + kTabOut) + 15) & ~(uintptr_t)15);
-  float** s_base_out = (float**)(s_base_in + kMaxArrays);
+  // W stages | fp32 activation tiles | barriers, 384 bytes | bias and scale per epilogue warp | transposes of row-major operands | table of the A mode | table of the scatter
+  constexpr int kRawOff = CF::kWBytes, kTailOff = kRawOff + (AMODE == A_TILE_T || AMODE == A_TILE_R ? kRawStages * kRawBytes : 0);
+  uint8_t* tail = smem + kTailOff;
+  const uint32_t bars = base + kTailOff;
+  // barriers: a_full [4] | a_empty [4] | w_full [6] | w_empty [6] | acc_full [2] | acc_empty [2] | cross_empty; then at 200
+  // the tensor-memory base, at 204 the abort flag, at 208 raw_full [4] | raw_empty [4], at 272 the checksum's warp sums
+  constexpr int kWStep = P16 ? CF::kWHalf : CF::kWStage;            // weight bytes per step
+  const uint32_t a_full = bars, a_empty = bars + 32, w_full = bars + 64, w_empty = bars + 112, acc_full = bars + 160, acc_empty = bars + 176,
+                 cross_empty = bars + 192, raw_full = bars + 208, raw_empty = bars + 240;
+  uint32_t* tmem_slot = (uint32_t*)(tail + 200);
+  volatile int* abort_flag = (volatile int*)(tail + 204);
+  constexpr bool kTile = AMODE == A_TILE_T || AMODE == A_TILE_R;
+  uint8_t* a_scratch = tail + kBarF + kEWarps * 2 * (NT / kESets) * 4;
+  uint8_t* c_scratch = a_scratch + (AMODE == A_ROW_MAJOR ? kPWarps * kTileScratch : 0);
+  uint8_t* tables = c_scratch + (P.c_mode == C_ROW_MAJOR ? kEWarps * kTileScratch : 0);
+  const int nkt = P.K_pad / kKt;
+  uint2* tab = (uint2*)tables;
+  const int ntab = AMODE == A_GATHER ? P.K_pad * (P16 ? 2 : 1) : AMODE == A_CONV8 ? nkt * (kKt / 8) : AMODE == A_CONV1 ? nkt * kKt : 0;
+  unsigned long long* o_tab = (unsigned long long*)(tab + ntab);      // scatter: 64-bit addresses, as the gather's
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ntn = P.N_pad / P.n_tile;
-  const long long ntm = (P.nrows + kM - 1) / kM, ntiles = ntm * ntn;
-  const int nkt = P.K_pad / kKt;
-  const uint32_t w_bytes = (uint32_t)(P.n_tile * kKt * 4);
+  const long long ntm = (P.nrows + kM - 1) / kM, ntiles = ntm * P.ntn;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStagesF; s++) { mbar_init(bar_full + 8 * s, 1 + kM); mbar_init(bar_empty + 8 * s, 1); }
-    mbar_init(bar_acc_full, 1);
-    mbar_init(bar_acc_empty, kM);
+    for (int s = 0; s < CF::kAStages; s++) { mbar_init(a_full + 8 * s, 4); mbar_init(a_empty + 8 * s, 1); }
+    for (int s = 0; s < CF::kWStages; s++) { mbar_init(w_full + 8 * s, 1); mbar_init(w_empty + 8 * s, 1); }
+    for (int s = 0; s < 2; s++) { mbar_init(acc_full + 8 * s, 1); mbar_init(acc_empty + 8 * s, kEWarps); }
+    mbar_init(cross_empty, kEWarps);
+    for (int s = 0; s < kRawStages; s++) { mbar_init(raw_full + 8 * s, 1); mbar_init(raw_empty + 8 * s, 4); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (threadIdx.x < kMaxArrays) {
-    s_base_in[threadIdx.x] = (const float*)P.TG.base[threadIdx.x];
-    s_base_out[threadIdx.x] = (float*)P.TS.base[threadIdx.x];
-  }
-  if (P.a_mode == A_GATHER)
-    for (int q = threadIdx.x; q < kTabIn; q += kThreadsF) {
-      uint8_t code = 0xFF; uint32_t off = 0;
+  if constexpr (AMODE == A_GATHER) {
+    for (int q = threadIdx.x; q < ntab; q += kThreadsF) {
+      unsigned long long e = 0;
       if (q < P.K_real) {
         const Access a = P.slots[q];
-        code = (uint8_t)(a.array | ((a.si == P.cin[0].si && a.sj == P.cin[0].sj && a.sk == P.cin[0].sk) ? 0 : 0x80));
-        off = (uint32_t)a.off0;
+        const bool c0 = a.si == P.cin[0].si && a.sj == P.cin[0].sj && a.sk == P.cin[0].sk;
+        e = (unsigned long long)((const float*)P.TG.base[a.array] + a.off0) | (c0 ? 0ull : 1ull);
       }
-      s_code[q] = code; s_off[q] = off;
+      reinterpret_cast<unsigned long long*>(tab)[q] = e;
     }
+  }
+  if constexpr (AMODE == A_CONV8 || AMODE == A_CONV1) {
+    const ConvGeom& g = P.cv;
+    constexpr int G = AMODE == A_CONV8 ? 8 : 1;
+    const int per_tap = (g.C + G - 1) / G, ntaps = g.KD * g.KH * g.KW;
+    for (int q = threadIdx.x; q < ntab; q += kThreadsF) {
+      uint2 e = make_uint2(0u, 0u);
+      if (q < ntaps * per_tap) {
+        const int tap = q / per_tap, c0 = (q - tap * per_tap) * G;
+        const int kd = tap / (g.KH * g.KW), kh = (tap / g.KW) % g.KH, kw = tap % g.KW;
+        const int n = g.C - c0 < G ? g.C - c0 : G;
+        e.x = (uint32_t)(int)((long long)kd * g.xs_d + (long long)kh * g.xs_h + (long long)kw * g.xs_w + (long long)c0 * g.xs_c);
+        e.y = (uint32_t)kd | ((uint32_t)kh << 8) | ((uint32_t)kw << 16) | ((uint32_t)n << 24);
+      }
+      tab[q] = e;
+    }
+  }
   if (P.c_mode == C_SCATTER)
     for (int n = threadIdx.x; n < kTabOut; n += kThreadsF) {
-      uint8_t code = 0xFF; uint32_t off = 0;
+      unsigned long long e = 0;
       if (n < P.N_real && P.store_by_slot[n].array >= 0) {
         const Access a = P.store_by_slot[n];
-        code = (uint8_t)(a.array | ((a.si == P.cout[0].si && a.sj == P.cout[0].sj && a.sk == P.cout[0].sk) ? 0 : 0x80));
-        off = (uint32_t)a.off0;
+        const bool c0 = a.si == P.cout[0].si && a.sj == P.cout[0].sj && a.sk == P.cout[0].sk;
+        e = (unsigned long long)((float*)P.TS.base[a.array] + a.off0) | (c0 ? 0ull : 1ull);
       }
-      o_code[n] = code; o_off[n] = off;
+      o_tab[n] = e;
     }
-  if (warp == 0 && lane < 2)
+  if (warp == kWarpW && lane < 2)
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(lane ? &P.map_lo : &P.map_hi)) : "memory");
-  if (warp == 1) {
+  if (warp == kWarpMma) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -176,226 +337,406 @@ __global__ void __launch_bounds__(kThreadsF, 1) linear_tf32x3_kernel(const __gri
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA: the W_hi / W_lo tiles of every stage
+  if (warp == kWarpW) {
+    // ------------------------------------------------------------------ TMA: the W_hi / W_lo tiles of every step
     uint32_t s = 0, ph = 0;
     bool stop = false;
     for (long long t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
-      const int n0 = (int)(t % ntn) * P.n_tile;
+      const int n0 = (int)(t % P.ntn) * NT;
       for (int kt = 0; kt < nkt; kt++) {
-        if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, P.status, FST_EMPTY)) { stop = true; break; }
-        mbar_expect_tx(bar_full + 8 * s, 2 * w_bytes);
-        const uint32_t st = base + s * kStageBytesF + 2 * kABytes;
-        tma_load_2d(st, &P.map_hi, kt * kKt, n0, bar_full + 8 * s);
-        tma_load_2d(st + kWBytes, &P.map_lo, kt * kKt, n0, bar_full + 8 * s);
-        if (++s == kStagesF) { s = 0; ph ^= 1; }
-      }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    uint32_t s = 0, ph = 0, chunk_it = 0;
-    const uint64_t desc_hi = make_kmajor_sw128_desc(0) & 0xFFFFFFFF00000000ull;
-    const uint32_t idesc = idesc_tf32(P.n_tile);
-    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-      for (int kt0 = 0; kt0 < nkt; kt0 += kChunkKt, chunk_it++) {
-        // the chunk accumulator (columns 0..255) is free again once the epilogue warps have taken the previous chunk over
-        mbar_wait(bar_acc_empty, (chunk_it & 1) ^ 1, abort_flag, P.status, FST_ACC_EMPTY);
-        tc_fence_after();
-        const int kt1 = kt0 + kChunkKt < nkt ? kt0 + kChunkKt : nkt;
-        for (int kt = kt0; kt < kt1; kt++) {
-          mbar_wait(bar_full + 8 * s, ph, abort_flag, P.status, FST_FULL);
-          tc_fence_after();
-          const uint32_t st = base + s * kStageBytesF;
-          const uint64_t ah = desc_hi | (uint64_t)((st >> 4) & 0x3FFF), al = desc_hi | (uint64_t)(((st + kABytes) >> 4) & 0x3FFF);
-          const uint64_t wh = desc_hi | (uint64_t)(((st + 2 * kABytes) >> 4) & 0x3FFF);
-          const uint64_t wl = desc_hi | (uint64_t)(((st + 2 * kABytes + kWBytes) >> 4) & 0x3FFF);
-#pragma unroll
-          for (int j = 0; j < kKt / 8; j++) {             // 8 tf32 = 32 bytes per k step: the address field moves by 2
-            mma_tf32_ss(tmem, ah + (uint64_t)(2 * j), wh + (uint64_t)(2 * j), idesc, (uint32_t)((kt - kt0) | j));
-            mma_tf32_ss(tmem, ah + (uint64_t)(2 * j), wl + (uint64_t)(2 * j), idesc, 1u);
-            mma_tf32_ss(tmem, al + (uint64_t)(2 * j), wh + (uint64_t)(2 * j), idesc, 1u);
-          }
-          tc_commit(bar_empty + 8 * s);
-          if (++s == kStagesF) { s = 0; ph ^= 1; }
-        }
-        tc_commit(bar_acc_full);
-      }
-    }
-  } else if (warp < 6) {
-    // ------------------------------------------------------------------ A producers: thread = row of the tile
-    asm volatile("griddepcontrol.wait;" ::: "memory");         // the previous layer's activations are complete and visible
-    const int r = (warp - 2) * 32 + lane;
-    uint32_t s = 0, ph = 0;
-    bool stop = false;
-    for (long long t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
-      const long long m0 = (t / ntn) * kM;
-      const long long row = m0 + r;
-      const bool live = row < P.nrows;
-      long long p0 = 0, p1 = 0;
-      if (P.a_mode == A_GATHER) {
-        long long ci = 0, cj = 0, kk = 0;
-        if (live) row_to_pos(P.g, row, &ci, &cj, &kk);
-        p0 = ci * P.cin[0].si + cj * P.cin[0].sj + kk * P.cin[0].sk;
-        p1 = ci * P.cin[1].si + cj * P.cin[1].sj + kk * P.cin[1].sk;
-      }
-      for (int kt = 0; kt < nkt; kt++) {
-        const int k0 = kt * kKt;
-        if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, P.status, FST_EMPTY)) { stop = true; break; }
-        uint8_t* a_hi = smem + s * kStageBytesF;
-        uint8_t* a_lo = a_hi + kABytes;
-        if (P.a_mode == A_ROW_MAJOR) {
-          // lanes run along k: one coalesced 128-byte read per row; element (row rr, k = lane) lands in 16-byte piece
-          // (lane / 4) ^ (rr % 8) of the row's 128-byte line
-          const int rb = (warp - 2) * 32;
-          const bool kin = k0 + lane < P.K_real;
-#pragma unroll 8
-          for (int rr = 0; rr < 32; rr++) {
-            const long long rw = m0 + rb + rr;
-            float x = 0.f;
-            if (kin && rw < P.nrows) {
-              x = __ldg(P.A + rw * P.lda + k0 + lane);
-              if (P.in_div) x = __fdiv_rn(x, __ldg(P.in_div + k0 + lane));
-            }
-            float hi, lo;
-            split_tf32(x, hi, lo);
-            const int off = (rb + rr) * 128 + ((((lane >> 2) ^ ((rb + rr) & 7)) << 4) | ((lane & 3) << 2));
-            *reinterpret_cast<float*>(a_hi + off) = hi;
-            *reinterpret_cast<float*>(a_lo + off) = lo;
-          }
+        if (!mbar_wait(w_empty + 8 * s, ph ^ 1, abort_flag, P.status, FST_W_EMPTY)) { stop = true; break; }
+        mbar_expect_tx(w_full + 8 * s, kWStep);
+        const uint32_t st = base + s * CF::kWStage;
+        if constexpr (P16 != 0) {
+          tma_load_2d(st, &P.map_hi, kt * 64, n0, w_full + 8 * s);
         } else {
-          float v[kKt];
-          if (P.a_mode == A_GATHER) {
+          tma_load_2d(st, &P.map_hi, kt * kKt, n0, w_full + 8 * s);
+          tma_load_2d(st + CF::kWHalf, &P.map_lo, kt * kKt, n0, w_full + 8 * s);
+        }
+        if (++s == CF::kWStages) { s = 0; ph ^= 1; }
+      }
+    }
+  } else if (warp == kWarpA) {
+    // ------------------------------------------------------------------ TMA: the fp32 activations of every step
+    if constexpr (kTile) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");       // the previous layer's activations are complete and visible
+      uint32_t s = 0, ph = 0;
+      bool stop = false;
+      for (long long t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
+        const int m0 = (int)((t / P.ntn) * kM);
+        for (int kt = 0; kt < nkt; kt++) {
+          if (!mbar_wait(raw_empty + 8 * s, ph ^ 1, abort_flag, P.status, FST_RAW_EMPTY)) { stop = true; break; }
+          mbar_expect_tx(raw_full + 8 * s, kRawBytes);
+          if constexpr (AMODE == A_TILE_T) tma_load_2d(base + kRawOff + s * kRawBytes, &P.map_a, m0, kt * kKt, raw_full + 8 * s);
+          else tma_load_2d(base + kRawOff + s * kRawBytes, &P.map_a, kt * kKt, m0, raw_full + 8 * s);
+          if (++s == kRawStages) { s = 0; ph ^= 1; }
+        }
+      }
+    }
+  } else if (warp == kWarpMma) {
+    // ------------------------------------------------------------------ MMA issuer
+    uint32_t as = 0, aph = 0, ws = 0, wph = 0, chunk_it = 0, tile_it = 0;
+    const uint64_t desc_hi = make_kmajor_sw128_desc(0) & 0xFFFFFFFF00000000ull;
+    constexpr uint32_t idesc = P16 == 0 ? idesc_tf32(NT) : idesc_16(NT, P16 == 2);
+    const uint32_t cross = tmem + CF::kColCross;
+    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x, tile_it++) {
+      for (int kt = 0; kt < nkt; kt++) {
+        const uint32_t in_chunk = P16 ? (uint32_t)kt : (uint32_t)(kt % kChunkKt), b = chunk_it & 1;
+        if (in_chunk == 0) mbar_wait(acc_empty + 8 * b, ((chunk_it >> 1) & 1) ^ 1, abort_flag, P.status, FST_ACC_EMPTY);
+        mbar_wait(w_full + 8 * ws, wph, abort_flag, P.status, FST_W_FULL);
+        mbar_wait(a_full + 8 * as, aph, abort_flag, P.status, FST_A_FULL);
+        tc_fence_after();
+        const uint32_t st = base + ws * CF::kWStage, acc = tmem + b * NT;
+        const uint64_t wh = desc_hi | (uint64_t)((st >> 4) & 0x3FFF), wl = desc_hi | (uint64_t)(((st + CF::kWHalf) >> 4) & 0x3FFF);
+        const uint32_t ah = tmem + CF::kColA + 64 * as, al = ah + 32;
+        if constexpr (P16 != 0) {
+          tc_mma_ts_first<idesc>(acc, ah, wh, in_chunk);
 #pragma unroll
-            for (int j = 0; j < kKt; j++) {
-              const uint32_t code = s_code[k0 + j];
-              v[j] = 0.f;
-              if (live && code != 0xFF)
-                v[j] = __ldg(s_base_in[code & 0x7F] + ((long long)s_off[k0 + j] + ((code & 0x80) ? p1 : p0)));
-            }
+          for (int j = 1; j < kKt / 8; j++) tc_mma_ts_acc<idesc>(acc, ah + 8 * j, wh + (uint64_t)(2 * j));    // 16 k = 32 bytes
+        } else {
+#pragma unroll
+          for (int j = 0; j < kKt / 8; j++)             // 8 tf32 = 32 bytes per k step: the address field moves by 2
+            mma_tf32_ts<idesc>(acc, ah + 8 * j, wh + (uint64_t)(2 * j), in_chunk | (uint32_t)j);
+          if (kt == 0) {                                // the previous tile's cross products have been read
+            mbar_wait(cross_empty, (tile_it & 1) ^ 1, abort_flag, P.status, FST_ACC_EMPTY);
+            tc_fence_after();
+          }
+#pragma unroll
+          for (int j = 0; j < kKt / 8; j++) {
+            mma_tf32_ts<idesc>(cross, ah + 8 * j, wl + (uint64_t)(2 * j), (uint32_t)(kt | j));
+            mma_tf32_ts<idesc>(cross, al + 8 * j, wh + (uint64_t)(2 * j), 1u);
+          }
+        }
+        tc_commit(a_empty + 8 * as);
+        tc_commit(w_empty + 8 * ws);
+        if ((!P16 && in_chunk == kChunkKt - 1) || kt == nkt - 1) { tc_commit(acc_full + 8 * b); chunk_it++; }
+        if (++as == CF::kAStages) { as = 0; aph ^= 1; }
+        if (++ws == CF::kWStages) { ws = 0; wph ^= 1; }
+      }
+    }
+  } else if (warp < kPWarps) {
+    // ------------------------------------------------------------------ A producers: thread = row of the tile
+    const int quad = warp & 3, r = quad * 32 + lane;
+    const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16) + CF::kColA;
+    uint32_t it = (uint32_t)(warp >> 2);                        // this set's k steps, counted over all tiles: every kPSets-th
+    // 16 inputs from `k` on: scale, split, tensor memory
+    auto publish16 = [&](float (&v)[16], int k, uint32_t dst) {
+      if (P.in_div) {
+#pragma unroll
+        for (int j = 0; j < 16; j++) if (k + j < P.K_real) v[j] = __fdiv_rn(v[j], __ldg(P.in_div + k + j));
+      }
+      uint32_t hi[16], lo[16];
+#pragma unroll
+      for (int j = 0; j < 16; j++) split_tf32(v[j], hi[j], lo[j]);
+      tmem_st16(dst, hi);
+      tmem_st16(dst + 32, lo);
+    };
+    auto arrive = [&](uint32_t bar) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    if constexpr (kTile) {
+      const long long steps = blockIdx.x < ntiles ? ((ntiles - 1 - blockIdx.x) / gridDim.x + 1) * nkt : 0;
+      int kt = (int)it;
+      while (kt >= nkt) kt -= nkt;
+      for (; it < steps; it += kPSets) {
+        const uint32_t s = it % CF::kAStages, rs = it % kRawStages;
+        if (!mbar_wait(raw_full + 8 * rs, (it / kRawStages) & 1, abort_flag, P.status, FST_RAW_FULL)) break;
+        const uint8_t* raw = smem + kRawOff + rs * kRawBytes;
+        bool ok = true;
+#pragma unroll 1
+        for (int h = 0; h < 2; h++) {
+          float v[16];
+          if constexpr (AMODE == A_TILE_T) {
+#pragma unroll
+            for (int j = 0; j < 16; j++) v[j] = *reinterpret_cast<const float*>(raw + (16 * h + j) * (kM * 4) + r * 4);
           } else {
 #pragma unroll
-            for (int j = 0; j < kKt; j++) v[j] = (live && k0 + j < P.K_real) ? __ldg(P.A + (long long)(k0 + j) * P.lda + row) : 0.f;
+            for (int i = 0; i < 4; i++) {
+              const float4 q = *reinterpret_cast<const float4*>(raw + r * 128 + (((4 * h + i) ^ (r & 7)) << 4));
+              v[4 * i] = q.x; v[4 * i + 1] = q.y; v[4 * i + 2] = q.z; v[4 * i + 3] = q.w;
+            }
           }
-          if (P.in_div) {
+          if (h == 0) {
+            ok = mbar_wait(a_empty + 8 * s, ((it / CF::kAStages) & 1) ^ 1, abort_flag, P.status, FST_A_EMPTY);
+            if (!ok) break;
+            tc_fence_after();
+          }
+          if constexpr (P16 != 0) {                              // pairs as they are
+            uint32_t pk[16];
 #pragma unroll
-            for (int j = 0; j < kKt; j++) if (k0 + j < P.K_real) v[j] = __fdiv_rn(v[j], __ldg(P.in_div + k0 + j));
-          }
-#pragma unroll
-          for (int kc = 0; kc < kKt / 4; kc++) {
-            float4 h4, l4;
-            split_tf32(v[4 * kc], h4.x, l4.x);
-            split_tf32(v[4 * kc + 1], h4.y, l4.y);
-            split_tf32(v[4 * kc + 2], h4.z, l4.z);
-            split_tf32(v[4 * kc + 3], h4.w, l4.w);
-            const int off = r * 128 + ((kc ^ (r & 7)) << 4);
-            *reinterpret_cast<float4*>(a_hi + off) = h4;
-            *reinterpret_cast<float4*>(a_lo + off) = l4;
-          }
+            for (int j = 0; j < 16; j++) pk[j] = __float_as_uint(v[j]);
+            tmem_st16(lane_addr + 64 * s + 16 * h, pk);
+          } else publish16(v, kt * kKt + 16 * h, lane_addr + 64 * s + 16 * h);
         }
-        // the tensor core reads shared memory through the async proxy: order these generic-proxy writes before it
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_arrive(bar_full + 8 * s);
-        if (++s == kStagesF) { s = 0; ph ^= 1; }
+        if (!ok) break;
+        tmem_st_wait();
+        arrive(a_full + 8 * s);
+        if (lane == 0) mbar_arrive(raw_empty + 8 * rs);
+        kt += kPSets;
+        while (kt >= nkt) kt -= nkt;
+      }
+    } else {
+      asm volatile("griddepcontrol.wait;" ::: "memory");       // the previous layer's activations are complete and visible
+      uint8_t* scratch = a_scratch + warp * kTileScratch;
+      ACursor<AMODE> c;
+      c.t = blockIdx.x; c.kt = (int)it;
+      while (c.kt >= nkt) { c.kt -= nkt; c.t += gridDim.x; }
+      if (c.t < ntiles) cursor_tile<AMODE>(P, c, r);
+      // 32 inputs from k0 on, in v[][]
+      auto load_block = [&](float (&v)[2][16], int k0) {
+        cursor_load<AMODE>(P, c, tab, quad, lane, k0, reinterpret_cast<float(&)[kKt]>(v));
+        if constexpr (AMODE == A_ROW_MAJOR) {
+          // element (row rr, k) lies in 16-byte piece (k / 4) ^ (rr % 8) of the row's 128-byte line: no bank conflicts either way
+#pragma unroll
+          for (int rr = 0; rr < 32; rr++)
+            *reinterpret_cast<float*>(scratch + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + ((lane & 3) << 2)) = v[rr >> 4][rr & 15];
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 8; i++) {
+            const float4 q = *reinterpret_cast<const float4*>(scratch + lane * 128 + ((i ^ (lane & 7)) << 4));
+            v[i >> 2][4 * (i & 3)] = q.x; v[i >> 2][4 * (i & 3) + 1] = q.y; v[i >> 2][4 * (i & 3) + 2] = q.z; v[i >> 2][4 * (i & 3) + 3] = q.w;
+          }
+          __syncwarp();
+        }
+      };
+      for (; c.t < ntiles; it += kPSets) {
+        const uint32_t s = it % CF::kAStages;
+        if constexpr (P16 != 0) {
+          bool ok = true;
+#pragma unroll 1
+          for (int h = 0; h < 2; h++) {
+            float v[2][16];
+            const int k0 = c.kt * 64 + 32 * h;
+            load_block(v, k0);
+            if (P.in_div) {
+#pragma unroll
+              for (int j = 0; j < 32; j++) if (k0 + j < P.K_real) v[j >> 4][j & 15] = __fdiv_rn(v[j >> 4][j & 15], __ldg(P.in_div + k0 + j));
+            }
+            uint32_t pk[16];
+#pragma unroll
+            for (int j = 0; j < 16; j++) pk[j] = pack_pair<P16 == 2>(v[j >> 3][(2 * j) & 15], v[j >> 3][(2 * j + 1) & 15]);
+            if (h == 0) {
+              ok = mbar_wait(a_empty + 8 * s, ((it / CF::kAStages) & 1) ^ 1, abort_flag, P.status, FST_A_EMPTY);
+              if (!ok) break;
+              tc_fence_after();
+            }
+            tmem_st16(lane_addr + 64 * s + 16 * h, pk);
+          }
+          if (!ok) break;
+        } else {
+          float v[2][16];
+          const int k0 = c.kt * kKt;
+          load_block(v, k0);
+          if (!mbar_wait(a_empty + 8 * s, ((it / CF::kAStages) & 1) ^ 1, abort_flag, P.status, FST_A_EMPTY)) break;
+          tc_fence_after();
+          publish16(v[0], k0, lane_addr + 64 * s);
+          publish16(v[1], k0 + 16, lane_addr + 64 * s + 16);
+        }
+        tmem_st_wait();
+        arrive(a_full + 8 * s);
+        cursor_advance<AMODE, kPSets>(P, c, nkt, ntiles, r);
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue: thread = row of the tile
+    // ------------------------------------------------------------------ epilogue: thread = row of the tile, half of the features
     asm volatile("griddepcontrol.wait;" ::: "memory");         // the buffer written here may still be read by the previous layer
-    const int quad = warp & 3;                                // the TMEM lanes this warp may read
+    constexpr int NH = NT / kESets, NL = 16;         // features per thread, columns per tensor-memory load
+    const int quad = warp & 3, half = (warp - kPWarps) >> 2;
     const int r = quad * 32 + lane;
-    const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16);
+    const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16) + half * NH;
+    uint8_t* scratch = c_scratch + (warp - kPWarps) * kTileScratch;
+    float* s_bias = (float*)(tail + kBarF) + (warp - kPWarps) * 2 * NH;
+    float* s_scale = s_bias + NH;
     uint32_t chunk_it = 0;
     double csum = 0.0;
-    const int nch = (nkt + kChunkKt - 1) / kChunkKt;
+    const int nch = P16 ? 1 : (nkt + kChunkKt - 1) / kChunkKt;
     for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-      const long long row = (t / ntn) * kM + r;
-      const int nt0 = (int)(t % ntn) * P.n_tile;
+      const long long m0 = (t / P.ntn) * kM, row = m0 + r;
+      const int nt0 = (int)(t % P.ntn) * NT + half * NH;
       const bool live = row < P.nrows;
-      long long op0 = 0, op1 = 0;
-      if (P.c_mode == C_SCATTER) {
-        long long ci = 0, cj = 0, kk = 0;
-        if (live) row_to_pos(P.g, row, &ci, &cj, &kk);
-        op0 = ci * P.cout[0].si + cj * P.cout[0].sj + kk * P.cout[0].sk;
-        op1 = ci * P.cout[1].si + cj * P.cout[1].sj + kk * P.cout[1].sk;
+      // bias (and scale) of this warp's features, for broadcast reads at the end of the tile: as loads from global memory
+      // there they cost 470 cycles a feature, 30 k of a 48 k-cycle tile
+      for (int j = lane; j < NH; j += 32) {
+        const bool real = nt0 + j < P.N_real;
+        s_bias[j] = P.bias && real ? __ldg(P.bias + nt0 + j) : 0.f;
+        if constexpr (P16 != 0) s_scale[j] = P.scale && real ? __ldg(P.scale + nt0 + j) : 1.f;
       }
+      __syncwarp();
+      float v[NH];
+#pragma unroll
+      for (int j = 0; j < NH; j++) v[j] = 0.f;
       for (int ch = 0; ch < nch; ch++, chunk_it++) {
-        const bool last = ch == nch - 1;
-        mbar_wait(bar_acc_full, chunk_it & 1, abort_flag, P.status, FST_ACC_FULL);
+        const uint32_t b = chunk_it & 1;
+        mbar_wait(acc_full + 8 * b, (chunk_it >> 1) & 1, abort_flag, P.status, FST_ACC_FULL);
         tc_fence_after();
-        for (int c0 = 0; c0 < P.n_tile; c0 += 32) {
-          uint32_t a[32], sm[32];
-          tmem_ld32(lane_addr + c0, a);                          // this chunk's partial sums
-          if (ch > 0) tmem_ld32(lane_addr + kNtMax + c0, sm);    // the running sum of the earlier chunks
+#pragma unroll
+        for (int c0 = 0; c0 < NH; c0 += NL) {
+          uint32_t a[NL];
+          tmem_ldn(lane_addr + b * NT + c0, a);
           tmem_ld_wait();
-          if (last && c0 + 32 >= P.n_tile) {                     // the chunk accumulator has been read completely
-            tc_fence_before();
-            mbar_arrive(bar_acc_empty);
+#pragma unroll
+          for (int j = 0; j < NL; j++) v[c0 + j] = __fadd_rn(v[c0 + j], __uint_as_float(a[j]));
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty + 8 * b);
+      }
+      if constexpr (P16 == 0) {
+#pragma unroll
+      for (int c0 = 0; c0 < NH; c0 += NL) {
+        uint32_t a[NL];
+        tmem_ldn(lane_addr + CF::kColCross + c0, a);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < NL; j++) v[c0 + j] = __fadd_rn(v[c0 + j], __uint_as_float(a[j]));
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(cross_empty);
+      }
+
+      if (P16 == 0 && P.c_mode == C_CONV) {
+        const ConvGeom& g = P.cv;
+        unsigned q = (unsigned)(live ? row : 0);
+        const int ow = (int)(q % (unsigned)g.Wo); q /= (unsigned)g.Wo;
+        const int oh = (int)(q % (unsigned)g.Ho); q /= (unsigned)g.Ho;
+        const int od = (int)(q % (unsigned)g.Do), on = (int)(q / (unsigned)g.Do);
+        const long long yo = (long long)on * g.ys_n + (long long)od * g.ys_d + (long long)oh * g.ys_h + (long long)ow * g.ys_w + nt0 * g.ys_c;
+        const long long ro = (long long)on * g.rs_n + (long long)od * g.rs_d + (long long)oh * g.rs_h + (long long)ow * g.rs_w + nt0 * g.rs_c;
+        if (!live) continue;
+#pragma unroll
+        for (int c0 = 0; c0 < NH; c0 += 16) {
+          float o[16];
+          if (P.residual) {
+#pragma unroll
+            for (int j = 0; j < 16; j++) o[j] = nt0 + c0 + j < P.N_real ? __ldg(P.residual + ro + (long long)(c0 + j) * g.rs_c) : 0.f;
           }
-          float v[32];
 #pragma unroll
-          for (int j = 0; j < 32; j++) v[j] = ch > 0 ? __fadd_rn(__uint_as_float(sm[j]), __uint_as_float(a[j])) : __uint_as_float(a[j]);
-          if (!last) {
+          for (int j = 0; j < 16; j++) v[c0 + j] += s_bias[c0 + j];
 #pragma unroll
-            for (int j = 0; j < 32; j++) a[j] = __float_as_uint(v[j]);
-            tmem_st32(lane_addr + kNtMax + c0, a);
-            continue;
+          for (int j = 0; j < 16; j++) o[j] = P.residual ? v[c0 + j] + o[j] : v[c0 + j];
+          act_f32(o, P.act, P.slope);
+          float* dst = P.C + yo + (long long)c0 * g.ys_c;
+#pragma unroll
+          for (int j = 0; j < 16; j++) {
+            if (nt0 + c0 + j < P.N_real) *dst = o[j];
+            dst += g.ys_c;
           }
-          const int n0 = nt0 + c0;
+        }
+        continue;
+      }
+      if constexpr (P16 != 0) {
+        // the fused kernel's expressions, hidden and last layer
+        if (!P.scale) {
 #pragma unroll
-          for (int j = 0; j < 32; j++) {
-            const float bj = P.bias ? __ldg(P.bias + n0 + j) : 0.f;
-            v[j] = act_slope(v[j] + bj, P.slope);
-          }
-          if (P.out_mul || P.relu_mask) {
+          for (int j = 0; j < NH; j++) v[j] = v[j] + s_bias[j];
+        } else if (P.C16) {
 #pragma unroll
-            for (int j = 0; j < 32; j++) {
-              const int n = n0 + j;
-              if (n < P.N_real) {
-                if (P.out_mul) v[j] *= __ldg(P.out_mul + n);
-                if (P.relu_mask && __ldg(P.relu_mask + n) != 0.f) v[j] = fmaxf(v[j], 0.f);
-              }
+          for (int j = 0; j < NH; j++) v[j] = fmaf(v[j], s_scale[j], s_bias[j]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < NH; j++) v[j] = v[j] * s_scale[j] + s_bias[j];
+        }
+#pragma unroll
+        for (int j = 0; j < NH; j++) v[j] = fmaxf(v[j], v[j] * P.slope);
+        if (P.C16) {
+          if (live) {
+            uint32_t* dst = P.C16 + (long long)(nt0 >> 1) * P.ldc + row;
+#pragma unroll
+            for (int j = 0; j < NH; j += 2) {
+              if (nt0 + j < P.N_real) *dst = pack_pair<P16 == 2>(v[j], v[j + 1]);
+              dst += P.ldc;
             }
           }
-          if (!live) continue;
-          if (P.c_mode == C_FEATURE_MAJOR) {
+          continue;
+        }
+      } else {
 #pragma unroll
-            for (int j = 0; j < 32; j++) if (n0 + j < P.N_real) P.C[(long long)(n0 + j) * P.ldc + row] = v[j];
-          } else if (P.c_mode == C_ROW_MAJOR) {
-            float* dst = P.C + row * P.ldc + n0;
-            if (n0 + 32 <= P.N_real && ((P.ldc & 3) == 0) && ((reinterpret_cast<uintptr_t>(P.C) & 15) == 0)) {
+        for (int j = 0; j < NH; j++) v[j] += s_bias[j];
+        act_f32(v, P.act, P.slope);
+      }
+      if (P.out_mul || P.relu_mask) {
 #pragma unroll
-              for (int j = 0; j < 8; j++) reinterpret_cast<float4*>(dst)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-            } else {
+        for (int j = 0; j < NH; j++) {
+          const int n = nt0 + j;
+          if (n < P.N_real) {
+            if (P.out_mul) v[j] *= __ldg(P.out_mul + n);
+            if (P.relu_mask && __ldg(P.relu_mask + n) != 0.f) v[j] = fmaxf(v[j], 0.f);
+          }
+        }
+      }
+      if (P.c_mode == C_FEATURE_MAJOR) {
+        if (live) {
+          float* dst = P.C + (long long)nt0 * P.ldc + row;
+          if (nt0 + NH <= P.N_real) {
 #pragma unroll
-              for (int j = 0; j < 32; j++) if (n0 + j < P.N_real) dst[j] = v[j];
-            }
+            for (int j = 0; j < NH; j++) { *dst = v[j]; dst += P.ldc; }
           } else {
 #pragma unroll
-            for (int j = 0; j < 32; j++) {
-              const uint32_t code = (n0 + j < kTabOut) ? o_code[n0 + j] : 0xFFu;
-              if (code != 0xFF) {
-                s_base_out[code & 0x7F][(long long)o_off[n0 + j] + ((code & 0x80) ? op1 : op0)] = v[j];
-                csum += (double)v[j];
-              }
+            for (int j = 0; j < NH; j++) {
+              if (nt0 + j < P.N_real) *dst = v[j];
+              dst += P.ldc;
             }
           }
         }
-        if (!last) {                                             // the running sum is in place: hand the chunk accumulator back
-          tmem_st_wait();
-          tc_fence_before();
-          mbar_arrive(bar_acc_empty);
+      } else if (P.c_mode == C_ROW_MAJOR) {
+        // blocks of 32 rows x NL features turned in shared memory: stores of whole lines
+#pragma unroll
+        for (int c0 = 0; c0 < NH; c0 += NL) {
+#pragma unroll
+          for (int i = 0; i < NL / 4; i++)
+            *reinterpret_cast<float4*>(scratch + lane * 128 + ((i ^ (lane & 7)) << 4)) =
+                make_float4(v[c0 + 4 * i], v[c0 + 4 * i + 1], v[c0 + 4 * i + 2], v[c0 + 4 * i + 3]);
+          __syncwarp();
+          const int n0 = nt0 + c0;
+          const long long mw = m0 + quad * 32;
+          if (P.c_vec) {
+            constexpr int LPR = NL / 4;                          // lanes per row
+            const int pc = lane % LPR;
+#pragma unroll
+            for (int i = 0; i < LPR; i++) {
+              const int rr = i * (32 / LPR) + lane / LPR;
+              const float4 q = *reinterpret_cast<const float4*>(scratch + rr * 128 + ((pc ^ (rr & 7)) << 4));
+              if (mw + rr < P.nrows && n0 + 4 * pc < P.N_real) *reinterpret_cast<float4*>(P.C + (mw + rr) * P.ldc + n0 + 4 * pc) = q;
+            }
+          } else {
+#pragma unroll 8
+            for (int rr = 0; rr < 32; rr++) {
+              const float q = *reinterpret_cast<const float*>(scratch + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + ((lane & 3) << 2));
+              if (lane < NL && mw + rr < P.nrows && n0 + lane < P.N_real) P.C[(mw + rr) * P.ldc + n0 + lane] = q;
+            }
+          }
+          __syncwarp();
+        }
+      } else if (live) {
+        long long ci, cj, kk;
+        row_to_pos(P.g, row, &ci, &cj, &kk);
+        const long long op0 = 4 * (ci * P.cout[0].si + cj * P.cout[0].sj + kk * P.cout[0].sk);
+        const long long op1 = 4 * (ci * P.cout[1].si + cj * P.cout[1].sj + kk * P.cout[1].sk);
+#pragma unroll
+        for (int j = 0; j < NH; j++) {
+          const unsigned long long e = nt0 + j < kTabOut ? o_tab[nt0 + j] : 0ull;
+          if (e != 0ull) {
+            *reinterpret_cast<float*>((e & ~1ull) + (unsigned long long)((e & 1ull) ? op1 : op0)) = v[j];
+            csum += (double)v[j];
+          }
         }
       }
     }
     if (P.partials) {
       // per-CTA checksum partial in a fixed order; the last CTA to finish folds all partials into the step checksum
-      double* wsum = (double*)(tail + 72);
+      double* wsum = (double*)(tail + 272);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) csum += __shfl_down_sync(0xffffffffu, csum, o);
-      if (lane == 0) wsum[quad] = csum;
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (quad == 0 && lane == 0) {
-        P.partials[blockIdx.x] = (wsum[0] + wsum[1]) + (wsum[2] + wsum[3]);
+      asm volatile("bar.sync 1, %0;" ::"n"(kEWarps * 32) : "memory");           // every epilogue warp has passed its last barrier wait
+      if (lane == 0) wsum[warp - kPWarps] = csum;
+      asm volatile("bar.sync 1, %0;" ::"n"(kEWarps * 32) : "memory");
+      if (warp == kPWarps && lane == 0) {
+        double part = 0.0;
+        for (int w = 0; w < kEWarps; w++) part += wsum[w];
+        P.partials[blockIdx.x] = part;
         if (P.sum) {
           __threadfence();
           if (atomicAdd(P.done, 1u) == gridDim.x - 1) {
@@ -414,21 +755,33 @@ __global__ void __launch_bounds__(kThreadsF, 1) linear_tf32x3_kernel(const __gri
   if (*abort_flag && threadIdx.x == 0)
     for (int i = 0; i < 2000; i++) __nanosleep(1000);        // let copies in flight land before the CTA gives its memory back
   __syncthreads();
-  if (warp == 1) {
+  if (warp == kWarpMma) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
 }
 
-// W (N, K) row-major on the device -> W_hi / W_lo [N_pad][K_pad] (zero padded): the split of fortis_gemm's weights,
-// which only exist on the device
-__global__ void split_weights_kernel(const float* __restrict__ W, int N, int K, float* __restrict__ hi, float* __restrict__ lo, int N_pad,
+// W (N, K) row-major on the device -> W_hi / W_lo [N_pad][K_pad] (zero padded)
+__global__ void split_weights_kernel(const float* __restrict__ W, int N, int K, uint32_t* __restrict__ hi, uint32_t* __restrict__ lo, int N_pad,
                                      int K_pad) {
   const long long n_el = (long long)N_pad * K_pad;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_el; i += (long long)gridDim.x * blockDim.x) {
     const int n = (int)(i / K_pad), k = (int)(i % K_pad);
-    float h = 0.f, l = 0.f;
+    uint32_t h = 0, l = 0;
     if (n < N && k < K) split_tf32(W[(long long)n * K + k], h, l);
+    hi[i] = h; lo[i] = l;
+  }
+}
+
+// the same for convolution weights (F, C, taps): reduction index = (tap, channel), channels padded to whole groups
+__global__ void split_conv_weights_kernel(const float* __restrict__ W, int F, int C, int taps, int group, uint32_t* __restrict__ hi,
+                                          uint32_t* __restrict__ lo, int N_pad, int K_pad) {
+  const long long n_el = (long long)N_pad * K_pad;
+  const int cp = (C + group - 1) / group * group;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_el; i += (long long)gridDim.x * blockDim.x) {
+    const int n = (int)(i / K_pad), k = (int)(i % K_pad), tap = k / cp, c = k - tap * cp;
+    uint32_t h = 0, l = 0;
+    if (n < F && tap < taps && c < C) split_tf32(W[((long long)n * C + c) * taps + tap], h, l);
     hi[i] = h; lo[i] = l;
   }
 }
@@ -448,68 +801,153 @@ EncodeTiledFnF encode_fn_f() {
 
 int round_up_f(int v, int m) { return (v + m - 1) / m * m; }
 
-// nearest TF32 value, ties away from zero (what cvt.rna.tf32.f32 returns)
-float tf32_rna_host(float x) {
-  uint32_t u;
-  std::memcpy(&u, &x, 4);
-  if ((u & 0x7f800000u) == 0x7f800000u) return x;            // inf / nan unchanged
-  u = (u + 0x1000u) & 0xFFFFE000u;
-  float r;
-  std::memcpy(&r, &u, 4);
-  return r;
-}
-
-struct LayerGeom { int K_real, N_real, K_pad, N_pad, n_tile; };
-LayerGeom layer_geom(int cin, int cout) {
-  LayerGeom g;
-  g.K_real = cin; g.N_real = cout;
-  g.K_pad = round_up_f(cin, kKt);
-  g.N_pad = round_up_f(cout, 64);
-  if (g.N_pad > kNtMax) g.N_pad = round_up_f(cout, kNtMax);
-  g.n_tile = g.N_pad < kNtMax ? g.N_pad : kNtMax;
-  return g;
-}
-
-bool make_w_maps(float* hi, float* lo, const LayerGeom& g, CUtensorMap* mh, CUtensorMap* ml) {
+// fp32 activations as the TMA reads them: `rows` x `K`, feature-major ([K][ld]) or row-major ([rows][K]).  False where the
+// rows do not start on 16-byte boundaries.
+bool make_a_map(bool feature_major, const float* A, long long rows, int K, long long ld, CUtensorMap* m) {
   EncodeTiledFnF enc = encode_fn_f();
-  if (!enc) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)g.K_pad, (cuuint64_t)g.N_pad};
-  const cuuint64_t strides[1] = {(cuuint64_t)g.K_pad * 4};
-  const cuuint32_t box[2] = {(cuuint32_t)kKt, (cuuint32_t)g.n_tile};
-  const cuuint32_t estr[2] = {1, 1};
-  for (int i = 0; i < 2; i++)
-    if (enc(i ? ml : mh, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, i ? lo : hi, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return false;
-  return true;
+  if (!enc || ((uintptr_t)A & 15) != 0 || (ld & 3) != 0 || rows >= (1LL << 31) - kM || ld * 4 >= (1LL << 40)) return false;
+  const cuuint64_t dims[2] = {(cuuint64_t)(feature_major ? rows : K), (cuuint64_t)(feature_major ? K : rows)};
+  const cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+  const cuuint32_t box[2] = {(cuuint32_t)(feature_major ? kM : kKt), (cuuint32_t)(feature_major ? kKt : kM)}, estr[2] = {1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(A), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             feature_major ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool prepare_kernel(std::string* err) {
-  static bool done = false;
-  if (done) return true;
-  if (cudaFuncSetAttribute(linear_tf32x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemF) != cudaSuccess) {
-    if (err) *err = "cannot reserve " + std::to_string(kSmemF) + " bytes of shared memory for the split-TF32 kernel";
+unsigned split_grid(size_t n_el) { return (unsigned)((n_el + 255) / 256 < 1184 ? (n_el + 255) / 256 : 1184); }
+
+int sm_count() {
+  static int sms = 0;
+  if (sms) return sms;
+  int n = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return sms = n;
+}
+
+// Split weights of one layer: W_hi / W_lo [N_pad][K_pad] and their tensor maps for the three tile widths.
+struct SplitW {
+  int K_real = 0, N_real = 0, K_pad = 0, N_pad = 0;
+  float *hi = nullptr, *lo = nullptr;
+  CUtensorMap map_hi[3], map_lo[3];        // box 32 x 32, 64, 128
+};
+
+void split_free(SplitW* w) { cudaFree(w->hi); cudaFree(w->lo); w->hi = w->lo = nullptr; }
+
+bool split_alloc(SplitW* w, int K, int N, std::string* err) {
+  w->K_real = K; w->N_real = N;
+  w->K_pad = round_up_f(K, kKt);
+  w->N_pad = round_up_f(N, 32);
+  const size_t n_el = (size_t)w->N_pad * w->K_pad;
+  if (cudaMalloc(&w->hi, n_el * 4) != cudaSuccess || cudaMalloc(&w->lo, n_el * 4) != cudaSuccess) {
+    cudaGetLastError();
+    split_free(w);
+    if (err) *err = "out of device memory for split weights";
     return false;
   }
-  done = true;
+  EncodeTiledFnF enc = encode_fn_f();
+  const cuuint64_t dims[2] = {(cuuint64_t)w->K_pad, (cuuint64_t)w->N_pad};
+  const cuuint64_t strides[1] = {(cuuint64_t)w->K_pad * 4};
+  const cuuint32_t estr[2] = {1, 1};
+  for (int i = 0; i < 6; i++) {
+    // a box that reaches behind the last feature is filled with zeros
+    const cuuint32_t box[2] = {(cuuint32_t)kKt, (cuuint32_t)(32 << (i >> 1))};
+    if (!enc || enc((i & 1) ? &w->map_lo[i >> 1] : &w->map_hi[i >> 1], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (i & 1) ? w->lo : w->hi, dims, strides, box,
+                    estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+      split_free(w);
+      if (err) *err = "cuTensorMapEncodeTiled failed for split weights";
+      return false;
+    }
+  }
   return true;
 }
 
-int grid_for(long long nrows, const LayerGeom& g) {
-  const long long tiles = ((nrows + kM - 1) / kM) * (g.N_pad / g.n_tile);
-  int sms = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return (int)(tiles < sms ? (tiles > 0 ? tiles : 1) : sms);
+// The tile width (0, 1, 2: 32, 64, 128 features).  A k step of a tile costs 6 clocks per feature of tensor time, or what
+// its producers need for 128 rows x 32 inputs if that is more, and the launch lasts as many rounds of tiles as the SM
+// that has the most.
+int pick_tile(long long nrows, int N, int step_floor) {
+  const long long ntm = (nrows + kM - 1) / kM, sms = sm_count();
+  long long best_cost = 0;
+  int best = -1;
+  for (int w = 2; w >= 0; w--) {
+    const int nt = 32 << w;
+    if (w > 0 && N <= nt / 2) continue;                     // more than half of the tile would be padding
+    const long long tiles = ntm * ((N + nt - 1) / nt), cost = ((tiles + sms - 1) / sms) * (6 * nt > step_floor ? 6 * nt : step_floor);
+    if (best < 0 || cost < best_cost) { best = w; best_cost = cost; }
+  }
+  return best;
+}
+
+template <int NT, int AMODE, int P16>
+size_t smem_bytes(const F32Params& P) {
+  using CF = TileCfg<NT>;
+  const int nkt = P.K_pad / kKt;
+  size_t n = CF::kWBytes + kBarF + kEWarps * 2 * (NT / kESets) * 4 + (AMODE == A_TILE_T || AMODE == A_TILE_R ? kRawStages * kRawBytes : 0);
+  if (AMODE == A_ROW_MAJOR) n += kPWarps * kTileScratch;
+  if (P.c_mode == C_ROW_MAJOR) n += kEWarps * kTileScratch;
+  if (AMODE == A_GATHER) n += (size_t)P.K_pad * (P16 ? 2 : 1) * 8;
+  if (AMODE == A_CONV8) n += (size_t)nkt * (kKt / 8) * 8;
+  if (AMODE == A_CONV1) n += (size_t)nkt * kKt * 8;
+  if (P.c_mode == C_SCATTER) n += kTabOut * 8;
+  return n;
+}
+constexpr int kSmemMaxF = 227 * 1024;
+
+// `early` = false for a launch whose WEIGHTS were produced by the kernel in front of it: the weight loads do not wait.
+// Otherwise the launch may start while the one before it in the stream drains (programmatic stream serialisation).
+template <int NT, int AMODE, int P16 = 0>
+bool launch_as(const F32Params& P, cudaStream_t s, bool early) {
+  static bool ready = false;
+  if (!ready) {
+    if (cudaFuncSetAttribute(f32tc_kernel<NT, AMODE, P16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMaxF) != cudaSuccess) return false;
+    ready = true;
+  }
+  const long long tiles = ((P.nrows + kM - 1) / kM) * P.ntn, sms = sm_count();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles < sms ? tiles : sms)); cfg.blockDim = dim3(kThreadsF);
+  cfg.dynamicSmemBytes = smem_bytes<NT, AMODE, P16>(P); cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  static const bool pdl = std::getenv("FORTIS_NO_PDL") == nullptr;
+  cfg.attrs = at; cfg.numAttrs = (pdl && early) ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, f32tc_kernel<NT, AMODE, P16>, P) == cudaSuccess;
+}
+
+template <int AMODE>
+bool launch_tile(F32Params& P, const SplitW& W, int step_floor, cudaStream_t s, bool early = true) {
+  const int w = pick_tile(P.nrows, W.N_real, step_floor);
+  P.map_hi = W.map_hi[w]; P.map_lo = W.map_lo[w];
+  P.K_pad = W.K_pad; P.K_real = W.K_real; P.N_real = W.N_real;
+  P.ntn = (W.N_real + (32 << w) - 1) / (32 << w);
+  return w == 2 ? launch_as<128, AMODE>(P, s, early) : w == 1 ? launch_as<64, AMODE>(P, s, early) : launch_as<32, AMODE>(P, s, early);
+}
+
+// clocks a k step's producers need at least (measured: see pick_tile)
+constexpr int kStepFloorLinear = 250, kStepFloorConv = 350;
+
+// a row-major operand: tiles through the TMA where rows start on 16-byte boundaries, else loads
+bool launch_rows(F32Params& P, const float* A, int K, const SplitW& W, cudaStream_t s, bool early) {
+  if (make_a_map(false, A, P.nrows, K, K, &P.map_a)) return launch_tile<A_TILE_R>(P, W, kStepFloorLinear, s, early);
+  P.A = A; P.lda = K;
+  return launch_tile<A_ROW_MAJOR>(P, W, kStepFloorLinear, s, early);
+}
+
+bool launched(bool ok, std::string* err) {
+  const cudaError_t e = cudaGetLastError();
+  if (ok && e == cudaSuccess) return true;
+  if (err) *err = std::string("split-TF32 kernel launch: ") + cudaGetErrorString(e);
+  return false;
 }
 
 }  // namespace
 
 struct F32TcModel {
   struct Layer {
-    LayerGeom g;
-    float *hi = nullptr, *lo = nullptr, *bias = nullptr;
-    CUtensorMap mh, ml;
-    float slope = 1.f;
+    SplitW w;
+    float* bias = nullptr;
+    int act = ACT_NONE;
+    float slope = 0.f;
   };
   std::vector<Layer> layers;
   float *in_div = nullptr, *out_mul = nullptr, *relu_mask = nullptr;
@@ -525,7 +963,7 @@ bool f32tc_supported(const ModelHost& M, std::string* why) {
 
 void f32tc_destroy(F32TcModel* m) {
   if (!m) return;
-  for (auto& L : m->layers) { cudaFree(L.hi); cudaFree(L.lo); cudaFree(L.bias); }
+  for (auto& L : m->layers) { split_free(&L.w); cudaFree(L.bias); }
   cudaFree(m->in_div); cudaFree(m->out_mul); cudaFree(m->relu_mask);
   delete m;
 }
@@ -533,69 +971,42 @@ void f32tc_destroy(F32TcModel* m) {
 F32TcModel* f32tc_create(const ModelHost& M, std::string* err) {
   std::string why;
   if (!f32tc_supported(M, &why)) { if (err) *err = why; return nullptr; }
-  if (!prepare_kernel(err)) return nullptr;
   F32TcModel* m = new F32TcModel();
   auto fail = [&](const std::string& w) { if (err) *err = w; f32tc_destroy(m); return (F32TcModel*)nullptr; };
-  for (auto& L : M.layers) {
-    F32TcModel::Layer T;
-    T.g = layer_geom(L.cin, L.cout);
-    std::vector<float> hi((size_t)T.g.N_pad * T.g.K_pad, 0.f), lo(hi.size(), 0.f), bias(T.g.N_pad, 0.f);
-    for (int n = 0; n < L.cout; n++) {
-      bias[n] = L.b[n];
-      for (int k = 0; k < L.cin; k++) {
-        const float w = L.W[(size_t)n * L.cin + k], h = tf32_rna_host(w);
-        hi[(size_t)n * T.g.K_pad + k] = h;
-        lo[(size_t)n * T.g.K_pad + k] = w - h;
-      }
-    }
-    if (cudaMalloc(&T.hi, hi.size() * 4) != cudaSuccess || cudaMalloc(&T.lo, lo.size() * 4) != cudaSuccess ||
-        cudaMalloc(&T.bias, bias.size() * 4) != cudaSuccess) {
-      cudaFree(T.hi); cudaFree(T.lo); cudaFree(T.bias);
-      return fail("out of device memory for split weights");
-    }
-    cudaMemcpy(T.hi, hi.data(), hi.size() * 4, cudaMemcpyHostToDevice);
-    cudaMemcpy(T.lo, lo.data(), lo.size() * 4, cudaMemcpyHostToDevice);
-    cudaMemcpy(T.bias, bias.data(), bias.size() * 4, cudaMemcpyHostToDevice);
-    T.slope = L.act == ACT_NONE ? 1.f : L.act == ACT_RELU ? 0.f : L.slope;
-    m->layers.push_back(T);
-    if (!make_w_maps(T.hi, T.lo, T.g, &m->layers.back().mh, &m->layers.back().ml)) return fail("cuTensorMapEncodeTiled failed for split weights");
-  }
   auto up = [&](const std::vector<float>& v) -> float* {
-    if (v.empty()) return nullptr;
     float* d = nullptr;
-    cudaMalloc(&d, v.size() * 4);
+    if (v.empty() || cudaMalloc(&d, v.size() * 4) != cudaSuccess) return nullptr;
     cudaMemcpy(d, v.data(), v.size() * 4, cudaMemcpyHostToDevice);
     return d;
   };
+  for (auto& L : M.layers) {
+    m->layers.push_back(F32TcModel::Layer());
+    F32TcModel::Layer& T = m->layers.back();
+    if (!split_alloc(&T.w, L.cin, L.cout, &why)) return fail(why);
+    float* raw = up(L.W);
+    T.bias = up(L.b);
+    if (!raw || !T.bias) { cudaFree(raw); cudaGetLastError(); return fail("out of device memory for split weights"); }
+    split_weights_kernel<<<split_grid((size_t)T.w.N_pad * T.w.K_pad), 256>>>(raw, L.cout, L.cin, (uint32_t*)T.w.hi, (uint32_t*)T.w.lo, T.w.N_pad, T.w.K_pad);
+    cudaStreamSynchronize(0);
+    cudaFree(raw);
+    T.act = L.act;
+    T.slope = L.slope;
+  }
   m->in_div = up(M.in_div); m->out_mul = up(M.out_mul); m->relu_mask = up(M.relu_mask);
+  if (cudaGetLastError() != cudaSuccess) return fail("splitting the weights failed");
   return m;
 }
 
 int f32tc_grid(long long nrows) {
-  int sms = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   (void)nrows;
-  return sms;
-}
-
-// one layer, allowed to start while the launch before it in the stream drains (programmatic stream serialisation)
-// (`early` = false for a launch whose WEIGHTS were produced by the kernel in front of it: the weight loads do not wait)
-static bool launch_layer(const F32Params& P, int grid, cudaStream_t s, bool early = true) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(kThreadsF); cfg.dynamicSmemBytes = kSmemF; cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  static const bool pdl = std::getenv("FORTIS_NO_PDL") == nullptr;
-  cfg.attrs = at; cfg.numAttrs = (pdl && early) ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, linear_tf32x3_kernel, P) == cudaSuccess;
+  return sm_count();
 }
 
 bool f32tc_forward(F32TcModel* m, const F32TcLaunch& L, cudaStream_t s, std::string* err) {
   const long long nrows = L.g.count * L.g.nk;
   if (nrows <= 0) return true;
   const int nl = (int)m->layers.size();
-  const int n_in = m->layers.front().g.K_real, n_out = m->layers.back().g.N_real;
+  const int n_in = m->layers.front().w.K_real, n_out = m->layers.back().w.N_real;
   const bool fast_in = L.fast_in && n_in <= kTabIn, fast_out = L.fast_out && n_out <= kTabOut;
   if (!fast_in && !L.X) { if (err) *err = "split-TF32 step: no input"; return false; }
   if (!fast_out && !L.Y) { if (err) *err = "split-TF32 step: no output"; return false; }
@@ -604,28 +1015,34 @@ bool f32tc_forward(F32TcModel* m, const F32TcLaunch& L, cudaStream_t s, std::str
     const F32TcModel::Layer& T = m->layers[l];
     F32Params P;
     std::memset(&P, 0, sizeof P);
-    P.map_hi = T.mh; P.map_lo = T.ml;
-    P.K_pad = T.g.K_pad; P.N_pad = T.g.N_pad; P.n_tile = T.g.n_tile; P.K_real = T.g.K_real; P.N_real = T.g.N_real;
-    P.bias = T.bias; P.slope = T.slope; P.nrows = nrows; P.g = L.g; P.status = L.status;
-    if (l == 0) {
-      P.in_div = m->in_div;
-      if (fast_in) {
-        P.a_mode = A_GATHER; P.slots = L.slots; P.TG = L.TG;
-        for (int i = 0; i < 2; i++) P.cin[i] = StrideClassF{L.cin[i][0], L.cin[i][1], L.cin[i][2]};
-      } else { P.a_mode = A_ROW_MAJOR; P.A = L.X; P.lda = n_in; }
-    } else { P.a_mode = A_FEATURE_MAJOR; P.A = L.act[(l - 1) & 1]; P.lda = L.act_ld; }
+    P.bias = T.bias; P.act = T.act; P.slope = T.slope; P.nrows = nrows; P.g = L.g; P.status = L.status;
     if (l == nl - 1) {
       P.out_mul = m->out_mul; P.relu_mask = m->relu_mask;
       if (fast_out) {
         P.c_mode = C_SCATTER; P.store_by_slot = L.store_by_slot; P.TS = L.TS;
         for (int i = 0; i < 2; i++) P.cout[i] = StrideClassF{L.cout[i][0], L.cout[i][1], L.cout[i][2]};
         P.partials = L.partials; P.sum = L.partials ? L.sum : nullptr; P.done = L.done;
-      } else { P.c_mode = C_ROW_MAJOR; P.C = L.Y; P.ldc = n_out; }
+      } else { P.c_mode = C_ROW_MAJOR; P.C = L.Y; P.ldc = n_out; P.c_vec = n_out % 4 == 0 && ((uintptr_t)L.Y & 15) == 0; }
     } else { P.c_mode = C_FEATURE_MAJOR; P.C = L.act[l & 1]; P.ldc = L.act_ld; }
-    if (!launch_layer(P, grid_for(nrows, T.g), s)) { if (err) *err = "split-TF32 kernel launch failed"; return false; }
+    bool ok;
+    if (l == 0) {
+      P.in_div = m->in_div;
+      if (fast_in) {
+        P.slots = L.slots; P.TG = L.TG;
+        for (int i = 0; i < 2; i++) P.cin[i] = StrideClassF{L.cin[i][0], L.cin[i][1], L.cin[i][2]};
+        ok = launch_tile<A_GATHER>(P, T.w, kStepFloorLinear, s);
+      } else {
+        ok = launch_rows(P, L.X, n_in, T.w, s, true);
+      }
+    } else {
+      if (!make_a_map(true, L.act[(l - 1) & 1], nrows, T.w.K_real, L.act_ld, &P.map_a)) {
+        if (err) *err = "split-TF32 step: activation rows must start on 16-byte boundaries";
+        return false;
+      }
+      ok = launch_tile<A_TILE_T>(P, T.w, kStepFloorLinear, s);
+    }
+    if (!launched(ok, err)) return false;
   }
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) { if (err) *err = std::string("split-TF32 kernel launch: ") + cudaGetErrorString(e); return false; }
   return true;
 }
 
@@ -634,38 +1051,166 @@ bool f32tc_forward(F32TcModel* m, const F32TcLaunch& L, cudaStream_t s, std::str
 // as the reference caches its transposed weights (runtime/fortis_rt.c:55-66).
 bool f32tc_gemm(const float* A, const float* W, float* C, long long M, int N, int K, int* status, cudaStream_t s, std::string* err) {
   if (M <= 0 || N <= 0 || K <= 0) return true;
-  if (!prepare_kernel(err)) return false;
-  struct Cached { const float* w; int N, K; float *hi, *lo; LayerGeom g; CUtensorMap mh, ml; };
+  struct Cached { const float* src = nullptr; SplitW w; };
   static std::vector<Cached> cache;
   static size_t victim = 0;
   Cached* c = nullptr;
-  for (auto& e : cache) if (e.w == W && e.N == N && e.K == K) c = &e;
+  bool fresh = false;
+  for (auto& e : cache) if (e.src == W && e.w.N_real == N && e.w.K_real == K) c = &e;
   if (!c) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(s, &cs);
     if (cs != cudaStreamCaptureStatusNone) { if (err) *err = "weights seen for the first time during graph capture; run one eager call first"; return false; }
-    if (cache.size() < 64) { cache.push_back(Cached{}); c = &cache.back(); c->hi = c->lo = nullptr; }
-    else { c = &cache[victim]; victim = (victim + 1) % cache.size(); cudaStreamSynchronize(s); cudaFree(c->hi); cudaFree(c->lo); c->hi = c->lo = nullptr; }
-    c->w = nullptr;
-    c->g = layer_geom(K, N);
-    const size_t n_el = (size_t)c->g.N_pad * c->g.K_pad;
-    if (cudaMalloc(&c->hi, n_el * 4) != cudaSuccess || cudaMalloc(&c->lo, n_el * 4) != cudaSuccess) { if (err) *err = "out of device memory for split weights"; return false; }
-    split_weights_kernel<<<(unsigned)((n_el + 255) / 256 < 1184 ? (n_el + 255) / 256 : 1184), 256, 0, s>>>(W, N, K, c->hi, c->lo, c->g.N_pad, c->g.K_pad);
-    if (!make_w_maps(c->hi, c->lo, c->g, &c->mh, &c->ml)) { if (err) *err = "cuTensorMapEncodeTiled failed"; return false; }
-    c->w = W; c->N = N; c->K = K;
+    if (cache.size() < 64) { cache.push_back(Cached()); c = &cache.back(); }
+    else { c = &cache[victim]; victim = (victim + 1) % cache.size(); cudaStreamSynchronize(s); split_free(&c->w); }
+    c->src = nullptr;
+    if (!split_alloc(&c->w, K, N, err)) return false;
+    split_weights_kernel<<<split_grid((size_t)c->w.N_pad * c->w.K_pad), 256, 0, s>>>(W, N, K, (uint32_t*)c->w.hi, (uint32_t*)c->w.lo, c->w.N_pad, c->w.K_pad);
+    c->src = W;
+    fresh = true;
   }
   F32Params P;
   std::memset(&P, 0, sizeof P);
-  P.map_hi = c->mh; P.map_lo = c->ml;
-  P.K_pad = c->g.K_pad; P.N_pad = c->g.N_pad; P.n_tile = c->g.n_tile; P.K_real = K; P.N_real = N;
-  P.slope = 1.f; P.nrows = M; P.status = status;
+  P.nrows = M; P.status = status;
   P.g.count = M; P.g.nk = 1; P.g.ni = 1; P.g.kk0 = 0;
-  P.a_mode = A_ROW_MAJOR; P.A = A; P.lda = K;
-  P.c_mode = C_ROW_MAJOR; P.C = C; P.ldc = N;
-  launch_layer(P, grid_for(M, c->g), s, false);
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) { if (err) *err = std::string("split-TF32 kernel launch: ") + cudaGetErrorString(e); return false; }
+  P.c_mode = C_ROW_MAJOR; P.C = C; P.ldc = N; P.c_vec = N % 4 == 0 && ((uintptr_t)C & 15) == 0;
+  return launched(launch_rows(P, A, K, c->w, s, !fresh), err);
+}
+
+// ---- 16-bit MLPs of few rows -----------------------------------------------------------------------------------
+// The fused kernel gives a 128-row tile to one SM, which streams all weights: a step of few tiles lasts as long as one
+// tile (70 us on 244-768x4-128) on a few SMs.  Here a layer's output tiles (128 rows x 64 or 128 features) are spread over
+// the SMs, layer by layer, the launches chained by programmatic dependent launch.
+
+struct RowsMlp {
+  struct Layer { F16Layer d; CUtensorMap map[2]; };     // box 64 inputs x 64 / 128 features
+  std::vector<Layer> layers;
+  const float *in_div = nullptr, *out_mul = nullptr, *relu_mask = nullptr;
+  bool f16 = false;
+};
+
+void rows_mlp_destroy(RowsMlp* m) { delete m; }
+
+RowsMlp* rows_mlp_create(const std::vector<F16Layer>& layers, bool f16, const float* in_div, const float* out_mul, const float* relu_mask,
+                         std::string* err) {
+  EncodeTiledFnF enc = encode_fn_f();
+  RowsMlp* m = new RowsMlp();
+  m->f16 = f16; m->in_div = in_div; m->out_mul = out_mul; m->relu_mask = relu_mask;
+  for (auto& d : layers) {
+    m->layers.push_back(RowsMlp::Layer());
+    RowsMlp::Layer& T = m->layers.back();
+    T.d = d;
+    const cuuint64_t dims[2] = {(cuuint64_t)d.K_pad, (cuuint64_t)d.N_pad};
+    const cuuint64_t strides[1] = {(cuuint64_t)d.K_pad * 2};
+    const cuuint32_t estr[2] = {1, 1};
+    for (int i = 0; i < 2; i++) {
+      const cuuint32_t box[2] = {64, (cuuint32_t)(64 << i)};
+      if (!enc || enc(&T.map[i], f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(d.w), dims, strides, box, estr,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+        if (err) *err = "cuTensorMapEncodeTiled failed for 16-bit weights";
+        delete m;
+        return nullptr;
+      }
+    }
+  }
+  return m;
+}
+
+template <int AMODE>
+static bool launch_rows16(F32Params& P, const RowsMlp::Layer& T, bool f16, cudaStream_t s) {
+  const long long ntm = (P.nrows + kM - 1) / kM, sms = sm_count();
+  const long long r64 = (ntm * ((T.d.n_real + 63) / 64) + sms - 1) / sms, r128 = (ntm * ((T.d.n_real + 127) / 128) + sms - 1) / sms;
+  const bool wide = T.d.n_real > 64 && 3 * r128 < 2 * r64;       // a wide tile's step takes up to 1.5 times as long
+  P.map_hi = T.map[wide];
+  P.K_real = T.d.k_real; P.N_real = T.d.n_real; P.K_pad = (T.d.k_real + 63) / 64 * 32;
+  P.ntn = wide ? (T.d.n_real + 127) / 128 : (T.d.n_real + 63) / 64;
+  if (wide) return f16 ? launch_as<128, AMODE, 2>(P, s, true) : launch_as<128, AMODE, 1>(P, s, true);
+  return f16 ? launch_as<64, AMODE, 2>(P, s, true) : launch_as<64, AMODE, 1>(P, s, true);
+}
+
+bool rows_mlp_forward(RowsMlp* m, const F32TcLaunch& L, cudaStream_t s, std::string* err) {
+  const long long nrows = L.g.count * L.g.nk;
+  if (nrows <= 0) return true;
+  const int nl = (int)m->layers.size();
+  for (int l = 0; l < nl; l++) {
+    const RowsMlp::Layer& T = m->layers[l];
+    F32Params P;
+    std::memset(&P, 0, sizeof P);
+    P.bias = T.d.bias; P.scale = T.d.scale; P.slope = T.d.slope; P.nrows = nrows; P.g = L.g; P.status = L.status;
+    if (l == nl - 1) {
+      P.out_mul = m->out_mul; P.relu_mask = m->relu_mask;
+      if (L.fast_out) {
+        P.c_mode = C_SCATTER; P.store_by_slot = L.store_by_slot; P.TS = L.TS;
+        for (int i = 0; i < 2; i++) P.cout[i] = StrideClassF{L.cout[i][0], L.cout[i][1], L.cout[i][2]};
+        P.partials = L.partials; P.sum = L.partials ? L.sum : nullptr; P.done = L.done;
+      } else { P.c_mode = C_ROW_MAJOR; P.C = L.Y; P.ldc = T.d.n_real; P.c_vec = T.d.n_real % 4 == 0 && ((uintptr_t)L.Y & 15) == 0; }
+    } else { P.c_mode = C_FEATURE_MAJOR; P.C16 = reinterpret_cast<uint32_t*>(L.act[l & 1]); P.ldc = L.act_ld; }
+    bool ok;
+    if (l == 0) {
+      P.in_div = m->in_div;
+      if (L.fast_in) {
+        P.slots = L.slots; P.TG = L.TG;
+        for (int i = 0; i < 2; i++) P.cin[i] = StrideClassF{L.cin[i][0], L.cin[i][1], L.cin[i][2]};
+        ok = launch_rows16<A_GATHER>(P, T, m->f16, s);
+      } else {
+        P.A = L.X; P.lda = T.d.k_real;
+        ok = launch_rows16<A_ROW_MAJOR>(P, T, m->f16, s);
+      }
+    } else {
+      // pairs of features are what a row of fp32 features is to the fp32 form
+      ok = make_a_map(true, L.act[(l - 1) & 1], nrows, (T.d.k_real + 1) / 2, L.act_ld, &P.map_a) && launch_rows16<A_TILE_T>(P, T, m->f16, s);
+    }
+    if (!launched(ok, err)) return false;
+  }
   return true;
+}
+
+// ---- convolutions ----------------------------------------------------------------------------------------------
+
+struct F32ConvW { SplitW w; int C = 0, taps = 0, group = 1; };
+
+// channels per table entry: groups of 8 share one test of a tap's position; with few channels that would mostly pad
+static int conv_group(int C) { return (C % 8 == 0 || C > 16) ? 8 : 1; }
+
+bool f32tc_conv_supported(const ConvGeom& g) {
+  if (g.dd != 1 || g.dh != 1 || g.dw != 1) return false;                       // transposed convolutions
+  if (g.KD > 32 || g.KH > 32 || g.KW > 32) return false;                       // one bit per tap and axis
+  const int G = conv_group(g.C);
+  const long long taps = (long long)g.KD * g.KH * g.KW, entries = taps * ((g.C + G - 1) / G);
+  if (entries * 8 + 32 * 8 > kConvTabMax) return false;
+  // row numbers and the offsets of taps and channels in 32 bits
+  const long long rows = (long long)g.N * g.Do * g.Ho * g.Wo;
+  const long long reach = (g.KD - 1) * g.xs_d + (g.KH - 1) * g.xs_h + (g.KW - 1) * g.xs_w + (g.C - 1) * g.xs_c;
+  return rows < (1LL << 31) - kM && reach < (1LL << 31);
+}
+
+void f32tc_conv_free(F32ConvW* w) {
+  if (!w) return;
+  split_free(&w->w);
+  delete w;
+}
+
+// w_dev: torch layout (F, C, taps) on the device; split on stream `s`
+F32ConvW* f32tc_conv_pack(const float* w_dev, int F, int C, int taps, cudaStream_t s, std::string* err) {
+  F32ConvW* w = new F32ConvW();
+  w->C = C; w->taps = taps; w->group = conv_group(C);
+  if (!split_alloc(&w->w, taps * ((C + w->group - 1) / w->group * w->group), F, err)) { delete w; return nullptr; }
+  split_conv_weights_kernel<<<split_grid((size_t)w->w.N_pad * w->w.K_pad), 256, 0, s>>>(w_dev, F, C, taps, w->group, (uint32_t*)w->w.hi, (uint32_t*)w->w.lo,
+                                                                                       w->w.N_pad, w->w.K_pad);
+  return w;
+}
+
+bool f32tc_conv(const F32ConvW* w, const float* x, const float* bias, const float* residual, float* y, const ConvGeom& g, int act,
+                float slope, int* status, cudaStream_t s, bool early, std::string* err) {
+  F32Params P;
+  std::memset(&P, 0, sizeof P);
+  P.nrows = (long long)g.N * g.Do * g.Ho * g.Wo;
+  if (P.nrows <= 0) return true;
+  P.status = status; P.bias = bias; P.act = act; P.slope = slope;
+  P.A = x; P.cv = g; P.residual = residual;
+  P.c_mode = C_CONV; P.C = y;
+  return launched(w->group == 8 ? launch_tile<A_CONV8>(P, w->w, kStepFloorConv, s, early) : launch_tile<A_CONV1>(P, w->w, kStepFloorConv, s, early), err);
 }
 
 }  // namespace fortis

@@ -1,0 +1,156 @@
+"""The split-TF32 tensor-core kernel (fp32 Linear layers and convolutions) at the edges of its tiles, steps and dispatch
+rules, against float64.
+
+Tolerance: every product keeps 21 bits of each operand and drops lo.lo, at most 2^-21 + 2^-22 of the
+product; the sums add 8 truncations per 64 k and one rounding per chunk, at most 8 * 2^-23 of the partial sums.  With
+zero-mean data both stay below 2^-20 = 9.5e-7 of the result's 2-norm.
+"""
+import ctypes
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import fortis_b200
+from fortis_b200 import descriptors
+
+TOL = 2.0 ** -20
+
+
+@pytest.fixture()
+def host():
+    h = fortis_b200.Host()
+    h.reset()
+    yield h
+    h.reset()
+
+
+def rel(a, b):
+    a, b = a.double(), b.double()
+    return float((a - b).norm() / b.norm())
+
+
+def memref(t):
+    return (t.data_ptr(), t.data_ptr(), 0) + tuple(t.shape) + tuple(t.stride())
+
+
+def randn(shape, seed, scale=1.0):
+    return torch.randn(shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(seed)) * scale
+
+
+_keep = []      # weights of the memref entries are constants of the program, told apart by their address
+
+
+@pytest.mark.parametrize("B,N,K", [(512, 1, 1), (512, 32, 32), (513, 33, 31), (640, 64, 33), (641, 65, 64), (1000, 96, 65), (767, 129, 130),
+                                   (2000, 257, 100), (19000, 200, 36)])
+def test_gemm_tile_and_step_edges(host, B, N, K):
+    A, W = randn((B, K), 1), randn((N, K), 2)
+    C = torch.full((B, N), float("nan"), device="cuda")
+    _keep.append(W)
+    f = host.L.fortis_gemm
+    f.argtypes, f.restype = ([ctypes.c_void_p] * 2 + [ctypes.c_long] * 5) * 3 + [ctypes.c_long] * 3, None
+    f(*memref(A), *memref(W), *memref(C), B, N, K)
+    host.sync()
+    assert rel(C, A.double() @ W.double().T) < TOL
+    assert host.L.fortis_device_status() == 0
+
+
+def conv_entry(host, x, w, y, stride, pad):
+    f = host.L.fortis_conv3d
+    f.argtypes, f.restype = ([ctypes.c_void_p] * 2 + [ctypes.c_long] * 11) * 3 + [ctypes.c_long] * 18, None
+    _keep.append(w)
+    f(*memref(x), *memref(w), *memref(y), x.shape[0], x.shape[1], *x.shape[2:], w.shape[0], *w.shape[2:], *y.shape[2:], *stride, *pad)
+    host.sync()
+
+
+def conv64(x, w, stride, pad):
+    return torch.nn.functional.conv3d(x.cpu().double(), w.cpu().double(), stride=stride, padding=pad).cuda()
+
+
+@pytest.mark.parametrize("C,F,K,stride,pad,shape", [
+    (1, 1, (1, 1, 1), (1, 1, 1), (0, 0, 0), (1, 3, 4, 5)),           # one tap, one channel
+    (7, 31, (3, 3, 3), (1, 1, 1), (1, 1, 1), (2, 5, 6, 7)),          # channels one by one
+    (8, 33, (2, 3, 4), (1, 2, 3), (0, 1, 3), (1, 6, 9, 11)),         # one group of channels, other extents per axis
+    (16, 64, (3, 3, 3), (2, 2, 2), (1, 1, 1), (1, 9, 9, 17)),
+    (17, 65, (3, 3, 3), (1, 1, 1), (2, 2, 2), (1, 4, 5, 6)),         # a ragged group; padding wider than K / 2
+    (39, 96, (1, 5, 5), (1, 1, 1), (0, 0, 0), (2, 1, 12, 9)),
+    (3, 130, (7, 1, 1), (1, 1, 1), (3, 0, 0), (1, 5, 8, 40)),
+    (64, 64, (3, 3, 3), (1, 1, 1), (1, 1, 1), (2, 8, 9, 10)),
+    (2, 3, (33, 1, 1), (1, 1, 1), (16, 0, 0), (1, 40, 3, 3)),        # more taps on an axis than the kernel takes: FFMA
+])
+def test_conv_groups_taps_and_strides(host, C, F, K, stride, pad, shape):
+    x, w = randn((shape[0], C) + shape[1:], 3), randn((F, C) + K, 4)
+    want = conv64(x, w, stride, pad)
+    y = torch.full(want.shape, float("nan"), device="cuda")
+    conv_entry(host, x, w, y, stride, pad)
+    assert rel(y, want) < TOL
+    assert host.L.fortis_device_status() == 0
+
+
+def test_conv_infinities_nans_and_the_largest_values(host):
+    """Where fp32 arithmetic gives an infinity or NaN so does the split form, and nowhere else; values that round past
+    the largest TF32 value stay finite."""
+    x, w = randn((1, 8, 6, 7, 40), 5), randn((5, 8, 3, 3, 3), 6)
+    w[0, 0, 0, 0, 0] = 0.5                                            # its low half is exactly zero
+    x[0, 1, 2, 3, 4], x[0, 2, 4, 5, 20], x[0, 3, 1, 1, 30] = float("inf"), float("-inf"), float("nan")
+    want = conv64(x, w, (1, 1, 1), (1, 1, 1))
+    y = torch.zeros(want.shape, device="cuda")
+    conv_entry(host, x, w, y, (1, 1, 1), (1, 1, 1))
+    assert torch.equal(torch.isnan(y), torch.isnan(want)) and torch.equal(torch.isinf(y), torch.isinf(want))
+    inf = torch.isinf(want)
+    assert torch.equal(torch.sign(y[inf]).double(), torch.sign(want[inf]))
+    fine = torch.isfinite(want)
+    assert rel(y[fine], want[fine]) < TOL
+    big = torch.full((1, 1, 1, 1, 4), 3.4028234e38, device="cuda")
+    w1 = torch.full((1, 1, 1, 1, 1), 0.25, device="cuda")
+    y1 = torch.zeros_like(big)
+    conv_entry(host, big, w1, y1, (1, 1, 1), (0, 0, 0))
+    assert rel(y1, big.double() * 0.25) < TOL
+
+
+def test_conv_net_whose_last_layer_adds_a_skip(host):
+    """Volumes between layers are channel-major, the program's arrays are channels-last: a skip added by the last layer
+    is read in the one layout and the result stored in the other."""
+    rng = np.random.default_rng(8)
+    conv = lambda ci, co: (0.2 * rng.standard_normal((co, ci, 3, 3, 3))).astype(np.float32)
+    layers = [dict(W=conv(5, 12), b=rng.standard_normal(12).astype(np.float32), act="leaky", slope=0.1, pad=1, save=True),
+              dict(W=conv(12, 20), b=np.zeros(20, np.float32), act="relu", pad=1),
+              dict(W=conv(20, 12), b=np.ones(12, np.float32), act="none", pad=1, add=True)]
+    x = randn((2, 5, 6, 7, 5), 9)
+    y = torch.zeros((2, 5, 6, 7, 12), device="cuda")
+    host.load_model(fortis_b200.write_blob(layers))
+    host.option("conv_shape", "2,5,6,7")
+    host.forward(x, y)
+    h, skip = x.double().permute(0, 4, 1, 2, 3), None
+    for L in layers:
+        h = conv64(h, torch.from_numpy(L["W"]), 1, 1) + torch.from_numpy(L["b"]).double().cuda().reshape(1, -1, 1, 1, 1)
+        if L.get("add"):
+            h = h + skip
+        h = {"none": lambda v: v, "relu": lambda v: v.clamp_min(0), "leaky": lambda v: torch.where(v > 0, v, v * 0.1)}[L["act"]](h)
+        if L.get("save"):
+            skip = h
+    assert rel(y, h.permute(0, 2, 3, 4, 1)) < 3 * TOL                # three layers
+
+
+@pytest.mark.parametrize("dims,rows", [([244, 768, 128], 1), ([244, 768, 128], 129), ([33, 65, 31, 7], 300), ([64, 1000, 5], 511), ([5, 3], 1)])
+def test_mlp_of_few_rows(host, dims, rows):
+    """Every row count of a model runs on the tensor cores: through the descriptors and through row-major arrays."""
+    layers = fortis_b200.mlp_layers(dims, seed=3, act="relu", bias="uniform", scale=0.1)
+    G, S, Lp, K = descriptors.identity(dims[0], dims[-1], rows)
+    x = randn((rows, dims[0]), 10)
+    host.configure(gather=G, scatter=S, loop=Lp)
+    host.load_model(fortis_b200.write_blob(layers))
+    y, z = (torch.full((rows, dims[-1]), float("nan"), device="cuda") for _ in range(2))
+    host.step([x], [y])
+    host.L.mlp_forward_batched(x.data_ptr(), z.data_ptr())
+    host.check()
+    want = x.double()
+    for i, L in enumerate(layers):
+        want = want @ torch.from_numpy(L["W"]).double().cuda().T + torch.from_numpy(L["b"]).double().cuda()
+        if i + 1 < len(layers):
+            want = want.clamp_min(0)
+    # one layer's bound per layer; an output near zero after cancellation is bounded against the largest sums it is made of
+    assert rel(y, want) < 4 * TOL * len(layers) and rel(z, want) < 4 * TOL * len(layers)
+    assert host.L.fortis_device_status() == 0
