@@ -1108,6 +1108,7 @@ struct TcModel {
   TcLayer layer[kMaxLayers];
   CUtensorMap maps[kMaxLayers];
   bool has_scale = false, f16 = false;
+  RowsMlp* rows = nullptr;         // the same weights for calls of few rows (cluster form's weights only)
   bool pair = false;               // run as two-CTA clusters (row-major weights + tensor maps are on the device as well)
 };
 
@@ -1116,12 +1117,14 @@ struct TcModel {
 // bf16 / fp16 and 8-9 % faster with FP8 weights.
 static int g_tc_pair = -1;
 void tc_set_pair_mode(int on) { g_tc_pair = on; }
-bool tc_pair_mode(int precision) {
+// 1 / 0: asked for by the option or the environment; -1: neither (clusters, or layer by layer where rows are few)
+static int tc_pair_chosen() {
   static const int env = [] { const char* e = std::getenv("FORTIS_TC_PAIR"); return e ? (std::atoi(e) != 0 ? 1 : 0) : -1; }();
-  if (g_tc_pair >= 0) return g_tc_pair != 0;
-  if (env >= 0) return env != 0;
+  return g_tc_pair >= 0 ? g_tc_pair : env;
+}
+bool tc_pair_mode(int precision) {
   (void)precision;
-  return true;
+  return tc_pair_chosen() != 0;
 }
 
 bool tc_model_supported(const ModelHost& M, std::string* why) {
@@ -1187,8 +1190,15 @@ void tc_model_destroy(TcModel* m) {
   for (float* p : m->bias) cudaFree(p);
   for (float* p : m->scale) cudaFree(p);
   cudaFree(m->in_div); cudaFree(m->out_mul); cudaFree(m->relu_mask);
+  rows_mlp_destroy(m->rows);
   delete m;
 }
+
+// Few rows run layer by layer (RowsMlp) instead of fused: the fused kernel gives a 128-row tile to one SM of a cluster, whose
+// time is its stream of all weights, while a layer of RowsMlp spreads its tiles over the SMs and pays a launch.  Measured
+// on 244-768x4-128, bf16, fused / layer by layer: 1000 rows 62.9 / 35.8 us, 2000 61.9 / 44.8, 4000 61.8 / 61.9, 8192 62.1 / 75.9;
+// at 3000 rows 64-256-256-64 29.9 / 23.6, 244-512-512-128 63.6 / 33.5, seven layers of 768 120.8 / 64.6.
+constexpr long long kFewRows = 3072;
 
 TcModel* tc_model_create(const ModelHost& M, int precision, cudaStream_t s, std::string* err) {
   (void)s;
@@ -1264,12 +1274,31 @@ TcModel* tc_model_create(const ModelHost& M, int precision, cudaStream_t s, std:
     return fail("cannot reserve " + std::to_string(kSmemBytes) + " bytes of shared memory for the tensor-core kernel");
   m->has_scale = precision == PREC_FP8W;
   m->f16 = precision == PREC_FP16;
+  if (pair && tc_pair_chosen() < 0) {
+    std::vector<F16Layer> rl;
+    for (int l = 0; l < m->nlayers; l++) {
+      const TcLayer& T = m->layer[l];
+      rl.push_back(F16Layer{m->w[l], T.K, T.N, M.layers[l].cin, T.n_real, T.bias, T.scale, T.slope});
+    }
+    m->rows = rows_mlp_create(rl, m->f16, m->in_div, m->out_mul, m->relu_mask, &why);
+    if (!m->rows) return fail(why);
+  }
   return m;
 }
 
 bool tc_forward(TcModel* m, const TcLaunch& L, cudaStream_t s, std::string* err) {
   const long long nrows = L.g.count * L.g.nk;
   if (nrows <= 0) return true;
+  const bool knobs = g_tc_test.wait_limit || g_tc_test.skip_stage || g_tc_test.no_stage;       // they address the fused kernel
+  if (m->rows && !knobs && L.act[0] && (m->nlayers < 3 || L.act[1]) && nrows <= kFewRows) {
+    F32TcLaunch R{};
+    R.fast_in = L.fast_in; R.slots = L.slots; R.TG = L.TG; R.X = L.X;
+    R.fast_out = L.fast_out; R.store_by_slot = L.store_by_slot; R.TS = L.TS; R.Y = L.Y;
+    std::memcpy(R.cin, L.cin, sizeof R.cin); std::memcpy(R.cout, L.cout, sizeof R.cout);
+    R.g = L.g; R.act[0] = L.act[0]; R.act[1] = L.act[1]; R.act_ld = L.act_ld;
+    R.partials = L.partials; R.sum = L.sum; R.done = L.done; R.status = L.status;
+    return rows_mlp_forward(m->rows, R, s, err);
+  }
   TcParams P;
   std::memset(&P, 0, sizeof P);
   for (int l = 0; l < m->nlayers; l++) { P.maps[l] = m->maps[l]; P.layer[l] = m->layer[l]; }
