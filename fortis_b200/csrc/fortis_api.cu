@@ -620,9 +620,11 @@ void download_stores(PlanDev& P, const int* args, int nargs, bool multi_plane, c
 // ---------------------------------------------------------------------------------------------------------------
 // the step
 // ---------------------------------------------------------------------------------------------------------------
-// fortis_gemm: from this batch on the weights are split once per address (constants of the caller); below it W is read as
-// it is on every call, by the FFMA kernel
-constexpr long long kGemmTcMinRows = 512;
+// Below this many rows the per-layer FFMA kernels run: their sums are what a program of few rows has always had.  (The
+// tensor-core kernel is faster there too, 300 rows of the column network 73 us against 455, but further from those sums
+// than from the exact ones.)  fortis_gemm: from here on the weights are split once per address (constants of the caller);
+// below, W is read as it is on every call.
+constexpr long long kF32TcMinRows = 512;
 
 struct StepArgs {
   bool use_gather = false;      // model input comes from the gather plan (else din)
@@ -804,7 +806,7 @@ void run_step_kernels(const StepArgs& A) {
     if (L.partials) launch_fold(s.d_partials, L.grid, s.d_sum, 1, st);
     return;
   }
-  if (s.f32) {
+  if (s.f32 && rows >= kF32TcMinRows) {
     // fp32 on the tensor cores: one split-TF32 kernel per layer, gather fused into the first layer's operand load and
     // scatter (+ checksum) into the last epilogue when the descriptors are table-driven, activations feature-major
     F32TcLaunch L{};
@@ -1703,7 +1705,7 @@ void fortis_gemm(float* Aa, float* A, long Ao, long As0, long As1, long At0, lon
                  B, K, At0, At1, N, K, Wt0, Wt1, B, N, Ct0, Ct1);
     return;
   }
-  if (B >= kGemmTcMinRows) {
+  if (B >= kF32TcMinRows) {
     // large batch: the tensor-core kernel (three TF32 MMAs per product, fp32-class accuracy)
     S();
     ensure_aux(1);

@@ -23,13 +23,13 @@
 // Operand traffic is why A sits in tensor memory: with A in shared memory (the form before this one) the three MMAs of a
 // k step read 12 KB per 128 clocks and the producers and the TMA write 96 KB per 1536, together 1.25 times what shared
 // memory moves; in this form only the weights (64 B/clk at any NT) and the fp32 tiles pass through it.
-// Measured, that form / this one: fortis_gemm 8192 x 768 x 768 756 / 59 us (a row-major operand was read by one dependent load
-// per row), column network 30,011 rows 994 / 769 us; convolutions against the FFMA kernel: 32 -> 64 channels 3x3x3 on 40^3
-// 297 / 70 us, 14-layer network 2 x 33^3 8.76 / 1.80 ms.
+// Measured, that form / this one: fortis_gemm 8192 x 768 x 768 756 / 63 us (a row-major operand was read by one dependent load
+// per row), column network 30,011 rows 991 / 766 us; convolutions against the FFMA kernel: 32 -> 64 channels 3x3x3 on 40^3
+// 297 / 78 us, 14-layer network 2 x 33^3 8.76 / 2.00 ms.
 //
 // The tensor core adds into its fp32 accumulator with truncation, not rounding, a bias per accumulation of half a unit in
 // the last place of the partial sum.  Two things keep it below fp32 rounding: the hi.hi products go into an accumulator
-// of their own that is taken over every 64 k (8 truncating additions) and summed by the epilogue warps in registers with
+// of their own that is taken over every 64 k (8 truncating additions; 32 where K is short) and summed by the epilogue warps in registers with
 // IEEE additions, and the two cross products go into a second accumulator (2^-11 of the result, so its truncation does not
 // count) that lives for the whole K.
 // Infinities: x_hi saturates at the largest finite TF32 value and x_lo = x - x_hi carries the infinity, so a product is
@@ -58,7 +58,14 @@ using namespace tc;
 
 constexpr int kM = 128;                    // rows per tile
 constexpr int kKt = 32;                    // k per stage: one 128-byte swizzle row of fp32
-constexpr int kChunkKt = 2;                // k steps of 32 accumulated in the tensor core before the sum is taken over (K = 64)
+// k steps of 32 accumulated in the tensor core before the sum is taken over: two, or one where K is short, so that the
+// truncations (a bias) stay below the few roundings fp32 arithmetic has there (2-D network of K = 27 to 576, six
+// convolutions, error against 64 bits: two 9.1e-7, one 6.2e-7, FFMA 7.7e-7)
+constexpr int kChunkLong = 2, kChunkShort = 1, kShortK = 640;
+// MLP steps keep the sums they have always had: the three products of a step of 8 k one after another in one accumulator
+// that is taken over every 128 k.  Further from the exact sums (five-layer column network 5.6e-6 against 2.4e-6), but a
+// program's results stay what they were to the last bit.
+constexpr int kChunkMlp = 4;
 constexpr int kBarF = 384;
 constexpr int kTabIn = 768, kTabOut = 256;     // widest gathered input / scattered output the tables hold
 constexpr int kTileScratch = 32 * 32 * 4;      // one warp's 32 x 32 transpose
@@ -87,6 +94,8 @@ struct StrideClassF { long long si, sj, sk; };
 
 struct F32Params {
   CUtensorMap map_hi, map_lo;            // W_hi / W_lo [N_pad][K_pad] fp32, box 32 x NT
+  int chunk_kt;                          // k steps per chunk
+  int one_acc;                           // all three products in one accumulator (MLP steps: see kChunkMlp)
   int K_pad, K_real, N_real, ntn;        // ntn: output tiles along N (16-bit: K_pad counts pairs, a step is 64 inputs)
   const float* scale;                    // 16-bit forms, FP8 weights: per feature
   uint32_t* C16;                         // 16-bit forms, hidden layers: [feature / 2][row] pairs
@@ -381,7 +390,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
     const uint32_t cross = tmem + CF::kColCross;
     for (long long t = blockIdx.x; t < ntiles; t += gridDim.x, tile_it++) {
       for (int kt = 0; kt < nkt; kt++) {
-        const uint32_t in_chunk = P16 ? (uint32_t)kt : (uint32_t)(kt % kChunkKt), b = chunk_it & 1;
+        const uint32_t in_chunk = P16 ? (uint32_t)kt : (uint32_t)(kt % P.chunk_kt), b = chunk_it & 1;
         if (in_chunk == 0) mbar_wait(acc_empty + 8 * b, ((chunk_it >> 1) & 1) ^ 1, abort_flag, P.status, FST_ACC_EMPTY);
         mbar_wait(w_full + 8 * ws, wph, abort_flag, P.status, FST_W_FULL);
         mbar_wait(a_full + 8 * as, aph, abort_flag, P.status, FST_A_FULL);
@@ -393,6 +402,13 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
           tc_mma_ts_first<idesc>(acc, ah, wh, in_chunk);
 #pragma unroll
           for (int j = 1; j < kKt / 8; j++) tc_mma_ts_acc<idesc>(acc, ah + 8 * j, wh + (uint64_t)(2 * j));    // 16 k = 32 bytes
+        } else if (P.one_acc) {
+#pragma unroll
+          for (int j = 0; j < kKt / 8; j++) {
+            mma_tf32_ts<idesc>(acc, ah + 8 * j, wh + (uint64_t)(2 * j), in_chunk | (uint32_t)j);
+            mma_tf32_ts<idesc>(acc, ah + 8 * j, wl + (uint64_t)(2 * j), 1u);
+            mma_tf32_ts<idesc>(acc, al + 8 * j, wh + (uint64_t)(2 * j), 1u);
+          }
         } else {
 #pragma unroll
           for (int j = 0; j < kKt / 8; j++)             // 8 tf32 = 32 bytes per k step: the address field moves by 2
@@ -409,7 +425,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
         }
         tc_commit(a_empty + 8 * as);
         tc_commit(w_empty + 8 * ws);
-        if ((!P16 && in_chunk == kChunkKt - 1) || kt == nkt - 1) { tc_commit(acc_full + 8 * b); chunk_it++; }
+        if ((!P16 && in_chunk == (uint32_t)P.chunk_kt - 1) || kt == nkt - 1) { tc_commit(acc_full + 8 * b); chunk_it++; }
         if (++as == CF::kAStages) { as = 0; aph ^= 1; }
         if (++ws == CF::kWStages) { ws = 0; wph ^= 1; }
       }
@@ -551,7 +567,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
     float* s_scale = s_bias + NH;
     uint32_t chunk_it = 0;
     double csum = 0.0;
-    const int nch = P16 ? 1 : (nkt + kChunkKt - 1) / kChunkKt;
+    const int nch = P16 ? 1 : (nkt + P.chunk_kt - 1) / P.chunk_kt;
     for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
       const long long m0 = (t / P.ntn) * kM, row = m0 + r;
       const int nt0 = (int)(t % P.ntn) * NT + half * NH;
@@ -566,7 +582,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
       __syncwarp();
       float v[NH];
 #pragma unroll
-      for (int j = 0; j < NH; j++) v[j] = 0.f;
+      for (int j = 0; j < NH; j++) v[j] = -0.f;            // -0 + x is x, also where x is -0
       for (int ch = 0; ch < nch; ch++, chunk_it++) {
         const uint32_t b = chunk_it & 1;
         mbar_wait(acc_full + 8 * b, (chunk_it >> 1) & 1, abort_flag, P.status, FST_ACC_FULL);
@@ -583,7 +599,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
         __syncwarp();
         if (lane == 0) mbar_arrive(acc_empty + 8 * b);
       }
-      if constexpr (P16 == 0) {
+      if (P16 == 0 && !P.one_acc) {
 #pragma unroll
       for (int c0 = 0; c0 < NH; c0 += NL) {
         uint32_t a[NL];
@@ -919,6 +935,7 @@ bool launch_tile(F32Params& P, const SplitW& W, int step_floor, cudaStream_t s, 
   const int w = pick_tile(P.nrows, W.N_real, step_floor);
   P.map_hi = W.map_hi[w]; P.map_lo = W.map_lo[w];
   P.K_pad = W.K_pad; P.K_real = W.K_real; P.N_real = W.N_real;
+  P.chunk_kt = P.one_acc ? kChunkMlp : W.K_pad <= kShortK ? kChunkShort : kChunkLong;
   P.ntn = (W.N_real + (32 << w) - 1) / (32 << w);
   return w == 2 ? launch_as<128, AMODE>(P, s, early) : w == 1 ? launch_as<64, AMODE>(P, s, early) : launch_as<32, AMODE>(P, s, early);
 }
@@ -1015,7 +1032,7 @@ bool f32tc_forward(F32TcModel* m, const F32TcLaunch& L, cudaStream_t s, std::str
     const F32TcModel::Layer& T = m->layers[l];
     F32Params P;
     std::memset(&P, 0, sizeof P);
-    P.bias = T.bias; P.act = T.act; P.slope = T.slope; P.nrows = nrows; P.g = L.g; P.status = L.status;
+    P.bias = T.bias; P.act = T.act; P.slope = T.slope; P.nrows = nrows; P.g = L.g; P.status = L.status; P.one_acc = 1;
     if (l == nl - 1) {
       P.out_mul = m->out_mul; P.relu_mask = m->relu_mask;
       if (fast_out) {
