@@ -202,8 +202,8 @@ bool upload_layer(const LayerHost& L, int taps, bool split, LayerDev* d, std::st
 }
 
 // A layer takes the tensor-core kernel wherever it can (f32tc_conv_supported: no input dilation, up to 32 taps per axis, a
-// table of taps and channels that fits shared memory): 14-layer network, 2 x 33^3 voxels, 2.00 ms against 8.76 on the FFMA
-// kernel; 32 -> 64 channels on 40^3 78 us against 297; and closer to the exact sums (2.1e-7 against 5.2e-7).
+// table of taps and channels that fits shared memory): 14-layer network, 2 x 33^3 voxels, 1.80 ms against 8.75 on the FFMA
+// kernel; 32 -> 64 channels on 40^3 71 us against 297; and closer to the exact sums (2.1e-7 against 5.2e-7).
 bool conv_layer(const F32ConvW* split, const float* wt, const float* bias, const float* x, const float* residual, float* y, const ConvGeom& g,
                 int act, float slope, int* status, cudaStream_t s, std::string* err) {
   if (split && f32tc_conv_supported(g)) return f32tc_conv(split, x, bias, residual, y, g, act, slope, status, s, true, err);

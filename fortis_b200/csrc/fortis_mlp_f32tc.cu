@@ -23,9 +23,9 @@
 // Operand traffic is why A sits in tensor memory: with A in shared memory (the form before this one) the three MMAs of a
 // k step read 12 KB per 128 clocks and the producers and the TMA write 96 KB per 1536, together 1.25 times what shared
 // memory moves; in this form only the weights (64 B/clk at any NT) and the fp32 tiles pass through it.
-// Measured, that form / this one: fortis_gemm 8192 x 768 x 768 756 / 63 us (a row-major operand was read by one dependent load
-// per row), column network 30,011 rows 991 / 766 us; convolutions against the FFMA kernel: 32 -> 64 channels 3x3x3 on 40^3
-// 297 / 78 us, 14-layer network 2 x 33^3 8.76 / 2.00 ms.
+// Measured, that form / this one: fortis_gemm 8192 x 768 x 768 756 / 60 us (a row-major operand was read by one dependent load
+// per row), column network 30,011 rows 991 / 730 us; convolutions against the FFMA kernel: 32 -> 64 channels 3x3x3 on 40^3
+// 297 / 71 us, 14-layer network 2 x 33^3 8.75 / 1.80 ms.
 //
 // The tensor core adds into its fp32 accumulator with truncation, not rounding, a bias per accumulation of half a unit in
 // the last place of the partial sum.  Two things keep it below fp32 rounding: the hi.hi products go into an accumulator
@@ -277,6 +277,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
                  cross_empty = bars + 192, raw_full = bars + 208, raw_empty = bars + 240;
   uint32_t* tmem_slot = (uint32_t*)(tail + 200);
   volatile int* abort_flag = (volatile int*)(tail + 204);
+  constexpr bool kMaybeOneAcc = AMODE != A_CONV8 && AMODE != A_CONV1;
   constexpr bool kTile = AMODE == A_TILE_T || AMODE == A_TILE_R;
   uint8_t* a_scratch = tail + kBarF + kEWarps * 2 * (NT / kESets) * 4;
   uint8_t* c_scratch = a_scratch + (AMODE == A_ROW_MAJOR ? kPWarps * kTileScratch : 0);
@@ -389,8 +390,9 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
     constexpr uint32_t idesc = P16 == 0 ? idesc_tf32(NT) : idesc_16(NT, P16 == 2);
     const uint32_t cross = tmem + CF::kColCross;
     for (long long t = blockIdx.x; t < ntiles; t += gridDim.x, tile_it++) {
+      uint32_t in_chunk = 0;                            // 16-bit forms: one chunk per tile
       for (int kt = 0; kt < nkt; kt++) {
-        const uint32_t in_chunk = P16 ? (uint32_t)kt : (uint32_t)(kt % P.chunk_kt), b = chunk_it & 1;
+        const uint32_t b = chunk_it & 1;
         if (in_chunk == 0) mbar_wait(acc_empty + 8 * b, ((chunk_it >> 1) & 1) ^ 1, abort_flag, P.status, FST_ACC_EMPTY);
         mbar_wait(w_full + 8 * ws, wph, abort_flag, P.status, FST_W_FULL);
         mbar_wait(a_full + 8 * as, aph, abort_flag, P.status, FST_A_FULL);
@@ -402,7 +404,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
           tc_mma_ts_first<idesc>(acc, ah, wh, in_chunk);
 #pragma unroll
           for (int j = 1; j < kKt / 8; j++) tc_mma_ts_acc<idesc>(acc, ah + 8 * j, wh + (uint64_t)(2 * j));    // 16 k = 32 bytes
-        } else if (P.one_acc) {
+        } else if (kMaybeOneAcc && P.one_acc) {
 #pragma unroll
           for (int j = 0; j < kKt / 8; j++) {
             mma_tf32_ts<idesc>(acc, ah + 8 * j, wh + (uint64_t)(2 * j), in_chunk | (uint32_t)j);
@@ -425,7 +427,8 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
         }
         tc_commit(a_empty + 8 * as);
         tc_commit(w_empty + 8 * ws);
-        if ((!P16 && in_chunk == (uint32_t)P.chunk_kt - 1) || kt == nkt - 1) { tc_commit(acc_full + 8 * b); chunk_it++; }
+        in_chunk++;
+        if ((!P16 && in_chunk == (uint32_t)P.chunk_kt) || kt == nkt - 1) { tc_commit(acc_full + 8 * b); chunk_it++; in_chunk = 0; }
         if (++as == CF::kAStages) { as = 0; aph ^= 1; }
         if (++ws == CF::kWStages) { ws = 0; wph ^= 1; }
       }
@@ -599,7 +602,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
         __syncwarp();
         if (lane == 0) mbar_arrive(acc_empty + 8 * b);
       }
-      if (P16 == 0 && !P.one_acc) {
+      if (P16 == 0 && !(kMaybeOneAcc && P.one_acc)) {
 #pragma unroll
       for (int c0 = 0; c0 < NH; c0 += NL) {
         uint32_t a[NL];
