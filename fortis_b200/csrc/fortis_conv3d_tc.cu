@@ -132,10 +132,6 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
   constexpr int kHalfRows = (kShiftA ? NOUT : 3 * NOUT) / 2;      // weight rows of one tile held by each CTA
   constexpr int kHalfBytes = kHalfRows * kC * 2;                  // 4 KB per tap (12 KB per group)
   extern __shared__ __align__(1024) uint8_t smem[];
-  // Programmatic dependent launch: the next layer's CTAs may be scheduled as soon as SMs free up.  They set up their
-  // barriers and tensor memory and load their weights while this layer's last tiles finish, and wait (griddep_wait below)
-  // for this grid to complete before they touch an activation buffer.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t base = smem_u32(smem);                           // resident weights at offset 0
   if (base & 1023u) {                                             // same in both CTAs of a pair: both leave
     if (threadIdx.x == 0) atomicCAS(P.status, 0, CST_ALIGN);
@@ -175,6 +171,12 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
   cluster_sync_all();                      // both CTAs' barriers exist before either signals the other's
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  // Programmatic dependent launch: the next layer's CTAs may be scheduled as soon as SMs free up.  They set up their
+  // barriers and tensor memory and load their weights while this layer's last tiles finish, and wait (griddepcontrol.wait below)
+  // for this grid to complete before they touch an activation buffer.
+  // Not before both CTAs have their tensor memory: a dependent CTA that fits the SM as well would take the columns first
+  // and keep them while it waits for this grid.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == 0) {
     // ---- TMA producer (one per CTA): this CTA's half of the weights once, then per tile 9 activation tiles.

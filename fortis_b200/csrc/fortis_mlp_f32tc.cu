@@ -258,9 +258,6 @@ template <int NT, int AMODE, int P16>
 __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_constant__ F32Params P) {
   using CF = TileCfg<NT>;
   extern __shared__ __align__(1024) uint8_t smem[];
-  // Programmatic dependent launch: the next layer's CTAs may be scheduled as SMs free up; they set up, start streaming
-  // their weights, and wait (griddepcontrol.wait in the warps that read or write activations) for this grid to finish.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t base = smem_u32(smem);
   if (base & 1023u) {
     if (threadIdx.x == 0) atomicCAS(P.status, 0, FST_ALIGN);
@@ -346,6 +343,11 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  // Programmatic dependent launch: the next layer's CTAs may be scheduled as SMs free up; they set up, start streaming
+  // their weights, and wait (griddepcontrol.wait in the warps that read or write activations) for this grid to finish.
+  // Not before this CTA has its tensor memory: a dependent CTA on the same SM would take the columns first and keep them
+  // while it waits for this grid.  (Registers, 96 x 608 threads, leave room for one CTA an SM; the order does not rely on it.)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == kWarpW) {
     // ------------------------------------------------------------------ TMA: the W_hi / W_lo tiles of every step

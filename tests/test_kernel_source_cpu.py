@@ -1,0 +1,24 @@
+"""Rules of the kernels that are launched programmatically (a grid may start while the one before it in the stream still
+runs), checked in their source: what breaks them shows up as a rare hang or a stale value, not as a failing comparison."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "fortis_b200", "csrc")
+
+
+def kernel(name, signature):
+    text = open(os.path.join(CSRC, name)).read()
+    start = text.index(signature)
+    return re.sub(r"//[^\n]*", "", text[start:text.index("\n}\n", start)])
+
+
+@pytest.mark.parametrize("name,signature", [("fortis_mlp_f32tc.cu", "f32tc_kernel(const __grid_constant__"),
+                                            ("fortis_conv3d_tc.cu", "conv3d_tc_kernel(const __grid_constant__")])
+def test_dependents_are_released_after_the_tensor_memory_is_allocated(name, signature):
+    """A dependent CTA that shares the SM could otherwise take the tensor-memory columns and wait for the grid whose CTA
+    still needs them."""
+    body = kernel(name, signature)
+    alloc, release = body.index("tcgen05.alloc"), body.index("griddepcontrol.launch_dependents")
+    assert alloc < release and "__syncthreads()" in body[alloc:release]
