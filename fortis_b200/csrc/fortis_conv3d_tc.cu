@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
     bool use_skip = !LAST && P.skip != nullptr && interior;
     if (use_skip) {
 #pragma unroll
-      for (int j = 0; j < CW / 8; j++) sk[j] = __ldg(reinterpret_cast<const uint4*>(P.skip + (size_t)p * kC + c0) + j);
+      for (int j = 0; j < CW / 8; j++) sk[j] = ld_global(reinterpret_cast<const uint4*>(P.skip + (size_t)p * kC + c0) + j);
     }
     uint32_t acc_it = 0;
     for (long long tp = pair0; tp < npairs; tp += pair_step, acc_it++) {
@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
         }
         if (nuse_skip) {                                           // these registers are free again: next tile's residual row
 #pragma unroll
-          for (int h = 0; h < CW / 8; h++) sk[h] = __ldg(reinterpret_cast<const uint4*>(P.skip + (size_t)np * kC + c0) + h);
+          for (int h = 0; h < CW / 8; h++) sk[h] = ld_global(reinterpret_cast<const uint4*>(P.skip + (size_t)np * kC + c0) + h);
         }
         if (writes) {
           uint4* dst = reinterpret_cast<uint4*>(P.out + (size_t)p * kC + c0);

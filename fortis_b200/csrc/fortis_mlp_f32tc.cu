@@ -156,10 +156,11 @@ template <int N> __device__ __forceinline__ void act_f32(float (&v)[N], int act,
   }
 }
 
-// a load that keeps its place in front of the wait that follows it; reads 0 where `ok` is 0
+// a load that keeps its place in front of the wait that follows it; reads 0 where `ok` is 0.  Not a read-only (.nc) load:
+// the grid in front may still write the activations while this one is resident.
 __device__ __forceinline__ float ld_ahead_if(const float* p, bool ok) {
   float v;
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@p ld.global.nc.f32 %0, [%1];\n\t}"
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@p ld.global.f32 %0, [%1];\n\t}"
                : "=f"(v) : "l"(p), "r"((int)ok));
   return v;
 }
@@ -632,7 +633,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
           float o[16];
           if (P.residual) {
 #pragma unroll
-            for (int j = 0; j < 16; j++) o[j] = nt0 + c0 + j < P.N_real ? __ldg(P.residual + ro + (long long)(c0 + j) * g.rs_c) : 0.f;
+            for (int j = 0; j < 16; j++) o[j] = ld_ahead_if(P.residual + ro + (long long)(c0 + j) * g.rs_c, nt0 + c0 + j < P.N_real);
           }
 #pragma unroll
           for (int j = 0; j < 16; j++) v[c0 + j] += s_bias[c0 + j];

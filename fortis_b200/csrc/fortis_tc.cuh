@@ -91,6 +91,14 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
 }
 
+// a load of data that the grid in front of a programmatically launched one may write while this grid is resident: the
+// read-only path (ld.global.nc, __ldg) is for memory nothing writes during a grid's lifetime
+__device__ __forceinline__ uint4 ld_global(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
 // linear bulk copy global -> shared (both 16-byte aligned, size a multiple of 16), completion counted on an mbarrier
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile(

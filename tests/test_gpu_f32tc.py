@@ -6,6 +6,10 @@ product; the sums add 8 truncations per 64 k and one rounding per chunk, at most
 zero-mean data both stay below 2^-20 = 9.5e-7 of the result's 2-norm.
 """
 import ctypes
+import hashlib
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -154,3 +158,37 @@ def test_mlp_on_either_side_of_the_row_limit(host, dims, rows):
     # MLP steps keep all three products in one accumulator for 128 k: 48 truncations instead of 8, under 4 * TOL per layer
     assert rel(y, want) < 4 * TOL * len(layers) and rel(z, want) < 4 * TOL * len(layers)
     assert host.L.fortis_device_status() == 0
+
+
+def chains():
+    """Checksums of chains of layers whose launches may overlap: conv networks that rotate three volumes and add skips, an
+    fp32 MLP and a 16-bit one of few rows, each called three times on other inputs."""
+    h, out = fortis_b200.Host(), []
+    for precision, shape in (("fp32", (1, 9, 10, 33)), ("fp32", (2, 17, 19, 21)), ("bf16", (1, 9, 10, 33))):
+        h.reset()
+        h.load_model(fortis_b200.write_blob(fortis_b200.conv_layers(3, 64, 3, nblocks=3, seed=6)))
+        h.option("precision", precision)
+        h.option("conv_shape", "%d,%d,%d,%d" % shape)
+        for call in range(3):
+            x = randn(shape + (3,), call)
+            y = torch.zeros_like(x)
+            h.forward(x, y)
+            out.append(y)
+    for precision, dims, rows in (("fp32", [33, 65, 31, 40, 7], 1300), ("bf16", [100, 200, 64, 96, 33], 700)):
+        h.reset()
+        h.load_model(fortis_b200.write_blob(fortis_b200.mlp_layers(dims, seed=3, act="leaky", slope=0.2, scale=0.2)))
+        h.option("precision", precision)
+        h.L.fortis_begin(rows)
+        for call in range(3):
+            x, y = randn((rows, dims[0]), call), torch.zeros((rows, dims[-1]), device="cuda")
+            h.forward_batched(x, y)
+            out.append(y)
+    assert h.L.fortis_device_status() == 0
+    h.reset()
+    return hashlib.sha256(b"".join(t.cpu().numpy().tobytes() for t in out)).hexdigest()
+
+
+def test_layers_that_overlap_give_the_bits_of_layers_run_one_by_one():
+    one_by_one = subprocess.run([sys.executable, "-c", "from tests import test_gpu_f32tc as t; print(t.chains())"], check=True, text=True,
+                                stdout=subprocess.PIPE, env=dict(os.environ, FORTIS_NO_PDL="1"), cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert chains() == one_by_one.stdout.split()[-1]

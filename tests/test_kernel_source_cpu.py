@@ -22,3 +22,13 @@ def test_dependents_are_released_after_the_tensor_memory_is_allocated(name, sign
     body = kernel(name, signature)
     alloc, release = body.index("tcgen05.alloc"), body.index("griddepcontrol.launch_dependents")
     assert alloc < release and "__syncthreads()" in body[alloc:release]
+
+
+@pytest.mark.parametrize("name,written", [("fortis_mlp_f32tc.cu", ["P.A", "P.residual", "c.rowp", "TG.base"]), ("fortis_conv3d_tc.cu", ["P.skip"])])
+def test_what_the_grid_in_front_may_write_is_not_read_as_constant(name, written):
+    """Read-only loads (ld.global.nc, __ldg) want memory that nothing writes during the grid's lifetime, and the wait for
+    the grid in front does not change that: activations and residuals are read by ordinary loads."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
+    assert "ld.global.nc" not in text
+    for line in text.splitlines():
+        assert not ("__ldg" in line and any(w in line for w in written)), line.strip()
