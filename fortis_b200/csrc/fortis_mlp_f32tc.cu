@@ -580,6 +580,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
       const bool live = row < P.nrows;
       // bias (and scale) of this warp's features, for broadcast reads at the end of the tile: as loads from global memory
       // there they cost 470 cycles a feature, 30 k of a 48 k-cycle tile
+      __syncwarp();                                            // every lane has read the previous tile's, also behind a `continue`
       for (int j = lane; j < NH; j += 32) {
         const bool real = nt0 + j < P.N_real;
         s_bias[j] = P.bias && real ? __ldg(P.bias + nt0 + j) : 0.f;

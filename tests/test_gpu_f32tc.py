@@ -192,3 +192,16 @@ def test_layers_that_overlap_give_the_bits_of_layers_run_one_by_one():
     one_by_one = subprocess.run([sys.executable, "-c", "from tests import test_gpu_f32tc as t; print(t.chains())"], check=True, text=True,
                                 stdout=subprocess.PIPE, env=dict(os.environ, FORTIS_NO_PDL="1"), cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     assert chains() == one_by_one.stdout.split()[-1]
+
+
+def test_biases_of_a_layer_with_more_feature_tiles_than_sms(host):
+    """A CTA then has several tiles whose rows are partly behind the last one, each with a bias table of its own."""
+    rng = np.random.default_rng(12)
+    C, F = 64, 19100
+    W, b = rng.standard_normal((F, C, 1, 1)).astype(np.float32), (10 * rng.standard_normal(F)).astype(np.float32)
+    x, y = randn((1, C, 10, 13), 13), torch.zeros((1, F, 10, 13), device="cuda")
+    host.load_model(fortis_b200.write_blob([dict(op="conv2d", W=W, b=b, stride=1, pad=0, act="none")]))
+    host.option("conv_shape", "1,1,10,13")
+    host.forward(x, y)
+    want = torch.from_numpy(W[:, :, 0, 0]).double().cuda() @ x.double().reshape(C, 130) + torch.from_numpy(b).double().cuda()[:, None]
+    assert rel(y.reshape(F, 130), want) < TOL

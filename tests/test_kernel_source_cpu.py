@@ -32,3 +32,10 @@ def test_what_the_grid_in_front_may_write_is_not_read_as_constant(name, written)
     assert "ld.global.nc" not in text
     for line in text.splitlines():
         assert not ("__ldg" in line and any(w in line for w in written)), line.strip()
+
+
+def test_a_tiles_bias_table_is_not_rewritten_before_every_lane_has_read_it():
+    """The table belongs to a warp; a lane that leaves a tile early (rows behind the last one) must wait for the others."""
+    body = kernel("fortis_mlp_f32tc.cu", "f32tc_kernel(const __grid_constant__")
+    tiles = body[:body.index("s_bias[j] =")]
+    assert "__syncwarp()" in tiles[tiles.rindex("for (long long t ="):]
