@@ -33,7 +33,8 @@
 // IEEE additions, and the two cross products go into a second accumulator (2^-11 of the result, so its truncation does not
 // count) that lives for the whole K.
 // Infinities: x_hi saturates at the largest finite TF32 value and x_lo = x - x_hi carries the infinity, so a product is
-// infinite, or NaN, where the fp32 product is.  Every barrier wait is bounded.
+// infinite, or NaN, where the fp32 product is.  Every barrier wait is bounded; a CTA
+// whose wait gives up records which one, lets its copies and MMAs in flight finish and returns.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -113,6 +114,8 @@ struct F32Params {
   long long nrows;
   double* partials; double* sum; unsigned int* done;
   int* status;
+  unsigned int wait_limit;               // polls before a barrier wait gives up
+  int test_skip_stage;                   // test only: CTA 0 never loads its first weight stage
 };
 
 // instruction descriptor of kind::tf32: D = f32, A = B = tf32 (format code 2), both K-major, M = 128
@@ -163,6 +166,12 @@ __device__ __forceinline__ float ld_ahead_if(const float* p, bool ok) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@p ld.global.f32 %0, [%1];\n\t}"
                : "=f"(v) : "l"(p), "r"((int)ok));
   return v;
+}
+// One poll after another until a phase is over, with a limit, whether or not another wait has given up: for copies and MMAs
+// still in flight when a CTA ends
+__device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t parity, uint32_t limit) {
+  for (uint32_t i = 0; i < limit; i++)
+    if (mbar_try_wait(bar, parity)) return;
 }
 // One step's activations of a producer thread, and where the next step lies.  `t`, `kt`: tile and k step.
 template <int AMODE>
@@ -269,8 +278,9 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
   uint8_t* tail = smem + kTailOff;
   const uint32_t bars = base + kTailOff;
   // barriers: a_full [4] | a_empty [4] | w_full [6] | w_empty [6] | acc_full [2] | acc_empty [2] | cross_empty; then at 200
-  // the tensor-memory base, at 204 the abort flag, at 208 raw_full [4] | raw_empty [4], at 272 the checksum's warp sums
+  // the tensor-memory base, at 204 the abort flag, at 208 raw_full [4] | raw_empty [4], at 272 the checksum's warp sums, at 336 drained
   constexpr int kWStep = P16 ? CF::kWHalf : CF::kWStage;            // weight bytes per step
+  const uint32_t drained = bars + 336;
   const uint32_t a_full = bars, a_empty = bars + 32, w_full = bars + 64, w_empty = bars + 112, acc_full = bars + 160, acc_empty = bars + 176,
                  cross_empty = bars + 192, raw_full = bars + 208, raw_empty = bars + 240;
   uint32_t* tmem_slot = (uint32_t*)(tail + 200);
@@ -292,7 +302,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
     for (int s = 0; s < CF::kAStages; s++) { mbar_init(a_full + 8 * s, 4); mbar_init(a_empty + 8 * s, 1); }
     for (int s = 0; s < CF::kWStages; s++) { mbar_init(w_full + 8 * s, 1); mbar_init(w_empty + 8 * s, 1); }
     for (int s = 0; s < 2; s++) { mbar_init(acc_full + 8 * s, 1); mbar_init(acc_empty + 8 * s, kEWarps); }
-    mbar_init(cross_empty, kEWarps);
+    mbar_init(cross_empty, kEWarps); mbar_init(drained, 1);
     for (int s = 0; s < kRawStages; s++) { mbar_init(raw_full + 8 * s, 1); mbar_init(raw_empty + 8 * s, 4); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -350,6 +360,11 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
   // while it waits for this grid.  (Registers, 96 x 608 threads, leave room for one CTA an SM; the order does not rely on it.)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
+  // Every lane of a warp goes on or gives up together: what follows a wait is executed by the whole warp.
+  auto wait = [&](uint32_t bar, uint32_t parity, int code) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, P.status, code, P.wait_limit)) != 0;
+  };
+
   if (warp == kWarpW) {
     // ------------------------------------------------------------------ TMA: the W_hi / W_lo tiles of every step
     uint32_t s = 0, ph = 0;
@@ -357,10 +372,12 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
     for (long long t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
       const int n0 = (int)(t % P.ntn) * NT;
       for (int kt = 0; kt < nkt; kt++) {
-        if (!mbar_wait(w_empty + 8 * s, ph ^ 1, abort_flag, P.status, FST_W_EMPTY)) { stop = true; break; }
-        mbar_expect_tx(w_full + 8 * s, kWStep);
+        if (!wait(w_empty + 8 * s, ph ^ 1, FST_W_EMPTY)) { stop = true; break; }
         const uint32_t st = base + s * CF::kWStage;
-        if constexpr (P16 != 0) {
+        const bool skip = P.test_skip_stage && blockIdx.x == 0 && t == 0 && kt == 0;
+        if (!skip) mbar_expect_tx(w_full + 8 * s, kWStep);
+        if (skip) {
+        } else if constexpr (P16 != 0) {
           tma_load_2d(st, &P.map_hi, kt * 64, n0, w_full + 8 * s);
         } else {
           tma_load_2d(st, &P.map_hi, kt * kKt, n0, w_full + 8 * s);
@@ -369,6 +386,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
         if (++s == CF::kWStages) { s = 0; ph ^= 1; }
       }
     }
+    for (uint32_t q = 0; q < CF::kWStages; q++) drain_wait(w_full + 8 * q, q < s ? ph : ph ^ 1, P.wait_limit);
   } else if (warp == kWarpA) {
     // ------------------------------------------------------------------ TMA: the fp32 activations of every step
     if constexpr (kTile) {
@@ -378,13 +396,14 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
       for (long long t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
         const int m0 = (int)((t / P.ntn) * kM);
         for (int kt = 0; kt < nkt; kt++) {
-          if (!mbar_wait(raw_empty + 8 * s, ph ^ 1, abort_flag, P.status, FST_RAW_EMPTY)) { stop = true; break; }
+          if (!wait(raw_empty + 8 * s, ph ^ 1, FST_RAW_EMPTY)) { stop = true; break; }
           mbar_expect_tx(raw_full + 8 * s, kRawBytes);
           if constexpr (AMODE == A_TILE_T) tma_load_2d(base + kRawOff + s * kRawBytes, &P.map_a, m0, kt * kKt, raw_full + 8 * s);
           else tma_load_2d(base + kRawOff + s * kRawBytes, &P.map_a, kt * kKt, m0, raw_full + 8 * s);
           if (++s == kRawStages) { s = 0; ph ^= 1; }
         }
       }
+      for (uint32_t q = 0; q < kRawStages; q++) drain_wait(raw_full + 8 * q, q < s ? ph : ph ^ 1, P.wait_limit);
     }
   } else if (warp == kWarpMma) {
     // ------------------------------------------------------------------ MMA issuer
@@ -392,13 +411,13 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
     const uint64_t desc_hi = make_kmajor_sw128_desc(0) & 0xFFFFFFFF00000000ull;
     constexpr uint32_t idesc = P16 == 0 ? idesc_tf32(NT) : idesc_16(NT, P16 == 2);
     const uint32_t cross = tmem + CF::kColCross;
-    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x, tile_it++) {
+    bool stop = false;
+    for (long long t = blockIdx.x; t < ntiles && !stop; t += gridDim.x, tile_it++) {
       uint32_t in_chunk = 0;                            // 16-bit forms: one chunk per tile
       for (int kt = 0; kt < nkt; kt++) {
         const uint32_t b = chunk_it & 1;
-        if (in_chunk == 0) mbar_wait(acc_empty + 8 * b, ((chunk_it >> 1) & 1) ^ 1, abort_flag, P.status, FST_ACC_EMPTY);
-        mbar_wait(w_full + 8 * ws, wph, abort_flag, P.status, FST_W_FULL);
-        mbar_wait(a_full + 8 * as, aph, abort_flag, P.status, FST_A_FULL);
+        if ((in_chunk == 0 && !wait(acc_empty + 8 * b, ((chunk_it >> 1) & 1) ^ 1, FST_ACC_EMPTY)) || !wait(w_full + 8 * ws, wph, FST_W_FULL) ||
+            !wait(a_full + 8 * as, aph, FST_A_FULL)) { stop = true; break; }
         tc_fence_after();
         const uint32_t st = base + ws * CF::kWStage, acc = tmem + b * NT;
         const uint64_t wh = desc_hi | (uint64_t)((st >> 4) & 0x3FFF), wl = desc_hi | (uint64_t)(((st + CF::kWHalf) >> 4) & 0x3FFF);
@@ -419,7 +438,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
           for (int j = 0; j < kKt / 8; j++)             // 8 tf32 = 32 bytes per k step: the address field moves by 2
             mma_tf32_ts<idesc>(acc, ah + 8 * j, wh + (uint64_t)(2 * j), in_chunk | (uint32_t)j);
           if (kt == 0) {                                // the previous tile's cross products have been read
-            mbar_wait(cross_empty, (tile_it & 1) ^ 1, abort_flag, P.status, FST_ACC_EMPTY);
+            if (!wait(cross_empty, (tile_it & 1) ^ 1, FST_ACC_EMPTY)) { stop = true; break; }
             tc_fence_after();
           }
 #pragma unroll
@@ -436,6 +455,8 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
         if (++ws == CF::kWStages) { ws = 0; wph ^= 1; }
       }
     }
+    tc_commit(drained);                                 // nothing may still read shared or tensor memory when the CTA ends
+    drain_wait(drained, 0, P.wait_limit);
   } else if (warp < kPWarps) {
     // ------------------------------------------------------------------ A producers: thread = row of the tile
     const int quad = warp & 3, r = quad * 32 + lane;
@@ -464,7 +485,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
       while (kt >= nkt) kt -= nkt;
       for (; it < steps; it += kPSets) {
         const uint32_t s = it % CF::kAStages, rs = it % kRawStages;
-        if (!mbar_wait(raw_full + 8 * rs, (it / kRawStages) & 1, abort_flag, P.status, FST_RAW_FULL)) break;
+        if (!wait(raw_full + 8 * rs, (it / kRawStages) & 1, FST_RAW_FULL)) break;
         const uint8_t* raw = smem + kRawOff + rs * kRawBytes;
         bool ok = true;
 #pragma unroll 1
@@ -481,7 +502,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
             }
           }
           if (h == 0) {
-            ok = mbar_wait(a_empty + 8 * s, ((it / CF::kAStages) & 1) ^ 1, abort_flag, P.status, FST_A_EMPTY);
+            ok = wait(a_empty + 8 * s, ((it / CF::kAStages) & 1) ^ 1, FST_A_EMPTY);
             if (!ok) break;
             tc_fence_after();
           }
@@ -540,7 +561,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
 #pragma unroll
             for (int j = 0; j < 16; j++) pk[j] = pack_pair<P16 == 2>(v[j >> 3][(2 * j) & 15], v[j >> 3][(2 * j + 1) & 15]);
             if (h == 0) {
-              ok = mbar_wait(a_empty + 8 * s, ((it / CF::kAStages) & 1) ^ 1, abort_flag, P.status, FST_A_EMPTY);
+              ok = wait(a_empty + 8 * s, ((it / CF::kAStages) & 1) ^ 1, FST_A_EMPTY);
               if (!ok) break;
               tc_fence_after();
             }
@@ -551,7 +572,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
           float v[2][16];
           const int k0 = c.kt * kKt;
           load_block(v, k0);
-          if (!mbar_wait(a_empty + 8 * s, ((it / CF::kAStages) & 1) ^ 1, abort_flag, P.status, FST_A_EMPTY)) break;
+          if (!wait(a_empty + 8 * s, ((it / CF::kAStages) & 1) ^ 1, FST_A_EMPTY)) break;
           tc_fence_after();
           publish16(v[0], k0, lane_addr + 64 * s);
           publish16(v[1], k0 + 16, lane_addr + 64 * s + 16);
@@ -588,11 +609,13 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
       }
       __syncwarp();
       float v[NH];
+      bool ok = true;
 #pragma unroll
       for (int j = 0; j < NH; j++) v[j] = -0.f;            // -0 + x is x, also where x is -0
       for (int ch = 0; ch < nch; ch++, chunk_it++) {
         const uint32_t b = chunk_it & 1;
-        mbar_wait(acc_full + 8 * b, (chunk_it >> 1) & 1, abort_flag, P.status, FST_ACC_FULL);
+        ok = wait(acc_full + 8 * b, (chunk_it >> 1) & 1, FST_ACC_FULL);
+        if (!ok) break;
         tc_fence_after();
 #pragma unroll
         for (int c0 = 0; c0 < NH; c0 += NL) {
@@ -606,6 +629,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
         __syncwarp();
         if (lane == 0) mbar_arrive(acc_empty + 8 * b);
       }
+      if (!ok) break;
       if (P16 == 0 && !(kMaybeOneAcc && P.one_acc)) {
 #pragma unroll
       for (int c0 = 0; c0 < NH; c0 += NL) {
@@ -775,9 +799,6 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
   }
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag && threadIdx.x == 0)
-    for (int i = 0; i < 2000; i++) __nanosleep(1000);        // let copies in flight land before the CTA gives its memory back
-  __syncthreads();
   if (warp == kWarpMma) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
@@ -919,7 +940,9 @@ constexpr int kSmemMaxF = 227 * 1024;
 // `early` = false for a launch whose WEIGHTS were produced by the kernel in front of it: the weight loads do not wait.
 // Otherwise the launch may start while the one before it in the stream drains (programmatic stream serialisation).
 template <int NT, int AMODE, int P16 = 0>
-bool launch_as(const F32Params& P, cudaStream_t s, bool early) {
+bool launch_as(F32Params& P, cudaStream_t s, bool early) {
+  P.wait_limit = g_tc_test.wait_limit ? g_tc_test.wait_limit : kWaitLimit;
+  P.test_skip_stage = g_tc_test.skip_stage;
   static bool ready = false;
   if (!ready) {
     if (cudaFuncSetAttribute(f32tc_kernel<NT, AMODE, P16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMaxF) != cudaSuccess) return false;

@@ -1289,8 +1289,7 @@ TcModel* tc_model_create(const ModelHost& M, int precision, cudaStream_t s, std:
 bool tc_forward(TcModel* m, const TcLaunch& L, cudaStream_t s, std::string* err) {
   const long long nrows = L.g.count * L.g.nk;
   if (nrows <= 0) return true;
-  const bool knobs = g_tc_test.wait_limit || g_tc_test.skip_stage || g_tc_test.no_stage;       // they address the fused kernel
-  if (m->rows && !knobs && L.act[0] && (m->nlayers < 3 || L.act[1]) && nrows <= kFewRows) {
+  if (m->rows && !g_tc_test.no_stage && L.act[0] && (m->nlayers < 3 || L.act[1]) && nrows <= kFewRows) {
     F32TcLaunch R{};
     R.fast_in = L.fast_in; R.slots = L.slots; R.TG = L.TG; R.X = L.X;
     R.fast_out = L.fast_out; R.store_by_slot = L.store_by_slot; R.TS = L.TS; R.Y = L.Y;

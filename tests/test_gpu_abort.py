@@ -77,3 +77,50 @@ def test_conv_pair_kernel_wait_gives_up_in_both_ctas_of_the_pair():
     assert h.L.fortis_device_status() == 0
     assert y2.tobytes() == y0.tobytes()
     h.reset()
+
+
+@pytest.mark.parametrize("case", ["fp32 step", "bf16 step of few rows", "fp32 conv network"])
+def test_layer_kernel_wait_gives_up_and_the_next_call_is_whole(case):
+    """The kernel that runs layer by layer (fp32 layers and convolutions, 16-bit MLPs of few rows): every layer's first CTA
+    misses its first weight stage, and the layers behind it run on what it left."""
+    h = fortis_b200.Host()
+    h.reset()
+    if case == "fp32 conv network":
+        shape = (1, 9, 10, 33)
+        x = torch.randn(shape + (3,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+        outs = [torch.zeros_like(x)]
+        h.load_model(fortis_b200.write_blob(fortis_b200.conv_layers(3, 64, 3, nblocks=2, seed=11)))
+        h.option("conv_shape", "%d,%d,%d,%d" % shape)
+        call = lambda: h.forward(x, outs[0])
+    else:
+        wl = W.column(1000)
+        h.configure(gather=wl["G"], scatter=wl["S"], loop=wl["Lp"])
+        h.load_model(fortis_b200.write_blob(wl["layers"]))
+        h.option("precision", case.split()[0])
+        h.option("checksum", 1)
+        d_in, outs = [dev(a) for a in wl["gin"]], [dev(a) for a in wl["sout"]]
+        call = lambda: h.step(d_in, outs)
+    call()
+    h.sync()
+    assert h.L.fortis_device_status() == 0
+    before = [t.clone() for t in outs]
+    checksum = h.step_checksum()
+    h.option("test_wait_limit", 4096)
+    h.option("test_skip_stage", 1)
+    call()
+    h.sync()
+    status = h.L.fortis_device_status()
+    assert 21 <= status <= 29 and status != 25, "expected a wait code of the layer kernel, got %d" % status
+    assert h.L.fortis_device_status() == 0
+    h.step_checksum()                                    # reading it clears it
+    h.option("test_skip_stage", 0)
+    h.option("test_wait_limit", 0)
+    for t in outs:
+        t.zero_()
+    call()
+    h.sync()
+    assert h.L.fortis_device_status() == 0
+    for a, b in zip(outs, before):
+        assert torch.equal(a, b)
+    assert h.step_checksum() == checksum
+    h.reset()
