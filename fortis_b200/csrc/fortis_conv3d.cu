@@ -18,6 +18,7 @@
 #include <string>
 #include <vector>
 
+#include "fortis_device.cuh"
 #include "fortis_kernels.h"
 #include "fortis_model.h"
 
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(256) conv3d_f32_kernel(const float* __restrict
       if (f >= g.F) continue;
       float o = acc[i][j] + (bias ? bias[f] : 0.f);
       if (residual) o += residual[ro + (long long)f * g.rs_c];
-      if (act == ACT_RELU) o = fmaxf(o, 0.f);
+      if (act == ACT_RELU) o = max_nan(o, 0.f);
       else if (act == ACT_LEAKY) o = o > 0.f ? o : o * slope;
       y[yo + (long long)f * g.ys_c] = o;
     }
@@ -221,7 +222,7 @@ __global__ void maxpool2d_kernel(const float* __restrict__ x, float* __restrict_
     const float* src = x + pl * H * W;
     float m = -INFINITY;
     for (int kh = 0; kh < KH; kh++)
-      for (int kw = 0; kw < KW; kw++) m = fmaxf(m, __ldg(src + (long long)(oh * sh + kh) * W + ow * sw + kw));
+      for (int kw = 0; kw < KW; kw++) m = max_nan(m, __ldg(src + (long long)(oh * sh + kh) * W + ow * sw + kw));
     y[i] = m;
   }
 }

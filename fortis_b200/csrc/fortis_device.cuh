@@ -9,6 +9,14 @@
 
 namespace fortis {
 
+// The larger value, NaN where one of the two is NaN (fmaxf would return the other one): what ReLU and max pooling mean in the
+// program a network was trained in, and the only way a host learns that its fields have blown up.
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 struct IoPlanDev {
   int n;                         // model inputs (gather) / outputs (scatter)
   int nscalars;

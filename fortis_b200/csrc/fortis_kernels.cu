@@ -131,7 +131,7 @@ void launch_scatter(const IoPlanDev* P, const StoreTarget* stores, int nout, con
 constexpr int LBM = 128, LBN = 64, LBK = 16;
 
 __device__ __forceinline__ float act_apply(float v, int act, float slope) {
-  if (act == ACT_RELU) return fmaxf(v, 0.f);
+  if (act == ACT_RELU) return max_nan(v, 0.f);
   if (act == ACT_LEAKY) return v > 0.f ? v : v * slope;
   return v;
 }
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict
       float v = acc[i][j] + (bias ? bias[nn] : 0.f);
       v = act_apply(v, act, slope);
       if (out_mul) v = v * out_mul[nn];
-      if (relu_mask && relu_mask[nn] != 0.f) v = fmaxf(v, 0.f);
+      if (relu_mask && relu_mask[nn] != 0.f) v = max_nan(v, 0.f);
       C[row * N + nn] = v;
     }
   }

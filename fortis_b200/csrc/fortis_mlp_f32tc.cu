@@ -152,7 +152,7 @@ template <bool F16> __device__ __forceinline__ uint32_t pack_pair(float lo, floa
 template <int N> __device__ __forceinline__ void act_f32(float (&v)[N], int act, float slope) {
   if (act == ACT_RELU) {
 #pragma unroll
-    for (int j = 0; j < N; j++) v[j] = fmaxf(v[j], 0.f);
+    for (int j = 0; j < N; j++) v[j] = max_nan(v[j], 0.f);
   } else if (act == ACT_LEAKY) {
 #pragma unroll
     for (int j = 0; j < N; j++) v[j] = v[j] > 0.f ? v[j] : v[j] * slope;
@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
           const int n = nt0 + j;
           if (n < P.N_real) {
             if (P.out_mul) v[j] *= __ldg(P.out_mul + n);
-            if (P.relu_mask && __ldg(P.relu_mask + n) != 0.f) v[j] = fmaxf(v[j], 0.f);
+            if (P.relu_mask && __ldg(P.relu_mask + n) != 0.f) v[j] = max_nan(v[j], 0.f);
           }
         }
       }

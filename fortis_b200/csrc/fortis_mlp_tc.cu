@@ -899,7 +899,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
                 const int n = n0 + j;
                 if (n < P.n_out) {
                   if (P.out_mul) v[j] *= __ldg(P.out_mul + n);
-                  if (P.relu_mask && __ldg(P.relu_mask + n) != 0.f) v[j] = fmaxf(v[j], 0.f);
+                  if (P.relu_mask && __ldg(P.relu_mask + n) != 0.f) v[j] = max_nan(v[j], 0.f);
                 }
               }
             }

@@ -19,6 +19,7 @@
 
 #include <cstring>
 
+#include "fortis_device.cuh"
 #include "fortis_kernels.h"
 
 namespace fortis {
@@ -46,7 +47,7 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 }
 
 template <bool RELU> __device__ __forceinline__ float act1(float v, float slope) {
-  if constexpr (RELU) return fmaxf(v, 0.f);
+  if constexpr (RELU) return max_nan(v, 0.f);
   else return fmaxf(v, v * slope);                   // none: slope 1, LeakyReLU: its slope
 }
 
