@@ -181,6 +181,7 @@ std::vector<float> repack_weights_taps(const float* w, int F, int C, int taps) {
 // split for that one.
 struct LayerDev { float *wt = nullptr, *bias = nullptr; F32ConvW* split = nullptr; };
 bool upload_layer(const LayerHost& L, int taps, bool split, LayerDev* d, std::string* err) {
+  split = split && (long long)L.cin * taps >= kF32TcConvMinProducts;
   const std::vector<float> wt = repack_weights_taps(L.W.data(), L.cout, L.cin, taps);
   float* raw = nullptr;
   auto fail = [&](const char* why) {
@@ -202,9 +203,9 @@ bool upload_layer(const LayerHost& L, int taps, bool split, LayerDev* d, std::st
   return true;
 }
 
-// A layer takes the tensor-core kernel wherever it can (f32tc_conv_supported: no input dilation, up to 32 taps per axis, a
-// table of taps and channels that fits shared memory): 14-layer network, 2 x 33^3 voxels, 1.80 ms against 8.75 on the FFMA
-// kernel; 32 -> 64 channels on 40^3 71 us against 297; and closer to the exact sums (2.1e-7 against 5.2e-7).
+// A layer takes the tensor-core kernel wherever it can and its sums are long enough (f32tc_conv_supported: no input dilation,
+// up to 32 taps per axis, a table of taps and channels that fits shared memory, kF32TcConvMinProducts): 14-layer network,
+// 2 x 33^3 voxels, 1.80 ms against 8.75 on the FFMA kernel; 32 -> 64 channels on 40^3 71 us against 297.
 bool conv_layer(const F32ConvW* split, const float* wt, const float* bias, const float* x, const float* residual, float* y, const ConvGeom& g,
                 int act, float slope, int* status, cudaStream_t s, std::string* err) {
   if (split && f32tc_conv_supported(g)) return f32tc_conv(split, x, bias, residual, y, g, act, slope, status, s, true, err);

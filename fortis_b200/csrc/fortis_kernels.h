@@ -155,6 +155,11 @@ void rows_mlp_destroy(RowsMlp* m);
 bool rows_mlp_forward(RowsMlp* m, const F32TcLaunch& L, cudaStream_t s, std::string* err);
 // one fp32 convolution layer on the same kernel (rows = output voxels, reduction = taps x channels)
 struct F32ConvW;                                       // split weights of one layer
+// Shorter reductions stay on the FFMA kernel: the split keeps 21 bits of an operand, which sums of few products show, while
+// the FFMA kernel's roundings grow with their number.  Error against 64 bits, relative 2-norm, split / FFMA, inputs normal and
+// normal.clamp_min(0), normal weights: 8 products 9.2e-8 / 5.3e-8 and 8.8e-8 / 4.2e-8, 27: 1.3e-7 / 9.4e-8 and 1.2e-7 / 7.0e-8,
+// 64: 1.4e-7 / 1.4e-7 and 1.2e-7 / 1.0e-7, 96: 1.35e-7 / 1.8e-7 and 1.23e-7 / 1.27e-7, 128: 1.4e-7 / 2.0e-7 and 1.3e-7 / 1.5e-7.
+constexpr int kF32TcConvMinProducts = 128;
 bool f32tc_conv_supported(const ConvGeom& g);
 F32ConvW* f32tc_conv_pack(const float* w_dev, int F, int C, int taps, cudaStream_t s, std::string* err);
 void f32tc_conv_free(F32ConvW* w);

@@ -1223,6 +1223,9 @@ static int conv_group(int C) { return (C % 8 == 0 || C > 16) ? 8 : 1; }
 bool f32tc_conv_supported(const ConvGeom& g) {
   if (g.dd != 1 || g.dh != 1 || g.dw != 1) return false;                       // transposed convolutions
   if (g.KD > 32 || g.KH > 32 || g.KW > 32) return false;                       // one bit per tap and axis
+  // the most products an output can have: taps that lie inside the volume, times channels
+  const long long inside = (long long)(g.KD < g.D ? g.KD : g.D) * (g.KH < g.H ? g.KH : g.H) * (g.KW < g.W ? g.KW : g.W);
+  if (inside * g.C < kF32TcConvMinProducts) return false;
   const int G = conv_group(g.C);
   const long long taps = (long long)g.KD * g.KH * g.KW, entries = taps * ((g.C + G - 1) / G);
   if (entries * 8 + 32 * 8 > kConvTabMax) return false;

@@ -205,3 +205,23 @@ def test_biases_of_a_layer_with_more_feature_tiles_than_sms(host):
     host.forward(x, y)
     want = torch.from_numpy(W[:, :, 0, 0]).double().cuda() @ x.double().reshape(C, 130) + torch.from_numpy(b).double().cuda()[:, None]
     assert rel(y.reshape(F, 130), want) < TOL
+
+
+@pytest.mark.parametrize("C,K", [(1, (1, 1, 1)), (8, (1, 1, 1)), (27, (1, 1, 1)), (1, (3, 3, 3)), (14, (3, 3, 1)), (15, (3, 3, 1)), (128, (1, 1, 1)), (64, (3, 3, 3))])
+@pytest.mark.parametrize("clamp", [False, True])
+def test_a_convolution_is_no_less_exact_than_its_fp32_sums(host, C, K, clamp):
+    """Against 64 bits, the error of a chain of fp32 fused multiply-adds over the same products (channels inside taps), for
+    reductions on both sides of the limit below which operands are not split.  5 % for the sample of 20,000 outputs."""
+    x, w = randn((1, C, 8, 10, 12), 14), randn((32, C) + K, 15)
+    if clamp:
+        x = x.clamp_min(0)
+    want = conv64(x, w, (1, 1, 1), (0, 0, 0))
+    y = torch.full(want.shape, float("nan"), device="cuda")
+    conv_entry(host, x, w, y, (1, 1, 1), (0, 0, 0))
+    chain = torch.zeros(want.shape, device="cuda")
+    D, H, W = want.shape[2:]
+    for kd, kh, kw in np.ndindex(K):
+        for c in range(C):          # a product of two fp32 values is exact in 64 bits, so this rounds once, as an FMA does
+            win = x[:, c, None, kd:kd + D, kh:kh + H, kw:kw + W].double()
+            chain = (chain.double() + win * w[None, :, c, kd, kh, kw, None, None, None].double()).float()
+    assert rel(y, want) <= 1.05 * rel(chain, want)
