@@ -1854,6 +1854,10 @@ int fortis_debug_pack_layer(const float* W, const float* b, int cout, int cin, i
   FORTIS_CATCH(return -1)
 }
 
+int fortis_debug_few_rows(const int* widths, int nlayers, int fp8w, long rows) {
+  return tc_rows_layer_by_layer(widths, widths + 1, nlayers, fp8w != 0, rows) ? 1 : 0;
+}
+
 int fortis_debug_eval_expr(const char* exprs_json, int tv_double, double tv, const double* scalars, const int* scalar_elt,
                            int nscalars, double* out) {
   FORTIS_TRY

@@ -112,6 +112,7 @@ struct TcLaunch {
 };
 int tc_grid(const TcModel* m, long long nrows);
 void tc_set_pair_mode(int on);                      // 1 / 0: two-CTA clusters or one CTA per SM for models created from now on; -1: the default (clusters)
+bool tc_rows_layer_by_layer(const int* K, const int* N, int nlayers, bool fp8w, long long nrows);   // which form a call takes
 bool tc_forward(TcModel* m, const TcLaunch& L, cudaStream_t s, std::string* err);
 
 // ---- fp32-class Linear layers on the tensor cores, three TF32 MMAs per product (fortis_mlp_f32tc.cu) ----------------
@@ -152,6 +153,7 @@ struct RowsMlp;
 RowsMlp* rows_mlp_create(const std::vector<F16Layer>& layers, bool f16, const float* in_div, const float* out_mul, const float* relu_mask,
                          std::string* err);
 void rows_mlp_destroy(RowsMlp* m);
+int rows_mlp_cost(const int* K, const int* N, int nlayers, long long nrows);     // estimated device time, 10 ns
 bool rows_mlp_forward(RowsMlp* m, const F32TcLaunch& L, cudaStream_t s, std::string* err);
 // one fp32 convolution layer on the same kernel (rows = output voxels, reduction = taps x channels)
 struct F32ConvW;                                       // split weights of one layer

@@ -1108,6 +1108,7 @@ struct TcModel {
   TcLayer layer[kMaxLayers];
   CUtensorMap maps[kMaxLayers];
   bool has_scale = false, f16 = false;
+  int widths[kMaxLayers + 1];      // inputs, then every layer's features
   RowsMlp* rows = nullptr;         // the same weights for calls of few rows (cluster form's weights only)
   bool pair = false;               // run as two-CTA clusters (row-major weights + tensor maps are on the device as well)
 };
@@ -1195,10 +1196,21 @@ void tc_model_destroy(TcModel* m) {
 }
 
 // Few rows run layer by layer (RowsMlp) instead of fused: the fused kernel gives a 128-row tile to one SM of a cluster, whose
-// time is its stream of all weights, while a layer of RowsMlp spreads its tiles over the SMs and pays a launch.  Measured
-// on 244-768x4-128, bf16, fused / layer by layer: 1000 rows 62.9 / 35.8 us, 2000 61.9 / 44.8, 4000 61.8 / 61.9, 8192 62.1 / 75.9;
-// at 3000 rows 64-256-256-64 29.9 / 23.6, 244-512-512-128 63.6 / 33.5, seven layers of 768 120.8 / 64.6.
+// time is its stream of all weights, while a layer of RowsMlp spreads its tiles over the SMs and pays a launch.  Device time
+// of bf16 steps, fused / layer by layer, us, at 1000 and 3072 rows: 244-768x4-128 60.3 / 34.1 and 59.0 / 42.1; 244-64x7-128
+// 32.9 / 29.4 and 32.5 / 29.8; 244-256x4-128 27.3 / 25.6 and 26.4 / 26.0; 244-256x7-128 35.9 / 38.0 and 35.0 / 37.4; seven
+// layers of 256 and 512 in turn 45.1 / 40.7 and 44.1 / 50.0.  So the form with the smaller estimate runs; the fused kernel's is
+// 12.7 us and, per layer, 1.65 us (FP8 weights 2.45) and 1.2 (1.3) per 256 x 256 block of weights; on
+// 933 networks and row counts (2 to 8 layers of 16 to 768 features, alternating widths among them) the form it picks is at
+// most 7 % behind the other one.  Above 3072 rows neither
+// estimate holds (244-768x4-128: 4000 rows 61.8 / 61.9, 8192 62.1 / 75.9).
 constexpr long long kFewRows = 3072;
+bool tc_rows_layer_by_layer(const int* K, const int* N, int nlayers, bool fp8w, long long nrows) {
+  if (nlayers < 2 || nrows > kFewRows) return false;             // (one layer is one launch either way)
+  int fused = 1270;
+  for (int l = 0; l < nlayers; l++) fused += (fp8w ? 245 : 165) + (fp8w ? 130 : 120) * ((K[l] + 255) / 256) * ((N[l] + 255) / 256);
+  return rows_mlp_cost(K, N, nlayers, nrows) < fused;
+}
 
 TcModel* tc_model_create(const ModelHost& M, int precision, cudaStream_t s, std::string* err) {
   (void)s;
@@ -1211,6 +1223,8 @@ TcModel* tc_model_create(const ModelHost& M, int precision, cudaStream_t s, std:
   TcModel* m = new TcModel();
   m->pair = pair;
   m->nlayers = (int)M.layers.size(); m->n_in = M.n_in(); m->n_out = M.n_out();
+  m->widths[0] = m->n_in;
+  for (int l = 0; l < m->nlayers; l++) m->widths[l + 1] = M.layers[l].cout;
   auto fail = [&](const std::string& w) { if (err) *err = w; tc_model_destroy(m); return (TcModel*)nullptr; };
   for (int l = 0; l < m->nlayers; l++) {
     const LayerHost& L = M.layers[l];
@@ -1289,7 +1303,8 @@ TcModel* tc_model_create(const ModelHost& M, int precision, cudaStream_t s, std:
 bool tc_forward(TcModel* m, const TcLaunch& L, cudaStream_t s, std::string* err) {
   const long long nrows = L.g.count * L.g.nk;
   if (nrows <= 0) return true;
-  if (m->rows && !g_tc_test.no_stage && L.act[0] && (m->nlayers < 3 || L.act[1]) && nrows <= kFewRows) {
+  if (m->rows && !g_tc_test.no_stage && L.act[0] && (m->nlayers < 3 || L.act[1]) &&
+      tc_rows_layer_by_layer(m->widths, m->widths + 1, m->nlayers, m->has_scale, nrows)) {
     F32TcLaunch R{};
     R.fast_in = L.fast_in; R.slots = L.slots; R.TG = L.TG; R.X = L.X;
     R.fast_out = L.fast_out; R.store_by_slot = L.store_by_slot; R.TS = L.TS; R.Y = L.Y;

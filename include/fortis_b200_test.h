@@ -22,6 +22,10 @@ int fortis_debug_plan(const char* desc_json, const char* loop_json, const char* 
 int fortis_debug_pack_layer(const float* W, const float* b, int cout, int cin, int last, int precision, unsigned short* image,
                             float* bias, float* scale, int* K, int* N);
 
+/* Host-only: does a 16-bit step of `rows` rows through an MLP of these widths (nlayers + 1 of them) run layer by layer (1) or
+ * as one fused kernel (0)?  `fp8w`: FP8 weights. */
+int fortis_debug_few_rows(const int* widths, int nlayers, int fp8w, long rows);
+
 /* Test-only keys of fortis_set_option (cleared by fortis_reset):
  *   "test_wait_limit"  N      polls before a bounded barrier wait of the tensor-core kernels gives up (0: the default)
  *   "test_skip_stage"  0 | 1  the first CTA's copy warp leaves out its first stage, so that a wait runs out: the
