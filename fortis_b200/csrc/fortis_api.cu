@@ -118,6 +118,7 @@ struct PlanDev {
   std::vector<const void*> reg;              // pinned registration: nullptr = none yet, (void*)1 = never again
   std::vector<const void*> cur;              // this call's pointers
   std::vector<char> on_dev;
+  bool mapped = false;                       // some array of this call is addressed in its pinned host pages
   void* vec_dev[kMaxVecs] = {};
   int *slot_head = nullptr, *store_next = nullptr;   // scatter: stores indexed by model output
   Access* store_by_slot = nullptr;                   // scatter: one store target per model output (fast path)
@@ -512,6 +513,7 @@ void bind_arrays(PlanDev& P, void* const* ptrs, const int* args, int nargs, bool
   Session& s = S();
   cudaStream_t st = stream();
   std::memset(T, 0, sizeof *T);
+  P.mapped = false;
   for (size_t ai = 0; ai < P.h.arrays.size(); ai++) {
     const ArrayInfo& a = P.h.arrays[ai];
     const size_t es = elt_size(a.elt);
@@ -527,7 +529,7 @@ void bind_arrays(PlanDev& P, void* const* ptrs, const int* args, int nargs, bool
       // The kernels address the pinned host pages themselves: loads and stores cross the bus inside the launch, no
       // staging copy on either side.
       void* dp = nullptr;
-      if (cudaHostGetDevicePointer(&dp, H, 0) == cudaSuccess && dp) { P.on_dev[ai] = true; T->base[ai] = (char*)dp + first * es; continue; }
+      if (cudaHostGetDevicePointer(&dp, H, 0) == cudaSuccess && dp) { P.on_dev[ai] = true; P.mapped = true; T->base[ai] = (char*)dp + first * es; continue; }
       cudaGetLastError();
     }
     if (P.stage_elems[ai] < need) {
@@ -760,6 +762,7 @@ void run_step_kernels(const StepArgs& A) {
     if (fuse_out) { L.SP = s.S.hdr; L.stores = (const StoreTarget*)s.S.items; L.TS = A.TS; L.fast_out = 1;
                     L.store_by_slot = s.S.store_by_slot; std::memcpy(L.cout, s.S.cls, sizeof L.cout); }
     L.Y = fuse_out ? nullptr : s.dout;
+    L.read_once = fuse_in && s.G.mapped;
     L.act[0] = s.act0; L.act[1] = s.act1; L.act_ld = act_ld(s.buf_rows);
     L.g = g;
     ensure_aux(std::max(tc_grid(s.tc, rows), f32tc_grid(rows)));
@@ -810,7 +813,8 @@ void run_step_kernels(const StepArgs& A) {
     // fp32 on the tensor cores: one split-TF32 kernel per layer, gather fused into the first layer's operand load and
     // scatter (+ checksum) into the last epilogue when the descriptors are table-driven, activations feature-major
     F32TcLaunch L{};
-    const bool fuse_in = A.use_gather && fuse && s.G.fast && s.model.n_in() <= 768;
+    // (a layer's tiles of 32 to 128 features each load all inputs of their rows: over the host link once is enough)
+    const bool fuse_in = A.use_gather && fuse && s.G.fast && s.model.n_in() <= 768 && !s.G.mapped;
     const bool fuse_out = A.fuse_scatter && fuse && s.S.fast && s.model.n_out() <= 256;
     if (fuse_in) { L.fast_in = 1; L.slots = (const Access*)s.G.items; L.TG = A.TG; std::memcpy(L.cin, s.G.cls, sizeof L.cin); }
     else {
@@ -1075,7 +1079,7 @@ bool overlapped_step(void* const* gptrs, void* const* sptrs, long long rows) {
       const ArrayInfo& a = P.h.arrays[ai];
       if (!a.used || P.on_dev[ai] || a.total != ncol || P.reg[ai] != ptrs[ai]) continue;
       void* dp = nullptr;
-      if (cudaHostGetDevicePointer(&dp, ptrs[ai], 0) == cudaSuccess && dp) { P.on_dev[ai] = true; T.base[ai] = dp; }
+      if (cudaHostGetDevicePointer(&dp, ptrs[ai], 0) == cudaSuccess && dp) { P.on_dev[ai] = true; P.mapped = true; T.base[ai] = dp; }
       else cudaGetLastError();
     }
   };

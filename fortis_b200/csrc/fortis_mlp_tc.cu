@@ -1303,7 +1303,7 @@ TcModel* tc_model_create(const ModelHost& M, int precision, cudaStream_t s, std:
 bool tc_forward(TcModel* m, const TcLaunch& L, cudaStream_t s, std::string* err) {
   const long long nrows = L.g.count * L.g.nk;
   if (nrows <= 0) return true;
-  if (m->rows && !g_tc_test.no_stage && L.act[0] && (m->nlayers < 3 || L.act[1]) &&
+  if (m->rows && !g_tc_test.no_stage && !L.read_once && L.act[0] && (m->nlayers < 3 || L.act[1]) &&
       tc_rows_layer_by_layer(m->widths, m->widths + 1, m->nlayers, m->has_scale, nrows)) {
     F32TcLaunch R{};
     R.fast_in = L.fast_in; R.slots = L.slots; R.TG = L.TG; R.X = L.X;

@@ -225,3 +225,26 @@ def test_a_convolution_is_no_less_exact_than_its_fp32_sums(host, C, K, clamp):
             win = x[:, c, None, kd:kd + D, kh:kh + H, kw:kw + W].double()
             chain = (chain.double() + win * w[None, :, c, kd, kh, kw, None, None, None].double()).float()
     assert rel(y, want) <= 1.05 * rel(chain, want)
+
+
+@pytest.mark.parametrize("dims", [[244, 128], [244, 64, 128]])
+def test_host_vectors_updated_in_place(host, dims):
+    """Column vectors that a step reads and writes stay in the host's pages; one layer's feature tiles must not read what
+    another tile has stored."""
+    rows, nlev = 9000, 60
+    G, S, Lp, K = descriptors.column(rows, nlev)
+    rng = np.random.default_rng(17)
+    fields = [np.asfortranarray(rng.standard_normal((rows, nlev)).astype(np.float32)) for _ in range(4)]
+    vectors = [rng.standard_normal(rows).astype(np.float32) for _ in range(8)]
+    blob = fortis_b200.write_blob(fortis_b200.mlp_layers(dims, seed=3, act="relu"))
+    got = []
+    for in_place in (False, True):
+        host.reset()
+        host.configure(gather=G, scatter=S, loop=Lp)
+        host.load_model(blob)
+        gin = [v.copy() for v in vectors[:4]]
+        out = [np.zeros((rows, nlev), np.float32, order="F") for _ in range(2)] + [v if in_place else v.copy() for v in gin] + [v.copy() for v in vectors[4:]]
+        host.step(fields + gin, out)
+        got.append([a.copy(order="F") for a in out])
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
