@@ -460,10 +460,11 @@ bool conv3d_ncdhw(const float* x, const float* w, float* y, int N, int C, int D,
   // weights are constants of the caller: repack each distinct (pointer, shape) once, as the reference caches its
   // transposed GEMM weights (runtime/fortis_rt.c:55-66)
   // The repack runs as a kernel on the caller's stream (no synchronisation, no host round trip).  The cache holds 64
-  // entries; when it is full the oldest entry is replaced and its buffer reused or freed.  A weight seen for the
-  // first time needs a buffer: that cannot happen while the stream is being captured into a graph, so such a call
-  // is refused (the reference captures on the second call for the same reason: the first call allocates).
-  struct Cached { const float* w; int F, C, taps; float* wt; F32ConvW* split; };
+  // entries and those a captured call uses (its graph holds their addresses); when it is full the oldest of the others is
+  // freed and replaced.  A weight seen for the first time needs a buffer: that cannot happen while the stream is being
+  // captured into a graph, so such a call is refused (the reference captures on the second call for the same reason: the
+  // first call allocates).
+  struct Cached { const float* w; int F, C, taps; float* wt; F32ConvW* split; bool captured; };
   static std::vector<Cached> cache;
   static size_t victim = 0;
   const int taps = K[0] * K[1] * K[2];
@@ -478,22 +479,26 @@ bool conv3d_ncdhw(const float* x, const float* w, float* y, int N, int C, int D,
   const bool tc = f32tc_conv_supported(g);
   Cached* c = nullptr;
   bool fresh = false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(s, &cs);
+  const bool capturing = cs != cudaStreamCaptureStatusNone;
   for (auto& q : cache) if (q.w == w && q.F == F && q.C == C && q.taps == taps) c = &q;
+  if (c && capturing) c->captured = true;
   if (!c || (tc ? (void*)c->split : (void*)c->wt) == nullptr) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(s, &cs);
-    if (cs != cudaStreamCaptureStatusNone) { if (err) *err = "conv weights seen for the first time during graph capture; run one eager call first"; return false; }
+    if (capturing) { if (err) *err = "conv weights seen for the first time during graph capture; run one eager call first"; return false; }
     if (!c) {
-      if (cache.size() < 64) { cache.push_back(Cached{}); c = &cache.back(); }
-      else { c = &cache[victim]; victim = (victim + 1) % cache.size(); cudaStreamSynchronize(s); cudaFree(c->wt); f32tc_conv_free(c->split); }
-      *c = Cached{w, F, C, taps, nullptr, nullptr};
+      for (size_t i = 0; i < cache.size() && cache.size() >= 64 && !c; i++, victim = (victim + 1) % cache.size())
+        if (!cache[victim].captured) c = &cache[victim];
+      if (c) { cudaStreamSynchronize(s); cudaFree(c->wt); f32tc_conv_free(c->split); }
+      else { cache.push_back(Cached{}); c = &cache.back(); }
+      *c = Cached{w, F, C, taps, nullptr, nullptr, false};
     }
     const size_t n = (size_t)F * C * taps;
     if (tc) {
       c->split = f32tc_conv_pack(w, F, C, taps, s, err);
-      if (!c->split) { cudaFree(c->wt); *c = Cached{}; return false; }
+      if (!c->split) return false;
     } else {
-      if (cudaMalloc(&c->wt, n * 4) != cudaSuccess) { cudaGetLastError(); f32tc_conv_free(c->split); *c = Cached{}; if (err) *err = "out of device memory for conv weights"; return false; }
+      if (cudaMalloc(&c->wt, n * 4) != cudaSuccess) { cudaGetLastError(); c->wt = nullptr; if (err) *err = "out of device memory for conv weights"; return false; }
       repack_weights_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(w, c->wt, F, C, taps);
     }
     fresh = true;

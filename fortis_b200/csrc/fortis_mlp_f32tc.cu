@@ -1098,18 +1098,23 @@ bool f32tc_forward(F32TcModel* m, const F32TcLaunch& L, cudaStream_t s, std::str
 // as the reference caches its transposed weights (runtime/fortis_rt.c:55-66).
 bool f32tc_gemm(const float* A, const float* W, float* C, long long M, int N, int K, int* status, cudaStream_t s, std::string* err) {
   if (M <= 0 || N <= 0 || K <= 0) return true;
-  struct Cached { const float* src = nullptr; SplitW w; };
+  struct Cached { const float* src = nullptr; SplitW w; bool captured = false; };
   static std::vector<Cached> cache;
   static size_t victim = 0;
   Cached* c = nullptr;
   bool fresh = false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(s, &cs);
+  const bool capturing = cs != cudaStreamCaptureStatusNone;
   for (auto& e : cache) if (e.src == W && e.w.N_real == N && e.w.K_real == K) c = &e;
+  if (c && capturing) c->captured = true;
   if (!c) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(s, &cs);
-    if (cs != cudaStreamCaptureStatusNone) { if (err) *err = "weights seen for the first time during graph capture; run one eager call first"; return false; }
-    if (cache.size() < 64) { cache.push_back(Cached()); c = &cache.back(); }
-    else { c = &cache[victim]; victim = (victim + 1) % cache.size(); cudaStreamSynchronize(s); split_free(&c->w); }
+    if (capturing) { if (err) *err = "weights seen for the first time during graph capture; run one eager call first"; return false; }
+    // 64 entries and those a captured call uses: its graph holds their addresses
+    for (size_t i = 0; i < cache.size() && cache.size() >= 64 && !c; i++, victim = (victim + 1) % cache.size())
+      if (!cache[victim].captured) c = &cache[victim];
+    if (c) { cudaStreamSynchronize(s); split_free(&c->w); }
+    else { cache.push_back(Cached()); c = &cache.back(); }
     c->src = nullptr;
     if (!split_alloc(&c->w, K, N, err)) return false;
     split_weights_kernel<<<split_grid((size_t)c->w.N_pad * c->w.K_pad), 256, 0, s>>>(W, N, K, (uint32_t*)c->w.hi, (uint32_t*)c->w.lo, c->w.N_pad, c->w.K_pad);

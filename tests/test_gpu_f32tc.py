@@ -62,11 +62,15 @@ def test_gemm_tile_and_step_edges(host, B, N, K):
 
 
 def conv_entry(host, x, w, y, stride, pad):
+    conv_call(host, x, w, y, stride, pad)
+    host.sync()
+
+
+def conv_call(host, x, w, y, stride, pad):
     f = host.L.fortis_conv3d
     f.argtypes, f.restype = ([ctypes.c_void_p] * 2 + [ctypes.c_long] * 11) * 3 + [ctypes.c_long] * 18, None
     _keep.append(w)
     f(*memref(x), *memref(w), *memref(y), x.shape[0], x.shape[1], *x.shape[2:], w.shape[0], *w.shape[2:], *y.shape[2:], *stride, *pad)
-    host.sync()
 
 
 def conv64(x, w, stride, pad):
@@ -248,3 +252,47 @@ def test_host_vectors_updated_in_place(host, dims):
         got.append([a.copy(order="F") for a in out])
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+def test_captured_calls_keep_their_weights(host):
+    """The memref entries keep the prepared weights of 64 layers by address; a graph that holds such an address is replayed
+    after more layers than that have been called."""
+    f = host.L.fortis_gemm
+    f.argtypes, f.restype = ([ctypes.c_void_p] * 2 + [ctypes.c_long] * 5) * 3 + [ctypes.c_long] * 3, None
+    gemm = lambda A, W, C: f(*memref(A), *memref(W), *memref(C), A.shape[0], W.shape[0], W.shape[1])
+    one, pad = (1, 1, 1), (1, 1, 1)
+    shapes = [(20, 16), (3, 5)]                                       # on the tensor cores, on the FFMA kernel
+    x = [randn((1, c, 4, 5, 6), 20) for c, _ in shapes]
+    w = [randn((o, c, 3, 3, 3), 21) for c, o in shapes]
+    y = [torch.zeros((1, o, 4, 5, 6), device="cuda") for _, o in shapes]
+    A, B, C = randn((600, 40), 22), randn((24, 40), 23), torch.zeros((600, 24), device="cuda")
+    _keep.append(B)
+    def calls():
+        for i in range(2):
+            conv_call(host, x[i], w[i], y[i], one, pad)
+        gemm(A, B, C)
+    calls()
+    host.sync()
+    host.L.mgpuStreamCreate.restype = ctypes.c_void_p
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(torch.cuda.ExternalStream(host.L.mgpuStreamCreate())):
+        graph.capture_begin(capture_error_mode="relaxed")
+        calls()
+        graph.capture_end()
+        other = [torch.zeros_like(y[0]), torch.zeros_like(y[1]), torch.zeros_like(C)]
+        for seed in range(70):
+            for i in range(2):
+                conv_call(host, x[i], randn(w[i].shape, 100 + seed), other[i], one, pad)
+            W = randn(B.shape, 300 + seed)
+            _keep.append(W)
+            gemm(A, W, other[2])
+        for t in x + [A]:
+            t.normal_()
+        for t in y + [C]:
+            t.zero_()
+        graph.replay()
+        torch.cuda.current_stream().synchronize()
+    for i in range(2):
+        assert rel(y[i], conv64(x[i], w[i], one, pad)) < TOL
+    assert rel(C, A.double() @ B.double().T) < TOL
+    assert host.L.fortis_device_status() == 0
