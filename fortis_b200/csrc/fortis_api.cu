@@ -809,7 +809,7 @@ void run_step_kernels(const StepArgs& A) {
     if (L.partials) launch_fold(s.d_partials, L.grid, s.d_sum, 1, st);
     return;
   }
-  if (s.f32 && rows >= kF32TcMinRows) {
+  if (s.f32 && rows >= kF32TcMinRows && rows <= kF32TcMaxRows) {
     // fp32 on the tensor cores: one split-TF32 kernel per layer, gather fused into the first layer's operand load and
     // scatter (+ checksum) into the last epilogue when the descriptors are table-driven, activations feature-major
     F32TcLaunch L{};

@@ -132,6 +132,7 @@ struct F32TcLaunch {
   int* status;
 };
 int f32tc_grid(long long nrows);
+constexpr long long kF32TcMaxRows = (1LL << 31) - 129;     // the activations' tiles are addressed by 32-bit row numbers
 bool f32tc_forward(F32TcModel* m, const F32TcLaunch& L, cudaStream_t s, std::string* err);
 // Extents and element strides of one convolution layer (cross-correlation, zero padding)
 struct ConvGeom {

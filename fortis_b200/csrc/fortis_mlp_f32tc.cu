@@ -849,7 +849,7 @@ int round_up_f(int v, int m) { return (v + m - 1) / m * m; }
 // rows do not start on 16-byte boundaries.
 bool make_a_map(bool feature_major, const float* A, long long rows, int K, long long ld, CUtensorMap* m) {
   EncodeTiledFnF enc = encode_fn_f();
-  if (!enc || ((uintptr_t)A & 15) != 0 || (ld & 3) != 0 || rows >= (1LL << 31) - kM || ld * 4 >= (1LL << 40)) return false;
+  if (!enc || ((uintptr_t)A & 15) != 0 || (ld & 3) != 0 || rows > kF32TcMaxRows || ld * 4 >= (1LL << 40)) return false;
   const cuuint64_t dims[2] = {(cuuint64_t)(feature_major ? rows : K), (cuuint64_t)(feature_major ? K : rows)};
   const cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
   const cuuint32_t box[2] = {(cuuint32_t)(feature_major ? kM : kKt), (cuuint32_t)(feature_major ? kKt : kM)}, estr[2] = {1, 1};

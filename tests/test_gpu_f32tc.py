@@ -192,10 +192,13 @@ def chains():
     return hashlib.sha256(b"".join(t.cpu().numpy().tobytes() for t in out)).hexdigest()
 
 
+def in_child(code, **env):
+    return subprocess.run([sys.executable, "-c", "from tests import test_gpu_f32tc as t; " + code], check=True, text=True, stdout=subprocess.PIPE,
+                          env=dict(os.environ, **env), cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__)))).stdout
+
+
 def test_layers_that_overlap_give_the_bits_of_layers_run_one_by_one():
-    one_by_one = subprocess.run([sys.executable, "-c", "from tests import test_gpu_f32tc as t; print(t.chains())"], check=True, text=True,
-                                stdout=subprocess.PIPE, env=dict(os.environ, FORTIS_NO_PDL="1"), cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
-    assert chains() == one_by_one.stdout.split()[-1]
+    assert chains() == in_child("print(t.chains())", FORTIS_NO_PDL="1").split()[-1]
 
 
 def test_biases_of_a_layer_with_more_feature_tiles_than_sms(host):
@@ -296,3 +299,25 @@ def test_captured_calls_keep_their_weights(host):
         assert rel(y[i], conv64(x[i], w[i], one, pad)) < TOL
     assert rel(C, A.double() @ B.double().T) < TOL
     assert host.L.fortis_device_status() == 0
+
+
+def very_many_rows():
+    rows, host = 2 ** 31 - 100, fortis_b200.Host()
+    layers = fortis_b200.mlp_layers([1, 2, 1], seed=3, act="relu", bias="uniform")
+    host.load_model(fortis_b200.write_blob(layers))
+    host.L.fortis_begin(rows)
+    x, y = torch.empty(rows, device="cuda").uniform_(-1, 1), torch.zeros(rows, device="cuda")
+    host.forward_batched(x, y)
+    for part in (slice(0, 1000), slice(rows - 1000, rows)):
+        want = x[part, None].double()
+        for i, L in enumerate(layers):
+            want = want @ torch.from_numpy(L["W"]).double().cuda().T + torch.from_numpy(L["b"]).double().cuda()
+            want = want if i else want.clamp_min(0)
+        assert rel(y[part], want[:, 0]) < TOL
+
+
+def test_more_rows_than_32_bit_tile_coordinates_hold():
+    """Such an MLP call runs on the FFMA kernels.  52 GB on the device, in a process of its own: the library pools memory."""
+    if torch.cuda.mem_get_info()[0] < 70e9:
+        pytest.skip("needs 70 GB of device memory")
+    in_child("t.very_many_rows()")
