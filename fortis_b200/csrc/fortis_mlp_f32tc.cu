@@ -67,6 +67,10 @@ constexpr int kChunkLong = 2, kChunkShort = 1, kShortK = 640;
 // that is taken over every 128 k.  Further from the exact sums (five-layer column network 5.6e-6 against 2.4e-6), but a
 // program's results stay what they were to the last bit.
 constexpr int kChunkMlp = 4;
+// Convolutions multiply x_lo by 2^10 (exact) and the cross sums by 2^-10: the tensor core takes subnormal operands as zero, and
+// unscaled x_lo is subnormal from |x| < 2^-102 on (2^-118: error 2.2e-6).  With it every normal value keeps its precision.
+// (x_lo is below 2^-10 of the largest value, so the product stays finite.)
+constexpr float kLoScale = 1024.f;
 constexpr int kBarF = 384;
 constexpr int kTabIn = 768, kTabOut = 256;     // widest gathered input / scattered output the tables hold
 constexpr int kTileScratch = 32 * 32 * 4;      // one warp's 32 x 32 transpose
@@ -470,7 +474,10 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
       }
       uint32_t hi[16], lo[16];
 #pragma unroll
-      for (int j = 0; j < 16; j++) split_tf32(v[j], hi[j], lo[j]);
+      for (int j = 0; j < 16; j++) {
+        split_tf32(v[j], hi[j], lo[j]);
+        if constexpr (!kMaybeOneAcc) lo[j] = __float_as_uint(__uint_as_float(lo[j]) * kLoScale);
+      }
       tmem_st16(dst, hi);
       tmem_st16(dst + 32, lo);
     };
@@ -637,7 +644,10 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
         tmem_ldn(lane_addr + CF::kColCross + c0, a);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < NL; j++) v[c0 + j] = __fadd_rn(v[c0 + j], __uint_as_float(a[j]));
+        for (int j = 0; j < NL; j++) {
+          if constexpr (kMaybeOneAcc) v[c0 + j] = __fadd_rn(v[c0 + j], __uint_as_float(a[j]));
+          else v[c0 + j] = fmaf(__uint_as_float(a[j]), 1.f / kLoScale, v[c0 + j]);
+        }
       }
       tc_fence_before();
       __syncwarp();
@@ -826,7 +836,7 @@ __global__ void split_conv_weights_kernel(const float* __restrict__ W, int F, in
     const int n = (int)(i / K_pad), k = (int)(i % K_pad), tap = k / cp, c = k - tap * cp;
     uint32_t h = 0, l = 0;
     if (n < F && tap < taps && c < C) split_tf32(W[((long long)n * C + c) * taps + tap], h, l);
-    hi[i] = h; lo[i] = l;
+    hi[i] = h; lo[i] = __float_as_uint(__uint_as_float(l) * kLoScale);
   }
 }
 

@@ -257,6 +257,16 @@ def test_host_vectors_updated_in_place(host, dims):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("xe,we", [(-117, 100), (-121, 100), (100, -117), (-60, -55), (120, -120)])
+def test_small_and_large_values_keep_their_low_halves(host, xe, we):
+    """The tensor core takes subnormal operands as zero; a value's low half is 2^-12 of it and its last bit 2^-23."""
+    x, w = randn((1, 64, 5, 8, 8), 24, 2.0 ** xe), randn((32, 64, 3, 3, 3), 25, 2.0 ** we)
+    want = conv64(x, w, (1, 1, 1), (0, 0, 0))
+    y = torch.full(want.shape, float("nan"), device="cuda")
+    conv_entry(host, x, w, y, (1, 1, 1), (0, 0, 0))
+    assert rel(y, want) < TOL
+
+
 def test_captured_calls_keep_their_weights(host):
     """The memref entries keep the prepared weights of 64 layers by address; a graph that holds such an address is replayed
     after more layers than that have been called."""
