@@ -26,9 +26,17 @@ BF16_TOL, FP8W_TOL, MODEL_TOL = 5e-3, 2e-2, 2e-3
 SLACK = 1.1
 
 
-@pytest.fixture()
-def host():
+@pytest.fixture(params=["default", "1", "0"])
+def host(request):
+    """The forms a 16-bit MLP call may take: by its size (few rows layer by layer), fused in two-CTA clusters, fused with one
+    CTA per SM."""
     h = fortis_b200.Host()
+    plain_reset = h.reset
+
+    def reset():
+        plain_reset()
+        h.option("tc_pair", request.param)
+    h.reset = reset
     h.reset()
     yield h
     assert h.L.fortis_device_status() == 0, "a bounded wait in the tensor-core kernel gave up"
@@ -308,7 +316,7 @@ def test_staged_tiles_random_layouts(host, seed):
 @pytest.mark.parametrize("seed", range(int(os.environ.get("FORTIS_TC_SWEEP", "10"))))
 def test_random_shapes_against_the_low_precision_model(host, seed):
     """Random depths (1-7 layers), widths (1-768, so every padding and chunk count), row counts (1-4000, so ragged
-    last tiles and CTAs with zero to several tiles), activations and precisions: the fused kernel against the oracle's
+    last tiles and CTAs with zero to several tiles), activations and precisions: every form of the call against the oracle's
     model of its arithmetic, in the array form and, for the fused step, through an identity-layout descriptor."""
     rng = np.random.default_rng(4200 + seed)
     nl = int(rng.integers(1, 8))
