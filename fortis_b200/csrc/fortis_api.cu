@@ -622,10 +622,9 @@ void download_stores(PlanDev& P, const int* args, int nargs, bool multi_plane, c
 // ---------------------------------------------------------------------------------------------------------------
 // the step
 // ---------------------------------------------------------------------------------------------------------------
-// Below this many rows the per-layer FFMA kernels run: their sums are what a program of few rows has always had.  (The
-// tensor-core kernel is faster there too, 300 rows of the column network 73 us against 455, but further from those sums
-// than from the exact ones.)  fortis_gemm: from here on the weights are split once per address (constants of the caller);
-// below, W is read as it is on every call.
+// Below this many rows the per-layer FFMA kernels run.  (The tensor-core kernel is faster there too, 300 rows of the column
+// network 73 us against 455, but its sums are others than a program of few rows has had.)  fortis_gemm: from here on the
+// weights are split once per address (constants of the caller); below, W is read as it is on every call.
 constexpr long long kF32TcMinRows = 512;
 
 struct StepArgs {

@@ -178,7 +178,7 @@ std::vector<float> repack_weights_taps(const float* w, int F, int C, int taps) {
 }
 
 // One layer's weights on the device: [tap][C][F] for the FFMA kernel and, where the tensor-core kernel may take the layer,
-// split for that one.
+// split for that one.  (Which of the two runs depends on the volume's extents too, so both stay.)
 struct LayerDev { float *wt = nullptr, *bias = nullptr; F32ConvW* split = nullptr; };
 bool upload_layer(const LayerHost& L, int taps, bool split, LayerDev* d, std::string* err) {
   split = split && (long long)L.cin * taps >= kF32TcConvMinProducts;
@@ -205,7 +205,7 @@ bool upload_layer(const LayerHost& L, int taps, bool split, LayerDev* d, std::st
 
 // A layer takes the tensor-core kernel wherever it can and its sums are long enough (f32tc_conv_supported: no input dilation,
 // up to 32 taps per axis, a table of taps and channels that fits shared memory, kF32TcConvMinProducts): 14-layer network,
-// 2 x 33^3 voxels, 1.80 ms against 8.75 on the FFMA kernel; 32 -> 64 channels on 40^3 71 us against 297.
+// 2 x 33^3 voxels, 2.02 ms against 8.75 on the FFMA kernel; 32 -> 64 channels on 40^3 73 us against 297.
 bool conv_layer(const F32ConvW* split, const float* wt, const float* bias, const float* x, const float* residual, float* y, const ConvGeom& g,
                 int act, float slope, int* status, cudaStream_t s, std::string* err) {
   if (split && f32tc_conv_supported(g)) return f32tc_conv(split, x, bias, residual, y, g, act, slope, status, s, true, err);

@@ -23,15 +23,16 @@
 // Operand traffic is why A sits in tensor memory: with A in shared memory (the form before this one) the three MMAs of a
 // k step read 12 KB per 128 clocks and the producers and the TMA write 96 KB per 1536, together 1.25 times what shared
 // memory moves; in this form only the weights (64 B/clk at any NT) and the fp32 tiles pass through it.
-// Measured, that form / this one: fortis_gemm 8192 x 768 x 768 756 / 60 us (a row-major operand was read by one dependent load
-// per row), column network 30,011 rows 991 / 730 us; convolutions against the FFMA kernel: 32 -> 64 channels 3x3x3 on 40^3
-// 297 / 71 us, 14-layer network 2 x 33^3 8.75 / 1.80 ms.
+// Measured, that form / this one: fortis_gemm 8192 x 768 x 768 756 / 62 us (a row-major operand was read by one dependent load
+// per row), column network 30,011 rows 991 / 750 us; convolutions against the FFMA kernel: 32 -> 64 channels 3x3x3 on 40^3
+// 297 / 73 us, 14-layer network 2 x 33^3 8.75 / 2.02 ms.
 //
 // The tensor core adds into its fp32 accumulator with truncation, not rounding, a bias per accumulation of half a unit in
-// the last place of the partial sum.  Two things keep it below fp32 rounding: the hi.hi products go into an accumulator
-// of their own that is taken over every 64 k (8 truncating additions; 32 where K is short) and summed by the epilogue warps in registers with
-// IEEE additions, and the two cross products go into a second accumulator (2^-11 of the result, so its truncation does not
-// count) that lives for the whole K.
+// the last place of the partial sum.  In convolutions and fortis_gemm two things keep it below fp32 rounding: the hi.hi
+// products go into an accumulator of their own that is taken over every 64 k (8 truncating additions; 32 where K is short)
+// and summed by the epilogue warps in registers with IEEE additions, and the two cross products go into a second accumulator
+// (2^-11 of the result, so its truncation does not count) that lives for the whole K.  MLP steps keep the three products in
+// one accumulator, taken over every 128 k (kChunkMlp).
 // Infinities: x_hi saturates at the largest finite TF32 value and x_lo = x - x_hi carries the infinity, so a product is
 // infinite, or NaN, where the fp32 product is.  Every barrier wait is bounded; a CTA
 // whose wait gives up records which one, lets its copies and MMAs in flight finish and returns.
@@ -64,8 +65,8 @@ constexpr int kKt = 32;                    // k per stage: one 128-byte swizzle 
 // convolutions, error against 64 bits: two 9.1e-7, one 6.2e-7, FFMA 7.7e-7)
 constexpr int kChunkLong = 2, kChunkShort = 1, kShortK = 640;
 // MLP steps keep the sums they have always had: the three products of a step of 8 k one after another in one accumulator
-// that is taken over every 128 k.  Further from the exact sums (five-layer column network 5.6e-6 against 2.4e-6), but a
-// program's results stay what they were to the last bit.
+// that is taken over every 128 k.  Further from the exact sums (five-layer column network 5.6e-6 against 2.4e-6), but the sums
+// a program has had of finite inputs.
 constexpr int kChunkMlp = 4;
 // Convolutions multiply x_lo by 2^10 (exact) and the cross sums by 2^-10: the tensor core takes subnormal operands as zero, and
 // unscaled x_lo is subnormal from |x| < 2^-102 on (2^-118: error 2.2e-6).  With it every normal value keeps its precision.
@@ -917,8 +918,12 @@ bool split_alloc(SplitW* w, int K, int N, std::string* err) {
 }
 
 // The tile width (0, 1, 2: 32, 64, 128 features).  A k step of a tile costs 6 clocks per feature of tensor time, or what
-// its producers need for 128 rows x 32 inputs if that is more, and the launch lasts as many rounds of tiles as the SM
-// that has the most.
+// its producers need for 128 rows x 32 inputs if that is more (step_floor), and the launch lasts as many rounds of tiles as
+// the SM that has the most.  The floors are estimates, and low ones: a step with its share of the tile's end measures 1140,
+// 1200, 1520 clocks at 32, 64, 128 features (fortis_gemm, K = 768), 2210, 2310, 2520 with rows off 16 bytes, 1240, 1280, 1430 in
+// convolutions of K = 1728 and 1960, 2100, 2460 of K = 405.  So the rule takes tiles that are too narrow: over 8 to 256 features
+// and 13 to 1138 row tiles the width it picks is within 5 % of the fastest for every convolution of up to 64 features and 147
+// of 240 wider ones (at worst 1.76 times the time), and for 276 of 390 products (8 to 1000 features; at worst 2.4 times).
 int pick_tile(long long nrows, int N, int step_floor) {
   const long long ntm = (nrows + kM - 1) / kM, sms = sm_count();
   long long best_cost = 0;
@@ -980,7 +985,7 @@ bool launch_tile(F32Params& P, const SplitW& W, int step_floor, cudaStream_t s, 
   return w == 2 ? launch_as<128, AMODE>(P, s, early) : w == 1 ? launch_as<64, AMODE>(P, s, early) : launch_as<32, AMODE>(P, s, early);
 }
 
-// clocks a k step's producers need at least (measured: see pick_tile)
+// clocks a k step's producers need at least (see pick_tile)
 constexpr int kStepFloorLinear = 250, kStepFloorConv = 350;
 
 // a row-major operand: tiles through the TMA where rows start on 16-byte boundaries, else loads

@@ -126,8 +126,9 @@ int fortis_load_model(const char* path);
 int fortis_load_model_mem(const void* blob, long nbytes);
 /* options:
  *   "precision"   "fp32" (default; large layers run as three TF32 tensor-core products per fp32 product with IEEE
- *                 running sums, <= 1e-5) | "bf16" | "fp16" (16-bit operands, fp32 accumulation) | "fp8w" (FP8-E4M3
- *                 weights with per-channel scales, bf16 activations; MLP models only)
+ *                 running sums, <= 1e-5; values below 2^-102, in convolutions 2^-126, lose precision there) |
+ *                 "bf16" | "fp16" (16-bit operands, fp32 accumulation) | "fp8w" (FP8-E4M3 weights with per-channel
+ *                 scales, bf16 activations; MLP models only)
  *   "fuse"        "0" | "1"   one launch per step where the descriptors allow it (default 1)
  *   "graph"       "0" | "1"   replay a step as a CUDA graph from its second call (FORTIS_GRAPH)
  *   "async"       "0" | "1"   return from a step without waiting for the stream (fortis_sync() waits)
@@ -137,9 +138,10 @@ int fortis_load_model_mem(const void* blob, long nbytes);
  *                 load from them as well); also FORTIS_HOST_ACCESS
  *   "stencil_tc"  "0" | "1"   3x3-stencil hosts with narrow MLPs: run the layers as TF32x3 tensor-core products instead
  *                 of packed FMAs (same <= 1e-5; measured slower for 27-20-20-3, default 0); also FORTIS_STENCIL_TC
- *   "tc_pair"     "1" (default) | "0" | "default"   wide MLPs in 16-bit / FP8-weight precision: run the fused
- *                 tensor-core kernel as clusters of two CTAs that share one stream of weights, or one CTA per SM (same
- *                 results bit for bit; the cluster form is 9-16 % faster); also FORTIS_TC_PAIR
+ *   "tc_pair"     "default" | "1" | "0"   wide MLPs in 16-bit / FP8-weight precision.  "default": calls of up to 3072 rows
+ *                 layer by layer where that is faster, others in one fused kernel of two-CTA clusters that share one
+ *                 stream of weights; "1": always the fused kernel in clusters; "0": always fused, one CTA per SM (9-16 %
+ *                 slower).  The same results bit for bit for finite values; also FORTIS_TC_PAIR (0 | 1)
  *   "conv_shape"  "N,D,H,W"   input extent of a conv3d model (NDHWC arrays); "N,1,H,W" for a network of 2-D operator
  *                 layers (Conv2d / transposed / pooling / upsampling; NCHW arrays in and out of mlp_forward)
  * The keys "test_wait_limit" and "test_skip_stage" exist for the tests of the bounded waits, "test_no_stage" for the test
