@@ -456,9 +456,14 @@ void ensure_buffers(long long rows) {
 void ensure_aux(long long npartials) {
   Session& s = S();
   if (!s.d_sum) {
-    s.d_sum = (double*)pool_alloc(sizeof(double));
-    s.d_status = (int*)pool_alloc(sizeof(int));
-    s.d_done = (unsigned int*)pool_alloc(sizeof(unsigned int));
+    double* sum = (double*)pool_alloc(sizeof(double));
+    int* status = (int*)pool_alloc(sizeof(int));
+    unsigned int* done = (unsigned int*)pool_alloc(sizeof(unsigned int));
+    if (!sum || !status || !done) {                 // a kernel would report through a null pointer
+      pool_free(sum); pool_free(status); pool_free(done);
+      throw std::runtime_error("out of device memory for the status words");
+    }
+    s.d_sum = sum; s.d_status = status; s.d_done = done;
     cudaMemset(s.d_done, 0, sizeof(unsigned int));
     cudaMemset(s.d_sum, 0, sizeof(double));
     cudaMemset(s.d_status, 0, sizeof(int));
@@ -466,7 +471,8 @@ void ensure_aux(long long npartials) {
   if (npartials > s.partials_cap) {
     pool_free(s.d_partials);
     s.d_partials = (double*)pool_alloc(npartials * (long long)sizeof(double));
-    s.partials_cap = npartials;
+    s.partials_cap = s.d_partials ? npartials : 0;
+    if (!s.d_partials) throw std::runtime_error("out of device memory for the checksum's partial sums");
     drop_graph();
   }
 }
@@ -1708,6 +1714,7 @@ void fortis_gemm(float* Aa, float* A, long Ao, long As0, long As1, long At0, lon
                  B, K, At0, At1, N, K, Wt0, Wt1, B, N, Ct0, Ct1);
     return;
   }
+  FORTIS_TRY
   if (B >= kF32TcMinRows) {
     // large batch: the tensor-core kernel (three TF32 MMAs per product, fp32-class accuracy)
     S();
@@ -1717,6 +1724,7 @@ void fortis_gemm(float* Aa, float* A, long Ao, long As0, long As1, long At0, lon
     std::fprintf(stderr, "fortis_gemm: %s; using the FFMA kernel\n", err.c_str());
   }
   launch_linear_f32(A + Ao, W + Wo, nullptr, C + Co, B, (int)N, (int)K, ACT_NONE, 0.f, nullptr, nullptr, nullptr, stream());
+  FORTIS_CATCH(return)
 }
 
 // dense NCDHW-style strides of a rank-5 memref (dimensions of extent 1 may carry any stride)
@@ -1745,11 +1753,13 @@ static void conv3d_entry(const char* who, float* x, long xo, float* w, long wo, 
     return;
   }
   const int K[3] = {(int)KD, (int)KH, (int)KW}, st[3] = {(int)sd, (int)sh, (int)sw}, pad[3] = {(int)pd, (int)ph, (int)pw};
+  FORTIS_TRY
   std::string err;
   S();
   ensure_aux(1);
   if (!conv3d_ncdhw(x + xo, w + wo, y + yo, (int)N, (int)C, (int)Din, (int)Hin, (int)Win, (int)F, K, st, pad, S().d_status, stream(), &err))
     std::fprintf(stderr, "%s: %s\n", who, err.c_str());
+  FORTIS_CATCH(return)
 }
 
 #define FORTIS_MEMREF5_UNUSED \

@@ -3,7 +3,10 @@ import ctypes
 import os
 import re
 
+import numpy as np
 import pytest
+
+torch = pytest.importorskip("torch")
 
 import fortis_b200
 from fortis_b200 import build as fb
@@ -86,3 +89,23 @@ def test_every_option_key_is_documented_in_a_header():
     docs = "\n".join(open(os.path.join(inc, f)).read() for f in sorted(os.listdir(inc)) if f.endswith(".h"))
     missing = [k for k in sorted(keys) if '"%s"' % k not in docs]
     assert not missing, "option keys without a line in include/*.h: %s" % missing
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="shows what a failed device allocation does: needs a host without a device")
+@pytest.mark.parametrize("entry", ["fortis_conv3d", "fortis_gemm"])
+def test_memref_entries_report_a_failed_allocation(entry):
+    """Without device memory for the word in which a kernel reports a wait that gave up, nothing is launched."""
+    L = fortis_b200.load()
+    L.fortis_reset()
+    buf = np.zeros(600 * 40, np.float32)
+    p = buf.ctypes.data
+    if entry == "fortis_gemm":
+        f, operands, extents = L.fortis_gemm, [(600, 40), (40, 40), (600, 40)], (600, 40, 40)
+    else:
+        f, operands, extents = L.fortis_conv3d, [(1, 1, 4, 4, 4), (1, 1, 1, 1, 1), (1, 1, 4, 4, 4)], (1, 1, 4, 4, 4, 1, 1, 1, 1, 4, 4, 4, 1, 1, 1, 0, 0, 0)
+    dense = lambda s: s + tuple(int(np.prod(s[i + 1:])) for i in range(len(s)))
+    args = [v for s in operands for v in (ctypes.c_void_p(p), ctypes.c_void_p(p), 0) + dense(s)] + list(extents)
+    f.restype = None
+    f(*[a if isinstance(a, ctypes.c_void_p) else ctypes.c_long(a) for a in args])
+    assert L.fortis_last_error() != 0 and b"memory" in ctypes.string_at(L.fortis_last_error_message())
+    L.fortis_reset()
