@@ -228,7 +228,7 @@ def test_a_convolution_is_no_less_exact_than_its_fp32_sums(host, C, K, clamp):
     chain = torch.zeros(want.shape, device="cuda")
     D, H, W = want.shape[2:]
     for kd, kh, kw in np.ndindex(K):
-        for c in range(C):          # a product of two fp32 values is exact in 64 bits, so this rounds once, as an FMA does
+        for c in range(C):          # a product of two fp32 values is exact in 64 bits: one fp32 rounding a step, as in an FMA
             win = x[:, c, None, kd:kd + D, kh:kh + H, kw:kw + W].double()
             chain = (chain.double() + win * w[None, :, c, kd, kh, kw, None, None, None].double()).float()
     assert rel(y, want) <= 1.05 * rel(chain, want)
