@@ -1,6 +1,6 @@
 // conv3d / conv2d (cross-correlation, zero padding, any kernel extent, stride and padding per axis), fp32: the network and
 // single-layer drivers, and the implicit GEMM on the CUDA cores (bias, residual add and activation fused into the epilogue)
-// for the layers the split-TF32 kernel of fortis_mlp_f32tc.cu does not take.
+// for the layers the tensor-core kernel of fortis_conv3d_f32.cu does not take.
 //
 // Replaces the reference's cuDNN lowerings fortis_conv2d / fortis_conv3d (runtime/fortis_rt.c:108-156: descriptors
 // rebuilt every call, heuristic algorithm, workspace from the pool, bias / activation / residual as further kernels:
@@ -173,10 +173,12 @@ __device__ __forceinline__ void voxel_at(const ConvGeom& g, unsigned v, int* n, 
 }
 
 // FG: warps of a block that share their voxels and take FN channels each (1, 2 or 4, FG * FN <= 64)
+// vol.base: the output goes into a split volume (fortis_conv3d_f32.cu), for a network's next layer
+struct ShortVol { float* base; long long plane; int pitch, Dq, Hq, Wq, pd, ph, pw; };
 template <int V, int FN>
 __global__ void __launch_bounds__(256, 2) conv_short_kernel(const float* __restrict__ x, const float* __restrict__ wt,   // wt [tap][C][F]
                                                             const float* __restrict__ bias, const float* __restrict__ residual,
-                                                            float* __restrict__ y, ConvGeom g, int FG, int act, float slope) {
+                                                            float* __restrict__ y, ConvGeom g, int FG, int act, float slope, ShortVol vol) {
   extern __shared__ __align__(16) float sw[];                 // [Kp][FB] weights | [Kp] {element offset, bits a voxel needs}
   const int K = g.KD * g.KH * g.KW * g.C, Kp = (K + kShortStep - 1) / kShortStep * kShortStep, FB = FG * FN;
   uint2* tab = reinterpret_cast<uint2*>(sw + Kp * FB);
@@ -262,6 +264,25 @@ __global__ void __launch_bounds__(256, 2) conv_short_kernel(const float* __restr
     if (v >= nvox) break;
     int on, od, oh, ow;
     voxel_at(g, (unsigned)v, &on, &od, &oh, &ow);
+    if (vol.base) {
+      float* op = vol.base + ((((long long)on * vol.Dq + od + vol.pd) * vol.Hq + oh + vol.ph) * vol.Wq + ow + vol.pw) * vol.pitch + ff;
+#pragma unroll
+      for (int j = 0; j < FN; j += 4) {
+        if (ff + j >= vol.pitch) break;
+        float h[4], l[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const int f = ff + j + e;
+          float o = (((j + e) & 1) ? acc[i][(j + e) / 2].y : acc[i][(j + e) / 2].x) + (bias && f < g.F ? __ldg(bias + f) : 0.f);
+          if (act == ACT_RELU) o = max_nan(o, 0.f);
+          else if (act == ACT_LEAKY) o = o > 0.f ? o : o * slope;
+          vol_split(f < g.F ? o : 0.f, h[e], l[e]);
+        }
+        *reinterpret_cast<float4*>(op + j) = make_float4(h[0], h[1], h[2], h[3]);
+        *reinterpret_cast<float4*>(op + vol.plane + j) = make_float4(l[0], l[1], l[2], l[3]);
+      }
+      continue;
+    }
     float* yp = y + ((long long)on * g.ys_n + (long long)od * g.ys_d + (long long)oh * g.ys_h + (long long)ow * g.ys_w);
     const float* rp = residual ? residual + ((long long)on * g.rs_n + (long long)od * g.rs_d + (long long)oh * g.rs_h + (long long)ow * g.rs_w) : nullptr;
 #pragma unroll
@@ -286,23 +307,24 @@ bool short_supported(const ConvGeom& g) {
 
 template <int V, int FN>
 void launch_short_as(const float* x, const float* wt, const float* bias, const float* residual, float* y, const ConvGeom& g, int act,
-                     float slope, cudaStream_t s) {
+                     float slope, const ShortVol& vol, cudaStream_t s) {
   const long long nvox = (long long)g.N * g.Do * g.Ho * g.Wo;
-  const int groups = (g.F + FN - 1) / FN, FG = groups > 2 && FN < 32 ? 4 : groups > 1 ? 2 : 1, FB = FG * FN, per_block = 32 * V * (8 / FG);
+  const int F = vol.base ? (g.F + 31) / 32 * 32 : g.F;         // a split volume's channels come in blocks of 32
+  const int groups = (F + FN - 1) / FN, FG = groups > 2 && FN < 32 ? 4 : groups > 1 ? 2 : 1, FB = FG * FN, per_block = 32 * V * (8 / FG);
   const int K = g.KD * g.KH * g.KW * g.C, Kp = (K + kShortStep - 1) / kShortStep * kShortStep;
-  const dim3 grid((unsigned)((nvox + per_block - 1) / per_block), (unsigned)((g.F + FB - 1) / FB));
-  conv_short_kernel<V, FN><<<grid, 256, (size_t)Kp * (FB * 4 + 8), s>>>(x, wt, bias, residual, y, g, FG, act, slope);
+  const dim3 grid((unsigned)((nvox + per_block - 1) / per_block), (unsigned)((F + FB - 1) / FB));
+  conv_short_kernel<V, FN><<<grid, 256, (size_t)Kp * (FB * 4 + 8), s>>>(x, wt, bias, residual, y, g, FG, act, slope, vol);
 }
 
 // More voxels and channels a thread: fewer loads, tests and weight reads per product; fewer: more warps in flight.  The most
 // voxels that leave 12 warps an SM, at most 64 outputs a thread.
 void launch_short(const float* x, const float* wt, const float* bias, const float* residual, float* y, const ConvGeom& g, int act,
-                  float slope, cudaStream_t s) {
+                  float slope, const ShortVol& vol, cudaStream_t s) {
   const long long nvox = (long long)g.N * g.Do * g.Ho * g.Wo;
   const int FN = g.F <= 4 ? 4 : g.F <= 8 ? 8 : (g.F + 31) / 32 * 2 == (g.F + 15) / 16 ? 32 : 16;   // 32 where that pads no more
   const long long warps1 = (nvox + 31) / 32 * ((g.F + FN - 1) / FN), enough = 148 * 12;
   const int V = warps1 >= 4 * enough && FN <= 16 ? 4 : warps1 >= 2 * enough ? 2 : 1;
-#define FORTIS_SHORT_CASE(A, B) if (V == A && FN == B) return launch_short_as<A, B>(x, wt, bias, residual, y, g, act, slope, s);
+#define FORTIS_SHORT_CASE(A, B) if (V == A && FN == B) return launch_short_as<A, B>(x, wt, bias, residual, y, g, act, slope, vol, s);
   FORTIS_SHORT_CASE(4, 4) FORTIS_SHORT_CASE(2, 4) FORTIS_SHORT_CASE(1, 4)
   FORTIS_SHORT_CASE(4, 8) FORTIS_SHORT_CASE(2, 8) FORTIS_SHORT_CASE(1, 8)
   FORTIS_SHORT_CASE(4, 16) FORTIS_SHORT_CASE(2, 16) FORTIS_SHORT_CASE(1, 16)
@@ -314,7 +336,7 @@ void launch_conv(const float* x, const float* wt, const float* bias, const float
                  float slope, cudaStream_t s) {
   const long long nvox = (long long)g.N * g.Do * g.Ho * g.Wo;
   if (nvox <= 0) return;
-  if (short_supported(g)) return launch_short(x, wt, bias, residual, y, g, act, slope, s);
+  if (short_supported(g)) return launch_short(x, wt, bias, residual, y, g, act, slope, ShortVol{}, s);
   dim3 grid((unsigned)((nvox + CBM - 1) / CBM), (unsigned)((g.F + CBN - 1) / CBN));
   conv3d_f32_kernel<<<grid, 256, 0, s>>>(x, wt, bias, residual, y, g, act, slope);
 }
@@ -339,16 +361,16 @@ std::vector<float> repack_weights_taps(const float* w, int F, int C, int taps) {
   return out;
 }
 
-// One layer's weights on the device: [tap][C][F] for the FFMA kernel and, where the tensor-core kernel may take the layer,
+// One layer's weights on the device: [tap][C][F] for the FFMA kernels and, where the tensor-core kernel may take the layer,
 // split for that one.  (Which of the two runs depends on the volume's extents too, so both stay.)
-struct LayerDev { float *wt = nullptr, *bias = nullptr; F32ConvW* split = nullptr; };
-bool upload_layer(const LayerHost& L, int taps, bool split, LayerDev* d, std::string* err) {
+struct LayerDev { float *wt = nullptr, *bias = nullptr; VolW* vw = nullptr; };
+bool upload_layer(const LayerHost& L, int taps, bool split, bool line, LayerDev* d, std::string* err) {
   split = split && (long long)L.cin * taps >= kF32TcConvMinProducts;
   const std::vector<float> wt = repack_weights_taps(L.W.data(), L.cout, L.cin, taps);
   float* raw = nullptr;
   auto fail = [&](const char* why) {
     if (err) *err = why;
-    cudaFree(d->wt); cudaFree(d->bias); cudaFree(raw); f32tc_conv_free(d->split);
+    cudaFree(d->wt); cudaFree(d->bias); cudaFree(raw); vol_weights_free(d->vw);
     cudaGetLastError();
     *d = LayerDev();
     return false;
@@ -359,18 +381,54 @@ bool upload_layer(const LayerHost& L, int taps, bool split, LayerDev* d, std::st
   if (!split) return true;
   if (cudaMalloc(&raw, L.W.size() * 4) != cudaSuccess) return fail("out of device memory for conv weights");
   cudaMemcpy(raw, L.W.data(), L.W.size() * 4, cudaMemcpyHostToDevice);
-  d->split = f32tc_conv_pack(raw, L.cout, L.cin, taps, 0, nullptr);
-  if (!d->split || cudaStreamSynchronize(0) != cudaSuccess) return fail("out of device memory for split conv weights");
+  d->vw = vol_weights_pack(raw, L.cout, L.cin, taps, line, 0, nullptr);
+  if (!d->vw || cudaStreamSynchronize(0) != cudaSuccess) return fail("out of device memory for split conv weights");
   cudaFree(raw);
   return true;
 }
 
-// A layer takes the tensor-core kernel wherever it can and its sums are long enough (f32tc_conv_supported: no input dilation,
-// up to 32 taps per axis, a table of taps and channels that fits shared memory, kF32TcConvMinProducts): 14-layer network,
-// 2 x 33^3 voxels, 2.02 ms against 8.75 on the FFMA kernel; 32 -> 64 channels on 40^3 73 us against 297.
-bool conv_layer(const F32ConvW* split, const float* wt, const float* bias, const float* x, const float* residual, float* y, const ConvGeom& g,
-                int act, float slope, int* status, cudaStream_t s, std::string* err) {
-  if (split && f32tc_conv_supported(g)) return f32tc_conv(split, x, bias, residual, y, g, act, slope, status, s, true, err);
+// The split volume of a layer whose input is a plain array.  One buffer for all such calls: they follow one another on the
+// library's one stream.  It grows to the largest call; a buffer that a captured graph addresses is not freed.
+float* vol_workspace(size_t bytes, cudaStream_t s) {
+  static float* buf = nullptr;
+  static size_t cap = 0;
+  static bool captured = false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(s, &cs);
+  const bool capturing = cs != cudaStreamCaptureStatusNone;
+  if (cap < bytes) {
+    if (buf && !captured && !capturing) { cudaStreamSynchronize(s); cudaFree(buf); }
+    buf = nullptr; cap = 0; captured = false;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // an allocation is no stream operation: allowed beside a capture
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const bool ok = cudaMalloc(&buf, bytes) == cudaSuccess;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (!ok) { cudaGetLastError(); buf = nullptr; return nullptr; }
+    cap = bytes;
+  }
+  if (capturing) captured = true;
+  return buf;
+}
+
+// A layer takes the tensor-core kernel wherever it can and its sums are long enough (vol_supported), unless its split volume
+// does not fit the device.
+bool conv_layer(const VolW* vw, const float* wt, const float* bias, const float* x, const VolSource* src, const float* residual, float* y,
+                const ConvGeom& g, int act, float slope, int* status, cudaStream_t s, bool early, std::string* err) {
+  if (vw && vol_supported(g)) {
+    const VolGeom vg = vol_geom(g, g.pd, g.ph, vol_front_w(g));
+    const int pitch = (g.C + 31) / 32 * 32;
+    float* vol = vol_workspace(vol_bytes(vg, pitch), s);
+    if (vol) {
+      const VolSource plain = {VolSource::PLAIN, 1, 1, 1, 1, g.xs_n, g.xs_d, g.xs_h, g.xs_w, g.xs_c};
+      vol_pack(x, vol, pitch, vg, src ? *src : plain, s);
+      VolOut o;
+      std::memset(&o, 0, sizeof o);
+      o.y = y; o.ys_n = g.ys_n; o.ys_d = g.ys_d; o.ys_h = g.ys_h; o.ys_w = g.ys_w; o.ys_c = g.ys_c;
+      o.res = residual; o.rs_n = g.rs_n; o.rs_d = g.rs_d; o.rs_h = g.rs_h; o.rs_w = g.rs_w; o.rs_c = g.rs_c;
+      return vol_conv(vw, vol, pitch, vg, o, bias, act, slope, status, s, early, err);
+    }
+  }
+  if (src || !wt) { if (err) *err = "out of device memory for a convolution's input"; return false; }
   launch_conv(x, wt, bias, residual, y, g, act, slope, s);
   return true;
 }
@@ -411,7 +469,7 @@ __global__ void upsample_nearest2d_kernel(const float* __restrict__ x, float* __
 struct OpNet {
   std::vector<LayerHost> meta;
   std::vector<float*> wt, bias;           // per layer (null for layers without weights)
-  std::vector<F32ConvW*> split;           // the weights as the tensor-core kernel takes them (null for layers without weights)
+  std::vector<VolW*> vw;                  // the weights as the tensor-core kernel takes them (null for layers without weights)
   float* buf[2] = {nullptr, nullptr};
   long long cap = 0;
 };
@@ -420,7 +478,7 @@ void opnet_destroy(OpNet* m) {
   if (!m) return;
   for (float* p : m->wt) cudaFree(p);
   for (float* p : m->bias) cudaFree(p);
-  for (F32ConvW* p : m->split) f32tc_conv_free(p);
+  for (VolW* p : m->vw) vol_weights_free(p);
   for (float* p : m->buf) cudaFree(p);
   delete m;
 }
@@ -460,13 +518,25 @@ OpNet* opnet_create(const ModelHost& M, std::string* err) {
     LayerHost meta = L; meta.W.clear(); meta.b.clear();
     m->meta.push_back(meta);
     LayerDev d;
-    if (L.kind == LAYER_CONV2D && !upload_layer(L, L.kh * L.kw, L.dil == 1, &d, err)) {
+    if (L.kind == LAYER_CONV2D && !upload_layer(L, L.kh * L.kw, L.dil == 1, L.kw == 3 && L.sw == 1 && L.pw <= 1, &d, err)) {
       opnet_destroy(m);
       return nullptr;
     }
-    m->wt.push_back(d.wt); m->bias.push_back(d.bias); m->split.push_back(d.split);
+    m->wt.push_back(d.wt); m->bias.push_back(d.bias); m->vw.push_back(d.vw);
   }
   return m;
+}
+
+static ConvGeom opnet_geom(const LayerHost& L, int N, int h, int w, int h2, int w2) {
+  ConvGeom g;
+  std::memset(&g, 0, sizeof g);
+  g.N = N; g.D = 1; g.H = h; g.W = w; g.C = L.cin; g.F = L.cout;
+  g.KD = 1; g.KH = L.kh; g.KW = L.kw; g.pd = 0; g.ph = L.ph; g.pw = L.pw; g.sd = 1; g.sh = L.sh; g.sw = L.sw;
+  g.dd = 1; g.dh = g.dw = L.dil;
+  g.Do = 1; g.Ho = h2; g.Wo = w2;
+  g.xs_w = 1; g.xs_h = w; g.xs_d = (long long)h * w; g.xs_c = (long long)h * w; g.xs_n = (long long)L.cin * h * w;
+  g.ys_w = 1; g.ys_h = w2; g.ys_d = (long long)h2 * w2; g.ys_c = (long long)h2 * w2; g.ys_n = (long long)L.cout * h2 * w2;
+  return g;
 }
 
 // x (N, Cin, H, W) -> y (N, Cout, Ho, Wo)
@@ -491,6 +561,8 @@ bool opnet_forward(OpNet* m, const float* x, float* y, int N, int H, int W, int*
     m->cap = mx;
   }
   const float* src = x;
+  VolSource pending;                      // pooling or upsampling left to the next layer
+  pending.op = VolSource::PLAIN;
   int h = H, w = W;
   const int nl = (int)m->meta.size();
   for (int l = 0; l < nl; l++) {
@@ -501,18 +573,24 @@ bool opnet_forward(OpNet* m, const float* x, float* y, int N, int H, int W, int*
     const long long planes = (long long)N * L.cin, nout = (long long)N * L.cout * h2 * w2;
     const unsigned blocks = (unsigned)((nout + 255) / 256 < 148 * 16 ? (nout + 255) / 256 : 148 * 16);
     if (L.kind == LAYER_CONV2D) {
-      ConvGeom g;
-      g.N = N; g.D = 1; g.H = h; g.W = w; g.C = L.cin; g.F = L.cout;
-      g.KD = 1; g.KH = L.kh; g.KW = L.kw; g.pd = 0; g.ph = L.ph; g.pw = L.pw; g.sd = 1; g.sh = L.sh; g.sw = L.sw;
-      g.dd = 1; g.dh = g.dw = L.dil;
-      g.Do = 1; g.Ho = h2; g.Wo = w2;
-      g.xs_w = 1; g.xs_h = w; g.xs_d = (long long)h * w; g.xs_c = (long long)h * w; g.xs_n = (long long)L.cin * h * w;
-      g.ys_w = 1; g.ys_h = w2; g.ys_d = (long long)h2 * w2; g.ys_c = (long long)h2 * w2; g.ys_n = (long long)L.cout * h2 * w2;
-      if (!conv_layer(m->split[l], m->wt[l], m->bias[l], src, nullptr, dst, g, L.act, L.slope, status, s, err)) return false;
-    } else if (L.kind == LAYER_MAXPOOL2D) {
-      maxpool2d_kernel<<<blocks, 256, 0, s>>>(src, dst, planes, h, w, L.kh, L.kw, L.sh, L.sw, h2, w2);
+      const ConvGeom g = opnet_geom(L, N, h, w, h2, w2);
+      if (!conv_layer(m->vw[l], m->wt[l], m->bias[l], src, pending.op ? &pending : nullptr, nullptr, dst, g, L.act, L.slope, status, s, true, err)) return false;
+      pending.op = VolSource::PLAIN;
     } else {
-      upsample_nearest2d_kernel<<<blocks, 256, 0, s>>>(src, dst, planes, h, w, L.sh, L.sw);
+      const bool pool = L.kind == LAYER_MAXPOOL2D;
+      // a convolution behind this layer that packs its input pools or repeats on the way
+      int h3, w3;
+      if (l + 1 < nl && m->meta[l + 1].kind == LAYER_CONV2D && m->vw[l + 1] && opnet_layer_shape(m->meta[l + 1], h2, w2, &h3, &w3)) {
+        const ConvGeom g = opnet_geom(m->meta[l + 1], N, h2, w2, h3, w3);
+        if (vol_supported(g) && vol_workspace(vol_bytes(vol_geom(g, 0, g.ph, vol_front_w(g)), (g.C + 31) / 32 * 32), s)) {
+          pending = VolSource{pool ? VolSource::MAXPOOL : VolSource::UPSAMPLE, pool ? L.kh : L.sh, pool ? L.kw : L.sw, L.sh, L.sw,
+                              (long long)L.cin * h * w, (long long)h * w, w, 1, (long long)h * w};
+          h = h2; w = w2;
+          continue;
+        }
+      }
+      if (pool) maxpool2d_kernel<<<blocks, 256, 0, s>>>(src, dst, planes, h, w, L.kh, L.kw, L.sh, L.sw, h2, w2);
+      else upsample_nearest2d_kernel<<<blocks, 256, 0, s>>>(src, dst, planes, h, w, L.sh, L.sw);
     }
     src = dst; h = h2; w = w2;
   }
@@ -525,9 +603,10 @@ struct ConvModel {
   ConvTcModel* tcm = nullptr;           // bf16 tensor-core network (precision bf16); the fields below serve fp32
   std::vector<LayerHost> meta;          // shapes and flags (weights dropped after upload)
   std::vector<float*> wt, bias;
-  std::vector<F32ConvW*> split;
+  std::vector<VolW*> vw;
   float *buf[3] = {nullptr, nullptr, nullptr};
-  long long buf_elems = 0;
+  size_t buf_bytes = 0;
+  int shape[4] = {0, 0, 0, 0};          // of the split volumes in buf, whose padding is zero (shape[0] = 0: none)
 };
 
 void conv_model_destroy(ConvModel* m) {
@@ -535,7 +614,7 @@ void conv_model_destroy(ConvModel* m) {
   conv_tc_destroy(m->tcm);
   for (float* p : m->wt) cudaFree(p);
   for (float* p : m->bias) cudaFree(p);
-  for (F32ConvW* p : m->split) f32tc_conv_free(p);
+  for (VolW* p : m->vw) vol_weights_free(p);
   for (float* p : m->buf) cudaFree(p);
   delete m;
 }
@@ -558,17 +637,105 @@ ConvModel* conv_model_create(const ModelHost& M, int precision, cudaStream_t s, 
     meta.W.clear(); meta.b.clear();
     m->meta.push_back(meta);
     LayerDev d;
-    if (!upload_layer(L, L.ksize * L.ksize * L.ksize, true, &d, err)) {
+    if (!upload_layer(L, L.ksize * L.ksize * L.ksize, true, L.ksize == 3 && L.pad == 1, &d, err)) {
       conv_model_destroy(m);
       return nullptr;
     }
-    m->wt.push_back(d.wt); m->bias.push_back(d.bias); m->split.push_back(d.split);
+    m->wt.push_back(d.wt); m->bias.push_back(d.bias); m->vw.push_back(d.vw);
   }
   return m;
 }
 
 // x (N, D, H, W, Cin) -> y (N, D, H, W, Cout); every layer keeps the spatial extent (pad = K / 2)
-// Between the layers the volumes are channel-major (NCDHW): one thread per voxel then loads and stores whole lines.
+static ConvGeom conv_geom(const LayerHost& L, int N, int D, int H, int W) {
+  ConvGeom g;
+  std::memset(&g, 0, sizeof g);
+  g.N = N; g.D = D; g.H = H; g.W = W; g.C = L.cin; g.F = L.cout;
+  g.KD = g.KH = g.KW = L.ksize; g.pd = g.ph = g.pw = L.pad; g.sd = g.sh = g.sw = 1; g.dd = g.dh = g.dw = 1;
+  g.Do = D; g.Ho = H; g.Wo = W;
+  return g;
+}
+static void set_strides(long long* n, long long* d, long long* h, long long* w, long long* c, bool channels_last, int C, int D, int H, int W) {
+  const long long vox = (long long)D * H * W, step = channels_last ? C : 1;
+  *c = channels_last ? 1 : vox; *w = step; *h = W * step; *d = (long long)H * W * step; *n = vox * C;
+}
+
+// A network whose layers behind the first all run on the tensor cores: every volume between them is a split volume of one grid
+// (zeros in front for the widest kernel), written by one layer as the next one reads it.  The first layer packs the input, or is a
+// short one that writes such a volume.  False where the network is not of that kind; *ok: how the call went.
+static bool conv_forward_volumes(ConvModel* m, const float* x, float* y, int N, int D, int H, int W, int* status, cudaStream_t s, bool* ok, std::string* err) {
+  const int nl = (int)m->meta.size();
+  int pad = 0, pad_w = 0, cmax = 0;
+  for (int l = 0; l < nl; l++) {
+    pad = m->meta[l].pad > pad ? m->meta[l].pad : pad;
+    const int fw = vol_front_w(conv_geom(m->meta[l], N, D, H, W));
+    if (l > 0 || m->vw[0]) pad_w = fw > pad_w ? fw : pad_w;
+    if (l < nl - 1 && m->meta[l].cout > cmax) cmax = m->meta[l].cout;
+  }
+  for (int l = 0; l < nl; l++) {
+    const LayerHost& L = m->meta[l];
+    ConvGeom g = conv_geom(L, N, D, H, W);
+    set_strides(&g.xs_n, &g.xs_d, &g.xs_h, &g.xs_w, &g.xs_c, true, L.cin, D, H, W);
+    if (!(m->vw[l] && vol_supported(g)) && !(l == 0 && nl > 1 && short_supported(g))) return false;
+    if (l == nl - 1 && (L.flags & (LFLAG_ADD_SKIP | LFLAG_SAVE_SKIP))) return false;
+    if (l == 0 && (L.flags & LFLAG_ADD_SKIP)) return false;
+    if ((long long)(D + pad) * (H + pad) * (W + pad) * N >= (1LL << 30)) return false;
+  }
+  const int pitch = (cmax + 31) / 32 * 32;
+  const size_t bytes = nl > 1 ? vol_bytes(vol_geom(conv_geom(m->meta[0], N, D, H, W), pad, pad, pad_w), pitch) : 0;
+  if (m->buf_bytes < bytes) {
+    for (float*& p : m->buf) { cudaFree(p); p = nullptr; }
+    m->buf_bytes = 0; m->shape[0] = 0;
+    for (float*& p : m->buf)
+      if (cudaMalloc(&p, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        for (float*& q : m->buf) { cudaFree(q); q = nullptr; }
+        return false;                                            // plain volumes take half as much
+      }
+    m->buf_bytes = bytes;
+  }
+  if (bytes && (m->shape[0] != N || m->shape[1] != D || m->shape[2] != H || m->shape[3] != W)) {
+    for (float* p : m->buf) cudaMemsetAsync(p, 0, bytes, s);     // the layers keep the padding zero from here on
+    m->shape[0] = N; m->shape[1] = D; m->shape[2] = H; m->shape[3] = W;
+  }
+  int cur = -1, skip = -1;
+  *ok = true;
+  for (int l = 0; l < nl && *ok; l++) {
+    const LayerHost& L = m->meta[l];
+    ConvGeom g = conv_geom(L, N, D, H, W);
+    set_strides(&g.xs_n, &g.xs_d, &g.xs_h, &g.xs_w, &g.xs_c, true, L.cin, D, H, W);
+    int dst = -1;
+    for (int b = 0; b < 3 && dst < 0; b++) if (b != cur && b != skip) dst = b;
+    if ((L.flags & LFLAG_ADD_SKIP) && skip < 0) { *ok = false; if (err) *err = "conv3d model: a layer adds a skip that was never saved"; return true; }
+    const VolGeom vg = vol_geom(g, pad, pad, pad_w);
+    VolOut o;
+    std::memset(&o, 0, sizeof o);
+    if (l < nl - 1) { o.vol = m->buf[dst]; o.pitch = pitch; o.skip = (L.flags & LFLAG_ADD_SKIP) ? m->buf[skip] : nullptr; }
+    else { o.y = y; set_strides(&o.ys_n, &o.ys_d, &o.ys_h, &o.ys_w, &o.ys_c, true, L.cout, D, H, W); }
+    if (l == 0 && !(m->vw[0] && vol_supported(g))) {
+      const ShortVol sv = {o.vol, vg.P * pitch, pitch, vg.Dq, vg.Hq, vg.Wq, pad, pad, pad_w};
+      launch_short(x, m->wt[0], m->bias[0], nullptr, nullptr, g, L.act, L.slope, sv, s);
+    } else {
+      const float* in = cur < 0 ? nullptr : m->buf[cur];
+      int in_pitch = pitch;
+      if (l == 0) {
+        in_pitch = (L.cin + 31) / 32 * 32;
+        float* vol = vol_workspace(vol_bytes(vg, in_pitch), s);
+        if (!vol) { *ok = false; if (err) *err = "out of device memory for conv activations"; return true; }
+        const VolSource src = {VolSource::PLAIN, 1, 1, 1, 1, g.xs_n, g.xs_d, g.xs_h, g.xs_w, g.xs_c};
+        vol_pack(x, vol, in_pitch, vg, src, s);
+        in = vol;
+      }
+      *ok = vol_conv(m->vw[l], in, in_pitch, vg, o, m->bias[l], L.act, L.slope, status, s, true, err);
+    }
+    if (L.flags & LFLAG_SAVE_SKIP) skip = dst;
+    cur = dst;
+  }
+  return true;
+}
+
+// Other networks: plain volumes between the layers, channel-major (NCDHW), so that one thread per voxel loads and stores whole
+// lines.
 bool conv_forward(ConvModel* m, const float* x, float* y, int N, int D, int H, int W, int* status, cudaStream_t s, std::string* err) {
   if (m->tcm) return conv_tc_forward(m->tcm, x, y, N, D, H, W, s, err);
   const long long nvox = (long long)N * D * H * W;
@@ -578,11 +745,20 @@ bool conv_forward(ConvModel* m, const float* x, float* y, int N, int D, int H, i
     if (L.pad * 2 + 1 != L.ksize) { if (err) *err = "conv3d model layers must keep the spatial extent (pad = K / 2)"; return false; }
     cmax = L.cout > cmax ? L.cout : cmax;
   }
-  if (m->buf_elems < nvox * cmax) {
+  bool ok = true;
+  if (conv_forward_volumes(m, x, y, N, D, H, W, status, s, &ok, err)) {
+    if (!ok) return false;
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) { if (err) *err = std::string("conv3d launch: ") + cudaGetErrorString(e); return false; }
+    return true;
+  }
+  m->shape[0] = 0;
+  if (m->buf_bytes < (size_t)nvox * cmax * 4) {
     for (float*& p : m->buf) { cudaFree(p); p = nullptr; }
+    m->buf_bytes = 0;
     for (float*& p : m->buf)
       if (cudaMalloc(&p, (size_t)nvox * cmax * 4) != cudaSuccess) { if (err) *err = "out of device memory for conv activations"; return false; }
-    m->buf_elems = nvox * cmax;
+    m->buf_bytes = (size_t)nvox * cmax * 4;
   }
   const float* src = x;
   const float* skip = nullptr;
@@ -596,18 +772,13 @@ bool conv_forward(ConvModel* m, const float* x, float* y, int N, int D, int H, i
       for (int b = 0; b < 3; b++)
         if (m->buf[b] != src && b != skip_buf) { dst = m->buf[b]; dst_buf = b; break; }
     }
-    ConvGeom g;
-    g.N = N; g.D = D; g.H = H; g.W = W; g.C = L.cin; g.F = L.cout;
-    g.KD = g.KH = g.KW = L.ksize; g.pd = g.ph = g.pw = L.pad; g.sd = g.sh = g.sw = 1; g.dd = g.dh = g.dw = 1;
-    g.Do = D; g.Ho = H; g.Wo = W;
-    const long long vox = (long long)D * H * W;
-    const long long xc = l == 0 ? L.cin : 1, yc = l == nl - 1 ? L.cout : 1;      // channels per voxel step: NDHWC at both ends
-    g.xs_c = l == 0 ? 1 : vox; g.xs_w = xc; g.xs_h = W * xc; g.xs_d = (long long)H * W * xc; g.xs_n = vox * L.cin;
-    g.ys_c = l == nl - 1 ? 1 : vox; g.ys_w = yc; g.ys_h = W * yc; g.ys_d = (long long)H * W * yc; g.ys_n = vox * L.cout;
-    g.rs_c = vox; g.rs_w = 1; g.rs_h = W; g.rs_d = (long long)H * W; g.rs_n = vox * L.cout;     // a skip is a layer's output, channel-major
+    ConvGeom g = conv_geom(L, N, D, H, W);
+    set_strides(&g.xs_n, &g.xs_d, &g.xs_h, &g.xs_w, &g.xs_c, l == 0, L.cin, D, H, W);          // NDHWC at both ends
+    set_strides(&g.ys_n, &g.ys_d, &g.ys_h, &g.ys_w, &g.ys_c, l == nl - 1, L.cout, D, H, W);
+    set_strides(&g.rs_n, &g.rs_d, &g.rs_h, &g.rs_w, &g.rs_c, false, L.cout, D, H, W);          // a skip is a layer's output, channel-major
     const float* res = (L.flags & LFLAG_ADD_SKIP) ? skip : nullptr;
     if ((L.flags & LFLAG_ADD_SKIP) && !skip) { if (err) *err = "conv3d model: a layer adds a skip that was never saved"; return false; }
-    if (!conv_layer(m->split[l], m->wt[l], m->bias[l], src, res, dst, g, L.act, L.slope, status, s, err)) return false;
+    if (!conv_layer(m->vw[l], m->wt[l], m->bias[l], src, nullptr, res, dst, g, L.act, L.slope, status, s, true, err)) return false;
     if (L.flags & LFLAG_SAVE_SKIP) { skip = dst; skip_buf = dst_buf; }
     src = dst;
   }
@@ -626,7 +797,8 @@ bool conv3d_ncdhw(const float* x, const float* w, float* y, int N, int C, int D,
   // freed and replaced.  A weight seen for the first time needs a buffer: that cannot happen while the stream is being
   // captured into a graph, so such a call is refused (the reference captures on the second call for the same reason: the
   // first call allocates).
-  struct Cached { const float* w; int F, C, taps; float* wt; F32ConvW* split; bool captured; };
+  // vw: the forms for layers that take a tap at a time and, of kernels three wide, a line's taps at a time: stride and padding decide
+  struct Cached { const float* w; int F, C, taps; float* wt; VolW* vw[2]; bool captured; };
   static std::vector<Cached> cache;
   static size_t victim = 0;
   const int taps = K[0] * K[1] * K[2];
@@ -638,7 +810,10 @@ bool conv3d_ncdhw(const float* x, const float* w, float* y, int N, int C, int D,
   g.Do = (D + 2 * pad[0] - K[0]) / stride[0] + 1; g.Ho = (H + 2 * pad[1] - K[1]) / stride[1] + 1; g.Wo = (W + 2 * pad[2] - K[2]) / stride[2] + 1;
   g.xs_w = 1; g.xs_h = W; g.xs_d = (long long)H * W; g.xs_c = (long long)D * H * W; g.xs_n = (long long)C * D * H * W;
   g.ys_w = 1; g.ys_h = g.Wo; g.ys_d = (long long)g.Ho * g.Wo; g.ys_c = (long long)g.Do * g.Ho * g.Wo; g.ys_n = (long long)F * g.Do * g.Ho * g.Wo;
-  const bool tc = f32tc_conv_supported(g);
+  const VolGeom vg = vol_geom(g, g.pd, g.ph, vol_front_w(g));
+  const int line = vg.line;
+  // the FFMA kernel, which needs no copy of x, where the copy does not fit the device
+  const bool tc = vol_supported(g) && vol_workspace(vol_bytes(vg, (C + 31) / 32 * 32), s) != nullptr;
   Cached* c = nullptr;
   bool fresh = false;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -646,27 +821,26 @@ bool conv3d_ncdhw(const float* x, const float* w, float* y, int N, int C, int D,
   const bool capturing = cs != cudaStreamCaptureStatusNone;
   for (auto& q : cache) if (q.w == w && q.F == F && q.C == C && q.taps == taps) c = &q;
   if (c && capturing) c->captured = true;
-  if (!c || (tc ? (void*)c->split : (void*)c->wt) == nullptr) {
+  if (!c || (tc ? (void*)c->vw[line] : (void*)c->wt) == nullptr) {
     if (capturing) { if (err) *err = "conv weights seen for the first time during graph capture; run one eager call first"; return false; }
     if (!c) {
       for (size_t i = 0; i < cache.size() && cache.size() >= 64 && !c; i++, victim = (victim + 1) % cache.size())
         if (!cache[victim].captured) c = &cache[victim];
-      if (c) { cudaStreamSynchronize(s); cudaFree(c->wt); f32tc_conv_free(c->split); }
+      if (c) { cudaStreamSynchronize(s); cudaFree(c->wt); vol_weights_free(c->vw[0]); vol_weights_free(c->vw[1]); }
       else { cache.push_back(Cached{}); c = &cache.back(); }
-      *c = Cached{w, F, C, taps, nullptr, nullptr, false};
+      *c = Cached{w, F, C, taps, nullptr, {nullptr, nullptr}, false};
     }
     const size_t n = (size_t)F * C * taps;
     if (tc) {
-      c->split = f32tc_conv_pack(w, F, C, taps, s, err);
-      if (!c->split) return false;
+      for (int form = 0; form < (K[2] == 3 ? 2 : 1); form++)
+        if (!c->vw[form] && !(c->vw[form] = vol_weights_pack(w, F, C, taps, form != 0, s, err))) return false;
     } else {
       if (cudaMalloc(&c->wt, n * 4) != cudaSuccess) { cudaGetLastError(); c->wt = nullptr; if (err) *err = "out of device memory for conv weights"; return false; }
       repack_weights_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(w, c->wt, F, C, taps);
     }
     fresh = true;
   }
-  if (tc) return f32tc_conv(c->split, x, nullptr, nullptr, y, g, ACT_NONE, 0.f, status, s, !fresh, err);
-  launch_conv(x, c->wt, nullptr, nullptr, y, g, ACT_NONE, 0.f, s);
+  if (!conv_layer(tc ? c->vw[line] : nullptr, c->wt, nullptr, x, nullptr, nullptr, y, g, ACT_NONE, 0.f, status, s, !fresh, err)) return false;
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { if (err) *err = std::string("conv3d launch: ") + cudaGetErrorString(e); return false; }
   return true;

@@ -1,0 +1,839 @@
+// fp32 convolutions on the tensor cores without threads in the operand path: y = act(conv(x, W) + b + residual) with every
+// product formed as three TF32 MMAs (x = x_hi + x_lo, W = W_hi + W_lo: hi.hi, hi.lo and lo.hi; the hi.hi sums taken over into
+// registers every 32 or 64 k with IEEE additions, the cross sums scaled by 2^10), both operands read from shared memory where the
+// TMA puts them.
+//
+// Replaces, for layers of 128 products and more, the reference's cuDNN lowerings fortis_conv2d / fortis_conv3d
+// (runtime/fortis_rt.c:108-156) and the further kernels for bias, residual and activation (compiler/FortisFuse.cpp:626-655).
+//
+// Activations lie in HBM as a SPLIT VOLUME: channels last, every value already split, [plane hi | lo][row][channels], one row per
+// position of a grid that holds the zero padding:
+//     row = ((n * Dq + d) * Hq + h) * Wq + w,      output (od, oh, ow) under tap (kd, kh, kw) reads row(out) + shift(tap)
+// For stride 1 a line's right padding is the next line's left padding (Wq = W + pad; the same for planes and volumes); for other
+// strides there is one such volume per residue of the position modulo the stride ("phase"), so that a tap is a shift again.  So an
+// operand tile is 128 consecutive rows, whatever the tap: no im2col, no masks, no bounds tests; rows that are padding are computed
+// too and written as zeros (the next layer's padding) or not at all.
+//
+//   * pairs of CTAs (cta_group::2), 128 rows each; a pair's leader issues the MMAs.  A stage of the activation ring holds the rows
+//     that all taps of one kd (or of one line, or one tap) read, 32 channels, hi and lo: taps read it through descriptors whose start
+//     address moves by whole rows (the 128-byte swizzle is a function of the address).
+//   * kernels three wide (LINE): one step multiplies the unshifted rows by the three taps of a line (N = 3 x 32 or 3 x 64 columns), and
+//     the epilogue adds the sums of neighbouring rows: an activation is read once for three taps, and lines need no padding.
+//     Others: one tap a step, x_hi . [W_hi | W_lo] as one MMA of twice the columns.
+//   * eight epilogue warps (thread = row, half of the features) hold the sums in registers and put finished rows into a stash in
+//     shared memory; four more warps add bias and residual, activate, split and store whole lines.
+// Bound: with 64 features the tensor core, 1152 clk a step of 3 taps x 32 channels, plus some 3000 clk at a tile's end, when the next
+// tile's second step waits for the epilogue (a step was measured at 1160); with few features and channels the tile's end.
+// Measured against the kernel before, whose threads loaded the taps and split them once per tap (a step of one tap 1240 clk): see
+// conv_layer in fortis_conv3d.cu.
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <cstdlib>
+#include <cstring>
+#include <string>
+#include <type_traits>
+
+#include "fortis_device.cuh"
+#include "fortis_kernels.h"
+#include "fortis_model.h"
+#include "fortis_tc.cuh"
+
+namespace fortis {
+
+namespace {
+
+using namespace tc;
+
+constexpr int kM = 128, kKt = 32;
+// The tensor core takes subnormal operands as zero: x_lo is stored times 2^10 (exact), so that it is normal wherever x is, and the
+// cross sums are multiplied by 2^-10.  Without it x_lo is lost from |x| < 2^-102 on (2^-118: error 2.2e-6).  (x_lo is below 2^-10 of
+// the largest value, so the product stays finite.)
+constexpr float kLoScale = 1024.f;
+// Steps of 32 k accumulated in the tensor core, which truncates, before the sums are taken over: two, or one where K is short (2-D
+// network of K = 27 to 576, six convolutions, error against 64 bits: two 9.1e-7, one 6.2e-7, FFMA 7.7e-7).  LINE: always one, at no
+// cost in time (14-layer network: 1.02e-6, with two 1.66e-6).
+constexpr int kChunkLong = 2, kChunkShort = 1, kShortK = 640;
+// warps: 0 activations, 1 weights (TMA), 2 and 3 MMA issuers, then the epilogue and the storers
+constexpr int kEWarps = 8, kWarpE0 = 4, kWarpS0 = kWarpE0 + kEWarps, kThreads = (kWarpS0 + 4) * 32;
+constexpr int kMaxStages = 8;
+constexpr int kBarBytes = 512;
+constexpr int kSmemMax = 227 * 1024;
+enum { VST_ALIGN = 31, VST_A_EMPTY = 32, VST_W_EMPTY = 33, VST_A_FULL = 34, VST_W_FULL = 35, VST_ACC_EMPTY = 36, VST_ACC_FULL = 37, VST_CROSS_FULL = 38,
+       VST_STASH_FULL = 39, VST_STASH_EMPTY = 40 };
+
+struct VolParams {
+  CUtensorMap amap;                            // [plane 2][row][channel], box 2 x box_rows x 32
+  CUtensorMap wmap;                            // [step][channel block][tile of features][CTA][row] rows of 32
+  VolGeom g;
+  int nchb, ntn, chunk_kt;
+  int ng, tpg, sub_w;                          // stages per channel block, steps per stage, steps of one line among them
+  int box_rows, a_stages, w_stages;
+  long long rows;                              // output rows up to the last one that is a real output
+  const float* bias; int act; float slope; int F;
+  // output: a split volume of the same grid (pitch: channels of a row) ...
+  float* out; long long out_plane; int out_pitch; long long out_shift;
+  const float* skip;                           // the residual, a split volume like `out`
+  // ... or a plain array, with a plain residual
+  float* y; long long ys_n, ys_d, ys_h, ys_w, ys_c;
+  const float* res; long long rs_n, rs_d, rs_h, rs_w, rs_c;
+  int* status;
+  unsigned int wait_limit; int test_skip_stage;
+};
+
+__host__ __device__ constexpr uint32_t idesc_tf32_pair(int n) {
+  return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)((2 * kM) >> 4) << 24);
+}
+// Low words of K-major 128-byte-swizzled shared-memory descriptors; the high word is the same for all of them
+constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_lo(uint32_t saddr) { return (saddr >> 4) & 0x3FFFu; }
+// D[tmem of both CTAs] (+)= A . B^T over a step of 32 k (FULL), or its first nk8 < 4 parts of 8 k (32 bytes of a row each), one
+// elected lane of the leader issues
+template <uint32_t IDESC, bool FULL>
+__device__ __forceinline__ void mma_step32(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t accumulate, int nk8) {
+  if constexpr (FULL)
+    asm volatile(
+        "{\n\t.reg .pred e, q;\n\t.reg .b64 a0, a1, a2, a3, b0, b1, b2, b3;\n\t"
+        "mov.b64 a0, {%1, %4};\n\tmov.b64 b0, {%2, %4};\n\t"
+        "add.s64 a1, a0, 2;\n\tadd.s64 b1, b0, 2;\n\tadd.s64 a2, a0, 4;\n\tadd.s64 b2, b0, 4;\n\tadd.s64 a3, a0, 6;\n\tadd.s64 b3, b0, 6;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\telect.sync _|e, 0xffffffff;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::tf32 [%0], a0, b0, %3, q;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::tf32 [%0], a1, b1, %3, 1;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::tf32 [%0], a2, b2, %3, 1;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::tf32 [%0], a3, b3, %3, 1;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "n"(IDESC), "n"(kDescHi), "r"(accumulate) : "memory");
+  else
+    for (int j = 0; j < nk8; j++)
+      asm volatile(
+          "{\n\t.reg .pred e, q;\n\t.reg .b64 a0, b0;\n\tmov.b64 a0, {%1, %4};\n\tmov.b64 b0, {%2, %4};\n\t"
+          "setp.ne.b32 q, %5, 0;\n\telect.sync _|e, 0xffffffff;\n\t"
+          "@e tcgen05.mma.cta_group::2.kind::tf32 [%0], a0, b0, %3, q;\n\t}"
+          ::"r"(d_tmem), "r"(a_lo + 2 * j), "r"(b_lo + 2 * j), "n"(IDESC), "n"(kDescHi), "r"(accumulate | (uint32_t)j) : "memory");
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {     // two IEEE additions
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
+  return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
+      "l"(*reinterpret_cast<unsigned long long*>(&c)));
+  return *reinterpret_cast<float2*>(&d);
+}
+// A bounded wait without a function call, which would empty the uniform registers and fix one register budget for all warps.  Every
+// lane of a warp goes on or gives up together; a CTA in which a wait has given up polls no more.
+__device__ __forceinline__ bool wait_polling(uint32_t bar, uint32_t parity, uint32_t limit, volatile int* abort_flag, int* status, int code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .u32 i;\n\tmov.u32 i, 0;\n"
+      "WAIT_LOOP_%=:\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "@p bra WAIT_DONE_%=;\n\t"
+      "add.u32 i, i, 1;\n\t"
+      "setp.lt.u32 q, i, %3;\n\t"
+      "@q bra WAIT_LOOP_%=;\n"
+      "WAIT_DONE_%=:\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok) : "r"(bar), "r"(parity), "r"(*abort_flag ? 1u : limit) : "memory");
+  if (__all_sync(0xffffffffu, ok)) return true;
+  if ((threadIdx.x & 31) == 0) {
+    *abort_flag = 1;
+    atomicCAS(status, 0, code);
+  }
+  return false;
+}
+__device__ __forceinline__ float4 ld_plain4(const float* p) {   // not read-only: the grid in front may have written it
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_plain(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t parity, uint32_t limit) {
+  for (uint32_t i = 0; i < limit; i++)
+    if (mbar_try_wait(bar, parity)) return;
+}
+
+// LINE: a step is the three taps of a line, and a tile has 126 output rows (the first and last computed ones only feed their
+// neighbours).  Otherwise a step is one tap.
+template <int NT, bool LINE> struct Form {
+  static constexpr int kTaps = LINE ? 3 : 1;
+  static constexpr int kRowsOut = LINE ? kM - 2 : kM, kHalo = LINE ? 1 : 0;
+  static constexpr int kWRows = LINE ? 3 * NT : NT;            // weight rows of a step held by one CTA, W_hi then W_lo
+  static constexpr int kWBytes = kWRows * kKt * 4, kWHalf = kWBytes / 2;
+  // tensor memory: two accumulators of kAcc columns, then the cross sums.  The accumulators take alternate chunks, or where there is
+  // no room for two (kHalves) 32 features each.
+  static constexpr bool kHalves = LINE && NT == 64;
+  static constexpr int kAcc = LINE ? 96 : 2 * NT, kCross = LINE ? 3 * NT : NT;
+  static constexpr uint32_t kColCross = 2 * kAcc;
+  static_assert(2 * kAcc + kCross <= 512, "tensor memory");
+  // LINE: a half's 96 rows (3 taps x 32 features) lie 48 in each CTA; the columns of the cross sums follow
+  static __device__ __forceinline__ int cross_col(int half, int n) { return kHalves ? (n < 48 ? half * 48 + n : half * 48 + n + 48) : n; }
+  static constexpr int kXchBytes = LINE ? 2 * 4 * NT * 4 : 0;          // rows exchanged between epilogue warps: [up | down][quadrant][feature]
+};
+
+// first row of stage g_ relative to the output row
+template <bool LINE>
+__device__ __forceinline__ long long stage_shift(const VolParams& P, int g_) {
+  const VolGeom& g = P.g;
+  const int nw = LINE ? 1 : g.KW, per_kd = P.tpg == g.KH * nw ? 1 : P.tpg == nw ? g.KH : g.KH * nw;      // stages of one kd
+  const int kd = g_ / per_kd, r = g_ - kd * per_kd, kh = per_kd == 1 ? 0 : P.tpg == nw ? r : r / nw, kw = P.tpg == 1 ? r % nw : 0;
+  const int phase = ((kd % g.sd) * g.fh + kh % g.sh) * g.fw + kw % g.sw;
+  return phase * g.P + ((long long)(g.od0 + kd / g.sd) * g.Hq + g.oh0 + kh / g.sh) * g.Wq + g.ow0 + (LINE ? 1 : kw / g.sw);
+}
+
+template <int NT, bool LINE>
+__global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vol_kernel(const __grid_constant__ VolParams P) {
+  using FM = Form<NT, LINE>;
+  constexpr int kWBytes = FM::kWBytes;
+  constexpr int NH = NT / 2;                                   // features per epilogue thread
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t base = smem_u32(smem);
+  if (base & 1023u) {                                          // the same in both CTAs of a pair
+    if (threadIdx.x == 0) atomicCAS(P.status, 0, VST_ALIGN);
+    return;
+  }
+  const uint32_t a_plane = (uint32_t)P.box_rows * kKt * 4, a_bytes = 2 * a_plane;
+  const uint32_t w_ring = base + P.a_stages * a_bytes, bars = w_ring + P.w_stages * kWBytes;
+  uint8_t* tail = smem + (bars - base);
+  // a_full [8] | a_empty [8] | w_full [8] | w_empty [8] | acc_full [2] | acc_empty [2] | cross_full | cross_empty | drained [2];
+  // at 320 the tensor-memory base, at 324 the abort flag, at 328 turn [8] | stash_full | stash_empty
+  const uint32_t a_full = bars, a_empty = bars + 64, w_full = bars + 128, w_empty = bars + 192, acc_full = bars + 256, acc_empty = bars + 272,
+                 cross_full = bars + 288, cross_empty = bars + 296, drained = bars + 304, turn = bars + 328, stash_full = bars + 392, stash_empty = bars + 400;
+  uint32_t* tmem_slot = (uint32_t*)(tail + 320);
+  volatile int* abort_flag = (volatile int*)(tail + 324);
+  // through a shuffle, so that the compiler knows the roles' branches, loops and addresses to be the same in a whole warp
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const uint32_t crank = cluster_ctarank();
+  const long long npairs = (P.rows + 2 * FM::kRowsOut - 1) / (2 * FM::kRowsOut), ntiles = npairs * P.ntn;
+  const long long t0 = blockIdx.x >> 1, t_step = gridDim.x >> 1;
+  const int nkt = P.ng * P.tpg * P.nchb;       // steps of a tile
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kMaxStages; s++) {
+      mbar_init(a_full + 8 * s, 1); mbar_init(a_empty + 8 * s, 2);
+      mbar_init(w_full + 8 * s, 1); mbar_init(w_empty + 8 * s, 2); mbar_init(turn + 8 * s, 1);
+    }
+    for (int s = 0; s < 2; s++) { mbar_init(acc_full + 8 * s, 1); mbar_init(acc_empty + 8 * s, FM::kHalves ? kEWarps : 2 * kEWarps); mbar_init(drained + 8 * s, 1); }
+    mbar_init(cross_full, 1); mbar_init(cross_empty, 2 * kEWarps); mbar_init(stash_full, kEWarps); mbar_init(stash_empty, 4);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0 && lane < 2)
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(lane ? &P.wmap : &P.amap)) : "memory");
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();                          // both CTAs' barriers exist before either signals the other's
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  // Programmatic dependent launch: the next layer's CTAs set up and load weights while this grid drains.  Not before both CTAs have
+  // their tensor memory.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+  auto wait = [&](uint32_t bar, uint32_t parity, int code) { return wait_polling(bar, parity, P.wait_limit, abort_flag, P.status, code); };
+  // The epilogue warps of the widest form hold 96 sums a thread and up to 96 loaded values.  56 x 256 + 200 x 256 = 128 x 512
+  // registers: what the block is launched with (checked before the launch).
+  if (warp < kWarpE0) {
+    if constexpr (FM::kHalves) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    if (warp == 0) {
+      // ---------------------------------------------------------------- TMA: activations, this CTA's rows
+      asm volatile("griddepcontrol.wait;" ::: "memory");        // what the kernel in front wrote is complete and visible
+      const uint32_t full0 = map_to_cta(a_full, 0);
+      uint32_t s = 0, ph = 0;
+      bool stop = false;
+      for (long long t = t0; t < ntiles && !stop; t += t_step) {
+        const long long m0 = (2 * (t / P.ntn) + crank) * FM::kRowsOut - FM::kHalo;
+        for (int g = 0; g < P.ng && !stop; g++) {
+          const int y0 = (int)(m0 + stage_shift<LINE>(P, g));
+          for (int cb = 0; cb < P.nchb; cb++) {
+            if (!wait(a_empty + 8 * s, ph ^ 1, VST_A_EMPTY)) { stop = true; break; }
+            const bool skip = P.test_skip_stage && blockIdx.x == 0 && t == t0 && g == 0 && cb == 0;    // test only: the stage never completes
+            if (crank == 0) mbar_expect_tx(a_full + 8 * s, 2 * a_bytes);
+            if (!skip) tma_load_3d_pair(base + s * a_bytes, &P.amap, cb * kKt, y0, 0, full0 + 8 * s);
+            if (++s == (uint32_t)P.a_stages) { s = 0; ph ^= 1; }
+          }
+        }
+      }
+      if (crank == 0)
+        for (uint32_t q = 0; q < (uint32_t)P.a_stages; q++) drain_wait(a_full + 8 * q, q < s ? ph : ph ^ 1, P.wait_limit);
+    } else if (warp == 1) {
+      // ---------------------------------------------------------------- TMA: weights, this CTA's half of the features
+      const uint32_t full0 = map_to_cta(w_full, 0);
+      uint32_t s = 0, ph = 0;
+      bool stop = false;
+      for (long long t = t0; t < ntiles && !stop; t += t_step) {
+        const int nt = (int)(t % P.ntn);
+        for (int g = 0; g < P.ng && !stop; g++)
+          for (int cb = 0; cb < P.nchb && !stop; cb++)
+            for (int tp = 0; tp < P.tpg; tp++) {
+              if (!wait(w_empty + 8 * s, ph ^ 1, VST_W_EMPTY)) { stop = true; break; }
+              if (crank == 0) mbar_expect_tx(w_full + 8 * s, 2 * kWBytes);
+              tma_load_2d_pair(w_ring + s * kWBytes, &P.wmap, 0, ((((g * P.tpg + tp) * P.nchb + cb) * P.ntn + nt) * 2 + (int)crank) * FM::kWRows, full0 + 8 * s);
+              if (++s == (uint32_t)P.w_stages) { s = 0; ph ^= 1; }
+            }
+      }
+      if (crank == 0)
+        for (uint32_t q = 0; q < (uint32_t)P.w_stages; q++) drain_wait(w_full + 8 * q, q < s ? ph : ph ^ 1, P.wait_limit);
+    } else if (crank == 0) {
+      // ---------------------------------------------------------------- MMA issuers (the leader's, for both CTAs).  A warp needs several
+      // hundred clocks for the waits, commits and counting of a step, in which it issues nothing, so two share a step: the first takes
+      // x_hi . [W_hi | W_lo], or with LINE x_hi . W_hi, into accumulators that the epilogue takes over chunk by chunk, the second the
+      // other cross products, each step when the first has issued its part: the cross products of a step then run while the epilogue
+      // takes over the sums (one warp: 1220 clk a step of 432 clk of MMAs; with LINE and no order the first waits for the epilogue
+      // behind the second's queued MMAs).
+      const uint32_t cross = tmem + FM::kColCross, line = (uint32_t)(P.g.Wq - P.sub_w + 1) * 8;
+      auto issue = [&](auto first_) {
+        constexpr bool kFirst = decltype(first_)::value;
+        uint32_t as = 0, aph = 0, ws = 0, wph = 0, chunk_it = 0, tile_it = 0;
+        for (long long t = t0; t < ntiles; t += t_step, tile_it++) {
+          int kt = 0, in_chunk = 0, cb = 0;
+          for (int st = P.ng * P.nchb; st > 0; st--) {
+            if (kFirst && !wait(a_full + 8 * as, aph, VST_A_FULL)) return;
+            const int left = P.g.C - cb * kKt, nk8 = left >= kKt ? 4 : (left + 7) >> 3;   // behind the last channel both operands are zero
+            if (++cb == P.nchb) cb = 0;
+            int dw = 0;
+            uint32_t row_ = desc_lo(base + as * a_bytes);        // the stage's row of the tile's first row under the present step
+            for (int tp = P.tpg; tp > 0; tp--, kt++) {
+              // the second follows the first: what the first has waited for is there
+              if (!wait((kFirst ? w_full : turn) + 8 * ws, wph, VST_W_FULL)) return;
+              // through shuffles: an MMA whose operands the compiler does not know to be the same in all lanes costs 18 clk and more
+              // to issue (7 otherwise)
+              const uint32_t row = __shfl_sync(0xffffffffu, row_, 0), wd = __shfl_sync(0xffffffffu, desc_lo(w_ring + ws * kWBytes), 0);
+              const uint32_t b = chunk_it & 1;
+              const bool ends = in_chunk + 1 == P.chunk_kt || kt == nkt - 1;
+              auto groups = [&](auto full_) {
+                constexpr bool kFull = decltype(full_)::value;
+                if constexpr (kFirst && FM::kHalves) {
+#pragma unroll
+                  for (int h = 0; h < 2; h++) {
+                    if (!wait(acc_empty + 8 * h, b ^ 1, VST_ACC_EMPTY)) return false;
+                    tc_fence_after();
+                    mma_step32<idesc_tf32_pair(FM::kAcc), kFull>(tmem + h * FM::kAcc, row, wd + h * (48 * 128 >> 4), 0u, nk8);
+                    tc_commit_pair(acc_full + 8 * h);
+                  }
+                } else if constexpr (kFirst) {
+                  if (in_chunk == 0 && !wait(acc_empty + 8 * b, ((chunk_it >> 1) & 1) ^ 1, VST_ACC_EMPTY)) return false;
+                  tc_fence_after();
+                  mma_step32<idesc_tf32_pair(FM::kAcc), kFull>(tmem + b * FM::kAcc, row, wd, (uint32_t)in_chunk, nk8);
+                  if (ends) tc_commit_pair(acc_full + 8 * b);
+                } else {
+                  if (kt == 0 && !wait(cross_empty, (tile_it & 1) ^ 1, VST_ACC_EMPTY)) return false;   // the previous tile's cross sums have been read
+                  tc_fence_after();
+                  if constexpr (LINE) mma_step32<idesc_tf32_pair(FM::kCross), kFull>(cross, row, wd + ((uint32_t)FM::kWHalf >> 4), (uint32_t)kt, nk8);
+                  mma_step32<idesc_tf32_pair(FM::kCross), kFull>(cross, row + (a_plane >> 4), wd, LINE ? 1u : (uint32_t)kt, nk8);
+                }
+                if constexpr (kFirst) {
+                  __syncwarp();
+                  if (lane == 0) mbar_arrive(turn + 8 * ws);
+                }
+                return true;
+              };
+              if (!(nk8 == 4 ? groups(std::true_type{}) : groups(std::false_type{}))) return;
+              if (ends) { chunk_it++; in_chunk = 0; } else in_chunk++;
+              tc_commit_pair(w_empty + 8 * ws);
+              if (++ws == (uint32_t)P.w_stages) { ws = 0; wph ^= 1; }
+              if (++dw == P.sub_w) { dw = 0; row_ += line; } else row_ += 8;
+            }
+            tc_commit_pair(a_empty + 8 * as);
+            if (++as == (uint32_t)P.a_stages) { as = 0; aph ^= 1; }
+          }
+          if constexpr (!kFirst) tc_commit_pair(cross_full);
+        }
+      };
+      if (warp == 2) issue(std::true_type{}); else issue(std::false_type{});
+      tc_commit_pair(drained + 8 * (warp - 2));                  // nothing may still read shared or tensor memory when the CTAs end
+      drain_wait(drained + 8 * (warp - 2), 0, P.wait_limit);
+    }
+  } else if (warp >= kWarpS0) {
+    if constexpr (FM::kHalves) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    // ------------------------------------------------------------------ storers: bias, residual, activation, and the tile's rows to
+    // global memory, from the stash, while the epilogue warps take over the next tile's sums
+    const VolGeom& G = P.g;
+    constexpr int LPR = NT / 4, RPI = 32 / LPR;                  // lanes per row, rows per access
+    const int quad = warp & 3;
+    const float* stash = (const float*)(tail + kBarBytes + FM::kXchBytes) + quad * 32 * NT;
+    auto activate = [&](float (&v)[4]) {
+      if (P.act == ACT_RELU) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) v[e] = max_nan(v[e], 0.f);
+      } else if (P.act == ACT_LEAKY) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) v[e] = v[e] > 0.f ? v[e] : v[e] * P.slope;
+      }
+    };
+    asm volatile("griddepcontrol.wait;" ::: "memory");           // before the first read of the residual and the first store
+    uint32_t tile_it = 0;
+    for (long long t = t0; t < ntiles; t += t_step, tile_it++) {
+      const int r = quad * 32 + lane, n0 = (int)(t % P.ntn) * NT;
+      const long long p = (2 * (t / P.ntn) + crank) * FM::kRowsOut - FM::kHalo + r;
+      const bool in_rows = p < P.rows && (!LINE || (r >= 1 && r <= FM::kRowsOut));
+      const uint32_t q0 = (uint32_t)(in_rows ? p : 0), q1 = q0 / (uint32_t)G.Wq, q2 = q1 / (uint32_t)G.Hq, q3 = q2 / (uint32_t)G.Dq;
+      const int ow = (int)(q0 - q1 * G.Wq), oh = (int)(q1 - q2 * G.Hq), od = (int)(q2 - q3 * G.Dq), on = (int)q3;
+      const bool live = in_rows && ow < G.Wo && oh < G.Ho && od < G.Do;
+      const uint32_t rows_mask = __ballot_sync(0xffffffffu, in_rows), live_mask = __ballot_sync(0xffffffffu, live);
+      if (!wait(stash_full, tile_it & 1, VST_STASH_FULL)) break;
+      if (P.out) {
+        // lanes along a row: whole lines of the split volume
+        const int c = lane % LPR, f = n0 + 4 * c;
+        const long long o0 = (p - lane + P.out_shift) * P.out_pitch + f;
+        const bool inside = f < P.out_pitch;
+        float b[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) b[e] = P.bias && f + e < P.F ? __ldg(P.bias + f + e) : 0.f;
+#pragma unroll 2
+        for (int i = 0; i < 32; i += RPI) {
+          const int rr = i + lane / LPR;
+          const bool mine = inside && ((rows_mask >> rr) & 1u), lv = (live_mask >> rr) & 1u;
+          const long long o = o0 + (long long)rr * P.out_pitch;
+          float4 sh = make_float4(0.f, 0.f, 0.f, 0.f), sl = sh;
+          if (P.skip && lv && inside) { sh = ld_plain4(P.skip + o); sl = ld_plain4(P.skip + P.out_plane + o); }
+          const float4 q = *reinterpret_cast<const float4*>(stash + rr * NT + ((c ^ (rr & 7)) << 2));
+          float v[4] = {q.x + b[0], q.y + b[1], q.z + b[2], q.w + b[3]}, h[4], l[4];
+          if (P.skip) {
+            v[0] += fmaf(sl.x, 1.f / kLoScale, sh.x); v[1] += fmaf(sl.y, 1.f / kLoScale, sh.y); v[2] += fmaf(sl.z, 1.f / kLoScale, sh.z); v[3] += fmaf(sl.w, 1.f / kLoScale, sh.w);
+          }
+          activate(v);
+#pragma unroll
+          for (int e = 0; e < 4; e++) vol_split(lv && f + e < P.F ? v[e] : 0.f, h[e], l[e]);   // the next layer's padding, and channels, are zero
+          if (mine) {
+            *reinterpret_cast<float4*>(P.out + o) = make_float4(h[0], h[1], h[2], h[3]);
+            *reinterpret_cast<float4*>(P.out + P.out_plane + o) = make_float4(l[0], l[1], l[2], l[3]);
+          }
+        }
+      } else {
+        // lane = row: whole lines of a channel-major array
+        float* dst = P.y + ((long long)on * P.ys_n + (long long)od * P.ys_d + (long long)oh * P.ys_h + (long long)ow * P.ys_w + (long long)n0 * P.ys_c);
+        const float* src = P.res ? P.res + ((long long)on * P.rs_n + (long long)od * P.rs_d + (long long)oh * P.rs_h + (long long)ow * P.rs_w + (long long)n0 * P.rs_c) : nullptr;
+        float b[NT / 32];                                            // of feature n0 + 32 i + lane
+#pragma unroll
+        for (int i = 0; i < NT / 32; i++) b[i] = P.bias && n0 + 32 * i + lane < P.F ? __ldg(P.bias + n0 + 32 * i + lane) : 0.f;
+#pragma unroll
+        for (int c = 0; c < LPR; c++) {
+          if (n0 + 4 * c >= P.F) break;
+          const float4 q = *reinterpret_cast<const float4*>(stash + lane * NT + ((c ^ (lane & 7)) << 2));
+          float v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            v[e] += __shfl_sync(0xffffffffu, b[c / 8], (4 * c + e) & 31);
+            if (src && live && n0 + 4 * c + e < P.F) v[e] += ld_plain(src + (4 * c + e) * P.rs_c);
+          }
+          activate(v);
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            if (live && n0 + 4 * c + e < P.F) *dst = v[e];
+            dst += P.ys_c;
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(stash_empty);
+    }
+  } else {
+    if constexpr (FM::kHalves) asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
+    // ------------------------------------------------------------------ epilogue: thread = row, half of the features.  A wait that gives
+    // up ends no warp here: the others would wait for it at the row exchange.  The waits behind it return at once.
+    const VolGeom& G = P.g;
+    const int quad = warp & 3, half = (warp - kWarpE0) >> 2;
+    const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16);
+    float* xch = (float*)(tail + kBarBytes);
+    float* stash = (float*)(tail + kBarBytes + FM::kXchBytes);
+    const uint32_t arr_acc = map_to_cta(acc_empty, 0), arr_cross = map_to_cta(cross_empty, 0);   // the leader's
+    const int nch = (nkt + P.chunk_kt - 1) / P.chunk_kt;
+    uint32_t chunk_it = 0, tile_it = 0;
+    for (long long t = t0; t < ntiles; t += t_step, tile_it++) {
+      const int r = quad * 32 + lane;
+      // the row's position in its line, for its neighbours
+      const long long p = (2 * (t / P.ntn) + crank) * FM::kRowsOut - FM::kHalo + r;
+      const int ow = LINE ? (int)((uint32_t)(p > 0 && p < P.rows ? p : 0) % (uint32_t)G.Wq) : 0;
+      float sum[FM::kTaps][NH], vx[LINE ? 1 : NH];
+#pragma unroll
+      for (int k = 0; k < FM::kTaps; k++)
+#pragma unroll
+        for (int j = 0; j < NH; j++) sum[k][j] = -0.f;           // -0 + x is x, also where x is -0
+      if constexpr (!LINE) {
+#pragma unroll
+        for (int j = 0; j < NH; j++) vx[j] = 0.f;
+      }
+      for (int ch = 0; ch < nch; ch++, chunk_it++) {
+        const uint32_t b = FM::kHalves ? half : chunk_it & 1;
+        wait(acc_full + 8 * b, (FM::kHalves ? chunk_it : chunk_it >> 1) & 1, VST_ACC_FULL);
+        tc_fence_after();
+        if constexpr (LINE) {
+          uint32_t a[3][NH];
+#pragma unroll
+          for (int k = 0; k < 3; k++) tmem_ldn(lane_addr + b * FM::kAcc + k * 32 + (FM::kHalves ? 0 : half * NH), a[k]);
+          tmem_ld_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster_relaxed(arr_acc + 8 * b);
+#pragma unroll
+          for (int k = 0; k < 3; k++)
+#pragma unroll
+            for (int j = 0; j < NH; j += 2) {
+              const float2 v = add2(make_float2(sum[k][j], sum[k][j + 1]), make_float2(__uint_as_float(a[k][j]), __uint_as_float(a[k][j + 1])));
+              sum[k][j] = v.x; sum[k][j + 1] = v.y;
+            }
+        } else {
+          uint32_t a[NH];
+          tmem_ldn(lane_addr + b * FM::kAcc + half * NT, a);     // a half's W_hi columns, then its W_lo columns
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < NH; j++) sum[0][j] = __fadd_rn(sum[0][j], __uint_as_float(a[j]));
+          tmem_ldn(lane_addr + b * FM::kAcc + half * NT + NH, a);
+          tmem_ld_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster_relaxed(arr_acc + 8 * b);
+#pragma unroll
+          for (int j = 0; j < NH; j++) vx[j] = __fadd_rn(vx[j], __uint_as_float(a[j]));
+        }
+      }
+      wait(cross_full, tile_it & 1, VST_CROSS_FULL);
+      tc_fence_after();
+      // What follows runs once a tile, so it is fetched instruction by instruction while the next tile's second step waits for these
+      // warps: as few instructions as possible (packed arithmetic, whole rows to and from shared memory, no branch per feature).
+      {
+        uint32_t a[FM::kTaps][NH / 16][16];
+#pragma unroll
+        for (int k = 0; k < FM::kTaps; k++)
+#pragma unroll
+          for (int c = 0; c < NH / 16; c++)
+            tmem_ldn(lane_addr + FM::kColCross + (LINE ? FM::cross_col(half, k * 32 + (FM::kHalves ? 0 : half * NH) + 16 * c) : half * NH + 16 * c), a[k][c]);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster_relaxed(arr_cross);
+#pragma unroll
+        for (int k = 0; k < FM::kTaps; k++)
+#pragma unroll
+          for (int j = 0; j < NH; j += 2) {
+            float2 x = make_float2(__uint_as_float(a[k][j / 16][j % 16]), __uint_as_float(a[k][j / 16][j % 16 + 1]));
+            if constexpr (!LINE) x = add2(make_float2(vx[j], vx[j + 1]), x);
+            const float2 v = fma2(x, make_float2(1.f / kLoScale, 1.f / kLoScale), make_float2(sum[k][j], sum[k][j + 1]));
+            sum[k][j] = v.x; sum[k][j + 1] = v.y;
+          }
+      }
+      float vh[NH];
+      if constexpr (LINE) {
+        // out[row] = sum0[row - 1] + sum1[row] + sum2[row + 1], where the neighbour is a position of the same line; rows on either side
+        // of a warp boundary go through shared memory
+        float* xu = xch + half * NH;                                 // tap 0's sums of each quadrant's last row
+        float* xd = xu + 4 * NT;                                     // tap 2's sums of each quadrant's first row
+        if (half == 0) asm volatile("bar.sync 1, 128;" ::: "memory"); else asm volatile("bar.sync 2, 128;" ::: "memory");   // the last tile's rows have been read
+        if (lane == 31) {
+#pragma unroll
+          for (int j = 0; j < NH; j += 4) *reinterpret_cast<float4*>(xu + quad * NT + j) = make_float4(sum[0][j], sum[0][j + 1], sum[0][j + 2], sum[0][j + 3]);
+        }
+        if (lane == 0) {
+#pragma unroll
+          for (int j = 0; j < NH; j += 4) *reinterpret_cast<float4*>(xd + quad * NT + j) = make_float4(sum[2][j], sum[2][j + 1], sum[2][j + 2], sum[2][j + 3]);
+        }
+        if (half == 0) asm volatile("bar.sync 1, 128;" ::: "memory"); else asm volatile("bar.sync 2, 128;" ::: "memory");
+        const bool has_up = ow + G.ow0 >= 0, has_dn = ow + G.ow0 + 2 < G.Wq;
+        const float* eu = xu + (quad > 0 ? quad - 1 : 0) * NT;       // what lanes 0 and 31 take instead (tile rows 0 and 127 are not outputs)
+        const float* ed = xd + (quad < 3 ? quad + 1 : 3) * NT;
+#pragma unroll
+        for (int j = 0; j < NH; j += 4) {
+          const float4 u4 = *reinterpret_cast<const float4*>(eu + j), d4 = *reinterpret_cast<const float4*>(ed + j);
+          const float u[4] = {u4.x, u4.y, u4.z, u4.w}, d[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            const float su = __shfl_up_sync(0xffffffffu, sum[0][j + e], 1), sd = __shfl_down_sync(0xffffffffu, sum[2][j + e], 1);
+            const float up = lane == 0 ? u[e] : su, dn = lane == 31 ? d[e] : sd;
+            vh[j + e] = sum[1][j + e] + (has_up ? up : 0.f) + (has_dn ? dn : 0.f);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < NH; j++) vh[j] = sum[0][j];
+      }
+      // 16-byte pieces at piece ^ (row % 8): no bank conflicts, whichever way the storers read
+      wait(stash_empty, (tile_it & 1) ^ 1, VST_STASH_EMPTY);
+#pragma unroll
+      for (int j = 0; j < NH; j += 4)
+        *reinterpret_cast<float4*>(stash + r * NT + ((((half * NH + j) >> 2) ^ (r & 7)) << 2)) = make_float4(vh[j], vh[j + 1], vh[j + 2], vh[j + 3]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(stash_full);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag && threadIdx.x == 0)
+    for (int i = 0; i < 2000; i++) __nanosleep(1000);          // let the partner's copies in flight land before the memory is given back
+  __syncthreads();
+  cluster_sync_all();                          // neither CTA leaves while its partner can still signal its barriers
+  if (warp == 2) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  }
+}
+
+// A strided fp32 array -> split volume: 64 rows x 32 channels per block, turned in shared memory; padding is written as zeros.  The
+// array is pooled or repeated on the way where the source says so (2-D networks), so that such a layer's output is never stored.
+__global__ void __launch_bounds__(256) pack_volume_kernel(const float* __restrict__ x, float* __restrict__ out, long long plane, int pitch, VolGeom g,
+                                                          VolSource src) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the layer may set up and load weights while this kernel runs
+  __shared__ float tile[64][33];
+  const uint32_t P32 = (uint32_t)g.P, R = P32 * (uint32_t)(g.fd * g.fh * g.fw), r0 = blockIdx.x * 64u;
+  const int c0 = blockIdx.y * 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const uint32_t r = r0 + i * 32 + lane;
+    const uint32_t ph = r / P32, q0 = r - ph * P32, q1 = q0 / (uint32_t)g.Wq, q2 = q1 / (uint32_t)g.Hq, q3 = q2 / (uint32_t)g.Dq;
+    const int w = (int)(q0 - q1 * g.Wq) * g.sw + (int)(ph % (uint32_t)g.fw) - g.pw;
+    const int h = (int)(q1 - q2 * g.Hq) * g.sh + (int)((ph / (uint32_t)g.fw) % (uint32_t)g.fh) - g.ph;
+    const int d = (int)(q2 - q3 * g.Dq) * g.sd + (int)(ph / (uint32_t)(g.fw * g.fh)) - g.pd;
+    const bool in = r < R && w >= 0 && w < g.W && h >= 0 && h < g.H && d >= 0 && d < g.D;
+    const float* p = x;
+    if (in)
+      p += (long long)q3 * src.xs_n + (long long)d * src.xs_d + (long long)(src.op == VolSource::UPSAMPLE ? (uint32_t)h / (uint32_t)src.kh : (uint32_t)(h * src.sh)) * src.xs_h +
+           (long long)(src.op == VolSource::UPSAMPLE ? (uint32_t)w / (uint32_t)src.kw : (uint32_t)(w * src.sw)) * src.xs_w;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int c = warp * 4 + k;
+      float v = 0.f;
+      if (in && c0 + c < g.C) {
+        const float* q = p + (long long)(c0 + c) * src.xs_c;
+        if (src.op != VolSource::MAXPOOL) v = __ldg(q);
+        else {
+          v = -INFINITY;
+          for (int a = 0; a < src.kh; a++)
+            for (int b = 0; b < src.kw; b++) v = max_nan(v, __ldg(q + a * src.xs_h + b * src.xs_w));
+        }
+      }
+      tile[i * 32 + lane][c] = v;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const int rr = i * 32 + (threadIdx.x >> 3), c = (threadIdx.x & 7) * 4;
+    if (r0 + rr >= R) continue;
+    float h[4], l[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) vol_split(tile[rr][c + e], h[e], l[e]);
+    float* o = out + (long long)(r0 + rr) * pitch + c0 + c;
+    *reinterpret_cast<float4*>(o) = make_float4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<float4*>(o + plane) = make_float4(l[0], l[1], l[2], l[3]);
+  }
+}
+
+// weights (F, C, taps) -> the steps' images [step][channel block][tile][CTA][W_hi rows | W_lo rows][32]; one tap: half of the tile's
+// features in each CTA; three taps: for every 32 features 96 rows [tap][feature], half of them in each CTA
+__global__ void pack_vol_weights_kernel(const float* __restrict__ W, int F, int C, int taps, int kw, int nchb, int ntn, int NT, float* __restrict__ out) {
+  const int half_rows = kw * NT / 2;                           // one CTA's
+  const long long n_el = (long long)(taps / kw) * nchb * ntn * 4 * half_rows * kKt;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_el; i += (long long)gridDim.x * blockDim.x) {
+    const int k = (int)(i % kKt);
+    long long rest = i / kKt;
+    const int row = (int)(rest % (2 * half_rows)); rest /= 2 * half_rows;
+    const int cta = (int)(rest & 1); rest >>= 1;
+    const int nt = (int)(rest % ntn); rest /= ntn;
+    const int cb = (int)(rest % nchb), step = (int)(rest / nchb);
+    const int r = row % half_rows, n = kw == 3 ? cta * 48 + r % 48 : cta * half_rows + r;
+    const int f = nt * NT + (kw == 3 ? r / 48 * 32 + n % 32 : n), tap = kw == 3 ? step * 3 + n / 32 : step, c = cb * kKt + k;
+    float h = 0.f, l = 0.f;
+    if (f < F && c < C) vol_split(W[((long long)f * C + c) * taps + tap], h, l);
+    out[i] = row < half_rows ? h : l;
+  }
+}
+
+typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                             const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeFn encode_fn() {
+  static EncodeFn fn = nullptr;
+  if (fn) return fn;
+  void* p = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || !p) return nullptr;
+  return fn = (EncodeFn)p;
+}
+
+int chunk_steps(const VolGeom& g) { return g.line || g.KD * g.KH * g.KW * ((g.C + 7) / 8 * 8) <= kShortK ? kChunkShort : kChunkLong; }
+
+// How a stage serves steps: those of a kd, of a line, or one; the widest sharing whose rows fit a box and leave two stages.  What
+// shared memory is left goes to the ring that reaches less far ahead, in steps.
+struct Sharing { int ng, tpg, sub_w, box_rows, a_stages, w_stages; size_t smem; };
+bool pick_sharing(const VolGeom& g, int NT, bool line, Sharing* o) {
+  const int nw = line ? 1 : g.KW, w_bytes = (line ? 3 : 1) * NT * kKt * 4;
+  const int fixed = kBarBytes + (line ? Form<32, true>::kXchBytes / 32 * NT : 0) + kM * NT * 4;
+  for (int level = 0; level < 3; level++) {
+    long long span;
+    if (level == 0) {
+      if (g.sh != 1 || (!line && g.sw != 1)) continue;
+      span = (long long)(g.KH - 1) * g.Wq + nw - 1;
+      o->ng = g.KD; o->tpg = g.KH * nw; o->sub_w = nw;
+    } else if (level == 1) {
+      if (!line && g.sw != 1) continue;
+      span = nw - 1;
+      o->ng = g.KD * g.KH; o->tpg = nw; o->sub_w = nw;
+    } else {
+      span = 0;
+      o->ng = g.KD * g.KH * nw; o->tpg = 1; o->sub_w = 1;
+    }
+    if (kM + span > 256) continue;
+    o->box_rows = (int)(kM + span + 7) / 8 * 8;
+    const int a_bytes = 2 * o->box_rows * kKt * 4;
+    int left = kSmemMax - fixed - 2 * a_bytes - 2 * w_bytes;
+    if (left < 0) continue;
+    o->a_stages = o->w_stages = 2;
+    for (;;) {
+      const bool a_ok = o->a_stages < kMaxStages && left >= a_bytes, w_ok = o->w_stages < kMaxStages && left >= w_bytes;
+      if (w_ok && (o->w_stages <= (o->a_stages - 1) * o->tpg || !a_ok)) { o->w_stages++; left -= w_bytes; }
+      else if (a_ok) { o->a_stages++; left -= a_bytes; }
+      else break;
+    }
+    o->smem = kSmemMax - left;
+    return true;
+  }
+  return false;
+}
+
+int sm_count() {
+  static int sms = 0;
+  if (sms) return sms;
+  int n = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return sms = n;
+}
+
+int vol_nt(int F) { return F <= 32 ? 32 : 64; }
+bool vol_line(int kw, int sw, int pw) { return kw == 3 && sw == 1 && pw <= 1; }       // the taps of a line in one step
+
+}  // namespace
+
+// `front`: zero positions in front of every line, plane and volume of the grid, at least the layer's own padding (a network whose
+// layers pad differently takes the widest for all); layers that take a line's taps in one step need none in front of lines
+VolGeom vol_geom(const ConvGeom& c, int front_d, int front_h, int front_w) {
+  VolGeom g;
+  std::memset(&g, 0, sizeof g);
+  g.N = c.N; g.D = c.D; g.H = c.H; g.W = c.W; g.C = c.C; g.Do = c.Do; g.Ho = c.Ho; g.Wo = c.Wo;
+  g.KD = c.KD; g.KH = c.KH; g.KW = c.KW; g.sd = c.sd; g.sh = c.sh; g.sw = c.sw;
+  g.pd = front_d; g.ph = front_h; g.pw = front_w;
+  // stride 1: a line's right padding is the next one's left padding; never fewer positions than outputs (padding of K and more)
+  auto axis = [](int ext, int front, int stride, int out) {
+    const int n = stride == 1 ? ext + front : (ext + 2 * front + stride - 1) / stride;
+    return n > out ? n : out;
+  };
+  g.Dq = axis(c.D, front_d, c.sd, c.Do); g.Hq = axis(c.H, front_h, c.sh, c.Ho); g.Wq = axis(c.W, front_w, c.sw, c.Wo);
+  g.fd = c.KD < c.sd ? c.KD : c.sd; g.fh = c.KH < c.sh ? c.KH : c.sh; g.fw = c.KW < c.sw ? c.KW : c.sw;
+  g.line = vol_line(c.KW, c.sw, c.pw);
+  g.od0 = front_d - c.pd; g.oh0 = front_h - c.ph; g.ow0 = front_w - c.pw;
+  g.P = (long long)g.N * g.Dq * g.Hq * g.Wq;
+  return g;
+}
+
+int vol_front_w(const ConvGeom& c) { return vol_line(c.KW, c.sw, c.pw) ? 0 : c.pw; }
+
+size_t vol_bytes(const VolGeom& g, int pitch) { return (size_t)g.P * g.fd * g.fh * g.fw * pitch * 8; }
+
+bool vol_supported(const ConvGeom& c) {
+  if (c.dd != 1 || c.dh != 1 || c.dw != 1) return false;                // transposed convolutions
+  // the most products an output can have: taps that lie inside the volume, times channels
+  const long long inside = (long long)(c.KD < c.D ? c.KD : c.D) * (c.KH < c.H ? c.KH : c.H) * (c.KW < c.W ? c.KW : c.W);
+  if (inside * c.C < kF32TcConvMinProducts) return false;
+  if ((long long)c.KD * c.KH * c.KW * ((c.C + 31) / 32) * ((c.F + 31) / 32) > (1 << 20)) return false;   // rows of the weight images in 32 bits
+  const VolGeom g = vol_geom(c, c.pd, c.ph, vol_front_w(c));
+  Sharing s;
+  // rows, and the last ones a tile may ask for, in 32 bits
+  return g.P * g.fd * g.fh * g.fw < (1LL << 30) && (long long)c.KD * g.Hq * g.Wq < (1LL << 29) && pick_sharing(g, vol_nt(c.F), g.line, &s);
+}
+
+struct VolW { int F = 0, C = 0, taps = 0, kw = 1, NT = 0, nchb = 0, ntn = 0; float* img = nullptr; CUtensorMap map; };     // kw: taps of a step
+
+void vol_weights_free(VolW* w) {
+  if (!w) return;
+  cudaFree(w->img);
+  delete w;
+}
+
+VolW* vol_weights_pack(const float* w_dev, int F, int C, int taps, bool line, cudaStream_t s, std::string* err) {
+  VolW* w = new VolW();
+  w->F = F; w->C = C; w->taps = taps; w->kw = line ? 3 : 1; w->NT = vol_nt(F); w->nchb = (C + kKt - 1) / kKt; w->ntn = (F + w->NT - 1) / w->NT;
+  const long long rows = (long long)(taps / w->kw) * w->nchb * w->ntn * (line ? 6 : 2) * w->NT;
+  if (cudaMalloc(&w->img, (size_t)rows * kKt * 4) != cudaSuccess) {
+    cudaGetLastError();
+    if (err) *err = "out of device memory for split conv weights";
+    delete w;
+    return nullptr;
+  }
+  const cuuint64_t dims[2] = {(cuuint64_t)kKt, (cuuint64_t)rows}, strides[1] = {kKt * 4};
+  const cuuint32_t box[2] = {kKt, (cuuint32_t)((line ? 3 : 1) * w->NT)}, estr[2] = {1, 1};
+  EncodeFn enc = encode_fn();
+  if (!enc || enc(&w->map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, w->img, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+    if (err) *err = "cuTensorMapEncodeTiled failed for split conv weights";
+    vol_weights_free(w);
+    return nullptr;
+  }
+  const long long n = rows * kKt;
+  pack_vol_weights_kernel<<<(unsigned)((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184), 256, 0, s>>>(w_dev, F, C, taps, w->kw, w->nchb, w->ntn, w->NT, w->img);
+  return w;
+}
+
+void vol_pack(const float* x, float* vol, int pitch, const VolGeom& g, const VolSource& src, cudaStream_t s) {
+  const long long R = g.P * g.fd * g.fh * g.fw;
+  pack_volume_kernel<<<dim3((unsigned)((R + 63) / 64), (unsigned)((g.C + 31) / 32)), 256, 0, s>>>(x, vol, R * pitch, pitch, g, src);
+}
+
+bool vol_conv(const VolW* w, const float* vol, int pitch, const VolGeom& g, const VolOut& o, const float* bias, int act, float slope, int* status,
+              cudaStream_t s, bool early, std::string* err) {
+  auto fail = [&](const char* why) { if (err) *err = why; return false; };
+  Sharing sh;
+  if (!pick_sharing(g, w->NT, g.line, &sh)) return fail("convolution: no stage layout");
+  VolParams P;
+  std::memset(&P, 0, sizeof P);
+  const long long R = g.P * g.fd * g.fh * g.fw;
+  const cuuint64_t dims[3] = {(cuuint64_t)pitch, (cuuint64_t)R, 2}, strides[2] = {(cuuint64_t)pitch * 4, (cuuint64_t)R * pitch * 4};
+  const cuuint32_t box[3] = {kKt, (cuuint32_t)sh.box_rows, 2}, estr[3] = {1, 1, 1};
+  EncodeFn enc = encode_fn();
+  if (!enc || enc(&P.amap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(vol), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return fail("cuTensorMapEncodeTiled failed for a split volume");
+  P.wmap = w->map; P.g = g; P.nchb = w->nchb; P.ntn = w->ntn;
+  P.chunk_kt = chunk_steps(g);
+  P.ng = sh.ng; P.tpg = sh.tpg; P.sub_w = sh.sub_w; P.box_rows = sh.box_rows; P.a_stages = sh.a_stages; P.w_stages = sh.w_stages;
+  P.rows = (((long long)(g.N - 1) * g.Dq + g.Do - 1) * g.Hq + g.Ho - 1) * g.Wq + g.Wo;
+  P.bias = bias; P.act = act; P.slope = slope; P.F = w->F;
+  P.out = o.vol; P.out_plane = g.P * o.pitch; P.out_pitch = o.pitch; P.out_shift = ((long long)g.pd * g.Hq + g.ph) * g.Wq + g.pw;
+  P.skip = o.skip; P.y = o.y; P.ys_n = o.ys_n; P.ys_d = o.ys_d; P.ys_h = o.ys_h; P.ys_w = o.ys_w; P.ys_c = o.ys_c;
+  P.res = o.res; P.rs_n = o.rs_n; P.rs_d = o.rs_d; P.rs_h = o.rs_h; P.rs_w = o.rs_w; P.rs_c = o.rs_c;
+  P.status = status;
+  P.wait_limit = g_tc_test.wait_limit ? g_tc_test.wait_limit : kWaitLimit;
+  P.test_skip_stage = g_tc_test.skip_stage;
+  typedef void (*Kernel)(VolParams);
+  static const Kernel kernels[4] = {conv_vol_kernel<32, false>, conv_vol_kernel<64, false>, conv_vol_kernel<32, true>, conv_vol_kernel<64, true>};
+  static bool ready = false;
+  if (!ready) {
+    for (Kernel k : kernels)
+      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess)
+        return fail("cannot reserve shared memory for the convolution kernel");
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, kernels[3]) != cudaSuccess || fa.numRegs != 128) return fail("the convolution kernel's register split does not add up");
+    ready = true;
+  }
+  const int per_pair = 2 * (g.line ? Form<64, true>::kRowsOut : Form<64, false>::kRowsOut);
+  const long long tiles = (P.rows + per_pair - 1) / per_pair * P.ntn, pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs))); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = sh.smem; cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  static const bool pdl = std::getenv("FORTIS_NO_PDL") == nullptr;
+  cfg.attrs = at; cfg.numAttrs = (pdl && early) ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernels[2 * g.line + (w->NT == 64)], P);
+  if (e != cudaSuccess) { if (err) *err = std::string("convolution launch: ") + cudaGetErrorString(e); return false; }
+  return true;
+}
+
+}  // namespace fortis

@@ -5,6 +5,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstdint>
+
 #include "fortis_plan.h"
 
 namespace fortis {
@@ -15,6 +17,14 @@ __device__ __forceinline__ float max_nan(float a, float b) {
   float r;
   asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
   return r;
+}
+
+// x = hi + lo * 2^-10 exactly: hi the nearest finite TF32 value
+__device__ __forceinline__ void vol_split(float x, float& hi, float& lo) {
+  uint32_t h;
+  asm("cvt.rna.satfinite.tf32.f32 %0, %1;" : "=r"(h) : "f"(x));
+  hi = __uint_as_float(h);
+  lo = (x - hi) * 1024.f;
 }
 
 struct IoPlanDev {

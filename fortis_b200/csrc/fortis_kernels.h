@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <string>
+#include <vector>
 
 #include "fortis_plan.h"
 
@@ -157,19 +158,45 @@ RowsMlp* rows_mlp_create(const std::vector<F16Layer>& layers, bool f16, const fl
 void rows_mlp_destroy(RowsMlp* m);
 int rows_mlp_cost(const int* K, const int* N, int nlayers, long long nrows);     // estimated device time, 10 ns
 bool rows_mlp_forward(RowsMlp* m, const F32TcLaunch& L, cudaStream_t s, std::string* err);
-// one fp32 convolution layer on the same kernel (rows = output voxels, reduction = taps x channels)
-struct F32ConvW;                                       // split weights of one layer
+// ---- fp32 convolutions on the tensor cores (fortis_conv3d_f32.cu): rows = positions of a grid that holds the padding ------
 // Shorter reductions stay on the FFMA kernel: the split keeps 21 bits of an operand, which sums of few products show, while
 // the FFMA kernel's roundings grow with their number.  Error against 64 bits, relative 2-norm, split / FFMA, inputs normal and
 // normal.clamp_min(0), normal weights: 8 products 9.2e-8 / 5.3e-8 and 8.8e-8 / 4.2e-8, 27: 1.3e-7 / 9.4e-8 and 1.2e-7 / 7.0e-8,
 // 64: 1.4e-7 / 1.4e-7 and 1.2e-7 / 1.0e-7, 96: 1.35e-7 / 1.8e-7 and 1.23e-7 / 1.27e-7, 128: 1.4e-7 / 2.0e-7 and 1.3e-7 / 1.5e-7.
 constexpr int kF32TcConvMinProducts = 128;
-bool f32tc_conv_supported(const ConvGeom& g);
-F32ConvW* f32tc_conv_pack(const float* w_dev, int F, int C, int taps, cudaStream_t s, std::string* err);
-void f32tc_conv_free(F32ConvW* w);
+struct VolGeom {
+  int N, D, H, W, C, Do, Ho, Wo;
+  int KD, KH, KW, sd, sh, sw;
+  int pd, ph, pw;                             // zero positions in front of every line, plane and volume
+  int Dq, Hq, Wq;                             // extents of the grid (of one phase)
+  int fd, fh, fw;                             // phases per axis: residues of a position modulo the stride that taps read
+  int od0, oh0, ow0;                          // where tap 0 of output 0 lies
+  int line;                                   // the three taps of a line in one step
+  long long P;                                // rows of one phase
+};
+VolGeom vol_geom(const ConvGeom& c, int front_d, int front_h, int front_w);
+int vol_front_w(const ConvGeom& c);                            // zero positions a layer needs in front of a line
+bool vol_supported(const ConvGeom& c);
+size_t vol_bytes(const VolGeom& g, int pitch);                 // of a split volume with `pitch` channels a row (a multiple of 32)
+struct VolW;                                                   // one layer's weights, split, as the kernel streams them
+// torch layout (F, C, taps); `line`: as vol_geom says of the layer
+VolW* vol_weights_pack(const float* w_dev, int F, int C, int taps, bool line, cudaStream_t s, std::string* err);
+void vol_weights_free(VolW* w);
+// where a split volume's values come from: an array, or an array pooled (windows kh x kw, steps sh x sw) or repeated (kh x kw times)
+struct VolSource {
+  enum { PLAIN = 0, MAXPOOL = 1, UPSAMPLE = 2 };
+  int op, kh, kw, sh, sw;
+  long long xs_n, xs_d, xs_h, xs_w, xs_c;
+};
+void vol_pack(const float* x, float* vol, int pitch, const VolGeom& g, const VolSource& src, cudaStream_t s);
+struct VolOut {
+  float* vol; int pitch; const float* skip;                    // a split volume of the same grid, the residual likewise, or ...
+  float* y; long long ys_n, ys_d, ys_h, ys_w, ys_c;            // ... a plain array ...
+  const float* res; long long rs_n, rs_d, rs_h, rs_w, rs_c;    // ... with a plain residual
+};
 // `early`: the launch may start (and read its weights) before the kernel in front of it in the stream has finished
-bool f32tc_conv(const F32ConvW* w, const float* x, const float* bias, const float* residual, float* y, const ConvGeom& g, int act,
-                float slope, int* status, cudaStream_t s, bool early, std::string* err);
+bool vol_conv(const VolW* w, const float* vol, int pitch, const VolGeom& g, const VolOut& o, const float* bias, int act, float slope, int* status,
+              cudaStream_t s, bool early, std::string* err);
 // C[M][N] = A[M][K] . W[N][K]^T, row-major device operands (the memref entry fortis_gemm)
 bool f32tc_gemm(const float* A, const float* W, float* C, long long M, int N, int K, int* status, cudaStream_t s, std::string* err);
 
