@@ -153,6 +153,7 @@ struct Session {
 
   long long buf_rows = 0;
   float *din = nullptr, *dout = nullptr, *act0 = nullptr, *act1 = nullptr;
+  long long pair_rows = 0;                        // rows act0 and act1 hold as split activations (0: none)
   float *X_pinned = nullptr, *Y_pinned = nullptr;
   long long pinned_rows = 0;
   bool pack_pending = false, gather_pending = false, gather_done = false;
@@ -432,13 +433,22 @@ long long out_floats(long long rows) {
   return (long long)s.conv_shape[0] * C * Ho * Wo;
 }
 
+// Below this many rows the per-layer FFMA kernels run.  (The tensor-core kernel is faster there too, 300 rows of the column
+// network 73 us against 455, but its sums are others than a program of few rows has had.)  fortis_gemm: from here on the
+// weights are split once per address (constants of the caller); below, W is read as it is on every call.
+constexpr long long kF32TcMinRows = 512;
+
 // row pitch of the feature-major activation buffers: every feature starts on a 16-byte boundary
 long long act_ld(long long rows) { return (rows + 3) / 4 * 4; }
 
 void ensure_buffers(long long rows) {
   Session& s = S();
-  if (rows <= s.buf_rows && s.din) return;
+  // fp32 layers on pairs of CTAs keep their activations split, twice the floats; without the memory for that they run as before
+  const bool pair = s.model.is_mlp() && s.f32 && rows >= kF32TcMinRows && rows <= kF32TcMaxRows && f32tc_pair_wanted(s.f32, rows);
+  if (rows <= s.buf_rows && s.din && (!pair || s.pair_rows != 0)) return;
+  if (rows < s.buf_rows) rows = s.buf_rows;
   pool_free(s.din); pool_free(s.dout); pool_free(s.act0); pool_free(s.act1);
+  s.act0 = s.act1 = nullptr;
   int wmax = 1;
   for (auto& L : s.model.layers) wmax = L.cout > wmax ? L.cout : wmax;
   const long long nin = s.model.n_in(), nout = s.model.n_out();
@@ -446,8 +456,19 @@ void ensure_buffers(long long rows) {
   s.dout = (float*)pool_alloc(out_floats(rows) * 4);
   (void)nout;
   const bool need_act = s.model.is_mlp() && s.model.layers.size() > 1;
-  s.act0 = need_act ? (float*)pool_alloc(act_ld(rows) * wmax * 4) : nullptr;
-  s.act1 = need_act && s.model.layers.size() > 2 ? (float*)pool_alloc(act_ld(rows) * wmax * 4) : nullptr;
+  const long long act_bytes = act_ld(rows) * wmax * 4;
+  s.pair_rows = pair ? -1 : 0;                    // asked for
+  if (pair) {
+    const long long bytes = std::max<long long>((long long)f32tc_pair_bytes(s.f32, rows), act_bytes);
+    s.act0 = (float*)pool_alloc(bytes);
+    s.act1 = s.act0 ? (float*)pool_alloc(bytes) : nullptr;
+    if (s.act1) s.pair_rows = rows;
+    else { pool_free(s.act0); s.act0 = nullptr; }
+  }
+  if (need_act && !s.act0) {
+    s.act0 = (float*)pool_alloc(act_bytes);
+    s.act1 = s.model.layers.size() > 2 ? (float*)pool_alloc(act_bytes) : nullptr;
+  }
   if (!s.din || !s.dout || (need_act && !s.act0)) throw std::runtime_error("out of device memory for the model buffers");
   s.buf_rows = rows;
   drop_graph();
@@ -628,11 +649,6 @@ void download_stores(PlanDev& P, const int* args, int nargs, bool multi_plane, c
 // ---------------------------------------------------------------------------------------------------------------
 // the step
 // ---------------------------------------------------------------------------------------------------------------
-// Below this many rows the per-layer FFMA kernels run.  (The tensor-core kernel is faster there too, 300 rows of the column
-// network 73 us against 455, but its sums are others than a program of few rows has had.)  fortis_gemm: from here on the
-// weights are split once per address (constants of the caller); below, W is read as it is on every call.
-constexpr long long kF32TcMinRows = 512;
-
 struct StepArgs {
   bool use_gather = false;      // model input comes from the gather plan (else din)
   bool fuse_scatter = false;    // outputs go straight to the host arrays (all planes)
@@ -830,6 +846,7 @@ void run_step_kernels(const StepArgs& A) {
     else L.Y = s.dout;
     L.g = g;
     L.act[0] = s.act0; L.act[1] = s.act1; L.act_ld = act_ld(s.buf_rows);
+    L.pair = s.pair_rows >= rows && f32tc_pair_wanted(s.f32, rows);
     ensure_aux(f32tc_grid(rows));
     if (fuse_out && s.want_checksum) { L.partials = s.d_partials; L.sum = s.d_sum; L.done = s.d_done; }
     L.status = s.d_status;

@@ -363,14 +363,15 @@ std::vector<float> repack_weights_taps(const float* w, int F, int C, int taps) {
 
 // One layer's weights on the device: [tap][C][F] for the FFMA kernels and, where the tensor-core kernel may take the layer,
 // split for that one.  (Which of the two runs depends on the volume's extents too, so both stay.)
-struct LayerDev { float *wt = nullptr, *bias = nullptr; VolW* vw = nullptr; };
-bool upload_layer(const LayerHost& L, int taps, bool split, bool line, LayerDev* d, std::string* err) {
+struct LayerDev { float *wt = nullptr, *bias = nullptr; VolW* vw = nullptr; F32ConvW* split = nullptr; };
+// line: the form of the split volumes' weights; both: the other kernel's weights too
+bool upload_layer(const LayerHost& L, int taps, bool split, bool line, bool both, LayerDev* d, std::string* err) {
   split = split && (long long)L.cin * taps >= kF32TcConvMinProducts;
   const std::vector<float> wt = repack_weights_taps(L.W.data(), L.cout, L.cin, taps);
   float* raw = nullptr;
   auto fail = [&](const char* why) {
     if (err) *err = why;
-    cudaFree(d->wt); cudaFree(d->bias); cudaFree(raw); vol_weights_free(d->vw);
+    cudaFree(d->wt); cudaFree(d->bias); cudaFree(raw); vol_weights_free(d->vw); f32tc_conv_free(d->split);
     cudaGetLastError();
     *d = LayerDev();
     return false;
@@ -382,7 +383,8 @@ bool upload_layer(const LayerHost& L, int taps, bool split, bool line, LayerDev*
   if (cudaMalloc(&raw, L.W.size() * 4) != cudaSuccess) return fail("out of device memory for conv weights");
   cudaMemcpy(raw, L.W.data(), L.W.size() * 4, cudaMemcpyHostToDevice);
   d->vw = vol_weights_pack(raw, L.cout, L.cin, taps, line, 0, nullptr);
-  if (!d->vw || cudaStreamSynchronize(0) != cudaSuccess) return fail("out of device memory for split conv weights");
+  if (both) d->split = f32tc_conv_pack(raw, L.cout, L.cin, taps, 0, nullptr);
+  if (!d->vw || (both && !d->split) || cudaStreamSynchronize(0) != cudaSuccess) return fail("out of device memory for split conv weights");
   cudaFree(raw);
   return true;
 }
@@ -410,11 +412,15 @@ float* vol_workspace(size_t bytes, cudaStream_t s) {
   return buf;
 }
 
-// A layer takes the tensor-core kernel wherever it can and its sums are long enough (vol_supported), unless its split volume
-// does not fit the device.
-bool conv_layer(const VolW* vw, const float* wt, const float* bias, const float* x, const VolSource* src, const float* residual, float* y,
-                const ConvGeom& g, int act, float slope, int* status, cudaStream_t s, bool early, std::string* err) {
-  if (vw && vol_supported(g)) {
+// Where a layer whose input is a plain array runs: over a split volume (packing, then no thread in the operand path), on the kernel whose
+// threads load the taps, or on the FFMA kernels (sums of few products: f32tc_conv_supported).  Small calls of few channels and many taps are
+// faster without packing (7 -> 47 channels 5x5x5 on 2 x 10x8x8 29 us, over a split volume 59; 10 -> 32 3x3x3 stride 2 15 and 28); large ones
+// over volumes (32 -> 64 on 40^3 73 and 53).
+bool takes_volume(const ConvGeom& g) { return vol_supported(g) && (!f32tc_conv_supported(g) || vol_cost(g) < f32tc_conv_cost(g)); }
+
+bool conv_layer(const VolW* vw, const F32ConvW* split, const float* wt, const float* bias, const float* x, const VolSource* src, const float* residual,
+                float* y, const ConvGeom& g, int act, float slope, int* status, cudaStream_t s, bool early, std::string* err) {
+  if (vw && (src || takes_volume(g))) {
     const VolGeom vg = vol_geom(g, g.pd, g.ph, vol_front_w(g));
     const int pitch = (g.C + 31) / 32 * 32;
     float* vol = vol_workspace(vol_bytes(vg, pitch), s);
@@ -427,8 +433,10 @@ bool conv_layer(const VolW* vw, const float* wt, const float* bias, const float*
       o.res = residual; o.rs_n = g.rs_n; o.rs_d = g.rs_d; o.rs_h = g.rs_h; o.rs_w = g.rs_w; o.rs_c = g.rs_c;
       return vol_conv(vw, vol, pitch, vg, o, bias, act, slope, status, s, early, err);
     }
+    if (src) { if (err) *err = "out of device memory for a convolution's input"; return false; }
   }
-  if (src || !wt) { if (err) *err = "out of device memory for a convolution's input"; return false; }
+  if (split && f32tc_conv_supported(g)) return f32tc_conv(split, x, bias, residual, y, g, act, slope, status, s, early, err);
+  if (!wt) { if (err) *err = "out of device memory for a convolution's input"; return false; }
   launch_conv(x, wt, bias, residual, y, g, act, slope, s);
   return true;
 }
@@ -469,7 +477,8 @@ __global__ void upsample_nearest2d_kernel(const float* __restrict__ x, float* __
 struct OpNet {
   std::vector<LayerHost> meta;
   std::vector<float*> wt, bias;           // per layer (null for layers without weights)
-  std::vector<VolW*> vw;                  // the weights as the tensor-core kernel takes them (null for layers without weights)
+  std::vector<VolW*> vw;                  // the weights as the tensor-core kernels take them (null for layers without weights)
+  std::vector<F32ConvW*> split;
   float* buf[2] = {nullptr, nullptr};
   long long cap = 0;
 };
@@ -479,6 +488,7 @@ void opnet_destroy(OpNet* m) {
   for (float* p : m->wt) cudaFree(p);
   for (float* p : m->bias) cudaFree(p);
   for (VolW* p : m->vw) vol_weights_free(p);
+  for (F32ConvW* p : m->split) f32tc_conv_free(p);
   for (float* p : m->buf) cudaFree(p);
   delete m;
 }
@@ -518,11 +528,11 @@ OpNet* opnet_create(const ModelHost& M, std::string* err) {
     LayerHost meta = L; meta.W.clear(); meta.b.clear();
     m->meta.push_back(meta);
     LayerDev d;
-    if (L.kind == LAYER_CONV2D && !upload_layer(L, L.kh * L.kw, L.dil == 1, L.kw == 3 && L.sw == 1 && L.pw <= 1, &d, err)) {
+    if (L.kind == LAYER_CONV2D && !upload_layer(L, L.kh * L.kw, L.dil == 1, L.kw == 3 && L.sw == 1 && L.pw <= 1, true, &d, err)) {
       opnet_destroy(m);
       return nullptr;
     }
-    m->wt.push_back(d.wt); m->bias.push_back(d.bias); m->vw.push_back(d.vw);
+    m->wt.push_back(d.wt); m->bias.push_back(d.bias); m->vw.push_back(d.vw); m->split.push_back(d.split);
   }
   return m;
 }
@@ -574,7 +584,7 @@ bool opnet_forward(OpNet* m, const float* x, float* y, int N, int H, int W, int*
     const unsigned blocks = (unsigned)((nout + 255) / 256 < 148 * 16 ? (nout + 255) / 256 : 148 * 16);
     if (L.kind == LAYER_CONV2D) {
       const ConvGeom g = opnet_geom(L, N, h, w, h2, w2);
-      if (!conv_layer(m->vw[l], m->wt[l], m->bias[l], src, pending.op ? &pending : nullptr, nullptr, dst, g, L.act, L.slope, status, s, true, err)) return false;
+      if (!conv_layer(m->vw[l], m->split[l], m->wt[l], m->bias[l], src, pending.op ? &pending : nullptr, nullptr, dst, g, L.act, L.slope, status, s, true, err)) return false;
       pending.op = VolSource::PLAIN;
     } else {
       const bool pool = L.kind == LAYER_MAXPOOL2D;
@@ -582,7 +592,7 @@ bool opnet_forward(OpNet* m, const float* x, float* y, int N, int H, int W, int*
       int h3, w3;
       if (l + 1 < nl && m->meta[l + 1].kind == LAYER_CONV2D && m->vw[l + 1] && opnet_layer_shape(m->meta[l + 1], h2, w2, &h3, &w3)) {
         const ConvGeom g = opnet_geom(m->meta[l + 1], N, h2, w2, h3, w3);
-        if (vol_supported(g) && vol_workspace(vol_bytes(vol_geom(g, 0, g.ph, vol_front_w(g)), (g.C + 31) / 32 * 32), s)) {
+        if (takes_volume(g) && vol_workspace(vol_bytes(vol_geom(g, 0, g.ph, vol_front_w(g)), (g.C + 31) / 32 * 32), s)) {
           pending = VolSource{pool ? VolSource::MAXPOOL : VolSource::UPSAMPLE, pool ? L.kh : L.sh, pool ? L.kw : L.sw, L.sh, L.sw,
                               (long long)L.cin * h * w, (long long)h * w, w, 1, (long long)h * w};
           h = h2; w = w2;
@@ -604,6 +614,7 @@ struct ConvModel {
   std::vector<LayerHost> meta;          // shapes and flags (weights dropped after upload)
   std::vector<float*> wt, bias;
   std::vector<VolW*> vw;
+  std::vector<F32ConvW*> split;
   float *buf[3] = {nullptr, nullptr, nullptr};
   size_t buf_bytes = 0;
   int shape[4] = {0, 0, 0, 0};          // of the split volumes in buf, whose padding is zero (shape[0] = 0: none)
@@ -615,6 +626,7 @@ void conv_model_destroy(ConvModel* m) {
   for (float* p : m->wt) cudaFree(p);
   for (float* p : m->bias) cudaFree(p);
   for (VolW* p : m->vw) vol_weights_free(p);
+  for (F32ConvW* p : m->split) f32tc_conv_free(p);
   for (float* p : m->buf) cudaFree(p);
   delete m;
 }
@@ -637,11 +649,11 @@ ConvModel* conv_model_create(const ModelHost& M, int precision, cudaStream_t s, 
     meta.W.clear(); meta.b.clear();
     m->meta.push_back(meta);
     LayerDev d;
-    if (!upload_layer(L, L.ksize * L.ksize * L.ksize, true, L.ksize == 3 && L.pad == 1, &d, err)) {
+    if (!upload_layer(L, L.ksize * L.ksize * L.ksize, true, L.ksize == 3 && L.pad == 1, true, &d, err)) {
       conv_model_destroy(m);
       return nullptr;
     }
-    m->wt.push_back(d.wt); m->bias.push_back(d.bias); m->vw.push_back(d.vw);
+    m->wt.push_back(d.wt); m->bias.push_back(d.bias); m->vw.push_back(d.vw); m->split.push_back(d.split);
   }
   return m;
 }
@@ -778,7 +790,7 @@ bool conv_forward(ConvModel* m, const float* x, float* y, int N, int D, int H, i
     set_strides(&g.rs_n, &g.rs_d, &g.rs_h, &g.rs_w, &g.rs_c, false, L.cout, D, H, W);          // a skip is a layer's output, channel-major
     const float* res = (L.flags & LFLAG_ADD_SKIP) ? skip : nullptr;
     if ((L.flags & LFLAG_ADD_SKIP) && !skip) { if (err) *err = "conv3d model: a layer adds a skip that was never saved"; return false; }
-    if (!conv_layer(m->vw[l], m->wt[l], m->bias[l], src, nullptr, res, dst, g, L.act, L.slope, status, s, true, err)) return false;
+    if (!conv_layer(m->vw[l], m->split[l], m->wt[l], m->bias[l], src, nullptr, res, dst, g, L.act, L.slope, status, s, true, err)) return false;
     if (L.flags & LFLAG_SAVE_SKIP) { skip = dst; skip_buf = dst_buf; }
     src = dst;
   }
@@ -798,7 +810,7 @@ bool conv3d_ncdhw(const float* x, const float* w, float* y, int N, int C, int D,
   // captured into a graph, so such a call is refused (the reference captures on the second call for the same reason: the
   // first call allocates).
   // vw: the forms for layers that take a tap at a time and, of kernels three wide, a line's taps at a time: stride and padding decide
-  struct Cached { const float* w; int F, C, taps; float* wt; VolW* vw[2]; bool captured; };
+  struct Cached { const float* w; int F, C, taps; float* wt; VolW* vw[2]; F32ConvW* split; bool captured; };
   static std::vector<Cached> cache;
   static size_t victim = 0;
   const int taps = K[0] * K[1] * K[2];
@@ -812,8 +824,7 @@ bool conv3d_ncdhw(const float* x, const float* w, float* y, int N, int C, int D,
   g.ys_w = 1; g.ys_h = g.Wo; g.ys_d = (long long)g.Ho * g.Wo; g.ys_c = (long long)g.Do * g.Ho * g.Wo; g.ys_n = (long long)F * g.Do * g.Ho * g.Wo;
   const VolGeom vg = vol_geom(g, g.pd, g.ph, vol_front_w(g));
   const int line = vg.line;
-  // the FFMA kernel, which needs no copy of x, where the copy does not fit the device
-  const bool tc = vol_supported(g) && vol_workspace(vol_bytes(vg, (C + 31) / 32 * 32), s) != nullptr;
+  const bool tc = vol_supported(g) || f32tc_conv_supported(g);
   Cached* c = nullptr;
   bool fresh = false;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -821,26 +832,29 @@ bool conv3d_ncdhw(const float* x, const float* w, float* y, int N, int C, int D,
   const bool capturing = cs != cudaStreamCaptureStatusNone;
   for (auto& q : cache) if (q.w == w && q.F == F && q.C == C && q.taps == taps) c = &q;
   if (c && capturing) c->captured = true;
-  if (!c || (tc ? (void*)c->vw[line] : (void*)c->wt) == nullptr) {
+  // every form the weights may be needed in, whatever the volume: a captured call packs none
+  auto complete = [&](const Cached* e) { return tc ? e->split && e->vw[0] && (K[2] != 3 || e->vw[1]) : e->wt != nullptr; };
+  if (!c || !complete(c)) {
     if (capturing) { if (err) *err = "conv weights seen for the first time during graph capture; run one eager call first"; return false; }
     if (!c) {
       for (size_t i = 0; i < cache.size() && cache.size() >= 64 && !c; i++, victim = (victim + 1) % cache.size())
         if (!cache[victim].captured) c = &cache[victim];
-      if (c) { cudaStreamSynchronize(s); cudaFree(c->wt); vol_weights_free(c->vw[0]); vol_weights_free(c->vw[1]); }
+      if (c) { cudaStreamSynchronize(s); cudaFree(c->wt); vol_weights_free(c->vw[0]); vol_weights_free(c->vw[1]); f32tc_conv_free(c->split); }
       else { cache.push_back(Cached{}); c = &cache.back(); }
-      *c = Cached{w, F, C, taps, nullptr, {nullptr, nullptr}, false};
+      *c = Cached{w, F, C, taps, nullptr, {nullptr, nullptr}, nullptr, false};
     }
     const size_t n = (size_t)F * C * taps;
     if (tc) {
       for (int form = 0; form < (K[2] == 3 ? 2 : 1); form++)
         if (!c->vw[form] && !(c->vw[form] = vol_weights_pack(w, F, C, taps, form != 0, s, err))) return false;
+      if (!c->split && !(c->split = f32tc_conv_pack(w, F, C, taps, s, err))) return false;
     } else {
       if (cudaMalloc(&c->wt, n * 4) != cudaSuccess) { cudaGetLastError(); c->wt = nullptr; if (err) *err = "out of device memory for conv weights"; return false; }
       repack_weights_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(w, c->wt, F, C, taps);
     }
     fresh = true;
   }
-  if (!conv_layer(tc ? c->vw[line] : nullptr, c->wt, nullptr, x, nullptr, nullptr, y, g, ACT_NONE, 0.f, status, s, !fresh, err)) return false;
+  if (!conv_layer(tc ? c->vw[line] : nullptr, tc ? c->split : nullptr, c->wt, nullptr, x, nullptr, nullptr, y, g, ACT_NONE, 0.f, status, s, !fresh, err)) return false;
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { if (err) *err = std::string("conv3d launch: ") + cudaGetErrorString(e); return false; }
   return true;

@@ -1,6 +1,6 @@
 // fp32 convolutions on the tensor cores without threads in the operand path: y = act(conv(x, W) + b + residual) with every
 // product formed as three TF32 MMAs (x = x_hi + x_lo, W = W_hi + W_lo: hi.hi, hi.lo and lo.hi; the hi.hi sums taken over into
-// registers every 32 or 64 k with IEEE additions, the cross sums scaled by 2^10), both operands read from shared memory where the
+// registers every 32 k with IEEE additions, the cross sums scaled by 2^10), both operands read from shared memory where the
 // TMA puts them.
 //
 // Replaces, for layers of 128 products and more, the reference's cuDNN lowerings fortis_conv2d / fortis_conv3d
@@ -51,23 +51,21 @@ constexpr int kM = 128, kKt = 32;
 // cross sums are multiplied by 2^-10.  Without it x_lo is lost from |x| < 2^-102 on (2^-118: error 2.2e-6).  (x_lo is below 2^-10 of
 // the largest value, so the product stays finite.)
 constexpr float kLoScale = 1024.f;
-// Steps of 32 k accumulated in the tensor core, which truncates, before the sums are taken over: two, or one where K is short (2-D
-// network of K = 27 to 576, six convolutions, error against 64 bits: two 9.1e-7, one 6.2e-7, FFMA 7.7e-7).  LINE: always one, at no
-// cost in time (14-layer network: 1.02e-6, with two 1.66e-6).
-constexpr int kChunkLong = 2, kChunkShort = 1, kShortK = 640;
+// The tensor core truncates as it accumulates, so the sums are taken over after every step of 32 k (14-layer network: error against 64 bits
+// 1.02e-6, every 64 k 1.66e-6; FFMA 2.5e-6).
 // warps: 0 activations, 1 weights (TMA), 2 and 3 MMA issuers, then the epilogue and the storers
 constexpr int kEWarps = 8, kWarpE0 = 4, kWarpS0 = kWarpE0 + kEWarps, kThreads = (kWarpS0 + 4) * 32;
 constexpr int kMaxStages = 8;
 constexpr int kBarBytes = 512;
 constexpr int kSmemMax = 227 * 1024;
-enum { VST_ALIGN = 31, VST_A_EMPTY = 32, VST_W_EMPTY = 33, VST_A_FULL = 34, VST_W_FULL = 35, VST_ACC_EMPTY = 36, VST_ACC_FULL = 37, VST_CROSS_FULL = 38,
-       VST_STASH_FULL = 39, VST_STASH_EMPTY = 40 };
+enum { VST_A_FULL = 21, VST_A_EMPTY = 22, VST_ACC_FULL = 23, VST_ACC_EMPTY = 24, VST_ALIGN = 25, VST_W_FULL = 26, VST_W_EMPTY = 27, VST_STASH_FULL = 28,
+       VST_STASH_EMPTY = 29 };                 // as the other fp32 kernel numbers its waits
 
 struct VolParams {
   CUtensorMap amap;                            // [plane 2][row][channel], box 2 x box_rows x 32
   CUtensorMap wmap;                            // [step][channel block][tile of features][CTA][row] rows of 32
   VolGeom g;
-  int nchb, ntn, chunk_kt;
+  int nchb, ntn;
   int ng, tpg, sub_w;                          // stages per channel block, steps per stage, steps of one line among them
   int box_rows, a_stages, w_stages;
   long long rows;                              // output rows up to the last one that is a real output
@@ -167,7 +165,7 @@ template <int NT, bool LINE> struct Form {
   static constexpr int kRowsOut = LINE ? kM - 2 : kM, kHalo = LINE ? 1 : 0;
   static constexpr int kWRows = LINE ? 3 * NT : NT;            // weight rows of a step held by one CTA, W_hi then W_lo
   static constexpr int kWBytes = kWRows * kKt * 4, kWHalf = kWBytes / 2;
-  // tensor memory: two accumulators of kAcc columns, then the cross sums.  The accumulators take alternate chunks, or where there is
+  // tensor memory: two accumulators of kAcc columns, then the cross sums.  The accumulators take alternate steps, or where there is
   // no room for two (kHalves) 32 features each.
   static constexpr bool kHalves = LINE && NT == 64;
   static constexpr int kAcc = LINE ? 96 : 2 * NT, kCross = LINE ? 3 * NT : NT;
@@ -287,7 +285,7 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
     } else if (crank == 0) {
       // ---------------------------------------------------------------- MMA issuers (the leader's, for both CTAs).  A warp needs several
       // hundred clocks for the waits, commits and counting of a step, in which it issues nothing, so two share a step: the first takes
-      // x_hi . [W_hi | W_lo], or with LINE x_hi . W_hi, into accumulators that the epilogue takes over chunk by chunk, the second the
+      // x_hi . [W_hi | W_lo], or with LINE x_hi . W_hi, into accumulators that the epilogue takes over step by step, the second the
       // other cross products, each step when the first has issued its part: the cross products of a step then run while the epilogue
       // takes over the sums (one warp: 1220 clk a step of 432 clk of MMAs; with LINE and no order the first waits for the epilogue
       // behind the second's queued MMAs).
@@ -296,7 +294,7 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
         constexpr bool kFirst = decltype(first_)::value;
         uint32_t as = 0, aph = 0, ws = 0, wph = 0, chunk_it = 0, tile_it = 0;
         for (long long t = t0; t < ntiles; t += t_step, tile_it++) {
-          int kt = 0, in_chunk = 0, cb = 0;
+          int kt = 0, cb = 0;
           for (int st = P.ng * P.nchb; st > 0; st--) {
             if (kFirst && !wait(a_full + 8 * as, aph, VST_A_FULL)) return;
             const int left = P.g.C - cb * kKt, nk8 = left >= kKt ? 4 : (left + 7) >> 3;   // behind the last channel both operands are zero
@@ -310,7 +308,6 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
               // to issue (7 otherwise)
               const uint32_t row = __shfl_sync(0xffffffffu, row_, 0), wd = __shfl_sync(0xffffffffu, desc_lo(w_ring + ws * kWBytes), 0);
               const uint32_t b = chunk_it & 1;
-              const bool ends = in_chunk + 1 == P.chunk_kt || kt == nkt - 1;
               auto groups = [&](auto full_) {
                 constexpr bool kFull = decltype(full_)::value;
                 if constexpr (kFirst && FM::kHalves) {
@@ -322,10 +319,10 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
                     tc_commit_pair(acc_full + 8 * h);
                   }
                 } else if constexpr (kFirst) {
-                  if (in_chunk == 0 && !wait(acc_empty + 8 * b, ((chunk_it >> 1) & 1) ^ 1, VST_ACC_EMPTY)) return false;
+                  if (!wait(acc_empty + 8 * b, ((chunk_it >> 1) & 1) ^ 1, VST_ACC_EMPTY)) return false;
                   tc_fence_after();
-                  mma_step32<idesc_tf32_pair(FM::kAcc), kFull>(tmem + b * FM::kAcc, row, wd, (uint32_t)in_chunk, nk8);
-                  if (ends) tc_commit_pair(acc_full + 8 * b);
+                  mma_step32<idesc_tf32_pair(FM::kAcc), kFull>(tmem + b * FM::kAcc, row, wd, 0u, nk8);
+                  tc_commit_pair(acc_full + 8 * b);
                 } else {
                   if (kt == 0 && !wait(cross_empty, (tile_it & 1) ^ 1, VST_ACC_EMPTY)) return false;   // the previous tile's cross sums have been read
                   tc_fence_after();
@@ -339,7 +336,7 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
                 return true;
               };
               if (!(nk8 == 4 ? groups(std::true_type{}) : groups(std::false_type{}))) return;
-              if (ends) { chunk_it++; in_chunk = 0; } else in_chunk++;
+              chunk_it++;
               tc_commit_pair(w_empty + 8 * ws);
               if (++ws == (uint32_t)P.w_stages) { ws = 0; wph ^= 1; }
               if (++dw == P.sub_w) { dw = 0; row_ += line; } else row_ += 8;
@@ -448,7 +445,6 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
     float* xch = (float*)(tail + kBarBytes);
     float* stash = (float*)(tail + kBarBytes + FM::kXchBytes);
     const uint32_t arr_acc = map_to_cta(acc_empty, 0), arr_cross = map_to_cta(cross_empty, 0);   // the leader's
-    const int nch = (nkt + P.chunk_kt - 1) / P.chunk_kt;
     uint32_t chunk_it = 0, tile_it = 0;
     for (long long t = t0; t < ntiles; t += t_step, tile_it++) {
       const int r = quad * 32 + lane;
@@ -464,7 +460,7 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
 #pragma unroll
         for (int j = 0; j < NH; j++) vx[j] = 0.f;
       }
-      for (int ch = 0; ch < nch; ch++, chunk_it++) {
+      for (int kt = 0; kt < nkt; kt++, chunk_it++) {
         const uint32_t b = FM::kHalves ? half : chunk_it & 1;
         wait(acc_full + 8 * b, (FM::kHalves ? chunk_it : chunk_it >> 1) & 1, VST_ACC_FULL);
         tc_fence_after();
@@ -498,7 +494,7 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
           for (int j = 0; j < NH; j++) vx[j] = __fadd_rn(vx[j], __uint_as_float(a[j]));
         }
       }
-      wait(cross_full, tile_it & 1, VST_CROSS_FULL);
+      wait(cross_full, tile_it & 1, VST_ACC_FULL);
       tc_fence_after();
       // What follows runs once a tile, so it is fetched instruction by instruction while the next tile's second step waits for these
       // warps: as few instructions as possible (packed arithmetic, whole rows to and from shared memory, no branch per feature).
@@ -659,8 +655,6 @@ EncodeFn encode_fn() {
   return fn = (EncodeFn)p;
 }
 
-int chunk_steps(const VolGeom& g) { return g.line || g.KD * g.KH * g.KW * ((g.C + 7) / 8 * 8) <= kShortK ? kChunkShort : kChunkLong; }
-
 // How a stage serves steps: those of a kd, of a line, or one; the widest sharing whose rows fit a box and leave two stages.  What
 // shared memory is left goes to the ring that reaches less far ahead, in steps.
 struct Sharing { int ng, tpg, sub_w, box_rows, a_stages, w_stages; size_t smem; };
@@ -749,6 +743,19 @@ bool vol_supported(const ConvGeom& c) {
   return g.P * g.fd * g.fh * g.fw < (1LL << 30) && (long long)c.KD * g.Hq * g.Wq < (1LL << 29) && pick_sharing(g, vol_nt(c.F), g.line, &s);
 }
 
+// Estimated device time of a layer whose input is packed first, ns: packing at 1.6 TB/s of what it writes, rounds of tiles, and in each the
+// steps (a tap each: stages shared or not; a line's taps: 32 or 64 features) and the tile's end.
+long long vol_cost(const ConvGeom& c) {
+  const VolGeom g = vol_geom(c, c.pd, c.ph, vol_front_w(c));
+  const int NT = vol_nt(c.F), pitch = (c.C + 31) / 32 * 32;
+  Sharing s;
+  if (!pick_sharing(g, NT, g.line, &s)) return 1LL << 60;
+  const long long rows = (((long long)(g.N - 1) * g.Dq + g.Do - 1) * g.Hq + g.Ho - 1) * g.Wq + g.Wo, per_pair = g.line ? 252 : 256, pairs = sm_count() / 2;
+  const long long tiles = (rows + per_pair - 1) / per_pair * ((c.F + NT - 1) / NT), rounds = (tiles + pairs - 1) / pairs, steps = (long long)s.ng * s.tpg * (pitch / 32);
+  const long long step = g.line ? (NT == 64 ? 680 : 600) : s.tpg > 1 ? 380 : 570, end = g.line ? 2600 : 1500;
+  return 4500 + (long long)(vol_bytes(g, pitch) / 1600) + rounds * (steps * step + end);
+}
+
 struct VolW { int F = 0, C = 0, taps = 0, kw = 1, NT = 0, nchb = 0, ntn = 0; float* img = nullptr; CUtensorMap map; };     // kw: taps of a step
 
 void vol_weights_free(VolW* w) {
@@ -801,7 +808,6 @@ bool vol_conv(const VolW* w, const float* vol, int pitch, const VolGeom& g, cons
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return fail("cuTensorMapEncodeTiled failed for a split volume");
   P.wmap = w->map; P.g = g; P.nchb = w->nchb; P.ntn = w->ntn;
-  P.chunk_kt = chunk_steps(g);
   P.ng = sh.ng; P.tpg = sh.tpg; P.sub_w = sh.sub_w; P.box_rows = sh.box_rows; P.a_stages = sh.a_stages; P.w_stages = sh.w_stages;
   P.rows = (((long long)(g.N - 1) * g.Dq + g.Do - 1) * g.Hq + g.Ho - 1) * g.Wq + g.Wo;
   P.bias = bias; P.act = act; P.slope = slope; P.F = w->F;

@@ -129,9 +129,12 @@ struct F32TcLaunch {
   float* Y;                                                                // ... or a (rows, n_out) output
   RowGeom g;
   float* act[2]; long long act_ld;                   // two feature-major activation buffers [max width][act_ld], act_ld >= rows
+  int pair;                                          // act[] hold f32tc_pair_bytes() each: the layers run on pairs of CTAs
   double* partials; double* sum; unsigned int* done; // optional checksum of the fused scatter (partials: f32tc_grid() doubles)
   int* status;
 };
+bool f32tc_pair_wanted(const F32TcModel* m, long long nrows);      // fortis_mlp_pair.cu
+size_t f32tc_pair_bytes(const F32TcModel* m, long long nrows);     // of each of its two buffers
 int f32tc_grid(long long nrows);
 constexpr long long kF32TcMaxRows = (1LL << 31) - 129;     // the activations' tiles are addressed by 32-bit row numbers
 bool f32tc_forward(F32TcModel* m, const F32TcLaunch& L, cudaStream_t s, std::string* err);
@@ -164,6 +167,15 @@ bool rows_mlp_forward(RowsMlp* m, const F32TcLaunch& L, cudaStream_t s, std::str
 // normal.clamp_min(0), normal weights: 8 products 9.2e-8 / 5.3e-8 and 8.8e-8 / 4.2e-8, 27: 1.3e-7 / 9.4e-8 and 1.2e-7 / 7.0e-8,
 // 64: 1.4e-7 / 1.4e-7 and 1.2e-7 / 1.0e-7, 96: 1.35e-7 / 1.8e-7 and 1.23e-7 / 1.27e-7, 128: 1.4e-7 / 2.0e-7 and 1.3e-7 / 1.5e-7.
 constexpr int kF32TcConvMinProducts = 128;
+// one fp32 convolution layer on the split-TF32 kernel of fortis_mlp_f32tc.cu, whose threads load the taps
+struct F32ConvW;                                       // split weights of one layer
+bool f32tc_conv_supported(const ConvGeom& g);
+long long f32tc_conv_cost(const ConvGeom& g);          // estimated device time, ns
+F32ConvW* f32tc_conv_pack(const float* w_dev, int F, int C, int taps, cudaStream_t s, std::string* err);
+void f32tc_conv_free(F32ConvW* w);
+bool f32tc_conv(const F32ConvW* w, const float* x, const float* bias, const float* residual, float* y, const ConvGeom& g, int act,
+                float slope, int* status, cudaStream_t s, bool early, std::string* err);
+// the same over split volumes
 struct VolGeom {
   int N, D, H, W, C, Do, Ho, Wo;
   int KD, KH, KW, sd, sh, sw;
@@ -177,6 +189,7 @@ struct VolGeom {
 VolGeom vol_geom(const ConvGeom& c, int front_d, int front_h, int front_w);
 int vol_front_w(const ConvGeom& c);                            // zero positions a layer needs in front of a line
 bool vol_supported(const ConvGeom& c);
+long long vol_cost(const ConvGeom& c);                         // estimated device time with the input packed, ns
 size_t vol_bytes(const VolGeom& g, int pitch);                 // of a split volume with `pitch` channels a row (a multiple of 32)
 struct VolW;                                                   // one layer's weights, split, as the kernel streams them
 // torch layout (F, C, taps); `line`: as vol_geom says of the layer

@@ -1,32 +1,34 @@
-// fp32-class Linear layers on the tensor cores: C = act(A . W^T + b) with every product formed as three
+// fp32-class Linear layers and convolutions on the tensor cores: C = act(A . W^T + b) with every product formed as three
 // TF32 MMAs
 //     A . W  ~=  A_hi . W_hi + A_hi . W_lo + A_lo . W_hi        (x_hi = tf32(x), x_lo = x - x_hi, accumulation in fp32)
 // which keeps 21 significant bits per operand at six bf16-MMA-equivalents per multiply-add instead of one FFMA per MAC.
 //
 // Replaces, for the fp32 precision, the reference's large-batch lowering of a Linear layer: fortis_gemm = cuBLAS SGEMM on
 // pre-transposed weights plus a separate bias / activation kernel (runtime/fortis_rt.c:45-75, compiler/FortisFuse.cpp:616-624,
-// 687-760), with fortis_gather_k in front and fortis_scatter_k behind (driver/fortis_gather_emit.py:52-62, 75-83): the gather
-// is fused into the first layer's operand load, bias + activation into every epilogue, the scatter (and the fp64 checksum)
-// into the last one.  Activations travel between layers in fp32, feature-major ([feature][row]: the memory order of a Fortran
-// (ncol, nlev) array), so both the epilogue's stores and the next layer's loads are coalesced with one thread per row.
-// (Convolutions: fortis_conv3d_f32.cu.)
+// 687-760), with fortis_gather_k in front and fortis_scatter_k behind (driver/fortis_gather_emit.py:52-62, 75-83), and its
+// cuDNN convolutions (runtime/fortis_rt.c:108-156): the gather is fused into the first layer's operand load, bias +
+// residual + activation into every epilogue, the scatter (and the fp64 checksum) into the last one.  Activations travel
+// between layers in fp32, feature-major ([feature][row]: the memory order of a Fortran (ncol, nlev) array and of an NCDHW
+// volume), so both the epilogue's stores and the next layer's loads are coalesced with one thread per row.
 //
 // One persistent CTA per SM, output tiles of 128 rows x NT (32, 64 or 128) features, K in steps of 32:
 //   * fp32 activations arrive as tiles through the TMA (a feature-major buffer, or a row-major matrix whose rows start on
-//     16-byte boundaries), or are loaded by the threads (host arrays through the slot table, other matrices); two sets of four warps (thread = row; the sets take alternate k steps) split them and write
+//     16-byte boundaries), or are loaded by the threads (host arrays through the slot table, other matrices, a volume at
+//     the taps' offsets); two sets of four warps (thread = row; the sets take alternate k steps) split them and write
 //     A_hi / A_lo into TENSOR MEMORY (lane = row);
 //   * one warp brings the matching W_hi / W_lo tiles (split once) into shared memory with two TMA loads;
 //   * one warp issues, per 8-wide k step, the three kind::tf32 MMAs (M = 128, N = NT, A from tensor memory);
-//   * two sets of four warps (thread = row, half of the features) read the accumulator, add the bias, apply the
+//   * two sets of four warps (thread = row, half of the features) read the accumulator, add bias (and residual), apply the
 //     activation and store.
 // Operand traffic is why A sits in tensor memory: with A in shared memory (the form before this one) the three MMAs of a
 // k step read 12 KB per 128 clocks and the producers and the TMA write 96 KB per 1536, together 1.25 times what shared
 // memory moves; in this form only the weights (64 B/clk at any NT) and the fp32 tiles pass through it.
 // Measured, that form / this one: fortis_gemm 8192 x 768 x 768 756 / 62 us (a row-major operand was read by one dependent load
-// per row), column network 30,011 rows 991 / 750 us.
+// per row), column network 30,011 rows 991 / 750 us; convolutions against the FFMA kernel: 32 -> 64 channels 3x3x3 on 40^3
+// 297 / 73 us, 14-layer network 2 x 33^3 8.75 / 2.02 ms.
 //
 // The tensor core adds into its fp32 accumulator with truncation, not rounding, a bias per accumulation of half a unit in
-// the last place of the partial sum.  In fortis_gemm two things keep it below fp32 rounding: the hi.hi
+// the last place of the partial sum.  In convolutions and fortis_gemm two things keep it below fp32 rounding: the hi.hi
 // products go into an accumulator of their own that is taken over every 64 k (8 truncating additions; 32 where K is short)
 // and summed by the epilogue warps in registers with IEEE additions, and the two cross products go into a second accumulator
 // (2^-11 of the result, so its truncation does not count) that lives for the whole K.  MLP steps keep the three products in
@@ -34,6 +36,7 @@
 // Infinities: x_hi saturates at the largest finite TF32 value and x_lo = x - x_hi carries the infinity, so a product is
 // infinite, or NaN, where the fp32 product is.  Every barrier wait is bounded; a CTA
 // whose wait gives up records which one, lets its copies and MMAs in flight finish and returns.
+// (Convolutions of many steps or voxels run on fortis_conv3d_f32.cu: conv_layer in fortis_conv3d.cu says which.)
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -47,6 +50,7 @@
 
 #include "fortis_device.cuh"
 #include "fortis_kernels.h"
+#include "fortis_mlp_pair.h"
 #include "fortis_model.h"
 #include "fortis_tc.cuh"
 
@@ -59,24 +63,31 @@ using namespace tc;
 constexpr int kM = 128;                    // rows per tile
 constexpr int kKt = 32;                    // k per stage: one 128-byte swizzle row of fp32
 // k steps of 32 accumulated in the tensor core before the sum is taken over: two, or one where K is short, so that the
-// truncations (a bias) stay below the few roundings fp32 arithmetic has there
+// truncations (a bias) stay below the few roundings fp32 arithmetic has there (2-D network of K = 27 to 576, six
+// convolutions, error against 64 bits: two 9.1e-7, one 6.2e-7, FFMA 7.7e-7)
 constexpr int kChunkLong = 2, kChunkShort = 1, kShortK = 640;
 // MLP steps keep the sums they have always had: the three products of a step of 8 k one after another in one accumulator
 // that is taken over every 128 k.  Further from the exact sums (five-layer column network 5.6e-6 against 2.4e-6), but the sums
 // a program has had of finite inputs.
 constexpr int kChunkMlp = 4;
+// Convolutions multiply x_lo by 2^10 (exact) and the cross sums by 2^-10: the tensor core takes subnormal operands as zero, and
+// unscaled x_lo is subnormal from |x| < 2^-102 on (2^-118: error 2.2e-6).  With it every normal value keeps its precision.
+// (x_lo is below 2^-10 of the largest value, so the product stays finite.)
+constexpr float kLoScale = 1024.f;
 constexpr int kBarF = 384;
 constexpr int kTabIn = 768, kTabOut = 256;     // widest gathered input / scattered output the tables hold
 constexpr int kTileScratch = 32 * 32 * 4;      // one warp's 32 x 32 transpose
+constexpr int kConvTabMax = 40 * 1024;         // widest table of taps a convolution may need
 // warps 0-7 produce A (two sets of four that take alternate k steps), 8-15 are the epilogue (two sets, half of the
-// features each), then the two TMA warps and the MMA warp.
+// features each), then the two TMA warps and the MMA warp.  (Three producer sets and one epilogue set for the
+// convolutions: 64 -> 64 channels 3 % slower.)
 constexpr int kPSets = 2, kPWarps = 8, kESets = 2, kEWarps = 8, kWarpW = 16, kWarpA = 17, kWarpMma = 18;
 constexpr int kThreadsF = 19 * 32;
 constexpr int kRawStages = 4;                  // fp32 activation tiles on their way to the producers, 16 KB each
 constexpr int kRawBytes = kM * kKt * 4;
 enum { FST_A_FULL = 21, FST_A_EMPTY = 22, FST_ACC_FULL = 23, FST_ACC_EMPTY = 24, FST_ALIGN = 25, FST_W_FULL = 26, FST_W_EMPTY = 27, FST_RAW_FULL = 28, FST_RAW_EMPTY = 29 };
-enum { A_TILE_T = 0, A_TILE_R = 1, A_ROW_MAJOR = 2, A_GATHER = 3 };   // the first two through the TMA
-enum { C_FEATURE_MAJOR = 0, C_ROW_MAJOR = 1, C_SCATTER = 2 };
+enum { A_TILE_T = 0, A_TILE_R = 1, A_ROW_MAJOR = 2, A_GATHER = 3, A_CONV8 = 4, A_CONV1 = 5 };   // the first two through the TMA
+enum { C_FEATURE_MAJOR = 0, C_ROW_MAJOR = 1, C_SCATTER = 2, C_CONV = 3 };
 
 template <int NT> struct TileCfg {
   static constexpr int kAStages = NT == 128 ? 2 : 4;     // 64 tensor-memory columns each (32 hi, 32 lo)
@@ -104,6 +115,7 @@ struct F32Params {
   CUtensorMap map_a;                     // A_TILE_T: [K][rows], box 128 rows x 32; A_TILE_R: [rows][K], box 32 x 128, 128-byte swizzle
   const float* A; long long lda;
   const Access* slots; ArrayTable TG; StrideClassF cin[2]; RowGeom g;
+  ConvGeom cv; const float* residual;    // A_CONV*: x = A, y = C
   int c_mode; float* C; long long ldc; int c_vec;
   const Access* store_by_slot; ArrayTable TS; StrideClassF cout[2];
   long long nrows;
@@ -173,8 +185,9 @@ template <int AMODE>
 struct ACursor {
   long long t;
   int kt;
-  const float* rowp;            // row-major: the tile's first row
+  const float* rowp;            // conv: the element tap 0 of this row reads (may lie outside the volume)
   long long p0, p1;             // gather: byte positions of the two stride classes
+  uint32_t md, mh, mw;          // conv: taps per axis that fall inside the volume
 };
 
 template <int AMODE>
@@ -189,6 +202,22 @@ __device__ __forceinline__ void cursor_tile(const F32Params& P, ACursor<AMODE>& 
     c.p0 = 4 * (ci * P.cin[0].si + cj * P.cin[0].sj + kk * P.cin[0].sk);
     c.p1 = 4 * (ci * P.cin[1].si + cj * P.cin[1].sj + kk * P.cin[1].sk);
   }
+  if constexpr (AMODE == A_CONV8 || AMODE == A_CONV1) {
+    const ConvGeom& g = P.cv;
+    unsigned q = (unsigned)row;
+    const int ow = (int)(q % (unsigned)g.Wo); q /= (unsigned)g.Wo;
+    const int oh = (int)(q % (unsigned)g.Ho); q /= (unsigned)g.Ho;
+    const int od = (int)(q % (unsigned)g.Do);
+    const int on = (int)(q / (unsigned)g.Do);
+    const int id = od * g.sd - g.pd, ih = oh * g.sh - g.ph, iw = ow * g.sw - g.pw;
+    c.rowp = P.A + ((long long)on * g.xs_n + (long long)id * g.xs_d + (long long)ih * g.xs_h + (long long)iw * g.xs_w);
+    auto inside = [](int first, int extent, int taps) {          // bit k: 0 <= first + k < extent
+      const int lo = first < 0 ? -first : 0, hi = extent - first < taps ? extent - first : taps;
+      const uint32_t upto = hi <= 0 ? 0u : (hi >= 32 ? 0xFFFFFFFFu : (1u << hi) - 1u);
+      return lo >= 32 ? 0u : (upto >> lo) << lo;
+    };
+    c.md = inside(id, g.D, g.KD); c.mh = inside(ih, g.H, g.KH); c.mw = inside(iw, g.W, g.KW);
+  }
 }
 
 template <int AMODE, int STEP>
@@ -199,7 +228,7 @@ __device__ __forceinline__ void cursor_advance(const F32Params& P, ACursor<AMODE
   if (c.t < ntiles) cursor_tile<AMODE>(P, c, r);
 }
 
-// `tab`: gather: 64-bit addresses (bit 0: stride class, 0: no such input)
+// `tab`: gather: 64-bit addresses (bit 0: stride class, 0: no such input); conv: {element offset, taps | channels << 24}
 template <int AMODE>
 __device__ __forceinline__ void cursor_load(const F32Params& P, const ACursor<AMODE>& c, const uint2* tab, int quad, int lane, int k0, float (&v)[kKt]) {
   if constexpr (AMODE == A_ROW_MAJOR) {
@@ -214,6 +243,28 @@ __device__ __forceinline__ void cursor_load(const F32Params& P, const ACursor<AM
     for (int j = 0; j < kKt; j++) {
       const unsigned long long e = *reinterpret_cast<const unsigned long long*>(tab + k0 + j);
       v[j] = ld_ahead_if(reinterpret_cast<const float*>((e & ~1ull) + (unsigned long long)((e & 1ull) ? c.p1 : c.p0)), e != 0ull);
+    }
+  } else if constexpr (AMODE == A_CONV8) {
+#pragma unroll
+    for (int gq = 0; gq < kKt / 8; gq++) {
+      const uint2 e = tab[k0 / 8 + gq];
+      const bool in = ((c.md >> (e.y & 0xFF)) & (c.mh >> ((e.y >> 8) & 0xFF)) & (c.mw >> ((e.y >> 16) & 0xFF)) & 1u) != 0u;
+      const float* p = c.rowp + (int)e.x;
+      const int n = (int)(e.y >> 24);
+      if (n == 8) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) { v[8 * gq + j] = ld_ahead_if(p, in); p += P.cv.xs_c; }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; j++) { v[8 * gq + j] = ld_ahead_if(p, in && j < n); p += P.cv.xs_c; }
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < kKt; j++) {
+      const uint2 e = tab[k0 + j];
+      const bool in = ((c.md >> (e.y & 0xFF)) & (c.mh >> ((e.y >> 8) & 0xFF)) & (c.mw >> ((e.y >> 16) & 0xFF)) & (e.y >> 24)) != 0u;
+      v[j] = ld_ahead_if(c.rowp + (int)e.x, in);
     }
   }
 }
@@ -241,13 +292,14 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
                  cross_empty = bars + 192, raw_full = bars + 208, raw_empty = bars + 240;
   uint32_t* tmem_slot = (uint32_t*)(tail + 200);
   volatile int* abort_flag = (volatile int*)(tail + 204);
+  constexpr bool kMaybeOneAcc = AMODE != A_CONV8 && AMODE != A_CONV1;
   constexpr bool kTile = AMODE == A_TILE_T || AMODE == A_TILE_R;
   uint8_t* a_scratch = tail + kBarF + kEWarps * 2 * (NT / kESets) * 4;
   uint8_t* c_scratch = a_scratch + (AMODE == A_ROW_MAJOR ? kPWarps * kTileScratch : 0);
   uint8_t* tables = c_scratch + (P.c_mode == C_ROW_MAJOR ? kEWarps * kTileScratch : 0);
   const int nkt = P.K_pad / kKt;
   uint2* tab = (uint2*)tables;
-  const int ntab = AMODE == A_GATHER ? P.K_pad * (P16 ? 2 : 1) : 0;
+  const int ntab = AMODE == A_GATHER ? P.K_pad * (P16 ? 2 : 1) : AMODE == A_CONV8 ? nkt * (kKt / 8) : AMODE == A_CONV1 ? nkt * kKt : 0;
   unsigned long long* o_tab = (unsigned long long*)(tab + ntab);      // scatter: 64-bit addresses, as the gather's
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -271,6 +323,22 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
         e = (unsigned long long)((const float*)P.TG.base[a.array] + a.off0) | (c0 ? 0ull : 1ull);
       }
       reinterpret_cast<unsigned long long*>(tab)[q] = e;
+    }
+  }
+  if constexpr (AMODE == A_CONV8 || AMODE == A_CONV1) {
+    const ConvGeom& g = P.cv;
+    constexpr int G = AMODE == A_CONV8 ? 8 : 1;
+    const int per_tap = (g.C + G - 1) / G, ntaps = g.KD * g.KH * g.KW;
+    for (int q = threadIdx.x; q < ntab; q += kThreadsF) {
+      uint2 e = make_uint2(0u, 0u);
+      if (q < ntaps * per_tap) {
+        const int tap = q / per_tap, c0 = (q - tap * per_tap) * G;
+        const int kd = tap / (g.KH * g.KW), kh = (tap / g.KW) % g.KH, kw = tap % g.KW;
+        const int n = g.C - c0 < G ? g.C - c0 : G;
+        e.x = (uint32_t)(int)((long long)kd * g.xs_d + (long long)kh * g.xs_h + (long long)kw * g.xs_w + (long long)c0 * g.xs_c);
+        e.y = (uint32_t)kd | ((uint32_t)kh << 8) | ((uint32_t)kw << 16) | ((uint32_t)n << 24);
+      }
+      tab[q] = e;
     }
   }
   if (P.c_mode == C_SCATTER)
@@ -365,7 +433,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
           tc_mma_ts_first<idesc>(acc, ah, wh, in_chunk);
 #pragma unroll
           for (int j = 1; j < kKt / 8; j++) tc_mma_ts_acc<idesc>(acc, ah + 8 * j, wh + (uint64_t)(2 * j));    // 16 k = 32 bytes
-        } else if (P.one_acc) {
+        } else if (kMaybeOneAcc && P.one_acc) {
 #pragma unroll
           for (int j = 0; j < kKt / 8; j++) {
             mma_tf32_ts<idesc>(acc, ah + 8 * j, wh + (uint64_t)(2 * j), in_chunk | (uint32_t)j);
@@ -411,6 +479,7 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
 #pragma unroll
       for (int j = 0; j < 16; j++) {
         split_tf32(v[j], hi[j], lo[j]);
+        if constexpr (!kMaybeOneAcc) lo[j] = __float_as_uint(__uint_as_float(lo[j]) * kLoScale);
       }
       tmem_st16(dst, hi);
       tmem_st16(dst + 32, lo);
@@ -571,20 +640,53 @@ __global__ void __launch_bounds__(kThreadsF, 1) f32tc_kernel(const __grid_consta
         if (lane == 0) mbar_arrive(acc_empty + 8 * b);
       }
       if (!ok) break;
-      if (P16 == 0 && !P.one_acc) {
+      if (P16 == 0 && !(kMaybeOneAcc && P.one_acc)) {
 #pragma unroll
       for (int c0 = 0; c0 < NH; c0 += NL) {
         uint32_t a[NL];
         tmem_ldn(lane_addr + CF::kColCross + c0, a);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < NL; j++) v[c0 + j] = __fadd_rn(v[c0 + j], __uint_as_float(a[j]));
+        for (int j = 0; j < NL; j++) {
+          if constexpr (kMaybeOneAcc) v[c0 + j] = __fadd_rn(v[c0 + j], __uint_as_float(a[j]));
+          else v[c0 + j] = fmaf(__uint_as_float(a[j]), 1.f / kLoScale, v[c0 + j]);
+        }
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(cross_empty);
       }
 
+      if (P16 == 0 && P.c_mode == C_CONV) {
+        const ConvGeom& g = P.cv;
+        unsigned q = (unsigned)(live ? row : 0);
+        const int ow = (int)(q % (unsigned)g.Wo); q /= (unsigned)g.Wo;
+        const int oh = (int)(q % (unsigned)g.Ho); q /= (unsigned)g.Ho;
+        const int od = (int)(q % (unsigned)g.Do), on = (int)(q / (unsigned)g.Do);
+        const long long yo = (long long)on * g.ys_n + (long long)od * g.ys_d + (long long)oh * g.ys_h + (long long)ow * g.ys_w + nt0 * g.ys_c;
+        const long long ro = (long long)on * g.rs_n + (long long)od * g.rs_d + (long long)oh * g.rs_h + (long long)ow * g.rs_w + nt0 * g.rs_c;
+        if (!live) continue;
+#pragma unroll
+        for (int c0 = 0; c0 < NH; c0 += 16) {
+          float o[16];
+          if (P.residual) {
+#pragma unroll
+            for (int j = 0; j < 16; j++) o[j] = ld_ahead_if(P.residual + ro + (long long)(c0 + j) * g.rs_c, nt0 + c0 + j < P.N_real);
+          }
+#pragma unroll
+          for (int j = 0; j < 16; j++) v[c0 + j] += s_bias[c0 + j];
+#pragma unroll
+          for (int j = 0; j < 16; j++) o[j] = P.residual ? v[c0 + j] + o[j] : v[c0 + j];
+          act_f32(o, P.act, P.slope);
+          float* dst = P.C + yo + (long long)c0 * g.ys_c;
+#pragma unroll
+          for (int j = 0; j < 16; j++) {
+            if (nt0 + c0 + j < P.N_real) *dst = o[j];
+            dst += g.ys_c;
+          }
+        }
+        continue;
+      }
       if constexpr (P16 != 0) {
         // the fused kernel's expressions, hidden and last layer
         if (!P.scale) {
@@ -728,6 +830,19 @@ __global__ void split_weights_kernel(const float* __restrict__ W, int N, int K, 
   }
 }
 
+// the same for convolution weights (F, C, taps): reduction index = (tap, channel), channels padded to whole groups
+__global__ void split_conv_weights_kernel(const float* __restrict__ W, int F, int C, int taps, int group, uint32_t* __restrict__ hi,
+                                          uint32_t* __restrict__ lo, int N_pad, int K_pad) {
+  const long long n_el = (long long)N_pad * K_pad;
+  const int cp = (C + group - 1) / group * group;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_el; i += (long long)gridDim.x * blockDim.x) {
+    const int n = (int)(i / K_pad), k = (int)(i % K_pad), tap = k / cp, c = k - tap * cp;
+    uint32_t h = 0, l = 0;
+    if (n < F && tap < taps && c < C) split_tf32(W[((long long)n * C + c) * taps + tap], h, l);
+    hi[i] = h; lo[i] = __float_as_uint(__uint_as_float(l) * kLoScale);
+  }
+}
+
 typedef CUresult (*EncodeTiledFnF)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                    const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -807,9 +922,10 @@ bool split_alloc(SplitW* w, int K, int N, std::string* err) {
 // The tile width (0, 1, 2: 32, 64, 128 features).  A k step of a tile costs 6 clocks per feature of tensor time, or what
 // its producers need for 128 rows x 32 inputs if that is more (step_floor), and the launch lasts as many rounds of tiles as
 // the SM that has the most.  The floors are estimates, and low ones: a step with its share of the tile's end measures 1140,
-// 1200, 1520 clocks at 32, 64, 128 features (fortis_gemm, K = 768), 2210, 2310, 2520 with rows off 16 bytes.  So the rule takes
-// tiles that are too narrow: the width it picks is within 5 % of the fastest for 276 of 390 products (8 to 1000 features, 13 to
-// 1138 row tiles; at worst 2.4 times the time).
+// 1200, 1520 clocks at 32, 64, 128 features (fortis_gemm, K = 768), 2210, 2310, 2520 with rows off 16 bytes, 1240, 1280, 1430 in
+// convolutions of K = 1728 and 1960, 2100, 2460 of K = 405.  So the rule takes tiles that are too narrow: over 8 to 256 features
+// and 13 to 1138 row tiles the width it picks is within 5 % of the fastest for every convolution of up to 64 features and 147
+// of 240 wider ones (at worst 1.76 times the time), and for 276 of 390 products (8 to 1000 features; at worst 2.4 times).
 int pick_tile(long long nrows, int N, int step_floor) {
   const long long ntm = (nrows + kM - 1) / kM, sms = sm_count();
   long long best_cost = 0;
@@ -826,10 +942,13 @@ int pick_tile(long long nrows, int N, int step_floor) {
 template <int NT, int AMODE, int P16>
 size_t smem_bytes(const F32Params& P) {
   using CF = TileCfg<NT>;
+  const int nkt = P.K_pad / kKt;
   size_t n = CF::kWBytes + kBarF + kEWarps * 2 * (NT / kESets) * 4 + (AMODE == A_TILE_T || AMODE == A_TILE_R ? kRawStages * kRawBytes : 0);
   if (AMODE == A_ROW_MAJOR) n += kPWarps * kTileScratch;
   if (P.c_mode == C_ROW_MAJOR) n += kEWarps * kTileScratch;
   if (AMODE == A_GATHER) n += (size_t)P.K_pad * (P16 ? 2 : 1) * 8;
+  if (AMODE == A_CONV8) n += (size_t)nkt * (kKt / 8) * 8;
+  if (AMODE == A_CONV1) n += (size_t)nkt * kKt * 8;
   if (P.c_mode == C_SCATTER) n += kTabOut * 8;
   return n;
 }
@@ -868,7 +987,8 @@ bool launch_tile(F32Params& P, const SplitW& W, int step_floor, cudaStream_t s, 
   return w == 2 ? launch_as<128, AMODE>(P, s, early) : w == 1 ? launch_as<64, AMODE>(P, s, early) : launch_as<32, AMODE>(P, s, early);
 }
 
-constexpr int kStepFloorLinear = 250;       // clocks a k step's producers need at least (see pick_tile)
+// clocks a k step's producers need at least (see pick_tile)
+constexpr int kStepFloorLinear = 250, kStepFloorConv = 350;
 
 // a row-major operand: tiles through the TMA where rows start on 16-byte boundaries, else loads
 bool launch_rows(F32Params& P, const float* A, int K, const SplitW& W, cudaStream_t s, bool early) {
@@ -941,6 +1061,44 @@ F32TcModel* f32tc_create(const ModelHost& M, std::string* err) {
   return m;
 }
 
+bool f32tc_pair_wanted(const F32TcModel* m, long long nrows) {
+  static const char* dev = std::getenv("FORTIS_PAIR_DEV");
+  if (dev) return dev[0] != '0' && m->layers.size() >= 2;
+  return m->layers.size() >= 2;
+}
+
+size_t f32tc_pair_bytes(const F32TcModel* m, long long nrows) {
+  int w = m->layers.front().w.K_real;
+  for (size_t l = 0; l + 1 < m->layers.size(); l++) w = m->layers[l].w.N_real > w ? m->layers[l].w.N_real : w;
+  return (size_t)nrows * round_up_f(w, 32) * 8;
+}
+
+static bool pair_forward(F32TcModel* m, const F32TcLaunch& L, bool fast_in, bool fast_out, cudaStream_t s, std::string* err) {
+  const long long nrows = L.g.count * L.g.nk;
+  const int nl = (int)m->layers.size(), n_in = m->layers.front().w.K_real;
+  if (fast_in) pair_split_gathered(L.slots, L.TG, L.g, n_in, m->in_div, L.act[1], nrows, s);
+  else pair_split_rows(L.X, n_in, m->in_div, L.act[1], nrows, s);
+  for (int l = 0; l < nl; l++) {
+    const F32TcModel::Layer& T = m->layers[l];
+    PairLayer p;
+    std::memset(&p, 0, sizeof p);
+    p.a = L.act[(l + 1) & 1]; p.nrows = nrows; p.K = T.w.K_real; p.N = T.w.N_real;
+    for (int i = 0; i < 2; i++) { p.map_hi[i] = &T.w.map_hi[i + 1]; p.map_lo[i] = &T.w.map_lo[i + 1]; }
+    p.bias = T.bias; p.act = T.act; p.slope = T.slope; p.status = L.status; p.g = L.g;
+    if (l < nl - 1) p.out = L.act[l & 1];
+    else {
+      p.out_mul = m->out_mul; p.relu_mask = m->relu_mask;
+      if (fast_out) {
+        p.store_by_slot = L.store_by_slot; p.TS = L.TS;
+        std::memcpy(p.cout, L.cout, sizeof p.cout);
+        p.partials = L.partials; p.sum = L.partials ? L.sum : nullptr; p.done = L.done;
+      } else p.Y = L.Y;
+    }
+    if (!pair_layer(p, s, err)) return false;
+  }
+  return launched(true, err);
+}
+
 int f32tc_grid(long long nrows) {
   (void)nrows;
   return sm_count();
@@ -955,6 +1113,7 @@ bool f32tc_forward(F32TcModel* m, const F32TcLaunch& L, cudaStream_t s, std::str
   if (!fast_in && !L.X) { if (err) *err = "split-TF32 step: no input"; return false; }
   if (!fast_out && !L.Y) { if (err) *err = "split-TF32 step: no output"; return false; }
   if (nl > 1 && (!L.act[0] || (nl > 2 && !L.act[1]))) { if (err) *err = "split-TF32 step: no activation buffers"; return false; }
+  if (L.pair) return pair_forward(m, L, fast_in, fast_out, s, err);
   for (int l = 0; l < nl; l++) {
     const F32TcModel::Layer& T = m->layers[l];
     F32Params P;
@@ -1132,6 +1291,66 @@ bool rows_mlp_forward(RowsMlp* m, const F32TcLaunch& L, cudaStream_t s, std::str
     if (!launched(ok, err)) return false;
   }
   return true;
+}
+
+// ---- convolutions ----------------------------------------------------------------------------------------------
+
+struct F32ConvW { SplitW w; int C = 0, taps = 0, group = 1; };
+
+// channels per table entry: groups of 8 share one test of a tap's position; with few channels that would mostly pad
+static int conv_group(int C) { return (C % 8 == 0 || C > 16) ? 8 : 1; }
+
+bool f32tc_conv_supported(const ConvGeom& g) {
+  if (g.dd != 1 || g.dh != 1 || g.dw != 1) return false;                       // transposed convolutions
+  if (g.KD > 32 || g.KH > 32 || g.KW > 32) return false;                       // one bit per tap and axis
+  // the most products an output can have: taps that lie inside the volume, times channels
+  const long long inside = (long long)(g.KD < g.D ? g.KD : g.D) * (g.KH < g.H ? g.KH : g.H) * (g.KW < g.W ? g.KW : g.W);
+  if (inside * g.C < kF32TcConvMinProducts) return false;
+  const int G = conv_group(g.C);
+  const long long taps = (long long)g.KD * g.KH * g.KW, entries = taps * ((g.C + G - 1) / G);
+  if (entries * 8 + 32 * 8 > kConvTabMax) return false;
+  // row numbers and the offsets of taps and channels in 32 bits
+  const long long rows = (long long)g.N * g.Do * g.Ho * g.Wo;
+  const long long reach = (g.KD - 1) * g.xs_d + (g.KH - 1) * g.xs_h + (g.KW - 1) * g.xs_w + (g.C - 1) * g.xs_c;
+  return rows < (1LL << 31) - kM && reach < (1LL << 31);
+}
+
+// Estimated device time of a layer, ns: rounds of tiles times steps of 32 k, a step as it measures in one round of tiles and in many (groups of
+// eight channels 0.56 to 0.75 us, single channels 0.73 to 1.3 us).
+long long f32tc_conv_cost(const ConvGeom& g) {
+  const int G = conv_group(g.C), w = pick_tile((long long)g.N * g.Do * g.Ho * g.Wo, g.F, kStepFloorConv), nt = 32 << w;
+  const long long steps = ((long long)g.KD * g.KH * g.KW * ((g.C + G - 1) / G * G) + kKt - 1) / kKt;
+  const long long tiles = (((long long)g.N * g.Do * g.Ho * g.Wo + kM - 1) / kM) * ((g.F + nt - 1) / nt), sms = sm_count(), rounds = (tiles + sms - 1) / sms;
+  static const int one[2] = {730, 560}, many[2][3] = {{1030, 1100, 1300}, {650, 670, 750}};
+  return rounds * (steps * (rounds == 1 ? one[G == 8] : many[G == 8][w]) + 1000);
+}
+
+void f32tc_conv_free(F32ConvW* w) {
+  if (!w) return;
+  split_free(&w->w);
+  delete w;
+}
+
+// w_dev: torch layout (F, C, taps) on the device; split on stream `s`
+F32ConvW* f32tc_conv_pack(const float* w_dev, int F, int C, int taps, cudaStream_t s, std::string* err) {
+  F32ConvW* w = new F32ConvW();
+  w->C = C; w->taps = taps; w->group = conv_group(C);
+  if (!split_alloc(&w->w, taps * ((C + w->group - 1) / w->group * w->group), F, err)) { delete w; return nullptr; }
+  split_conv_weights_kernel<<<split_grid((size_t)w->w.N_pad * w->w.K_pad), 256, 0, s>>>(w_dev, F, C, taps, w->group, (uint32_t*)w->w.hi, (uint32_t*)w->w.lo,
+                                                                                       w->w.N_pad, w->w.K_pad);
+  return w;
+}
+
+bool f32tc_conv(const F32ConvW* w, const float* x, const float* bias, const float* residual, float* y, const ConvGeom& g, int act,
+                float slope, int* status, cudaStream_t s, bool early, std::string* err) {
+  F32Params P;
+  std::memset(&P, 0, sizeof P);
+  P.nrows = (long long)g.N * g.Do * g.Ho * g.Wo;
+  if (P.nrows <= 0) return true;
+  P.status = status; P.bias = bias; P.act = act; P.slope = slope;
+  P.A = x; P.cv = g; P.residual = residual;
+  P.c_mode = C_CONV; P.C = y;
+  return launched(w->group == 8 ? launch_tile<A_CONV8>(P, w->w, kStepFloorConv, s, early) : launch_tile<A_CONV1>(P, w->w, kStepFloorConv, s, early), err);
 }
 
 }  // namespace fortis
