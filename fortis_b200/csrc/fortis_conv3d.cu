@@ -416,7 +416,10 @@ float* vol_workspace(size_t bytes, cudaStream_t s) {
 // threads load the taps, or on the FFMA kernels (sums of few products: f32tc_conv_supported).  Small calls of few channels and many taps are
 // faster without packing (7 -> 47 channels 5x5x5 on 2 x 10x8x8 29 us, over a split volume 59; 10 -> 32 3x3x3 stride 2 15 and 28); large ones
 // over volumes (32 -> 64 on 40^3 73 and 53).
-bool takes_volume(const ConvGeom& g) { return vol_supported(g) && (!f32tc_conv_supported(g) || vol_cost(g) < f32tc_conv_cost(g)); }
+// `in_front`: what a kernel costs that packing makes unnecessary, ns.
+bool takes_volume(const ConvGeom& g, long long in_front = 0) {
+  return vol_supported(g) && (!f32tc_conv_supported(g) || vol_cost(g) < f32tc_conv_cost(g) + in_front);
+}
 
 bool conv_layer(const VolW* vw, const F32ConvW* split, const float* wt, const float* bias, const float* x, const VolSource* src, const float* residual,
                 float* y, const ConvGeom& g, int act, float slope, int* status, cudaStream_t s, bool early, std::string* err) {
@@ -592,7 +595,9 @@ bool opnet_forward(OpNet* m, const float* x, float* y, int N, int H, int W, int*
       int h3, w3;
       if (l + 1 < nl && m->meta[l + 1].kind == LAYER_CONV2D && m->vw[l + 1] && opnet_layer_shape(m->meta[l + 1], h2, w2, &h3, &w3)) {
         const ConvGeom g = opnet_geom(m->meta[l + 1], N, h2, w2, h3, w3);
-        if (takes_volume(g) && vol_workspace(vol_bytes(vol_geom(g, 0, g.ph, vol_front_w(g)), (g.C + 31) / 32 * 32), s)) {
+        // pooling measures 11 us for 16.6 MB in, repeating 53 us for 33 MB out
+        const long long in_front = 2500 + (pool ? 4 * planes * h * w / 1900 : 4 * nout / 650);
+        if (takes_volume(g, in_front) && vol_workspace(vol_bytes(vol_geom(g, 0, g.ph, vol_front_w(g)), (g.C + 31) / 32 * 32), s)) {
           pending = VolSource{pool ? VolSource::MAXPOOL : VolSource::UPSAMPLE, pool ? L.kh : L.sh, pool ? L.kw : L.sw, L.sh, L.sw,
                               (long long)L.cin * h * w, (long long)h * w, w, 1, (long long)h * w};
           h = h2; w = w2;

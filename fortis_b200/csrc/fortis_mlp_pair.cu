@@ -319,28 +319,26 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) mlp_pai
         }
         continue;
       }
-      // blocks of 32 rows x 32 features turned in shared memory: whole lines of a row, eight lanes each
+      // blocks of 32 rows x 32 features turned in shared memory: whole lines of a row, eight lanes each.  One compact loop, the sums moved
+      // down after each block: straight code for all blocks took longer to fetch (26,000 clk a tile) than two chunks to multiply.
       const int c = lane & 7;
+      float b[NH / 32][4];
 #pragma unroll
+      for (int k = 0; k < NH / 32; k++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) b[k][e] = P.bias && n0 + 32 * k + 4 * c + e < P.N_real ? __ldg(P.bias + n0 + 32 * k + 4 * c + e) : 0.f;
+#pragma unroll 1
       for (int c0 = 0; c0 < NH; c0 += 32) {
 #pragma unroll
         for (int i = 0; i < 8; i++)
-          *reinterpret_cast<float4*>(scratch + lane * 32 + ((i ^ (lane & 7)) << 2)) = make_float4(v[c0 + 4 * i], v[c0 + 4 * i + 1], v[c0 + 4 * i + 2], v[c0 + 4 * i + 3]);
+          *reinterpret_cast<float4*>(scratch + lane * 32 + ((i ^ (lane & 7)) << 2)) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
         __syncwarp();
         const int n = n0 + c0 + 4 * c;
-        float b[4], m[4], r[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const bool real = n + e < P.N_real;
-          b[e] = P.bias && real ? __ldg(P.bias + n + e) : 0.f;
-          m[e] = P.out_mul && real ? __ldg(P.out_mul + n + e) : 1.f;
-          r[e] = P.relu_mask && real ? __ldg(P.relu_mask + n + e) : 0.f;
-        }
-#pragma unroll
+#pragma unroll 2
         for (int i = 0; i < 8; i++) {
           const int rr = 4 * i + (lane >> 3);
           const float4 q = *reinterpret_cast<const float4*>(scratch + rr * 32 + ((c ^ (rr & 7)) << 2));
-          float o[4] = {q.x + b[0], q.y + b[1], q.z + b[2], q.w + b[3]};
+          float o[4] = {q.x + b[0][0], q.y + b[0][1], q.z + b[0][2], q.w + b[0][3]};
           act4(o);
           if (P.out) {
             float h[4], l[4];
@@ -351,16 +349,23 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) mlp_pai
               *reinterpret_cast<float4*>(dst) = make_float4(h[0], h[1], h[2], h[3]);
               *reinterpret_cast<float4*>(dst + P.out_plane) = make_float4(l[0], l[1], l[2], l[3]);
             }
-          } else {
+          } else if (mw + rr < P.nrows) {
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-              if (P.out_mul) o[e] *= m[e];
-              if (r[e] != 0.f) o[e] = max_nan(o[e], 0.f);
-              if (mw + rr < P.nrows && n + e < P.N_real) P.Y[(mw + rr) * P.ldc + n + e] = o[e];
+              if (n + e >= P.N_real) continue;
+              if (P.out_mul) o[e] *= __ldg(P.out_mul + n + e);
+              if (P.relu_mask && __ldg(P.relu_mask + n + e) != 0.f) o[e] = max_nan(o[e], 0.f);
+              P.Y[(mw + rr) * P.ldc + n + e] = o[e];
             }
           }
         }
         __syncwarp();
+#pragma unroll
+        for (int j = 0; j + 32 < NH; j++) v[j] = v[j + 32];
+#pragma unroll
+        for (int k = 0; k + 1 < NH / 32; k++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) b[k][e] = b[k + 1][e];
       }
     }
     if (P.partials) {
@@ -399,34 +404,41 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) mlp_pai
   }
 }
 
-// Model inputs -> split rows: 64 rows x 32 inputs per block, turned in shared memory.  From host arrays through the slot table (lane =
-// row: a load reads 32 neighbouring elements) ...
+// Model inputs -> split rows: 128 rows x 32 inputs per block, turned in shared memory.  From host arrays through the slot table (lane =
+// row: a load reads 32 neighbouring elements; a thread has 16 in flight) ...
 __global__ void __launch_bounds__(256) gather_split_kernel(const Access* __restrict__ slots, ArrayTable T, RowGeom g, int n_in, const float* __restrict__ in_div,
                                                            float* __restrict__ out, long long plane, int pitch, long long nrows) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the first layer may set up while this kernel runs
-  __shared__ float tile[64][33];
-  const long long r0 = (long long)blockIdx.x * 64;
+  __shared__ float tile[128][33];
+  const long long r0 = (long long)blockIdx.x * 128;
   const int c0 = blockIdx.y * 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  long long ci[4], cj[4], kk[4];
 #pragma unroll
-  for (int i = 0; i < 2; i++) {
-    const long long r = r0 + i * 32 + lane < nrows ? r0 + i * 32 + lane : nrows - 1;
-    long long ci, cj, kk;
-    row_to_pos(g, r, &ci, &cj, &kk);
+  for (int i = 0; i < 4; i++) row_to_pos(g, r0 + i * 32 + lane < nrows ? r0 + i * 32 + lane : nrows - 1, &ci[i], &cj[i], &kk[i]);
+  float v[4][4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int c = warp * 4 + k;
-      float v = 0.f;
-      if (c0 + c < n_in) {
-        const Access a = slots[c0 + c];
-        v = __ldg((const float*)T.base[a.array] + access_offset(a, ci, cj, kk));
-        if (in_div) v = __fdiv_rn(v, __ldg(in_div + c0 + c));
-      }
-      tile[i * 32 + lane][c] = v;
+  for (int k = 0; k < 4; k++) {
+    const int c = c0 + warp * 4 + k;
+    const bool real = c < n_in;
+    const Access a = slots[real ? c : 0];
+    const float* base = (const float*)T.base[a.array] + a.off0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[k][i] = real ? __ldg(base + (ci[i] * a.si + cj[i] * a.sj + kk[i] * a.sk)) : 0.f;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int c = c0 + warp * 4 + k;
+    if (in_div && c < n_in) {
+      const float d = __ldg(in_div + c);
+#pragma unroll
+      for (int i = 0; i < 4; i++) v[k][i] = __fdiv_rn(v[k][i], d);
     }
+#pragma unroll
+    for (int i = 0; i < 4; i++) tile[i * 32 + lane][warp * 4 + k] = v[k][i];
   }
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < 2; i++) {
+  for (int i = 0; i < 4; i++) {
     const int rr = i * 32 + (threadIdx.x >> 3), c = (threadIdx.x & 7) * 4;
     if (r0 + rr >= nrows) continue;
     float h[4], l[4];
@@ -514,7 +526,7 @@ bool pair_wide(long long nrows, int N, bool scatter) {
 
 void pair_split_gathered(const Access* slots, const ArrayTable& T, const RowGeom& g, int n_in, const float* in_div, float* out, long long nrows, cudaStream_t s) {
   const int pitch = (n_in + 31) / 32 * 32;
-  gather_split_kernel<<<dim3((unsigned)((nrows + 63) / 64), (unsigned)(pitch / 32)), 256, 0, s>>>(slots, T, g, n_in, in_div, out, nrows * pitch, pitch, nrows);
+  gather_split_kernel<<<dim3((unsigned)((nrows + 127) / 128), (unsigned)(pitch / 32)), 256, 0, s>>>(slots, T, g, n_in, in_div, out, nrows * pitch, pitch, nrows);
 }
 void pair_split_rows(const float* X, int n_in, const float* in_div, float* out, long long nrows, cudaStream_t s) {
   const int pitch = (n_in + 31) / 32 * 32;
