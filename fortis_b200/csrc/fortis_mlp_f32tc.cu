@@ -919,21 +919,19 @@ bool split_alloc(SplitW* w, int K, int N, std::string* err) {
   return true;
 }
 
-// The tile width (0, 1, 2: 32, 64, 128 features).  A k step of a tile costs 6 clocks per feature of tensor time, or what
-// its producers need for 128 rows x 32 inputs if that is more (step_floor), and the launch lasts as many rounds of tiles as
-// the SM that has the most.  The floors are estimates, and low ones: a step with its share of the tile's end measures 1140,
-// 1200, 1520 clocks at 32, 64, 128 features (fortis_gemm, K = 768), 2210, 2310, 2520 with rows off 16 bytes, 1240, 1280, 1430 in
-// convolutions of K = 1728 and 1960, 2100, 2460 of K = 405.  So the rule takes tiles that are too narrow: over 8 to 256 features
-// and 13 to 1138 row tiles the width it picks is within 5 % of the fastest for every convolution of up to 64 features and 147
-// of 240 wider ones (at worst 1.76 times the time), and for 276 of 390 products (8 to 1000 features; at worst 2.4 times).
-int pick_tile(long long nrows, int N, int step_floor) {
+// The tile width (0, 1, 2: 32, 64, 128 features).  The launch lasts as many rounds of tiles as the SM that has the most, and a k step of a
+// tile, its share of the tile's end included, as many clocks as it measures: fortis_gemm, K = 768; rows off 16 bytes; inputs gathered from
+// host arrays; convolutions of K = 1728 (groups of eight channels) and of K = 405 (single channels).
+constexpr int kStepLinear[3] = {1140, 1200, 1520}, kStepLoads[3] = {2210, 2310, 2520}, kStepGather[3] = {1900, 2000, 2100}, kStepConv8[3] = {1240, 1280, 1430},
+              kStepConv1[3] = {1960, 2100, 2460};
+int pick_tile(long long nrows, int N, const int (&step)[3]) {
   const long long ntm = (nrows + kM - 1) / kM, sms = sm_count();
   long long best_cost = 0;
   int best = -1;
   for (int w = 2; w >= 0; w--) {
     const int nt = 32 << w;
     if (w > 0 && N <= nt / 2) continue;                     // more than half of the tile would be padding
-    const long long tiles = ntm * ((N + nt - 1) / nt), cost = ((tiles + sms - 1) / sms) * (6 * nt > step_floor ? 6 * nt : step_floor);
+    const long long tiles = ntm * ((N + nt - 1) / nt), cost = ((tiles + sms - 1) / sms) * step[w];
     if (best < 0 || cost < best_cost) { best = w; best_cost = cost; }
   }
   return best;
@@ -978,8 +976,8 @@ bool launch_as(F32Params& P, cudaStream_t s, bool early) {
 }
 
 template <int AMODE>
-bool launch_tile(F32Params& P, const SplitW& W, int step_floor, cudaStream_t s, bool early = true) {
-  const int w = pick_tile(P.nrows, W.N_real, step_floor);
+bool launch_tile(F32Params& P, const SplitW& W, const int (&step)[3], cudaStream_t s, bool early = true) {
+  const int w = pick_tile(P.nrows, W.N_real, step);
   P.map_hi = W.map_hi[w]; P.map_lo = W.map_lo[w];
   P.K_pad = W.K_pad; P.K_real = W.K_real; P.N_real = W.N_real;
   P.chunk_kt = P.one_acc ? kChunkMlp : W.K_pad <= kShortK ? kChunkShort : kChunkLong;
@@ -987,14 +985,11 @@ bool launch_tile(F32Params& P, const SplitW& W, int step_floor, cudaStream_t s, 
   return w == 2 ? launch_as<128, AMODE>(P, s, early) : w == 1 ? launch_as<64, AMODE>(P, s, early) : launch_as<32, AMODE>(P, s, early);
 }
 
-// clocks a k step's producers need at least (see pick_tile)
-constexpr int kStepFloorLinear = 250, kStepFloorConv = 350;
-
 // a row-major operand: tiles through the TMA where rows start on 16-byte boundaries, else loads
 bool launch_rows(F32Params& P, const float* A, int K, const SplitW& W, cudaStream_t s, bool early) {
-  if (make_a_map(false, A, P.nrows, K, K, &P.map_a)) return launch_tile<A_TILE_R>(P, W, kStepFloorLinear, s, early);
+  if (make_a_map(false, A, P.nrows, K, K, &P.map_a)) return launch_tile<A_TILE_R>(P, W, kStepLinear, s, early);
   P.A = A; P.lda = K;
-  return launch_tile<A_ROW_MAJOR>(P, W, kStepFloorLinear, s, early);
+  return launch_tile<A_ROW_MAJOR>(P, W, kStepLoads, s, early);
 }
 
 bool launched(bool ok, std::string* err) {
@@ -1064,7 +1059,10 @@ F32TcModel* f32tc_create(const ModelHost& M, std::string* err) {
 bool f32tc_pair_wanted(const F32TcModel* m, long long nrows) {
   static const char* dev = std::getenv("FORTIS_PAIR_DEV");
   if (dev) return dev[0] != '0' && m->layers.size() >= 2;
-  return m->layers.size() >= 2;
+  if (m->layers.size() < 2) return false;
+  long long narrow = 1 << 30;
+  for (size_t l = 0; l + 1 < m->layers.size(); l++) narrow = m->layers[l].w.N_real < narrow ? m->layers[l].w.N_real : narrow;
+  return narrow >= 320 && narrow * nrows >= 6000000;
 }
 
 size_t f32tc_pair_bytes(const F32TcModel* m, long long nrows) {
@@ -1133,7 +1131,7 @@ bool f32tc_forward(F32TcModel* m, const F32TcLaunch& L, cudaStream_t s, std::str
       if (fast_in) {
         P.slots = L.slots; P.TG = L.TG;
         for (int i = 0; i < 2; i++) P.cin[i] = StrideClassF{L.cin[i][0], L.cin[i][1], L.cin[i][2]};
-        ok = launch_tile<A_GATHER>(P, T.w, kStepFloorLinear, s);
+        ok = launch_tile<A_GATHER>(P, T.w, kStepGather, s);
       } else {
         ok = launch_rows(P, L.X, n_in, T.w, s, true);
       }
@@ -1142,7 +1140,7 @@ bool f32tc_forward(F32TcModel* m, const F32TcLaunch& L, cudaStream_t s, std::str
         if (err) *err = "split-TF32 step: activation rows must start on 16-byte boundaries";
         return false;
       }
-      ok = launch_tile<A_TILE_T>(P, T.w, kStepFloorLinear, s);
+      ok = launch_tile<A_TILE_T>(P, T.w, kStepLinear, s);
     }
     if (!launched(ok, err)) return false;
   }
@@ -1318,7 +1316,7 @@ bool f32tc_conv_supported(const ConvGeom& g) {
 // Estimated device time of a layer, ns: rounds of tiles times steps of 32 k, a step as it measures in one round of tiles and in many (groups of
 // eight channels 0.56 to 0.75 us, single channels 0.73 to 1.3 us).
 long long f32tc_conv_cost(const ConvGeom& g) {
-  const int G = conv_group(g.C), w = pick_tile((long long)g.N * g.Do * g.Ho * g.Wo, g.F, kStepFloorConv), nt = 32 << w;
+  const int G = conv_group(g.C), w = pick_tile((long long)g.N * g.Do * g.Ho * g.Wo, g.F, G == 8 ? kStepConv8 : kStepConv1), nt = 32 << w;
   const long long steps = ((long long)g.KD * g.KH * g.KW * ((g.C + G - 1) / G * G) + kKt - 1) / kKt;
   const long long tiles = (((long long)g.N * g.Do * g.Ho * g.Wo + kM - 1) / kM) * ((g.F + nt - 1) / nt), sms = sm_count(), rounds = (tiles + sms - 1) / sms;
   static const int one[2] = {730, 560}, many[2][3] = {{1030, 1100, 1300}, {650, 670, 750}};
@@ -1350,7 +1348,7 @@ bool f32tc_conv(const F32ConvW* w, const float* x, const float* bias, const floa
   P.status = status; P.bias = bias; P.act = act; P.slope = slope;
   P.A = x; P.cv = g; P.residual = residual;
   P.c_mode = C_CONV; P.C = y;
-  return launched(w->group == 8 ? launch_tile<A_CONV8>(P, w->w, kStepFloorConv, s, early) : launch_tile<A_CONV1>(P, w->w, kStepFloorConv, s, early), err);
+  return launched(w->group == 8 ? launch_tile<A_CONV8>(P, w->w, kStepConv8, s, early) : launch_tile<A_CONV1>(P, w->w, kStepConv1, s, early), err);
 }
 
 }  // namespace fortis
