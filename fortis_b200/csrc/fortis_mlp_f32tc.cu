@@ -24,7 +24,7 @@
 // k step read 12 KB per 128 clocks and the producers and the TMA write 96 KB per 1536, together 1.25 times what shared
 // memory moves; in this form only the weights (64 B/clk at any NT) and the fp32 tiles pass through it.
 // Measured, that form / this one: fortis_gemm 8192 x 768 x 768 756 / 62 us (a row-major operand was read by one dependent load
-// per row), column network 30,011 rows 991 / 750 us; convolutions against the FFMA kernel: 32 -> 64 channels 3x3x3 on 40^3
+// per row), column network 30,011 rows 991 / 750 us (on pairs of CTAs, fortis_mlp_pair.cu, 592); convolutions against the FFMA kernel: 32 -> 64 channels 3x3x3 on 40^3
 // 297 / 73 us, 14-layer network 2 x 33^3 8.75 / 2.02 ms.
 //
 // The tensor core adds into its fp32 accumulator with truncation, not rounding, a bias per accumulation of half a unit in
@@ -1056,13 +1056,15 @@ F32TcModel* f32tc_create(const ModelHost& M, std::string* err) {
   return m;
 }
 
+// Pairs of CTAs (fortis_mlp_pair.cu) for wide layers of many rows; the results are the same bits.  Their tiles are 256 x 256, their launches
+// cost 4 us more each, and the split activations move twice the bytes.  Device time of whole calls, this kernel / pairs (us): hidden layers
+// of 768: 2000 rows 115 / 113, 4000 164 / 168, 8000 224 / 206, 30,011 631 / 570; 1024: 4000 115 / 118, 8000 177 / 164; 2048: 3000 200 / 177, 5000
+// 293 / 255; 900: 7000 131 / 146, 12,000 206 / 188; 512: 30,011 192 / 216; 400 and 640 in turn: 30,011 256 / 274.
 bool f32tc_pair_wanted(const F32TcModel* m, long long nrows) {
-  static const char* dev = std::getenv("FORTIS_PAIR_DEV");
-  if (dev) return dev[0] != '0' && m->layers.size() >= 2;
   if (m->layers.size() < 2) return false;
   long long narrow = 1 << 30;
   for (size_t l = 0; l + 1 < m->layers.size(); l++) narrow = m->layers[l].w.N_real < narrow ? m->layers[l].w.N_real : narrow;
-  return narrow >= 320 && narrow * nrows >= 6000000;
+  return narrow >= 768 && narrow * nrows >= 7000000;
 }
 
 size_t f32tc_pair_bytes(const F32TcModel* m, long long nrows) {

@@ -3,7 +3,7 @@
 //
 // The arithmetic of an MLP step is that of f32tc_kernel (fortis_mlp_f32tc.cu), sum by sum: the three products of 8 k one after another
 // (hi.hi, hi.lo, lo.hi) in one accumulator that is taken over every 128 k with IEEE additions.  The results are the same bits; this
-// form takes over where there are rows enough for its wide tiles (pair_wanted).
+// form takes over where there are rows and features enough for its wide tiles (f32tc_pair_wanted).
 //
 // Replaces the same reference lowering: fortis_gemm = cuBLAS SGEMM per layer with further kernels for bias and activation
 // (runtime/fortis_rt.c:45-75, compiler/FortisFuse.cpp:616-624, 687-760), fortis_gather_k in front and fortis_scatter_k behind.
@@ -16,7 +16,8 @@
 //     CTA; one MMA of N = 256 takes 128 clk and reads 8 KB of shared memory a CTA, the copies write 43 B/clk: bound by the tensor core.
 //   * one warp copies, one issues (12 MMAs a step), two accumulators of NT columns; eight epilogue warps (thread = row, half of the
 //     features) hold up to 128 sums a thread, so that the next tile's first two chunks (12,288 clk) run under a tile's end.
-// Measured: see f32tc_forward.
+// Measured: column network 244 -> 768 x4 -> 128, 30,011 rows 757 -> 592 us; a hidden layer 185 -> 151 (MMAs alone 97 at 1.9 GHz): what is left is
+// the tiles' ends, 262 KB of split activations stored by every CTA at about the same time.
 #include <cuda.h>
 #include <cuda_runtime.h>
 

@@ -1,0 +1,73 @@
+"""fp32 MLP steps on pairs of CTAs (fortis_mlp_pair.cu): calls of many rows run there, calls of few rows on the split-TF32 kernel, with
+the same sums, so a row's outputs are the same bits however many rows are in the call.  The edges of its tiles (128 and 256 rows, 128 and
+256 features, 32 k and chunks of 128), both kinds of input and output, all activations."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import fortis_b200
+from fortis_b200 import descriptors as D
+from fortis_b200.model import mlp_layers, write_blob
+
+
+@pytest.fixture()
+def host():
+    h = fortis_b200.Host()
+    h.reset()
+    yield h
+    h.reset()
+
+
+def forward(host, x, n_out):
+    y = torch.full((x.shape[0], n_out), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    host.L.fortis_begin(x.shape[0])
+    host.forward_batched(x, y)
+    return y
+
+
+@pytest.mark.parametrize("dims,rows,act", [
+    ([33, 768, 1], 9217, "leaky"), ([244, 800, 768, 130], 9344, "relu"), ([1, 1023, 1025, 256], 7000, "leaky"), ([768, 768, 300], 9343, "leaky"),
+    ([129, 2049, 31], 3500, "relu"),
+])
+def test_rows_have_the_same_bits_in_calls_of_any_size(host, dims, rows, act):
+    layers = mlp_layers(dims, seed=2, act=act, bias="uniform")
+    in_div = np.linspace(0.5, 2.0, dims[0]).astype(np.float32)
+    out_mul = np.linspace(-1.0, 3.0, dims[-1]).astype(np.float32)
+    host.load_model(write_blob(layers, in_div=in_div, out_mul=out_mul))
+    x = torch.randn((rows, dims[0]), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    y = forward(host, x, dims[-1])
+    # 1500 rows at a time: below what pairs of CTAs take
+    parts = torch.cat([forward(host, x[r:r + 1500].contiguous(), dims[-1]) for r in range(0, rows - 1500, 1500)])
+    assert torch.equal(y[:parts.shape[0]], parts)
+    v = x.double() / torch.from_numpy(in_div).cuda().double()
+    for k, l in enumerate(layers):
+        v = v @ torch.from_numpy(l["W"]).cuda().double().T + torch.from_numpy(l["b"]).cuda().double()
+        if l.get("act") == "relu": v = v.clamp_min(0)
+        elif l.get("act") == "leaky": v = torch.where(v > 0, v, v * float(np.float32(l["slope"])))
+    v = v * torch.from_numpy(out_mul).cuda().double()
+    assert float((y.double() - v).norm() / v.norm()) < 1e-5
+
+
+def test_gathered_step_and_its_checksum(host):
+    """The column step over device arrays: inputs through the slot table, outputs scattered, the checksum folded in the launch."""
+    ncol = 9601
+    G, S, L, K = D.column(ncol, 60)
+    host.configure(gather=G, scatter=S, loop=L, kdist=K)
+    layers = mlp_layers([244, 768, 768, 128], seed=0)
+    host.load_model(write_blob(layers))
+    g = torch.Generator(device="cuda").manual_seed(3)
+    gin = [torch.randn((60, ncol), device="cuda", generator=g) for _ in range(4)] + [torch.randn(ncol, device="cuda", generator=g) for _ in range(4)]
+    out = [torch.zeros((60, ncol), device="cuda") for _ in range(2)] + [torch.zeros(ncol, device="cuda") for _ in range(8)]
+    host.option("checksum", "1")
+    torch.cuda.synchronize()
+    host.step(gin, out)
+    host.sync()
+    x = torch.cat([f.T for f in gin[:4]] + [v[:, None] for v in gin[4:]], dim=1).double()
+    for l in layers:
+        x = x @ torch.from_numpy(l["W"]).cuda().double().T + torch.from_numpy(l["b"]).cuda().double()
+        if l.get("act") == "leaky": x = torch.where(x > 0, x, x * float(np.float32(l["slope"])))
+    y = torch.cat([out[0].T, out[1].T] + [v[:, None] for v in out[2:]], dim=1)
+    assert float((y.double() - x).norm() / x.norm()) < 1e-5
