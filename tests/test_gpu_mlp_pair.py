@@ -71,3 +71,4 @@ def test_gathered_step_and_its_checksum(host):
         if l.get("act") == "leaky": x = torch.where(x > 0, x, x * float(np.float32(l["slope"])))
     y = torch.cat([out[0].T, out[1].T] + [v[:, None] for v in out[2:]], dim=1)
     assert float((y.double() - x).norm() / x.norm()) < 1e-5
+    assert abs(host.step_checksum() - float(y.double().sum())) <= 1e-12 * float(y.double().abs().sum())
