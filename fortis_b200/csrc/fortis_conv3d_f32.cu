@@ -743,7 +743,7 @@ bool vol_supported(const ConvGeom& c) {
   return g.P * g.fd * g.fh * g.fw < (1LL << 30) && (long long)c.KD * g.Hq * g.Wq < (1LL << 29) && pick_sharing(g, vol_nt(c.F), g.line, &s);
 }
 
-// Estimated device time of a layer whose input is packed first, ns: packing at 1.6 TB/s of what it writes, rounds of tiles, and in each the
+// Estimated device time of a layer whose input is packed first, ns: one launch more, packing at 1.6 TB/s of what it writes, rounds of tiles, and in each the
 // steps (a tap each: stages shared or not; a line's taps: 32 or 64 features) and the tile's end.
 long long vol_cost(const ConvGeom& c) {
   const VolGeom g = vol_geom(c, c.pd, c.ph, vol_front_w(c));
@@ -753,7 +753,7 @@ long long vol_cost(const ConvGeom& c) {
   const long long rows = (((long long)(g.N - 1) * g.Dq + g.Do - 1) * g.Hq + g.Ho - 1) * g.Wq + g.Wo, per_pair = g.line ? 252 : 256, pairs = sm_count() / 2;
   const long long tiles = (rows + per_pair - 1) / per_pair * ((c.F + NT - 1) / NT), rounds = (tiles + pairs - 1) / pairs, steps = (long long)s.ng * s.tpg * (pitch / 32);
   const long long step = g.line ? (NT == 64 ? 680 : 600) : s.tpg > 1 ? 380 : 570, end = g.line ? 2600 : 1500;
-  return 4500 + (long long)(vol_bytes(g, pitch) / 1600) + rounds * (steps * step + end);
+  return 6500 + (long long)(vol_bytes(g, pitch) / 1600) + rounds * (steps * step + end);
 }
 
 struct VolW { int F = 0, C = 0, taps = 0, kw = 1, NT = 0, nchb = 0, ntn = 0; float* img = nullptr; CUtensorMap map; };     // kw: taps of a step
