@@ -68,7 +68,9 @@ struct VolParams {
   int nchb, ntn;
   int ng, tpg, sub_w;                          // stages per channel block, steps per stage, steps of one line among them
   int box_rows, a_stages, w_stages;
-  long long rows;                              // output rows up to the last one that is a real output
+  // the rows in pieces (the whole volume, or the images of a batch) of `rows` output rows up to the last one that is a real output,
+  // piece_stride apart, each in pairs of tiles of its own
+  int pieces, pairs_piece; long long rows, piece_stride;
   const float* bias; int act; float slope; int F;
   // output: a split volume of the same grid (pitch: channels of a row) ...
   float* out; long long out_plane; int out_pitch; long long out_shift;
@@ -209,7 +211,12 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
   // through a shuffle, so that the compiler knows the roles' branches, loops and addresses to be the same in a whole warp
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t crank = cluster_ctarank();
-  const long long npairs = (P.rows + 2 * FM::kRowsOut - 1) / (2 * FM::kRowsOut), ntiles = npairs * P.ntn;
+  const long long ntiles = (long long)P.pieces * P.pairs_piece * P.ntn;
+  // a tile's piece and its first computed row there
+  auto piece_of = [&](long long t) { return (uint32_t)(t / P.ntn) / (uint32_t)P.pairs_piece; };
+  auto first_row = [&](long long t, uint32_t piece) {
+    return (2 * ((long long)(uint32_t)(t / P.ntn) - (long long)piece * P.pairs_piece) + crank) * FM::kRowsOut - FM::kHalo;
+  };
   const long long t0 = blockIdx.x >> 1, t_step = gridDim.x >> 1;
   const int nkt = P.ng * P.tpg * P.nchb;       // steps of a tile
 
@@ -250,7 +257,8 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
       uint32_t s = 0, ph = 0;
       bool stop = false;
       for (long long t = t0; t < ntiles && !stop; t += t_step) {
-        const long long m0 = (2 * (t / P.ntn) + crank) * FM::kRowsOut - FM::kHalo;
+        const uint32_t piece = piece_of(t);
+        const long long m0 = piece * P.piece_stride + first_row(t, piece);
         for (int g = 0; g < P.ng && !stop; g++) {
           const int y0 = (int)(m0 + stage_shift<LINE>(P, g));
           for (int cb = 0; cb < P.nchb; cb++) {
@@ -372,8 +380,9 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
     uint32_t tile_it = 0;
     for (long long t = t0; t < ntiles; t += t_step, tile_it++) {
       const int r = quad * 32 + lane, n0 = (int)(t % P.ntn) * NT;
-      const long long p = (2 * (t / P.ntn) + crank) * FM::kRowsOut - FM::kHalo + r;
-      const bool in_rows = p < P.rows && (!LINE || (r >= 1 && r <= FM::kRowsOut));
+      const uint32_t piece = piece_of(t);
+      const long long local = first_row(t, piece) + r, p = piece * P.piece_stride + local;
+      const bool in_rows = local < P.rows && (!LINE || (r >= 1 && r <= FM::kRowsOut));
       const uint32_t q0 = (uint32_t)(in_rows ? p : 0), q1 = q0 / (uint32_t)G.Wq, q2 = q1 / (uint32_t)G.Hq, q3 = q2 / (uint32_t)G.Dq;
       const int ow = (int)(q0 - q1 * G.Wq), oh = (int)(q1 - q2 * G.Hq), od = (int)(q2 - q3 * G.Dq), on = (int)q3;
       const bool live = in_rows && ow < G.Wo && oh < G.Ho && od < G.Do;
@@ -449,8 +458,8 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
     for (long long t = t0; t < ntiles; t += t_step, tile_it++) {
       const int r = quad * 32 + lane;
       // the row's position in its line, for its neighbours
-      const long long p = (2 * (t / P.ntn) + crank) * FM::kRowsOut - FM::kHalo + r;
-      const int ow = LINE ? (int)((uint32_t)(p > 0 && p < P.rows ? p : 0) % (uint32_t)G.Wq) : 0;
+      const long long local = LINE ? first_row(t, piece_of(t)) + r : 0;      // pieces start at a line's start
+      const int ow = LINE ? (int)((uint32_t)(local > 0 && local < P.rows ? local : 0) % (uint32_t)G.Wq) : 0;
       float sum[FM::kTaps][NH], vx[LINE ? 1 : NH];
 #pragma unroll
       for (int k = 0; k < FM::kTaps; k++)
@@ -743,6 +752,17 @@ bool vol_supported(const ConvGeom& c) {
   return g.P * g.fd * g.fh * g.fw < (1LL << 30) && (long long)c.KD * g.Hq * g.Wq < (1LL << 29) && pick_sharing(g, vol_nt(c.F), g.line, &s);
 }
 
+// The rows as one piece, or image by image (which leaves the padding planes between them out) where that takes fewer rounds of tiles:
+// 14-layer network, 2 x 33^3: 299 pairs of tiles, 4.04 rounds, or 294, 3.97.
+struct Pieces { int n, pairs; long long rows, stride; };
+Pieces pick_pieces(const VolGeom& g, int ntn) {
+  const long long per_pair = 2 * (g.line ? Form<64, true>::kRowsOut : Form<64, false>::kRowsOut), on_device = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
+  const long long stride = (long long)g.Dq * g.Hq * g.Wq, image = ((long long)(g.Do - 1) * g.Hq + g.Ho - 1) * g.Wq + g.Wo, all = (g.N - 1) * stride + image;
+  const long long one = (all + per_pair - 1) / per_pair, each = (image + per_pair - 1) / per_pair;
+  if ((each * g.N * ntn + on_device - 1) / on_device < (one * ntn + on_device - 1) / on_device) return Pieces{g.N, (int)each, image, stride};
+  return Pieces{1, (int)one, all, 0};
+}
+
 // Estimated device time of a layer whose input is packed first, ns: one launch more, packing at 1.6 TB/s of what it writes, rounds of tiles, and in each the
 // steps (a tap each: stages shared or not; a line's taps: 32 or 64 features) and the tile's end.
 long long vol_cost(const ConvGeom& c) {
@@ -750,8 +770,8 @@ long long vol_cost(const ConvGeom& c) {
   const int NT = vol_nt(c.F), pitch = (c.C + 31) / 32 * 32;
   Sharing s;
   if (!pick_sharing(g, NT, g.line, &s)) return 1LL << 60;
-  const long long rows = (((long long)(g.N - 1) * g.Dq + g.Do - 1) * g.Hq + g.Ho - 1) * g.Wq + g.Wo, per_pair = g.line ? 252 : 256, pairs = sm_count() / 2;
-  const long long tiles = (rows + per_pair - 1) / per_pair * ((c.F + NT - 1) / NT), rounds = (tiles + pairs - 1) / pairs, steps = (long long)s.ng * s.tpg * (pitch / 32);
+  const Pieces pc = pick_pieces(g, (c.F + NT - 1) / NT);
+  const long long pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1, tiles = (long long)pc.n * pc.pairs * ((c.F + NT - 1) / NT), rounds = (tiles + pairs - 1) / pairs, steps = (long long)s.ng * s.tpg * (pitch / 32);
   const long long step = g.line ? (NT == 64 ? 680 : 600) : s.tpg > 1 ? 380 : 570, end = g.line ? 2600 : 1500;
   return 6500 + (long long)(vol_bytes(g, pitch) / 1600) + rounds * (steps * step + end);
 }
@@ -809,7 +829,8 @@ bool vol_conv(const VolW* w, const float* vol, int pitch, const VolGeom& g, cons
     return fail("cuTensorMapEncodeTiled failed for a split volume");
   P.wmap = w->map; P.g = g; P.nchb = w->nchb; P.ntn = w->ntn;
   P.ng = sh.ng; P.tpg = sh.tpg; P.sub_w = sh.sub_w; P.box_rows = sh.box_rows; P.a_stages = sh.a_stages; P.w_stages = sh.w_stages;
-  P.rows = (((long long)(g.N - 1) * g.Dq + g.Do - 1) * g.Hq + g.Ho - 1) * g.Wq + g.Wo;
+  const Pieces pc = pick_pieces(g, w->ntn);
+  P.pieces = pc.n; P.pairs_piece = pc.pairs; P.rows = pc.rows; P.piece_stride = pc.stride;
   P.bias = bias; P.act = act; P.slope = slope; P.F = w->F;
   P.out = o.vol; P.out_plane = g.P * o.pitch; P.out_pitch = o.pitch; P.out_shift = ((long long)g.pd * g.Hq + g.ph) * g.Wq + g.pw;
   P.skip = o.skip; P.y = o.y; P.ys_n = o.ys_n; P.ys_d = o.ys_d; P.ys_h = o.ys_h; P.ys_w = o.ys_w; P.ys_c = o.ys_c;
@@ -828,8 +849,7 @@ bool vol_conv(const VolW* w, const float* vol, int pitch, const VolGeom& g, cons
     if (cudaFuncGetAttributes(&fa, kernels[3]) != cudaSuccess || fa.numRegs != 128) return fail("the convolution kernel's register split does not add up");
     ready = true;
   }
-  const int per_pair = 2 * (g.line ? Form<64, true>::kRowsOut : Form<64, false>::kRowsOut);
-  const long long tiles = (P.rows + per_pair - 1) / per_pair * P.ntn, pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
+  const long long tiles = (long long)pc.n * pc.pairs * P.ntn, pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs))); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = sh.smem; cfg.stream = s;
   cudaLaunchAttribute at[1];
