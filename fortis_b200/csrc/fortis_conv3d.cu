@@ -418,6 +418,7 @@ float* vol_workspace(size_t bytes, cudaStream_t s) {
 // over volumes (32 -> 64 on 40^3 73 and 53).
 // `in_front`: what a kernel costs that packing makes unnecessary, ns.
 bool takes_volume(const ConvGeom& g, long long in_front = 0) {
+  if (g_tc_test.conv_route) return g_tc_test.conv_route == 1 && vol_supported(g);
   return vol_supported(g) && (!f32tc_conv_supported(g) || vol_cost(g) < f32tc_conv_cost(g) + in_front);
 }
 
@@ -682,6 +683,7 @@ static void set_strides(long long* n, long long* d, long long* h, long long* w, 
 // short one that writes such a volume.  False where the network is not of that kind; *ok: how the call went.
 static bool conv_forward_volumes(ConvModel* m, const float* x, float* y, int N, int D, int H, int W, int* status, cudaStream_t s, bool* ok, std::string* err) {
   const int nl = (int)m->meta.size();
+  if (g_tc_test.conv_route == 2) return false;
   int pad = 0, pad_w = 0, cmax = 0;
   for (int l = 0; l < nl; l++) {
     pad = m->meta[l].pad > pad ? m->meta[l].pad : pad;

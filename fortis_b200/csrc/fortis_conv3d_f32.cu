@@ -881,6 +881,7 @@ bool vol_conv(const VolW* w, const float* vol, int pitch, const VolGeom& g, cons
   cfg.attrs = at; cfg.numAttrs = (pdl && early) ? 1 : 0;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernels[2 * g.line + (w->NT == 64)], P);
   if (e != cudaSuccess) { if (err) *err = std::string("convolution launch: ") + cudaGetErrorString(e); return false; }
+  g_launches.vol_conv++;
   return true;
 }
 

@@ -82,8 +82,15 @@ bool launch_stencil_tc(StencilTcModel* m, const StencilLaunch& S, int* status, c
 // Test knobs of the tensor-core kernels (set through fortis_set_option "test_wait_limit" / "test_skip_stage"; both 0
 // in normal operation): a short poll limit for the bounded barrier waits, and "the first CTA's TMA warp does not load
 // its first stage", which makes a wait run out so that the give-up path can be exercised without hanging anything.
-struct TcTestKnobs { unsigned int wait_limit; int skip_stage; int no_stage; };   // no_stage: fused MLP kernel, move every tile's inputs and outputs element by element
+struct TcTestKnobs {
+  unsigned int wait_limit; int skip_stage;
+  int no_stage;                                      // fused MLP kernel: move every tile's inputs and outputs element by element
+  int conv_route;                                    // fp32 convolutions: 0 by estimate, 1 over split volumes wherever they can, 2 never
+};
 extern TcTestKnobs g_tc_test;
+// launches since the library was loaded, so that a test can tell which kernel served a call
+struct LaunchCounts { long vol_conv, mlp_pair; };
+extern LaunchCounts g_launches;
 
 // ---- tensor-core fused MLP (fortis_mlp_tc.cu) ----------------------------------------------------------------
 struct ModelHost;

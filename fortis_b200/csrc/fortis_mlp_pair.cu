@@ -513,6 +513,7 @@ bool launch(PairParams& P, cudaStream_t s, std::string* err) {
   cfg.attrs = at; cfg.numAttrs = pdl ? 1 : 0;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, mlp_pair_kernel<NT>, P);
   if (e != cudaSuccess) { if (err) *err = std::string("pair kernel launch: ") + cudaGetErrorString(e); return false; }
+  g_launches.mlp_pair++;
   return true;
 }
 

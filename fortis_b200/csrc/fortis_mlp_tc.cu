@@ -1040,7 +1040,8 @@ float e4m3_round(float v) {
 
 }  // namespace
 
-TcTestKnobs g_tc_test = {0u, 0, 0};
+TcTestKnobs g_tc_test = {};
+LaunchCounts g_launches = {};
 
 // One Linear layer converted for the tensor-core kernel: padded, rounded to the 16-bit operand type (FP8 weights: the
 // nearest E4M3 code of w / scale, which bf16 represents exactly), as row-major [N][K] (`rowmajor`, optional) and as

@@ -26,7 +26,8 @@ def host():
 
 
 # (N, C, F, D, H, W), kernel, stride, padding.  One voxel, a ragged warp, every group of channels (1, 4, 5, 8, 9, 16, 17, 33, 65),
-# every number of voxels a thread takes (one, two and four: 57,000, 114,000 and 228,000 warps' worth of outputs)
+# every number of voxels a thread takes with 4, 8 and 16 channels (one; two from 3552 warps of 32 voxels and one group of channels on; four
+# from 7104), one and two with 32
 @pytest.mark.parametrize("shape,K,stride,pad", [
     ((1, 1, 1, 1, 1, 1), (1, 1, 1), (1, 1, 1), (0, 0, 0)),
     ((2, 3, 64, 5, 7, 9), (3, 3, 3), (1, 1, 1), (1, 1, 1)),
@@ -40,6 +41,9 @@ def host():
     ((1, 4, 8, 1, 500, 500), (1, 3, 3), (1, 1, 1), (0, 1, 1)),
     ((1, 4, 4, 4, 239, 239), (1, 2, 2), (1, 1, 1), (0, 0, 0)),
     ((1, 3, 16, 30, 60, 65), (1, 3, 3), (1, 1, 1), (0, 1, 1)),
+    ((1, 4, 4, 4, 241, 241), (1, 2, 2), (1, 1, 1), (0, 0, 0)),
+    ((1, 2, 7, 1, 340, 345), (1, 3, 3), (1, 1, 1), (0, 1, 1)),
+    ((1, 3, 16, 30, 90, 91), (1, 3, 3), (1, 1, 1), (0, 1, 1)),
 ])
 def test_short_sums(host, shape, K, stride, pad):
     N, C, F, D, H, W = shape

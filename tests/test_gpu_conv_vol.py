@@ -33,10 +33,17 @@ def rel(a, b):
     return float((a - b).norm() / b.norm())
 
 
+def on_device(host, route):
+    host.option("test_conv_route", {"volume": 1, "loads": 2}[route])
+    return lambda: host.L.fortis_debug_launches(b"conv_vol_kernel")
+
+
 # (N, C, F, D, H, W), kernel, stride, padding: one line's taps a step (three wide, stride 1, padding 0 and 1) and a tap a step (others);
 # stages of a plane, of a line (wide volumes), of a tap (strides); phases; padding of K and more; rows 126, 127, 252, 253 of a tile and
-# a pair; channels 8 to 100 in blocks of 32, features 1 to 130 in tiles of 32 and 64; lines of one and two positions
+# a pair; channels 8 to 100 in blocks of 32, features 1 to 130 in tiles of 32 and 64; lines of one and two positions.  Every case
+# runs on both kernels, whatever the estimate would choose; sums of fewer than 128 products run on neither
 @pytest.mark.gpu
+@pytest.mark.parametrize("route", ["volume", "loads"])
 @pytest.mark.parametrize("shape,K,stride,pad", [
     ((1, 32, 64, 3, 6, 7), (3, 3, 3), (1, 1, 1), (1, 1, 1)),
     ((1, 16, 1, 1, 1, 126), (1, 3, 3), (1, 1, 1), (0, 1, 1)),
@@ -57,9 +64,14 @@ def rel(a, b):
     ((1, 130, 12, 4, 4, 5), (1, 1, 1), (2, 1, 2), (1, 2, 3)),
     ((1, 32, 16, 3, 3, 3), (2, 2, 3), (1, 1, 1), (3, 2, 4)),
     ((1, 40, 64, 1, 7, 200), (1, 3, 3), (1, 2, 1), (0, 1, 0)),
+    ((1, 48, 20, 1, 1, 126), (1, 3, 3), (1, 1, 1), (0, 1, 1)),
+    ((1, 16, 65, 7, 6, 1), (3, 3, 3), (1, 1, 1), (1, 1, 1)),
+    ((2, 24, 30, 9, 9, 12), (3, 3, 3), (2, 2, 2), (1, 1, 1)),
+    ((1, 33, 96, 10, 7, 9), (3, 3, 3), (3, 2, 2), (0, 1, 2)),
+    ((1, 32, 32, 11, 5, 6), (4, 1, 2), (2, 1, 3), (1, 0, 1)),
     ((2, 64, 64, 33, 33, 33), (3, 3, 3), (1, 1, 1), (1, 1, 1)),
 ])
-def test_layers(host, shape, K, stride, pad):
+def test_layers(host, shape, K, stride, pad, route):
     from tests.test_gpu_conv import _conv_entry
     from tests.test_gpu_f32tc import memref, randn
     N, C, F, D, H, W = shape
@@ -68,9 +80,13 @@ def test_layers(host, shape, K, stride, pad):
     want = torch.nn.functional.conv3d(x.double(), w.double(), stride=stride, padding=pad)
     y = torch.full(want.shape, float("nan"), device="cuda")
     torch.cuda.synchronize()                                  # the library runs on a stream of its own
+    launches = on_device(host, route)
+    before = launches()
     _conv_entry(host.L, "fortis_conv3d", 5)(*memref(x), *memref(w), *memref(y), N, C, D, H, W, F, *K, *want.shape[2:], *stride, *pad)
     host.sync()
     assert rel(y, want) < TOL
+    products = C * min(K[0], D) * min(K[1], H) * min(K[2], W)
+    assert launches() - before == (route == "volume" and products >= 128)
 
 
 def conv3d_layer(rng, ci, co, k, act="none", **flags):
