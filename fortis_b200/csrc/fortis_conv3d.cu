@@ -389,15 +389,19 @@ bool upload_layer(const LayerHost& L, int taps, bool split, bool line, bool both
   return true;
 }
 
+bool stream_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(s, &cs);
+  return cs != cudaStreamCaptureStatusNone;
+}
+
 // The split volume of a layer whose input is a plain array.  One buffer for all such calls: they follow one another on the
 // library's one stream.  It grows to the largest call; a buffer that a captured graph addresses is not freed.
 float* vol_workspace(size_t bytes, cudaStream_t s) {
   static float* buf = nullptr;
   static size_t cap = 0;
   static bool captured = false;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  cudaStreamIsCapturing(s, &cs);
-  const bool capturing = cs != cudaStreamCaptureStatusNone;
+  const bool capturing = stream_capturing(s);
   if (cap < bytes) {
     if (buf && !captured && !capturing) { cudaStreamSynchronize(s); cudaFree(buf); }
     buf = nullptr; cap = 0; captured = false;
@@ -623,6 +627,7 @@ struct ConvModel {
   std::vector<F32ConvW*> split;
   float *buf[3] = {nullptr, nullptr, nullptr};
   size_t buf_bytes = 0;
+  size_t refused = 0;                   // bytes of split volumes that there was no memory for: not asked for again (0: none)
   int shape[4] = {0, 0, 0, 0};          // of the split volumes in buf, whose padding is zero (shape[0] = 0: none)
 };
 
@@ -678,6 +683,26 @@ static void set_strides(long long* n, long long* d, long long* h, long long* w, 
   *c = channels_last ? 1 : vox; *w = step; *h = W * step; *d = (long long)H * W * step; *n = vox * C;
 }
 
+// Three buffers of `bytes` each for what lies between the layers, split volumes or plain ones.  Nothing is freed or allocated while the
+// stream is captured (the eager call in front of a captured one has sized the buffers), and split volumes that did not fit are not asked
+// for again, so that such a network does not pay for freeing and allocating on every call.
+static bool conv_buffers(ConvModel* m, size_t bytes, bool split, cudaStream_t s) {
+  if (m->buf_bytes >= bytes) return true;
+  if (stream_capturing(s) || (split && m->refused && bytes >= m->refused)) return false;
+  for (float*& p : m->buf) { cudaFree(p); p = nullptr; }
+  m->buf_bytes = 0; m->shape[0] = 0;
+  for (float*& p : m->buf) {
+    if (split ? vol_alloc((void**)&p, bytes) : cudaMalloc(&p, bytes) == cudaSuccess) continue;
+    cudaGetLastError();
+    p = nullptr;
+    for (float*& q : m->buf) { cudaFree(q); q = nullptr; }
+    if (split) m->refused = bytes;
+    return false;
+  }
+  m->buf_bytes = bytes;
+  return true;
+}
+
 // A network whose layers behind the first all run on the tensor cores: every volume between them is a split volume of one grid
 // (zeros in front for the widest kernel), written by one layer as the next one reads it.  The first layer packs the input, or is a
 // short one that writes such a volume.  False where the network is not of that kind; *ok: how the call went.
@@ -702,17 +727,12 @@ static bool conv_forward_volumes(ConvModel* m, const float* x, float* y, int N, 
   }
   const int pitch = (cmax + 31) / 32 * 32;
   const size_t bytes = nl > 1 ? vol_bytes(vol_geom(conv_geom(m->meta[0], N, D, H, W), pad, pad, pad_w), pitch) : 0;
-  if (m->buf_bytes < bytes) {
-    for (float*& p : m->buf) { cudaFree(p); p = nullptr; }
-    m->buf_bytes = 0; m->shape[0] = 0;
-    for (float*& p : m->buf)
-      if (cudaMalloc(&p, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        for (float*& q : m->buf) { cudaFree(q); q = nullptr; }
-        return false;                                            // plain volumes take half as much
-      }
-    m->buf_bytes = bytes;
-  }
+  const bool first_short = !(m->vw[0] && vol_supported(conv_geom(m->meta[0], N, D, H, W)));
+  const VolGeom vg0 = vol_geom(conv_geom(m->meta[0], N, D, H, W), pad, pad, pad_w);
+  const int in_pitch0 = (m->meta[0].cin + 31) / 32 * 32;
+  float* packed = nullptr;                                       // the first layer's input, where that is not a short layer
+  if (!first_short && !(packed = vol_workspace(vol_bytes(vg0, in_pitch0), s))) return false;
+  if (!conv_buffers(m, bytes, true, s)) return false;            // plain volumes take half as much, less where channels are padded to 32
   if (bytes && (m->shape[0] != N || m->shape[1] != D || m->shape[2] != H || m->shape[3] != W)) {
     for (float* p : m->buf) cudaMemsetAsync(p, 0, bytes, s);     // the layers keep the padding zero from here on
     m->shape[0] = N; m->shape[1] = D; m->shape[2] = H; m->shape[3] = W;
@@ -731,19 +751,17 @@ static bool conv_forward_volumes(ConvModel* m, const float* x, float* y, int N, 
     std::memset(&o, 0, sizeof o);
     if (l < nl - 1) { o.vol = m->buf[dst]; o.pitch = pitch; o.skip = (L.flags & LFLAG_ADD_SKIP) ? m->buf[skip] : nullptr; }
     else { o.y = y; set_strides(&o.ys_n, &o.ys_d, &o.ys_h, &o.ys_w, &o.ys_c, true, L.cout, D, H, W); }
-    if (l == 0 && !(m->vw[0] && vol_supported(g))) {
+    if (l == 0 && first_short) {
       const ShortVol sv = {o.vol, vg.P * pitch, pitch, vg.Dq, vg.Hq, vg.Wq, pad, pad, pad_w};
       launch_short(x, m->wt[0], m->bias[0], nullptr, nullptr, g, L.act, L.slope, sv, s);
     } else {
       const float* in = cur < 0 ? nullptr : m->buf[cur];
       int in_pitch = pitch;
       if (l == 0) {
-        in_pitch = (L.cin + 31) / 32 * 32;
-        float* vol = vol_workspace(vol_bytes(vg, in_pitch), s);
-        if (!vol) { *ok = false; if (err) *err = "out of device memory for conv activations"; return true; }
+        in_pitch = in_pitch0;
         const VolSource src = {VolSource::PLAIN, 1, 1, 1, 1, g.xs_n, g.xs_d, g.xs_h, g.xs_w, g.xs_c};
-        vol_pack(x, vol, in_pitch, vg, src, s);
-        in = vol;
+        vol_pack(x, packed, in_pitch, vg, src, s);
+        in = packed;
       }
       *ok = vol_conv(m->vw[l], in, in_pitch, vg, o, m->bias[l], L.act, L.slope, status, s, true, err);
     }
@@ -772,13 +790,7 @@ bool conv_forward(ConvModel* m, const float* x, float* y, int N, int D, int H, i
     return true;
   }
   m->shape[0] = 0;
-  if (m->buf_bytes < (size_t)nvox * cmax * 4) {
-    for (float*& p : m->buf) { cudaFree(p); p = nullptr; }
-    m->buf_bytes = 0;
-    for (float*& p : m->buf)
-      if (cudaMalloc(&p, (size_t)nvox * cmax * 4) != cudaSuccess) { if (err) *err = "out of device memory for conv activations"; return false; }
-    m->buf_bytes = (size_t)nvox * cmax * 4;
-  }
+  if (!conv_buffers(m, (size_t)nvox * cmax * 4, false, s)) { if (err) *err = "out of device memory for conv activations"; return false; }
   const float* src = x;
   const float* skip = nullptr;
   int skip_buf = -1;
@@ -834,9 +846,7 @@ bool conv3d_ncdhw(const float* x, const float* w, float* y, int N, int C, int D,
   const bool tc = vol_supported(g) || f32tc_conv_supported(g);
   Cached* c = nullptr;
   bool fresh = false;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  cudaStreamIsCapturing(s, &cs);
-  const bool capturing = cs != cudaStreamCaptureStatusNone;
+  const bool capturing = stream_capturing(s);
   for (auto& q : cache) if (q.w == w && q.F == F && q.C == C && q.taps == taps) c = &q;
   if (c && capturing) c->captured = true;
   // every form the weights may be needed in, whatever the volume: a captured call packs none

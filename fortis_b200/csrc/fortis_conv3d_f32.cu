@@ -758,6 +758,14 @@ int vol_front_w(const ConvGeom& c) { return vol_line(c.KW, c.sw, c.pw) ? 0 : c.p
 
 size_t vol_bytes(const VolGeom& g, int pitch) { return (size_t)g.P * g.fd * g.fh * g.fw * pitch * 8; }
 
+bool vol_alloc(void** p, size_t bytes) {
+  g_launches.volume_allocs++;
+  if (!(g_tc_test.volume_limit && bytes > g_tc_test.volume_limit) && cudaMalloc(p, bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  *p = nullptr;
+  return false;
+}
+
 bool vol_supported(const ConvGeom& c) {
   if (c.dd != 1 || c.dh != 1 || c.dw != 1) return false;                // transposed convolutions
   // the most products an output can have: taps that lie inside the volume, times channels

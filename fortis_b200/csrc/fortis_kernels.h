@@ -86,10 +86,11 @@ struct TcTestKnobs {
   unsigned int wait_limit; int skip_stage;
   int no_stage;                                      // fused MLP kernel: move every tile's inputs and outputs element by element
   int conv_route;                                    // fp32 convolutions: 0 by estimate, 1 over split volumes wherever they can, 2 never
+  unsigned long long volume_limit;                   // bytes: an allocation for split volumes or their weights beyond it fails (0: no limit)
 };
 extern TcTestKnobs g_tc_test;
 // launches since the library was loaded, so that a test can tell which kernel served a call
-struct LaunchCounts { long vol_conv, mlp_pair; };
+struct LaunchCounts { long vol_conv, mlp_pair, volume_allocs; };     // volume_allocs: tries to allocate split volumes
 extern LaunchCounts g_launches;
 
 // ---- tensor-core fused MLP (fortis_mlp_tc.cu) ----------------------------------------------------------------
@@ -198,6 +199,7 @@ int vol_front_w(const ConvGeom& c);                            // zero positions
 bool vol_supported(const ConvGeom& c);
 long long vol_cost(const ConvGeom& c);                         // estimated device time with the input packed, ns
 size_t vol_bytes(const VolGeom& g, int pitch);                 // of a split volume with `pitch` channels a row (a multiple of 32)
+bool vol_alloc(void** p, size_t bytes);                        // device memory for split volumes and their weights
 struct VolW;                                                   // one layer's weights, split, as the kernel streams them
 // torch layout (F, C, taps); `line`: as vol_geom says of the layer
 VolW* vol_weights_pack(const float* w_dev, int F, int C, int taps, bool line, cudaStream_t s, std::string* err);

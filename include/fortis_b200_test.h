@@ -33,10 +33,12 @@ int fortis_debug_few_rows(const int* widths, int nlayers, int fp8w, long rows);
  *   "test_no_stage"    0 | 1  fused MLP kernel: fetch every tile's inputs and store its outputs element by element
  *                             instead of staging whole tiles by bulk copies (same bits; for the comparison of the paths)
  *   "test_conv_route"  0 | 1 | 2  fp32 convolutions: by estimate (0), over split volumes wherever the layer's shape
- *                             allows it (1), never over split volumes (2) */
+ *                             allows it (1), never over split volumes (2)
+ *   "test_volume_limit"  N    bytes: a device allocation for split volumes or their weights beyond it fails (0: no limit) */
 
 /* Launches of one kernel since the library was loaded ("conv_vol_kernel", "mlp_pair_kernel"; -1: no such counter), so that a
- * test can tell which kernel served a call.  Launches replayed by a graph are not counted. */
+ * test can tell which kernel served a call.  Launches replayed by a graph are not counted.  "volume_allocs": tries to allocate
+ * device memory for split volumes or their weights. */
 long fortis_debug_launches(const char* kernel);
 
 #ifdef __cplusplus
