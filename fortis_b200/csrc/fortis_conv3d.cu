@@ -361,11 +361,11 @@ std::vector<float> repack_weights_taps(const float* w, int F, int C, int taps) {
   return out;
 }
 
-// One layer's weights on the device: [tap][C][F] for the FFMA kernels and, where the tensor-core kernel may take the layer,
-// split for that one.  (Which of the two runs depends on the volume's extents too, so both stay.)
+// One layer's weights on the device: [tap][C][F] for the FFMA kernels and, where a tensor-core kernel may take the layer, split for
+// that one and, memory permitting, for split volumes.  (Which of them runs depends on the volume's extents too, so all stay.)
 struct LayerDev { float *wt = nullptr, *bias = nullptr; VolW* vw = nullptr; F32ConvW* split = nullptr; };
-// line: the form of the split volumes' weights; both: the other kernel's weights too
-bool upload_layer(const LayerHost& L, int taps, bool split, bool line, bool both, LayerDev* d, std::string* err) {
+// line: the form of the split volumes' weights
+bool upload_layer(const LayerHost& L, int taps, bool split, bool line, LayerDev* d, std::string* err) {
   split = split && (long long)L.cin * taps >= kF32TcConvMinProducts;
   const std::vector<float> wt = repack_weights_taps(L.W.data(), L.cout, L.cin, taps);
   float* raw = nullptr;
@@ -383,8 +383,8 @@ bool upload_layer(const LayerHost& L, int taps, bool split, bool line, bool both
   if (cudaMalloc(&raw, L.W.size() * 4) != cudaSuccess) return fail("out of device memory for conv weights");
   cudaMemcpy(raw, L.W.data(), L.W.size() * 4, cudaMemcpyHostToDevice);
   d->vw = vol_weights_pack(raw, L.cout, L.cin, taps, line, 0, nullptr);
-  if (both) d->split = f32tc_conv_pack(raw, L.cout, L.cin, taps, 0, nullptr);
-  if (!d->vw || (both && !d->split) || cudaStreamSynchronize(0) != cudaSuccess) return fail("out of device memory for split conv weights");
+  d->split = f32tc_conv_pack(raw, L.cout, L.cin, taps, 0, nullptr);
+  if (!d->split || cudaStreamSynchronize(0) != cudaSuccess) return fail("out of device memory for split conv weights");
   cudaFree(raw);
   return true;
 }
@@ -407,9 +407,9 @@ float* vol_workspace(size_t bytes, cudaStream_t s) {
     buf = nullptr; cap = 0; captured = false;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // an allocation is no stream operation: allowed beside a capture
     cudaThreadExchangeStreamCaptureMode(&mode);
-    const bool ok = cudaMalloc(&buf, bytes) == cudaSuccess;
+    const bool ok = vol_alloc((void**)&buf, bytes);
     cudaThreadExchangeStreamCaptureMode(&mode);
-    if (!ok) { cudaGetLastError(); buf = nullptr; return nullptr; }
+    if (!ok) return nullptr;
     cap = bytes;
   }
   if (capturing) captured = true;
@@ -426,9 +426,11 @@ bool takes_volume(const ConvGeom& g, long long in_front = 0) {
   return vol_supported(g) && (!f32tc_conv_supported(g) || vol_cost(g) < f32tc_conv_cost(g) + in_front);
 }
 
+// vw: the layer runs over a split volume (takes_volume), or from `src`; where there is no memory for the volume, and for vw = null, on the
+// kernels that need none, whose weights are `split` where f32tc_conv_supported says so and `wt` otherwise
 bool conv_layer(const VolW* vw, const F32ConvW* split, const float* wt, const float* bias, const float* x, const VolSource* src, const float* residual,
                 float* y, const ConvGeom& g, int act, float slope, int* status, cudaStream_t s, bool early, std::string* err) {
-  if (vw && (src || takes_volume(g))) {
+  if (vw) {
     const VolGeom vg = vol_geom(g, g.pd, g.ph, vol_front_w(g));
     const int pitch = (g.C + 31) / 32 * 32;
     float* vol = vol_workspace(vol_bytes(vg, pitch), s);
@@ -444,7 +446,6 @@ bool conv_layer(const VolW* vw, const F32ConvW* split, const float* wt, const fl
     if (src) { if (err) *err = "out of device memory for a convolution's input"; return false; }
   }
   if (split && f32tc_conv_supported(g)) return f32tc_conv(split, x, bias, residual, y, g, act, slope, status, s, early, err);
-  if (!wt) { if (err) *err = "out of device memory for a convolution's input"; return false; }
   launch_conv(x, wt, bias, residual, y, g, act, slope, s);
   return true;
 }
@@ -536,7 +537,7 @@ OpNet* opnet_create(const ModelHost& M, std::string* err) {
     LayerHost meta = L; meta.W.clear(); meta.b.clear();
     m->meta.push_back(meta);
     LayerDev d;
-    if (L.kind == LAYER_CONV2D && !upload_layer(L, L.kh * L.kw, L.dil == 1, L.kw == 3 && L.sw == 1 && L.pw <= 1, true, &d, err)) {
+    if (L.kind == LAYER_CONV2D && !upload_layer(L, L.kh * L.kw, L.dil == 1, L.kw == 3 && L.sw == 1 && L.pw <= 1, &d, err)) {
       opnet_destroy(m);
       return nullptr;
     }
@@ -592,7 +593,7 @@ bool opnet_forward(OpNet* m, const float* x, float* y, int N, int H, int W, int*
     const unsigned blocks = (unsigned)((nout + 255) / 256 < 148 * 16 ? (nout + 255) / 256 : 148 * 16);
     if (L.kind == LAYER_CONV2D) {
       const ConvGeom g = opnet_geom(L, N, h, w, h2, w2);
-      if (!conv_layer(m->vw[l], m->split[l], m->wt[l], m->bias[l], src, pending.op ? &pending : nullptr, nullptr, dst, g, L.act, L.slope, status, s, true, err)) return false;
+      if (!conv_layer(pending.op || takes_volume(g) ? m->vw[l] : nullptr, m->split[l], m->wt[l], m->bias[l], src, pending.op ? &pending : nullptr, nullptr, dst, g, L.act, L.slope, status, s, true, err)) return false;
       pending.op = VolSource::PLAIN;
     } else {
       const bool pool = L.kind == LAYER_MAXPOOL2D;
@@ -660,7 +661,7 @@ ConvModel* conv_model_create(const ModelHost& M, int precision, cudaStream_t s, 
     meta.W.clear(); meta.b.clear();
     m->meta.push_back(meta);
     LayerDev d;
-    if (!upload_layer(L, L.ksize * L.ksize * L.ksize, true, L.ksize == 3 && L.pad == 1, true, &d, err)) {
+    if (!upload_layer(L, L.ksize * L.ksize * L.ksize, true, L.ksize == 3 && L.pad == 1, &d, err)) {
       conv_model_destroy(m);
       return nullptr;
     }
@@ -809,7 +810,7 @@ bool conv_forward(ConvModel* m, const float* x, float* y, int N, int D, int H, i
     set_strides(&g.rs_n, &g.rs_d, &g.rs_h, &g.rs_w, &g.rs_c, false, L.cout, D, H, W);          // a skip is a layer's output, channel-major
     const float* res = (L.flags & LFLAG_ADD_SKIP) ? skip : nullptr;
     if ((L.flags & LFLAG_ADD_SKIP) && !skip) { if (err) *err = "conv3d model: a layer adds a skip that was never saved"; return false; }
-    if (!conv_layer(m->vw[l], m->split[l], m->wt[l], m->bias[l], src, nullptr, res, dst, g, L.act, L.slope, status, s, true, err)) return false;
+    if (!conv_layer(takes_volume(g) ? m->vw[l] : nullptr, m->split[l], m->wt[l], m->bias[l], src, nullptr, res, dst, g, L.act, L.slope, status, s, true, err)) return false;
     if (L.flags & LFLAG_SAVE_SKIP) { skip = dst; skip_buf = dst_buf; }
     src = dst;
   }
@@ -828,8 +829,13 @@ bool conv3d_ncdhw(const float* x, const float* w, float* y, int N, int C, int D,
   // freed and replaced.  A weight seen for the first time needs a buffer: that cannot happen while the stream is being
   // captured into a graph, so such a call is refused (the reference captures on the second call for the same reason: the
   // first call allocates).
-  // vw: the forms for layers that take a tap at a time and, of kernels three wide, a line's taps at a time: stride and padding decide
-  struct Cached { const float* w; int F, C, taps; float* wt; VolW* vw[2]; F32ConvW* split; bool captured; };
+  // Which weights a call needs depends on its extents, stride and padding.  `split` (f32tc_conv_supported) or `wt` are packed for every
+  // call: a captured call, which packs none, finds them whatever its volume.  vw (a tap at a time, or of kernels three wide a line's taps)
+  // is packed for the first eager call that runs over split volumes in that form; without it, or without memory for it (no_vw), a call
+  // runs on the others.
+  // plan: where the call with these extents runs, so that a repeated one (10.5 us) does not estimate again (0.3 us).
+  struct Plan { ConvGeom g; bool valid, volume, split; };
+  struct Cached { const float* w; int F, C, taps; float* wt; VolW* vw[2]; bool no_vw[2]; F32ConvW* split; bool captured; Plan plan; };
   static std::vector<Cached> cache;
   static size_t victim = 0;
   const int taps = K[0] * K[1] * K[2];
@@ -841,37 +847,45 @@ bool conv3d_ncdhw(const float* x, const float* w, float* y, int N, int C, int D,
   g.Do = (D + 2 * pad[0] - K[0]) / stride[0] + 1; g.Ho = (H + 2 * pad[1] - K[1]) / stride[1] + 1; g.Wo = (W + 2 * pad[2] - K[2]) / stride[2] + 1;
   g.xs_w = 1; g.xs_h = W; g.xs_d = (long long)H * W; g.xs_c = (long long)D * H * W; g.xs_n = (long long)C * D * H * W;
   g.ys_w = 1; g.ys_h = g.Wo; g.ys_d = (long long)g.Ho * g.Wo; g.ys_c = (long long)g.Do * g.Ho * g.Wo; g.ys_n = (long long)F * g.Do * g.Ho * g.Wo;
-  const VolGeom vg = vol_geom(g, g.pd, g.ph, vol_front_w(g));
-  const int line = vg.line;
-  const bool tc = vol_supported(g) || f32tc_conv_supported(g);
   Cached* c = nullptr;
   bool fresh = false;
   const bool capturing = stream_capturing(s);
   for (auto& q : cache) if (q.w == w && q.F == F && q.C == C && q.taps == taps) c = &q;
   if (c && capturing) c->captured = true;
-  // every form the weights may be needed in, whatever the volume: a captured call packs none
-  auto complete = [&](const Cached* e) { return tc ? e->split && e->vw[0] && (K[2] != 3 || e->vw[1]) : e->wt != nullptr; };
-  if (!c || !complete(c)) {
+  if (!c && !capturing) {
+    for (size_t i = 0; i < cache.size() && cache.size() >= 64 && !c; i++, victim = (victim + 1) % cache.size())
+      if (!cache[victim].captured) c = &cache[victim];
+    if (c) { cudaStreamSynchronize(s); cudaFree(c->wt); vol_weights_free(c->vw[0]); vol_weights_free(c->vw[1]); f32tc_conv_free(c->split); }
+    else { cache.push_back(Cached{}); c = &cache.back(); }
+    *c = Cached{};
+    c->w = w; c->F = F; c->C = C; c->taps = taps;
+  }
+  if (c && (!c->plan.valid || std::memcmp(&c->plan.g, &g, sizeof g) != 0 || g_tc_test.conv_route)) {
+    std::memcpy(&c->plan.g, &g, sizeof g); c->plan.valid = !g_tc_test.conv_route;
+    c->plan.volume = takes_volume(g); c->plan.split = f32tc_conv_supported(g);
+  }
+  if (!c || (c->plan.split ? (void*)c->split : (void*)c->wt) == nullptr) {
     if (capturing) { if (err) *err = "conv weights seen for the first time during graph capture; run one eager call first"; return false; }
-    if (!c) {
-      for (size_t i = 0; i < cache.size() && cache.size() >= 64 && !c; i++, victim = (victim + 1) % cache.size())
-        if (!cache[victim].captured) c = &cache[victim];
-      if (c) { cudaStreamSynchronize(s); cudaFree(c->wt); vol_weights_free(c->vw[0]); vol_weights_free(c->vw[1]); f32tc_conv_free(c->split); }
-      else { cache.push_back(Cached{}); c = &cache.back(); }
-      *c = Cached{w, F, C, taps, nullptr, {nullptr, nullptr}, nullptr, false};
-    }
-    const size_t n = (size_t)F * C * taps;
-    if (tc) {
-      for (int form = 0; form < (K[2] == 3 ? 2 : 1); form++)
-        if (!c->vw[form] && !(c->vw[form] = vol_weights_pack(w, F, C, taps, form != 0, s, err))) return false;
-      if (!c->split && !(c->split = f32tc_conv_pack(w, F, C, taps, s, err))) return false;
+    if (c->plan.split) {
+      if (!(c->split = f32tc_conv_pack(w, F, C, taps, s, err))) return false;
     } else {
+      const size_t n = (size_t)F * C * taps;
       if (cudaMalloc(&c->wt, n * 4) != cudaSuccess) { cudaGetLastError(); c->wt = nullptr; if (err) *err = "out of device memory for conv weights"; return false; }
       repack_weights_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(w, c->wt, F, C, taps);
     }
     fresh = true;
   }
-  if (!conv_layer(tc ? c->vw[line] : nullptr, tc ? c->split : nullptr, c->wt, nullptr, x, nullptr, nullptr, y, g, ACT_NONE, 0.f, status, s, !fresh, err)) return false;
+  VolW* vw = nullptr;
+  if (c->plan.volume) {
+    const int line = vol_geom(g, g.pd, g.ph, vol_front_w(g)).line;
+    if (!c->vw[line] && !c->no_vw[line] && !capturing) {
+      c->vw[line] = vol_weights_pack(w, F, C, taps, line != 0, s, nullptr);
+      c->no_vw[line] = !c->vw[line];
+      fresh = true;
+    }
+    vw = c->vw[line];
+  }
+  if (!conv_layer(vw, c->plan.split ? c->split : nullptr, c->wt, nullptr, x, nullptr, nullptr, y, g, ACT_NONE, 0.f, status, s, !fresh, err)) return false;
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { if (err) *err = std::string("conv3d launch: ") + cudaGetErrorString(e); return false; }
   return true;

@@ -815,8 +815,7 @@ VolW* vol_weights_pack(const float* w_dev, int F, int C, int taps, bool line, cu
   VolW* w = new VolW();
   w->F = F; w->C = C; w->taps = taps; w->kw = line ? 3 : 1; w->NT = vol_nt(F); w->nchb = (C + kKt - 1) / kKt; w->ntn = (F + w->NT - 1) / w->NT;
   const long long rows = (long long)(taps / w->kw) * w->nchb * w->ntn * (line ? 6 : 2) * w->NT;
-  if (cudaMalloc(&w->img, (size_t)rows * kKt * 4) != cudaSuccess) {
-    cudaGetLastError();
+  if (!vol_alloc((void**)&w->img, (size_t)rows * kKt * 4)) {
     if (err) *err = "out of device memory for split conv weights";
     delete w;
     return nullptr;

@@ -58,3 +58,54 @@ def test_network_without_room_for_split_volumes(host, cin, graph):
     assert host.L.fortis_debug_launches(b"conv_vol_kernel") == launches
     call((1, 6, 7, 8))                                         # fits what there is
     call((2, 12, 11, 13))
+
+
+def layer(host, x, w, pad):
+    from tests.test_gpu_f32tc import conv_call
+    y = torch.full([x.shape[0], w.shape[0]] + [n + 2 * p - k + 1 for n, p, k in zip(x.shape[2:], pad, w.shape[2:])], float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    conv_call(host, x, w, y, (1, 1, 1), pad)
+    host.sync()
+    return y
+
+
+# a kernel that the split-TF32 kernel takes, and one of more taps in a row than that has tables for
+@pytest.mark.parametrize("K", [(3, 3, 3), (1, 1, 40)])
+@pytest.mark.parametrize("limit", [1, 1 << 19])                # no room for the weights; room for them, not for the volume
+def test_layer_without_room_for_a_split_volume(host, K, limit):
+    from tests.test_gpu_f32tc import conv64, randn
+    pad = tuple(min(1, k // 2) for k in K)
+    x, w = randn((1, 32, 9, 33, 60), 1), randn((8, 32) + K, 2)
+    host.option("test_conv_route", 1)
+    host.option("test_volume_limit", limit)
+    launches = host.L.fortis_debug_launches(b"conv_vol_kernel")
+    y = layer(host, x, w, pad)
+    assert host.L.fortis_debug_launches(b"conv_vol_kernel") == launches
+    # sums of up to 1280 products: on the FFMA kernel one rounding each, at random 2^-24 * sqrt(1280 / 3) of the 2-norm = 1.2e-6
+    assert rel(y, conv64(x, w, (1, 1, 1), pad)) < 2 * TOL
+    assert host.L.fortis_last_error() == 0
+
+
+def test_model_without_room_for_split_volume_weights(host):
+    rng = np.random.default_rng(4)
+    layers = [conv3d_layer(rng, ci, co, 3, a) for ci, co, a in [(3, 32, "leaky"), (32, 32, "leaky"), (32, 5, "none")]]
+    host.option("test_volume_limit", 1)
+    host.load_model(write_blob(layers))
+    host.option("conv_shape", "1,6,7,8")
+    x, y = rng.standard_normal((1, 6, 7, 8, 3)).astype(np.float32), np.zeros((1, 6, 7, 8, 5), np.float32)
+    host.forward(x, y)
+    assert rel(torch.from_numpy(y), network64(layers, x)) < 3 * TOL
+
+
+def test_weights_are_kept_once_per_form_that_calls_take(host):
+    """A layer called with one stride and padding packs one form of its weights for split volumes, and repeats nothing."""
+    from tests.test_gpu_f32tc import conv64, randn
+    x, w = randn((1, 32, 9, 10, 11), 1), randn((64, 32, 3, 3, 3), 2)
+    host.option("test_conv_route", 1)
+    allocs = lambda: host.L.fortis_debug_launches(b"volume_allocs")
+    layer(host, x, randn((64, 32, 3, 3, 3), 3), (1, 1, 1))      # sizes the workspace
+    before = allocs()
+    for _ in range(3):
+        y = layer(host, x, w, (1, 1, 1))
+    assert allocs() == before + 1
+    assert rel(y, conv64(x, w, (1, 1, 1), (1, 1, 1))) < TOL
