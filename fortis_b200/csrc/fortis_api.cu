@@ -94,6 +94,7 @@ void* pool_alloc(long n) {
         break;
       }
     cudaGetLastError();
+    if (g_stream) conv_workspace_release(g_stream);
     for (int i = 0; i < kPool; i++)
       if (g_pool[i].p && !g_pool[i].used) { cudaFree(g_pool[i].p); g_pool[i].p = nullptr; g_pool[i].n = 0; }
   }
@@ -207,6 +208,8 @@ void free_plan(PlanDev& P) {
   P = PlanDev();
 }
 
+void set_capturing(bool on) { fortis_capturing = on; g_own_capture = on; }
+
 void drop_graph() {
   Session& s = S();
   if (s.gexec) { cudaGraphExecDestroy(s.gexec); s.gexec = nullptr; }
@@ -215,6 +218,7 @@ void drop_graph() {
   if (s.ov_gexec) { cudaGraphExecDestroy(s.ov_gexec); s.ov_gexec = nullptr; }
   s.ov_key.clear();
   s.ov_calls = 0;
+  if (g_stream) conv_graphs_dropped(g_stream);
 }
 
 void free_model_dev() {
@@ -888,14 +892,14 @@ void run_step(const StepArgs& A) {
   if (key != s.gkey) { drop_graph(); s.gkey = key; }
   const bool cap = (++s.ncalls == 2);
   if (!cap) { run_step_kernels(A); return; }
-  fortis_capturing = 1;
+  set_capturing(true);
   if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-    cudaGetLastError(); fortis_capturing = 0; run_step_kernels(A); return;
+    cudaGetLastError(); set_capturing(false); run_step_kernels(A); return;
   }
   bool threw = false; std::string what;
   try { run_step_kernels(A); } catch (const std::exception& e) { threw = true; what = e.what(); }
   cudaGraph_t gr = nullptr;
-  fortis_capturing = 0;
+  set_capturing(false);
   const bool ok = cudaStreamEndCapture(st, &gr) == cudaSuccess && !threw &&
                   cudaGraphInstantiate(&s.gexec, gr, 0) == cudaSuccess;
   if (gr) cudaGraphDestroy(gr);
@@ -1141,7 +1145,7 @@ bool overlapped_step(void* const* gptrs, void* const* sptrs, long long rows) {
 
   bool capturing = (++s.ov_calls == 2) && !std::getenv("FORTIS_NO_STAGING_GRAPH");
   if (capturing && cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { cudaGetLastError(); capturing = false; }
-  if (capturing) fortis_capturing = 1;
+  if (capturing) set_capturing(true);
   bool threw = false; std::string what;
   try {
     // fork: both copy streams start behind everything already on the persistent stream (the previous step included)
@@ -1195,7 +1199,7 @@ bool overlapped_step(void* const* gptrs, void* const* sptrs, long long rows) {
     cudaStreamWaitEvent(st, g_ev_join_out, 0);
   } catch (const std::exception& e) { threw = true; what = e.what(); }
   if (capturing) {
-    fortis_capturing = 0;
+    set_capturing(false);
     cudaGraph_t gr = nullptr;
     const bool ok = cudaStreamEndCapture(st, &gr) == cudaSuccess && !threw && cudaGraphInstantiate(&s.ov_gexec, gr, 0) == cudaSuccess;
     if (gr) cudaGraphDestroy(gr);
@@ -1257,7 +1261,7 @@ bool overlapped_planes_step(void* const* gptrs, void* const* sptrs) {
   const LoopInfo saved = s.loop;
   bool capturing = (++s.ov_calls == 2) && !std::getenv("FORTIS_NO_STAGING_GRAPH");
   if (capturing && cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { cudaGetLastError(); capturing = false; }
-  if (capturing) fortis_capturing = 1;
+  if (capturing) set_capturing(true);
   bool threw = false; std::string what;
   try {
     cudaEventRecord(g_ev_fork, st);
@@ -1292,7 +1296,7 @@ bool overlapped_planes_step(void* const* gptrs, void* const* sptrs) {
     cudaStreamWaitEvent(st, g_ev_join_out, 0);
   } catch (const std::exception& e) { threw = true; what = e.what(); s.loop = saved; }
   if (capturing) {
-    fortis_capturing = 0;
+    set_capturing(false);
     cudaGraph_t gr = nullptr;
     const bool ok = cudaStreamEndCapture(st, &gr) == cudaSuccess && !threw && cudaGraphInstantiate(&s.ov_gexec, gr, 0) == cudaSuccess;
     if (gr) cudaGraphDestroy(gr);
@@ -1497,6 +1501,7 @@ void fortis_reset(void) {
   if (g_stream) cudaStreamSynchronize(g_stream);
   Session& s = S();
   drop_graph();
+  if (g_stream) conv_workspace_release(g_stream);
   free_plan(s.G); free_plan(s.S);
   free_model_dev();
   pool_free(s.din); pool_free(s.dout); pool_free(s.act0); pool_free(s.act1);

@@ -396,24 +396,37 @@ bool stream_capturing(cudaStream_t s) {
 }
 
 // The split volume of a layer whose input is a plain array.  One buffer for all such calls: they follow one another on the
-// library's one stream.  It grows to the largest call; a buffer that a captured graph addresses is not freed.
+// library's one stream.  It grows to the largest call and goes back to the device when the library is reset or short of memory.  A buffer
+// that a graph addresses is not freed: one of the library's own graphs gives it back when it is dropped; of a graph that the caller
+// has captured the end is not known.
+struct Workspace {
+  float* buf = nullptr;
+  size_t cap = 0, refused = 0;            // refused: bytes that there was no memory for, not asked for again before the next release
+  bool in_own_graph = false, in_callers_graph = false;
+  std::vector<float*> retired;            // outgrown buffers of the library's own graphs
+} g_work;
+
 float* vol_workspace(size_t bytes, cudaStream_t s) {
-  static float* buf = nullptr;
-  static size_t cap = 0;
-  static bool captured = false;
+  Workspace& k = g_work;
   const bool capturing = stream_capturing(s);
-  if (cap < bytes) {
-    if (buf && !captured && !capturing) { cudaStreamSynchronize(s); cudaFree(buf); }
-    buf = nullptr; cap = 0; captured = false;
+  if (k.cap < bytes) {
+    if (k.refused && bytes >= k.refused) return nullptr;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // an allocation is no stream operation: allowed beside a capture
     cudaThreadExchangeStreamCaptureMode(&mode);
-    const bool ok = vol_alloc((void**)&buf, bytes);
+    if (k.buf && k.in_own_graph && !k.in_callers_graph) k.retired.push_back(k.buf);
+    else if (k.buf && !k.in_callers_graph) {
+      // (kernels in flight still use it; while the stream is captured nothing may wait for them)
+      if (capturing) k.retired.push_back(k.buf);
+      else { cudaStreamSynchronize(s); cudaFree(k.buf); }
+    }
+    k.buf = nullptr; k.cap = 0; k.in_own_graph = k.in_callers_graph = false;
+    const bool ok = vol_alloc((void**)&k.buf, bytes);
     cudaThreadExchangeStreamCaptureMode(&mode);
-    if (!ok) return nullptr;
-    cap = bytes;
+    if (!ok) { k.refused = bytes; return nullptr; }
+    k.cap = bytes;
   }
-  if (capturing) captured = true;
-  return buf;
+  if (capturing) (g_own_capture ? k.in_own_graph : k.in_callers_graph) = true;
+  return k.buf;
 }
 
 // Where a layer whose input is a plain array runs: over a split volume (packing, then no thread in the operand path), on the kernel whose
@@ -476,6 +489,25 @@ __global__ void upsample_nearest2d_kernel(const float* __restrict__ x, float* __
 }
 
 }  // namespace
+
+// the library's own graphs are gone: so may be the buffers that they addressed
+void conv_graphs_dropped(cudaStream_t s) {
+  Workspace& k = g_work;
+  if (k.retired.empty() && !k.in_own_graph) return;
+  if (stream_capturing(s)) return;
+  for (float* p : k.retired) cudaFree(p);                     // waits for the kernels in flight
+  k.retired.clear();
+  k.in_own_graph = false;
+}
+
+void conv_workspace_release(cudaStream_t s) {
+  Workspace& k = g_work;
+  if (stream_capturing(s)) return;
+  k.refused = 0;
+  if (!k.buf || k.in_own_graph || k.in_callers_graph) return;
+  cudaFree(k.buf);
+  k.buf = nullptr; k.cap = 0;
+}
 
 // ---------------------------------------------------------------------------------------------------------------
 // Networks of 2-D operator layers, NCHW fp32: Conv2d (any kernel, stride, padding; transposed convolutions as the

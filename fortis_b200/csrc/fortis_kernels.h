@@ -92,6 +92,11 @@ extern TcTestKnobs g_tc_test;
 // launches since the library was loaded, so that a test can tell which kernel served a call
 struct LaunchCounts { long vol_conv, mlp_pair, volume_allocs; };     // volume_allocs: tries to allocate split volumes
 extern LaunchCounts g_launches;
+extern bool g_own_capture;                           // the stream is captured for one of the library's own graphs, not the caller's
+// The buffer for split volumes of single layers (fortis_conv3d.cu): given back to the device unless a graph addresses it; and what
+// the library's own graphs addressed, once they are dropped
+void conv_workspace_release(cudaStream_t s);
+void conv_graphs_dropped(cudaStream_t s);
 
 // ---- tensor-core fused MLP (fortis_mlp_tc.cu) ----------------------------------------------------------------
 struct ModelHost;

@@ -1042,6 +1042,7 @@ float e4m3_round(float v) {
 
 TcTestKnobs g_tc_test = {};
 LaunchCounts g_launches = {};
+bool g_own_capture = false;
 
 // One Linear layer converted for the tensor-core kernel: padded, rounded to the 16-bit operand type (FP8 weights: the
 // nearest E4M3 code of w / scale, which bf16 represents exactly), as row-major [N][K] (`rowmajor`, optional) and as

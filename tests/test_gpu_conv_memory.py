@@ -109,3 +109,42 @@ def test_weights_are_kept_once_per_form_that_calls_take(host):
         y = layer(host, x, w, (1, 1, 1))
     assert allocs() == before + 1
     assert rel(y, conv64(x, w, (1, 1, 1), (1, 1, 1))) < TOL
+
+
+def device_free():
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+def test_the_workspace_of_single_layers_goes_back_to_the_device(host, graph):
+    """A layer's split volume (68 MB) is given back by a reset; one that a graph of the library addresses, also after it was outgrown by
+    a larger layer (270 MB), with the graph."""
+    from tests.test_gpu_f32tc import randn
+    rng = np.random.default_rng(6)
+    host.option("test_conv_route", 1)
+    x, w = [randn((1, 32, d, 64, 64), 1) for d in (63, 255)], randn((8, 32, 3, 3, 3), 2)
+    layer(host, x[0][:, :, :5].contiguous(), w, (1, 1, 1))
+    host.reset()
+    torch.cuda.empty_cache()
+    before = device_free()
+    host.option("test_conv_route", 1)
+    if graph:                                                  # one layer, 32 channels: its input is packed into the workspace
+        host.load_model(write_blob([conv3d_layer(rng, 32, 3, 3)]))
+        host.option("conv_shape", "1,63,64,64")
+        host.option("graph", 1)
+        xn = rng.standard_normal((1, 63, 64, 64, 32)).astype(np.float32)
+        yn = [np.zeros((1, 63, 64, 64, 3), np.float32) for _ in range(3)]
+        host.forward(xn, yn[0])
+        host.forward(xn, yn[1])                                # captured
+    y = [layer(host, v, w, (1, 1, 1)) for v in x]
+    if graph:
+        host.forward(xn, yn[2])                                # replayed: in the buffer that was outgrown
+        assert yn[1].tobytes() == yn[0].tobytes() and yn[2].tobytes() == yn[0].tobytes()
+    assert before - device_free() > 270 << 20
+    host.reset()
+    del y
+    torch.cuda.empty_cache()
+    kept = before - device_free()
+    # (what the pool of model buffers keeps for the next model: the network's input and output)
+    assert kept < (64 << 20)
