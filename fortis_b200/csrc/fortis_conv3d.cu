@@ -661,6 +661,8 @@ struct ConvModel {
   float *buf[3] = {nullptr, nullptr, nullptr};
   size_t buf_bytes = 0;
   size_t refused = 0;                   // bytes of split volumes that there was no memory for: not asked for again (0: none)
+  int planned[4] = {0, 0, 0, 0};        // the extents for which `volumes` says whether the network runs over split volumes
+  bool volumes = false;
   int shape[4] = {0, 0, 0, 0};          // of the split volumes in buf, whose padding is zero (shape[0] = 0: none)
 };
 
@@ -736,29 +738,62 @@ static bool conv_buffers(ConvModel* m, size_t bytes, bool split, cudaStream_t s)
   return true;
 }
 
-// A network whose layers behind the first all run on the tensor cores: every volume between them is a split volume of one grid
-// (zeros in front for the widest kernel), written by one layer as the next one reads it.  The first layer packs the input, or is a
-// short one that writes such a volume.  False where the network is not of that kind; *ok: how the call went.
-static bool conv_forward_volumes(ConvModel* m, const float* x, float* y, int N, int D, int H, int W, int* status, cudaStream_t s, bool* ok, std::string* err) {
+// the grid of a network's split volumes: zeros in front for the widest kernel, channels for the widest volume
+struct NetGrid { int pad = 0, pad_w = 0, pitch = 0; };
+static NetGrid net_grid(const ConvModel* m, int N, int D, int H, int W) {
   const int nl = (int)m->meta.size();
-  if (g_tc_test.conv_route == 2) return false;
-  int pad = 0, pad_w = 0, cmax = 0;
+  NetGrid q;
   for (int l = 0; l < nl; l++) {
-    pad = m->meta[l].pad > pad ? m->meta[l].pad : pad;
+    q.pad = m->meta[l].pad > q.pad ? m->meta[l].pad : q.pad;
     const int fw = vol_front_w(conv_geom(m->meta[l], N, D, H, W));
-    if (l > 0 || m->vw[0]) pad_w = fw > pad_w ? fw : pad_w;
-    if (l < nl - 1 && m->meta[l].cout > cmax) cmax = m->meta[l].cout;
+    if (l > 0 || m->vw[0]) q.pad_w = fw > q.pad_w ? fw : q.pad_w;
+    if (l < nl - 1 && (m->meta[l].cout + 31) / 32 * 32 > q.pitch) q.pitch = (m->meta[l].cout + 31) / 32 * 32;
   }
+  return q;
+}
+
+// Does a network run over split volumes from layer to layer?  All layers behind the first have to run on the tensor cores, and the
+// estimate has to say that it is faster than layer by layer on the kernel that loads the taps: volumes pad channels to 32, which few
+// channels with many taps pay for.  Four hidden layers, 2 x 33^3, over volumes / layer by layer: 64 channels 3x3x3 357 / 758 us, 16
+// channels 180 / 240, 8 channels 174 / 146, 8 channels 5x5x5 1410 / 486, 128 channels 1x1x1 231 / 180.
+static bool takes_volumes(const ConvModel* m, int N, int D, int H, int W) {
+  if (g_tc_test.conv_route == 2) return false;
+  const int nl = (int)m->meta.size();
+  const NetGrid q = net_grid(m, N, D, H, W);
+  long long over = 0, layers = 0;
   for (int l = 0; l < nl; l++) {
     const LayerHost& L = m->meta[l];
     ConvGeom g = conv_geom(L, N, D, H, W);
-    set_strides(&g.xs_n, &g.xs_d, &g.xs_h, &g.xs_w, &g.xs_c, true, L.cin, D, H, W);
+    set_strides(&g.xs_n, &g.xs_d, &g.xs_h, &g.xs_w, &g.xs_c, l == 0, L.cin, D, H, W);
     if (!(m->vw[l] && vol_supported(g)) && !(l == 0 && nl > 1 && short_supported(g))) return false;
     if (l == nl - 1 && (L.flags & (LFLAG_ADD_SKIP | LFLAG_SAVE_SKIP))) return false;
     if (l == 0 && (L.flags & LFLAG_ADD_SKIP)) return false;
-    if ((long long)(D + pad) * (H + pad) * (W + pad) * N >= (1LL << 30)) return false;
+    if ((long long)(D + q.pad) * (H + q.pad) * (W + q.pad) * N >= (1LL << 30)) return false;
+    const VolGeom vg = vol_geom(g, q.pad, q.pad, q.pad_w);
+    if (!(m->vw[l] && vol_supported(g))) {                       // the same kernel either way, that writes more
+      const long long more = (long long)vol_bytes(vg, q.pitch) - 4LL * N * D * H * W * L.cout;
+      over += more > 0 ? more / 2500 : 0;
+      continue;
+    }
+    over += vol_kernel_cost(vg, L.cout) + 1000 + (l == 0 ? vol_pack_cost(vg) : 0);     // a cluster's launch: 1 us more
+    layers += f32tc_conv_supported(g) ? f32tc_conv_cost(g) : 1LL << 50;
   }
-  const int pitch = (cmax + 31) / 32 * 32;
+  return g_tc_test.conv_route == 1 || over < layers;
+}
+
+// A network whose layers behind the first all run on the tensor cores: every volume between them is a split volume of one grid, written
+// by one layer as the next one reads it.  The first layer packs the input, or is a short one that writes such a volume.  False where
+// the network does not run like that; *ok: how the call went.
+static bool conv_forward_volumes(ConvModel* m, const float* x, float* y, int N, int D, int H, int W, int* status, cudaStream_t s, bool* ok, std::string* err) {
+  const int nl = (int)m->meta.size(), extents[4] = {N, D, H, W};
+  if (g_tc_test.conv_route || std::memcmp(m->planned, extents, sizeof extents) != 0) {
+    m->volumes = takes_volumes(m, N, D, H, W);
+    std::memcpy(m->planned, extents, sizeof extents);
+    if (g_tc_test.conv_route) m->planned[0] = 0;
+  }
+  if (!m->volumes) return false;
+  const NetGrid q = net_grid(m, N, D, H, W);
+  const int pad = q.pad, pad_w = q.pad_w, pitch = q.pitch;
   const size_t bytes = nl > 1 ? vol_bytes(vol_geom(conv_geom(m->meta[0], N, D, H, W), pad, pad, pad_w), pitch) : 0;
   const bool first_short = !(m->vw[0] && vol_supported(conv_geom(m->meta[0], N, D, H, W)));
   const VolGeom vg0 = vol_geom(conv_geom(m->meta[0], N, D, H, W), pad, pad, pad_w);

@@ -789,18 +789,24 @@ Pieces pick_pieces(const VolGeom& g, int ntn) {
   return Pieces{1, (int)one, all, 0};
 }
 
-// Estimated device time of a layer whose input is packed first, ns: one launch more, packing at 1.6 TB/s of what it writes (slower than it measures now: a call near the line
-// stays with the general kernel), rounds of tiles, and in each the
-// steps (a tap each: stages shared or not; a line's taps: 32 or 64 features) and the tile's end.
-long long vol_cost(const ConvGeom& c) {
-  const VolGeom g = vol_geom(c, c.pd, c.ph, vol_front_w(c));
-  const int NT = vol_nt(c.F), pitch = (c.C + 31) / 32 * 32;
+// Estimated device time of a layer, ns: rounds of tiles, and in each the steps and the tile's end.  The constants are those of 520 timed
+// layers and networks, on the high side of the fits (a line's taps 365 and 610 ns a step, a tap 330 to 380 with shared stages and 510 to
+// 530 without, packing 5.4 TB/s of what it writes and 6 us), so that a call near the line stays with the general kernel.  A block of up to
+// 24 channels issues its MMAs one by one: 24 -> 24 channels 5x5x5 on 2 x 40^3 450 us, on the general kernel 409, without that term taken
+// for 421 and 435.
+long long vol_kernel_cost(const VolGeom& g, int F) {
+  const int NT = vol_nt(F), blocks = (g.C + 31) / 32, last = g.C % 32;
   Sharing s;
   if (!pick_sharing(g, NT, g.line, &s)) return 1LL << 60;
-  const Pieces pc = pick_pieces(g, (c.F + NT - 1) / NT);
-  const long long pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1, tiles = (long long)pc.n * pc.pairs * ((c.F + NT - 1) / NT), rounds = (tiles + pairs - 1) / pairs, steps = (long long)s.ng * s.tpg * (pitch / 32);
-  const long long step = g.line ? (NT == 64 ? 680 : 600) : s.tpg > 1 ? 380 : 570, end = g.line ? 2600 : 1500;
-  return 6500 + (long long)(vol_bytes(g, pitch) / 1600) + rounds * (steps * step + end);
+  const Pieces pc = pick_pieces(g, (F + NT - 1) / NT);
+  const long long pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1, tiles = (long long)pc.n * pc.pairs * ((F + NT - 1) / NT), rounds = (tiles + pairs - 1) / pairs;
+  const long long taps = s.ng * s.tpg, step = g.line ? (NT == 64 ? 680 : 500) : s.tpg > 1 ? 380 : 570, end = g.line ? (NT == 64 ? 2600 : 2000) : 1500;
+  return rounds * (taps * (blocks * step + (!g.line && last > 0 && last <= 24 ? 50 : 0)) + end);
+}
+long long vol_pack_cost(const VolGeom& g) { return 6500 + (long long)(vol_bytes(g, (g.C + 31) / 32 * 32) / 1600); }
+long long vol_cost(const ConvGeom& c) {
+  const VolGeom g = vol_geom(c, c.pd, c.ph, vol_front_w(c));
+  return vol_pack_cost(g) + vol_kernel_cost(g, c.F);
 }
 
 struct VolW { int F = 0, C = 0, taps = 0, kw = 1, NT = 0, nchb = 0, ntn = 0; float* img = nullptr; CUtensorMap map; };     // kw: taps of a step

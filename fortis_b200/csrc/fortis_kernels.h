@@ -202,7 +202,10 @@ struct VolGeom {
 VolGeom vol_geom(const ConvGeom& c, int front_d, int front_h, int front_w);
 int vol_front_w(const ConvGeom& c);                            // zero positions a layer needs in front of a line
 bool vol_supported(const ConvGeom& c);
-long long vol_cost(const ConvGeom& c);                         // estimated device time with the input packed, ns
+// estimated device times, ns: of a layer over a volume, of packing its input, and of both
+long long vol_kernel_cost(const VolGeom& g, int F);
+long long vol_pack_cost(const VolGeom& g);
+long long vol_cost(const ConvGeom& c);
 size_t vol_bytes(const VolGeom& g, int pitch);                 // of a split volume with `pitch` channels a row (a multiple of 32)
 bool vol_alloc(void** p, size_t bytes);                        // device memory for split volumes and their weights
 struct VolW;                                                   // one layer's weights, split, as the kernel streams them

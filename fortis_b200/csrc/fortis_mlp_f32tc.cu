@@ -1322,7 +1322,10 @@ long long f32tc_conv_cost(const ConvGeom& g) {
   const long long steps = ((long long)g.KD * g.KH * g.KW * ((g.C + G - 1) / G * G) + kKt - 1) / kKt;
   const long long tiles = (((long long)g.N * g.Do * g.Ho * g.Wo + kM - 1) / kM) * ((g.F + nt - 1) / nt), sms = sm_count(), rounds = (tiles + sms - 1) / sms;
   static const int one[2] = {730, 560}, many[2][3] = {{1030, 1100, 1300}, {650, 670, 750}};
-  return rounds * (steps * (rounds == 1 ? one[G == 8] : many[G == 8][w]) + 1000);
+  const long long cost = rounds * (steps * (rounds == 1 ? one[G == 8] : many[G == 8][w]) + (w == 2 ? 2000 : 1000));
+  // channels innermost (a network's input): every load of a group of eight touches a line per row, 1.5 to 1.8 times the time (16 to 40
+  // channels 3x3x3 and 5x5x5), and from where a tile's rows leave the L1 cache on (28 KB) 4 times (96 and 128 channels 5x5x5)
+  return g.xs_w > 1 && G == 8 ? (g.C > 56 ? 4 * cost : cost + cost / 2) : cost;
 }
 
 void f32tc_conv_free(F32ConvW* w) {

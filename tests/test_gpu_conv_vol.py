@@ -96,13 +96,17 @@ def conv3d_layer(rng, ci, co, k, act="none", **flags):
 
 # widths that are no multiples of 32, kernels of one and two widths, a first layer that is short and one that is not, residuals
 @pytest.mark.gpu
+@pytest.mark.parametrize("route", ["volume", "loads"])
 @pytest.mark.parametrize("spec", [
     [(3, 24, 3), (24, 24, 3), (24, 5, 3)],
     [(6, 40, 3), (40, 40, 5), (40, 40, 3), (40, 2, 3)],
     [(2, 70, 5), (70, 70, 3), (70, 33, 3)],
+    [(130, 20, 1), (20, 36, 3), (36, 36, 5), (36, 3, 3)],
 ])
-def test_networks_change_their_extents(host, spec):
+def test_networks_change_their_extents(host, spec, route):
     """Volumes of other extents in the same buffers: the padding is zero again, whatever lay there before."""
+    launches = on_device(host, route)
+    before = launches()
     rng = np.random.default_rng(3)
     layers = [conv3d_layer(rng, ci, co, k, "leaky" if l < len(spec) - 1 else "none") for l, (ci, co, k) in enumerate(spec)]
     layers[0]["save"] = True
@@ -120,6 +124,30 @@ def test_networks_change_their_extents(host, spec):
             if l["act"] == "leaky": v = torch.where(v > 0, v, v * float(np.float32(0.2)))
             if l.get("save"): skip = v
         assert rel(torch.from_numpy(y), v.permute(0, 2, 3, 4, 1)) < len(layers) * TOL
+    on_volumes = sum(ci * min(k, 6) ** 3 >= 128 for ci, _, k in spec)
+    assert launches() - before == (3 * on_volumes if route == "volume" else 0)
+
+
+# few channels with many taps, 1x1x1 layers: volumes pad channels to 32, and the general kernel is up to three times as fast
+@pytest.mark.gpu
+@pytest.mark.parametrize("width,k,cin,extents,over_volumes", [
+    (8, 5, 3, (1, 20, 20, 20), False), (8, 5, 8, (2, 33, 33, 33), False), (24, 5, 3, (1, 8, 9, 10), False), (160, 1, 3, (2, 33, 33, 33), False),
+    (32, 3, 3, (1, 20, 20, 20), True), (64, 3, 3, (2, 12, 13, 14), True), (64, 3, 64, (1, 8, 9, 10), True), (128, 5, 128, (1, 8, 9, 10), True),
+])
+def test_networks_run_over_volumes_where_that_is_faster(host, width, k, cin, extents, over_volumes):
+    rng = np.random.default_rng(3)
+    host.load_model(write_blob([conv3d_layer(rng, ci, co, k) for ci, co in [(cin, width), (width, width), (width, width), (width, 3)]]))
+    host.option("conv_shape", "%d,%d,%d,%d" % extents)
+    x = torch.randn(extents + (cin,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    y, general = [torch.zeros(extents + (3,), device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    before = host.L.fortis_debug_launches(b"conv_vol_kernel")
+    host.forward(x, y)
+    launched = host.L.fortis_debug_launches(b"conv_vol_kernel") - before
+    assert launched == (3 + (cin * k ** 3 >= 128) if over_volumes else 0)
+    host.option("test_conv_route", 2)
+    host.forward(x, general)
+    assert rel(y, general) < 2 * 4 * TOL
 
 
 @pytest.mark.gpu
