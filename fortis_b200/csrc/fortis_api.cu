@@ -154,7 +154,7 @@ struct Session {
 
   long long buf_rows = 0;
   float *din = nullptr, *dout = nullptr, *act0 = nullptr, *act1 = nullptr;
-  long long pair_rows = 0;                        // rows act0 and act1 hold as split activations (0: none)
+  long long act_bytes = 0, pair_refused = 0;      // of act0 and act1 each; bytes of split activations that there was no memory for (0: none)
   float *X_pinned = nullptr, *Y_pinned = nullptr;
   long long pinned_rows = 0;
   bool pack_pending = false, gather_pending = false, gather_done = false;
@@ -447,35 +447,52 @@ long long act_ld(long long rows) { return (rows + 3) / 4 * 4; }
 
 void ensure_buffers(long long rows) {
   Session& s = S();
-  // fp32 layers on pairs of CTAs keep their activations split, twice the floats; without the memory for that they run as before
-  const bool pair = s.model.is_mlp() && s.f32 && rows >= kF32TcMinRows && rows <= kF32TcMaxRows && f32tc_pair_wanted(s.f32, rows);
-  if (rows <= s.buf_rows && s.din && (!pair || s.pair_rows != 0)) return;
-  if (rows < s.buf_rows) rows = s.buf_rows;
-  pool_free(s.din); pool_free(s.dout); pool_free(s.act0); pool_free(s.act1);
-  s.act0 = s.act1 = nullptr;
-  int wmax = 1;
-  for (auto& L : s.model.layers) wmax = L.cout > wmax ? L.cout : wmax;
-  const long long nin = s.model.n_in(), nout = s.model.n_out();
-  s.din = (float*)pool_alloc(rows * nin * 4);
+  if (rows <= s.buf_rows && s.din) return;
+  pool_free(s.din); pool_free(s.dout);
+  s.din = (float*)pool_alloc(rows * s.model.n_in() * 4);
   s.dout = (float*)pool_alloc(out_floats(rows) * 4);
-  (void)nout;
-  const bool need_act = s.model.is_mlp() && s.model.layers.size() > 1;
-  const long long act_bytes = act_ld(rows) * wmax * 4;
-  s.pair_rows = pair ? -1 : 0;                    // asked for
-  if (pair) {
-    const long long bytes = std::max<long long>((long long)f32tc_pair_bytes(s.f32, rows), act_bytes);
-    s.act0 = (float*)pool_alloc(bytes);
-    s.act1 = s.act0 ? (float*)pool_alloc(bytes) : nullptr;
-    if (s.act1) s.pair_rows = rows;
-    else { pool_free(s.act0); s.act0 = nullptr; }
-  }
-  if (need_act && !s.act0) {
-    s.act0 = (float*)pool_alloc(act_bytes);
-    s.act1 = s.model.layers.size() > 2 ? (float*)pool_alloc(act_bytes) : nullptr;
-  }
-  if (!s.din || !s.dout || (need_act && !s.act0)) throw std::runtime_error("out of device memory for the model buffers");
+  if (!s.din || !s.dout) throw std::runtime_error("out of device memory for the model buffers");
   s.buf_rows = rows;
   drop_graph();
+}
+
+bool runs_on_pairs(long long rows) {
+  Session& s = S();
+  return s.model.is_mlp() && s.f32 && rows >= kF32TcMinRows && rows <= kF32TcMaxRows && f32tc_pair_wanted(s.f32, rows);
+}
+
+// What lies between the layers of an MLP, for launches of up to `rows` rows each (a step over host arrays runs in chunks).  fp32 layers on
+// pairs of CTAs keep their activations split, twice the floats; without the memory for that they run as others do, and it is not asked
+// for again before the next model.
+void ensure_activations(long long rows) {
+  Session& s = S();
+  if (!s.model.is_mlp() || s.model.layers.size() < 2) return;
+  int wmax = 1;
+  for (auto& L : s.model.layers) wmax = L.cout > wmax ? L.cout : wmax;
+  const long long plain = act_ld(rows) * wmax * 4, split = runs_on_pairs(rows) ? std::max<long long>((long long)f32tc_pair_bytes(s.f32, rows), plain) : 0;
+  bool pair = split > 0 && (!s.pair_refused || split < s.pair_refused);
+  long long bytes = pair ? split : plain;
+  bool two = pair || s.model.layers.size() > 2;
+  if (s.act0 && (s.act1 || !two) && s.act_bytes >= bytes) return;
+  pool_free(s.act0); pool_free(s.act1);
+  s.act0 = s.act1 = nullptr; s.act_bytes = 0;
+  drop_graph();
+  auto get = [&]() {
+    s.act0 = (float*)pool_alloc(bytes);
+    if (s.act0 && two) s.act1 = (float*)pool_alloc(bytes);
+    if (s.act0 && (s.act1 || !two)) return true;
+    pool_free(s.act0);
+    s.act0 = nullptr;
+    return false;
+  };
+  bool ok = get();
+  if (!ok && pair) {
+    s.pair_refused = split;
+    pair = false; bytes = plain; two = s.model.layers.size() > 2;
+    ok = get();
+  }
+  if (!ok) throw std::runtime_error("out of device memory for the model buffers");
+  s.act_bytes = bytes;
 }
 
 void ensure_aux(long long npartials) {
@@ -788,7 +805,7 @@ void run_step_kernels(const StepArgs& A) {
                     L.store_by_slot = s.S.store_by_slot; std::memcpy(L.cout, s.S.cls, sizeof L.cout); }
     L.Y = fuse_out ? nullptr : s.dout;
     L.read_once = fuse_in && s.G.mapped;
-    L.act[0] = s.act0; L.act[1] = s.act1; L.act_ld = act_ld(s.buf_rows);
+    L.act[0] = s.act0; L.act[1] = s.act1; L.act_ld = act_ld(rows);
     L.g = g;
     ensure_aux(std::max(tc_grid(s.tc, rows), f32tc_grid(rows)));
     L.partials = (fuse_out && s.want_checksum) ? s.d_partials : nullptr;
@@ -849,8 +866,8 @@ void run_step_kernels(const StepArgs& A) {
     if (fuse_out) { L.fast_out = 1; L.store_by_slot = s.S.store_by_slot; L.TS = A.TS; std::memcpy(L.cout, s.S.cls, sizeof L.cout); }
     else L.Y = s.dout;
     L.g = g;
-    L.act[0] = s.act0; L.act[1] = s.act1; L.act_ld = act_ld(s.buf_rows);
-    L.pair = s.pair_rows >= rows && f32tc_pair_wanted(s.f32, rows);
+    L.act[0] = s.act0; L.act[1] = s.act1; L.act_ld = act_ld(rows);
+    L.pair = s.act1 && runs_on_pairs(rows) && s.act_bytes >= (long long)f32tc_pair_bytes(s.f32, rows);
     ensure_aux(f32tc_grid(rows));
     if (fuse_out && s.want_checksum) { L.partials = s.d_partials; L.sum = s.d_sum; L.done = s.d_done; }
     L.status = s.d_status;
@@ -886,6 +903,7 @@ std::string step_key(const StepArgs& A) {
 void run_step(const StepArgs& A) {
   Session& s = S();
   cudaStream_t st = stream();
+  ensure_activations(A.rows);
   if (!s.graph) { run_step_kernels(A); return; }
   const std::string key = step_key(A);
   if (s.gexec && key == s.gkey) { cuda_ok(cudaGraphLaunch(s.gexec, st), "cudaGraphLaunch"); return; }
@@ -1086,31 +1104,6 @@ bool overlapped_step(void* const* gptrs, void* const* sptrs, long long rows) {
     if (!s.async) cudaStreamSynchronize(st);
     return true;
   }
-  if (key != s.ov_key) {
-    if (s.ov_gexec) { cudaGraphExecDestroy(s.ov_gexec); s.ov_gexec = nullptr; }
-    s.ov_key = key; s.ov_calls = 0;
-  }
-  int args[8] = {1, 1, 1, 1, 1, 1, 1, 1};
-  StepArgs A;
-  A.use_gather = true; A.fuse_scatter = true;
-  // pins the arrays, sizes the staging buffers; the copies themselves are issued per chunk below
-  bind_arrays(s.G, gptrs, args, 0, false, false, &A.TG);
-  bind_arrays(s.S, sptrs, args, 0, false, false, &A.TS);
-  // Per-column vectors (one element per column) are not staged at all: a copy of a few hundred KB costs a copy's
-  // latency (7-10 us each, and copies of one direction run one after another whatever their stream), which for a dozen
-  // vectors is a tenth of the step.  The kernels load and store them through the pinned host pages instead; their
-  // bytes cross the bus inside the launches, beside the chunk copies.
-  auto map_vectors = [&](PlanDev& P, void* const* ptrs, ArrayTable& T) {
-    for (size_t ai = 0; ai < P.h.arrays.size(); ai++) {
-      const ArrayInfo& a = P.h.arrays[ai];
-      if (!a.used || P.on_dev[ai] || a.total != ncol || P.reg[ai] != ptrs[ai]) continue;
-      void* dp = nullptr;
-      if (cudaHostGetDevicePointer(&dp, ptrs[ai], 0) == cudaSuccess && dp) { P.on_dev[ai] = true; P.mapped = true; T.base[ai] = dp; }
-      else cudaGetLastError();
-    }
-  };
-  if (!std::getenv("FORTIS_STAGE_VECTORS")) { map_vectors(s.G, gptrs, A.TG); map_vectors(s.S, sptrs, A.TS); }
-  const ArrayTable TG0 = A.TG, TS0 = A.TS;
   // Chunk schedule: large chunks first, small ones last, so that what is left after the last upload (one forward
   // and one download) is short.  FORTIS_STAGING_CHUNKS overrides it with a list of relative weights ("2,2,2,1,1").
   std::vector<long long> weights;
@@ -1142,7 +1135,34 @@ bool overlapped_step(void* const* gptrs, void* const* sptrs, long long rows) {
   }
   const int nchunks = (int)cuts.size();
   cuts.push_back(ncol);
-
+  long long largest = 0;
+  for (int c = 0; c < nchunks; c++) largest = std::max(largest, cuts[c + 1] - cuts[c]);
+  ensure_activations(largest);
+  if (key != s.ov_key) {
+    if (s.ov_gexec) { cudaGraphExecDestroy(s.ov_gexec); s.ov_gexec = nullptr; }
+    s.ov_key = key; s.ov_calls = 0;
+  }
+  int args[8] = {1, 1, 1, 1, 1, 1, 1, 1};
+  StepArgs A;
+  A.use_gather = true; A.fuse_scatter = true;
+  // pins the arrays, sizes the staging buffers; the copies themselves are issued per chunk below
+  bind_arrays(s.G, gptrs, args, 0, false, false, &A.TG);
+  bind_arrays(s.S, sptrs, args, 0, false, false, &A.TS);
+  // Per-column vectors (one element per column) are not staged at all: a copy of a few hundred KB costs a copy's
+  // latency (7-10 us each, and copies of one direction run one after another whatever their stream), which for a dozen
+  // vectors is a tenth of the step.  The kernels load and store them through the pinned host pages instead; their
+  // bytes cross the bus inside the launches, beside the chunk copies.
+  auto map_vectors = [&](PlanDev& P, void* const* ptrs, ArrayTable& T) {
+    for (size_t ai = 0; ai < P.h.arrays.size(); ai++) {
+      const ArrayInfo& a = P.h.arrays[ai];
+      if (!a.used || P.on_dev[ai] || a.total != ncol || P.reg[ai] != ptrs[ai]) continue;
+      void* dp = nullptr;
+      if (cudaHostGetDevicePointer(&dp, ptrs[ai], 0) == cudaSuccess && dp) { P.on_dev[ai] = true; P.mapped = true; T.base[ai] = dp; }
+      else cudaGetLastError();
+    }
+  };
+  if (!std::getenv("FORTIS_STAGE_VECTORS")) { map_vectors(s.G, gptrs, A.TG); map_vectors(s.S, sptrs, A.TS); }
+  const ArrayTable TG0 = A.TG, TS0 = A.TS;
   bool capturing = (++s.ov_calls == 2) && !std::getenv("FORTIS_NO_STAGING_GRAPH");
   if (capturing && cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { cudaGetLastError(); capturing = false; }
   if (capturing) set_capturing(true);
@@ -1248,6 +1268,7 @@ bool overlapped_planes_step(void* const* gptrs, void* const* sptrs) {
     if (!s.async) cudaStreamSynchronize(st);
     return true;
   }
+  ensure_activations(s.loop.count);
   if (key != s.ov_key) {
     if (s.ov_gexec) { cudaGraphExecDestroy(s.ov_gexec); s.ov_gexec = nullptr; }
     s.ov_key = key; s.ov_calls = 0;
@@ -1442,7 +1463,7 @@ int fortis_load_model_mem(const void* blob, long nbytes) {
   s.model = std::move(M);
   s.have_model = true;
   pool_free(s.din); pool_free(s.dout); pool_free(s.act0); pool_free(s.act1);
-  s.din = s.dout = s.act0 = s.act1 = nullptr; s.buf_rows = 0;
+  s.din = s.dout = s.act0 = s.act1 = nullptr; s.buf_rows = 0; s.act_bytes = s.pair_refused = 0;
   g_err = 0;
   return 0;
   FORTIS_CATCH(return -1)
@@ -1668,7 +1689,7 @@ void mlp_forward(void* in, void* out) {
     StepArgs A; A.rows = 1;
     const LoopInfo saved = s.loop;
     s.loop.nk = 1; s.loop.count = 1; s.loop.ni = 1;
-    try { run_step_kernels(A); } catch (...) { s.loop = saved; throw; }
+    try { ensure_activations(1); run_step_kernels(A); } catch (...) { s.loop = saved; throw; }
     s.loop = saved; (void)keep; (void)had_l;
     cuda_ok(cudaMemcpyAsync(out, s.dout, nout * 4, cudaMemcpyDefault, st), "D2H of one row");
     cudaStreamSynchronize(st);

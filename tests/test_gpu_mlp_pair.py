@@ -72,3 +72,32 @@ def test_gathered_step_and_its_checksum(host):
     y = torch.cat([out[0].T, out[1].T] + [v[:, None] for v in out[2:]], dim=1)
     assert float((y.double() - x).norm() / x.norm()) < 1e-5
     assert abs(host.step_checksum() - float(y.double().sum())) <= 1e-12 * float(y.double().abs().sum())
+
+
+def staged_step():
+    import fortis_b200
+    ncol = 20000
+    h = fortis_b200.Host()
+    G, S, L, K = D.column(ncol, 60)
+    h.configure(gather=G, scatter=S, loop=L, kdist=K)
+    h.load_model(write_blob(mlp_layers([244, 768, 768, 128], seed=0)))
+    rng = np.random.default_rng(1)
+    gin = [np.asfortranarray(rng.standard_normal((ncol, 60)).astype(np.float32)) for _ in range(4)] + [rng.standard_normal(ncol).astype(np.float32) for _ in range(4)]
+    out = [np.zeros((ncol, 60), np.float32, order="F") for _ in range(2)] + [np.zeros(ncol, np.float32) for _ in range(8)]
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    for _ in range(3):
+        h.step(gin, out)
+    used = before - torch.cuda.mem_get_info()[0]
+    # staged inputs and outputs 30 MB, the model's 30, weights 15; activations of a chunk of up to 6784 columns two times 21 (of all 20,000,
+    # split, two times 123); 32 MB for what the runtime allocates with the first launches
+    assert used < (30 + 30 + 15 + 42 + 32) << 20, used >> 20
+    assert np.isfinite(out[0]).all() and np.abs(out[0]).max() > 0
+
+
+def test_a_staged_step_holds_activations_for_its_chunks():
+    """Of a step over host arrays the chunks decide which kernel runs and how much lies between the layers, not the whole call.  In a
+    process of its own: the library pools memory."""
+    import os, subprocess, sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", "import tests.test_gpu_mlp_pair as t; t.staged_step()"], cwd=root, check=True, timeout=300)
