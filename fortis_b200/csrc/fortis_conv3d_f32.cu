@@ -758,6 +758,23 @@ int vol_front_w(const ConvGeom& c) { return vol_line(c.KW, c.sw, c.pw) ? 0 : c.p
 
 size_t vol_bytes(const VolGeom& g, int pitch) { return (size_t)g.P * g.fd * g.fh * g.fw * pitch * 8; }
 
+typedef void (*VolKernel)(VolParams);
+const VolKernel kVolKernels[4] = {conv_vol_kernel<32, false>, conv_vol_kernel<64, false>, conv_vol_kernel<32, true>, conv_vol_kernel<64, true>};
+
+// The widest form (the one that moves registers between its warps) needs the number the compiler gave it (128 a thread); with another
+// compiler's the layers stay on the other kernels.
+bool vol_available() {
+  static const bool ok = [] {
+    cudaFuncAttributes fa;
+    for (VolKernel k : kVolKernels)
+      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess) { cudaGetLastError(); return false; }
+    if (cudaFuncGetAttributes(&fa, kVolKernels[3]) == cudaSuccess && fa.numRegs == 128) return true;
+    cudaGetLastError();
+    return false;
+  }();
+  return ok;
+}
+
 bool vol_alloc(void** p, size_t bytes) {
   g_launches.volume_allocs++;
   if (!(g_tc_test.volume_limit && bytes > g_tc_test.volume_limit) && cudaMalloc(p, bytes) == cudaSuccess) return true;
@@ -775,7 +792,7 @@ bool vol_supported(const ConvGeom& c) {
   const VolGeom g = vol_geom(c, c.pd, c.ph, vol_front_w(c));
   Sharing s;
   // rows, and the last ones a tile may ask for, in 32 bits
-  return g.P * g.fd * g.fh * g.fw < (1LL << 30) && (long long)c.KD * g.Hq * g.Wq < (1LL << 29) && pick_sharing(g, vol_nt(c.F), g.line, &s);
+  return g.P * g.fd * g.fh * g.fw < (1LL << 30) && (long long)c.KD * g.Hq * g.Wq < (1LL << 29) && pick_sharing(g, vol_nt(c.F), g.line, &s) && vol_available();
 }
 
 // The rows as one piece, or image by image (which leaves the padding planes between them out) where that takes fewer rounds of tiles:
@@ -873,17 +890,7 @@ bool vol_conv(const VolW* w, const float* vol, int pitch, const VolGeom& g, cons
   P.status = status;
   P.wait_limit = g_tc_test.wait_limit ? g_tc_test.wait_limit : kWaitLimit;
   P.test_skip_stage = g_tc_test.skip_stage;
-  typedef void (*Kernel)(VolParams);
-  static const Kernel kernels[4] = {conv_vol_kernel<32, false>, conv_vol_kernel<64, false>, conv_vol_kernel<32, true>, conv_vol_kernel<64, true>};
-  static bool ready = false;
-  if (!ready) {
-    for (Kernel k : kernels)
-      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess)
-        return fail("cannot reserve shared memory for the convolution kernel");
-    cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, kernels[3]) != cudaSuccess || fa.numRegs != 128) return fail("the convolution kernel's register split does not add up");
-    ready = true;
-  }
+  if (!vol_available()) return fail("convolution: shared memory or register split not available");
   const long long tiles = (long long)pc.n * pc.pairs * P.ntn, pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs))); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = sh.smem; cfg.stream = s;
@@ -892,7 +899,7 @@ bool vol_conv(const VolW* w, const float* vol, int pitch, const VolGeom& g, cons
   at[0].val.programmaticStreamSerializationAllowed = 1;
   static const bool pdl = std::getenv("FORTIS_NO_PDL") == nullptr;
   cfg.attrs = at; cfg.numAttrs = (pdl && early) ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernels[2 * g.line + (w->NT == 64)], P);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kVolKernels[2 * g.line + (w->NT == 64)], P);
   if (e != cudaSuccess) { if (err) *err = std::string("convolution launch: ") + cudaGetErrorString(e); return false; }
   g_launches.vol_conv++;
   return true;

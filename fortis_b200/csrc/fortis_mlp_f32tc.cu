@@ -1064,7 +1064,7 @@ bool f32tc_pair_wanted(const F32TcModel* m, long long nrows) {
   if (m->layers.size() < 2) return false;
   long long narrow = 1 << 30;
   for (size_t l = 0; l + 1 < m->layers.size(); l++) narrow = m->layers[l].w.N_real < narrow ? m->layers[l].w.N_real : narrow;
-  return narrow >= 768 && narrow * nrows >= 7000000;
+  return narrow >= 768 && narrow * nrows >= 7000000 && pair_available();
 }
 
 size_t f32tc_pair_bytes(const F32TcModel* m, long long nrows) {

@@ -491,16 +491,7 @@ int pairs_on_device() {
 
 template <int NT>
 bool launch(PairParams& P, cudaStream_t s, std::string* err) {
-  static bool ready = false;
-  if (!ready) {
-    cudaFuncAttributes fa;
-    if (cudaFuncSetAttribute(mlp_pair_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<NT>::kSmem) != cudaSuccess ||
-        cudaFuncGetAttributes(&fa, mlp_pair_kernel<NT>) != cudaSuccess || fa.numRegs != 168) {
-      if (err) *err = "pair kernel: shared memory or register split not available";
-      return false;
-    }
-    ready = true;
-  }
+  if (!pair_available()) { if (err) *err = "pair kernel: shared memory or register split not available"; return false; }
   P.wait_limit = g_tc_test.wait_limit ? g_tc_test.wait_limit : kWaitLimit;
   P.test_skip_stage = g_tc_test.skip_stage;
   const long long tiles = (P.nrows + 2 * kM - 1) / (2 * kM) * P.ntn, pairs = pairs_on_device();
@@ -517,7 +508,23 @@ bool launch(PairParams& P, cudaStream_t s, std::string* err) {
   return true;
 }
 
+template <int NT>
+bool available() {
+  cudaFuncAttributes fa;
+  const bool ok = cudaFuncSetAttribute(mlp_pair_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<NT>::kSmem) == cudaSuccess &&
+                  cudaFuncGetAttributes(&fa, mlp_pair_kernel<NT>) == cudaSuccess && fa.numRegs == 168;
+  if (!ok) cudaGetLastError();
+  return ok;
+}
+
 }  // namespace
+
+// The register split adds up only with what the compiler gave the kernel (168 a thread); with another compiler's number the layers stay
+// on f32tc_kernel.
+bool pair_available() {
+  static const bool ok = available<256>() && available<128>();
+  return ok;
+}
 
 // 256 features a tile, or 128 where that takes fewer rounds of tiles (a step 1536 or 900 clk) or the outputs are scattered
 bool pair_wide(long long nrows, int N, bool scatter) {

@@ -21,6 +21,8 @@ struct PairLayer {
   double* partials; double* sum; unsigned int* done;
   int* status;
 };
+bool pair_available();                               // the kernels' shared memory and register splits are to be had
+bool pair_wide(long long nrows, int N, bool scatter);      // tiles of 256 features, not 128
 bool pair_layer(const PairLayer& L, cudaStream_t s, std::string* err);
 void pair_split_gathered(const Access* slots, const ArrayTable& T, const RowGeom& g, int n_in, const float* in_div, float* out, long long nrows, cudaStream_t s);
 void pair_split_rows(const float* X, int n_in, const float* in_div, float* out, long long nrows, cudaStream_t s);

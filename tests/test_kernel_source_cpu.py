@@ -15,7 +15,9 @@ def kernel(name, signature):
 
 
 @pytest.mark.parametrize("name,signature", [("fortis_mlp_f32tc.cu", "f32tc_kernel(const __grid_constant__"),
-                                            ("fortis_conv3d_tc.cu", "conv3d_tc_kernel(const __grid_constant__")])
+                                            ("fortis_conv3d_tc.cu", "conv3d_tc_kernel(const __grid_constant__"),
+                                            ("fortis_conv3d_f32.cu", "conv_vol_kernel(const __grid_constant__"),
+                                            ("fortis_mlp_pair.cu", "mlp_pair_kernel(const __grid_constant__")])
 def test_dependents_are_released_after_the_tensor_memory_is_allocated(name, signature):
     """A dependent CTA that shares the SM could otherwise take the tensor-memory columns and wait for the grid whose CTA
     still needs them."""
@@ -32,6 +34,20 @@ def test_what_the_grid_in_front_may_write_is_not_read_as_constant(name, written)
     assert "ld.global.nc" not in text
     for line in text.splitlines():
         assert not ("__ldg" in line and any(w in line for w in written)), line.strip()
+
+
+@pytest.mark.parametrize("name,signature,threads,registers,launch,available", [
+    ("fortis_conv3d_f32.cu", "conv_vol_kernel(const __grid_constant__", 512, 128, "bool vol_supported(", "vol_available()"),
+    ("fortis_mlp_pair.cu", "mlp_pair_kernel(const __grid_constant__", 384, 168, "bool f32tc_pair_wanted(", "pair_available()")])
+def test_register_splits_add_up(name, signature, threads, registers, launch, available):
+    """setmaxnreg draws on the registers that the block was launched with: more than those, and a warp waits for good.  Eight epilogue
+    warps take what the others give; with another number than the split assumes the rule that chooses the kernel chooses another."""
+    body = kernel(name, signature)
+    dec, inc = [[int(v) for v in re.findall(r"setmaxnreg\.%s\.sync\.aligned\.u32 (\d+)" % k, body)] for k in ("dec", "inc")]
+    assert len(inc) == 1 and len(set(dec)) == 1
+    assert inc[0] * 256 + dec[0] * (threads - 256) <= threads * registers
+    assert "numRegs == %d" % registers in open(os.path.join(CSRC, name)).read()
+    assert available in kernel(name if "vol" in launch else "fortis_mlp_f32tc.cu", launch)
 
 
 def test_a_tiles_bias_table_is_not_rewritten_before_every_lane_has_read_it():
