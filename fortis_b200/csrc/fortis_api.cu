@@ -1505,6 +1505,7 @@ int fortis_set_option(const char* key, const char* value) {
   else if (k == "test_skip_stage") { g_tc_test.skip_stage = v != "0"; drop_graph(); }
   else if (k == "test_no_stage") { g_tc_test.no_stage = v != "0"; drop_graph(); }
   else if (k == "test_conv_route") { g_tc_test.conv_route = std::atoi(v.c_str()); drop_graph(); }
+  else if (k == "test_mlp_pair") { g_tc_test.mlp_pair = std::atoi(v.c_str()); drop_graph(); }
   else if (k == "test_volume_limit") { g_tc_test.volume_limit = std::strtoull(v.c_str(), nullptr, 10); }
   else if (k == "conv_shape") {
     if (std::sscanf(v.c_str(), "%d,%d,%d,%d", &s.conv_shape[0], &s.conv_shape[1], &s.conv_shape[2], &s.conv_shape[3]) != 4)

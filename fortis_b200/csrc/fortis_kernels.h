@@ -86,6 +86,7 @@ struct TcTestKnobs {
   unsigned int wait_limit; int skip_stage;
   int no_stage;                                      // fused MLP kernel: move every tile's inputs and outputs element by element
   int conv_route;                                    // fp32 convolutions: 0 by estimate, 1 over split volumes wherever they can, 2 never
+  int mlp_pair;                                      // fp32 MLPs of two and more layers: 0 by estimate, 1 on pairs of CTAs, 2 never
   unsigned long long volume_limit;                   // bytes: an allocation for split volumes or their weights beyond it fails (0: no limit)
 };
 extern TcTestKnobs g_tc_test;

@@ -1056,15 +1056,30 @@ F32TcModel* f32tc_create(const ModelHost& M, std::string* err) {
   return m;
 }
 
-// Pairs of CTAs (fortis_mlp_pair.cu) for wide layers of many rows; the results are the same bits.  Their tiles are 256 x 256, their launches
-// cost 4 us more each, and the split activations move twice the bytes.  Device time of whole calls, this kernel / pairs (us): hidden layers
-// of 768: 2000 rows 115 / 113, 4000 164 / 168, 8000 224 / 206, 30,011 631 / 570; 1024: 4000 115 / 118, 8000 177 / 164; 2048: 3000 200 / 177, 5000
-// 293 / 255; 900: 7000 131 / 146, 12,000 206 / 188; 512: 30,011 192 / 216; 400 and 640 in turn: 30,011 256 / 274.
+// Pairs of CTAs (fortis_mlp_pair.cu) for wide layers of many rows; the results are the same bits.  From 768 features and seven million
+// activations of the narrowest layer on, where the estimate says that they are faster: their tiles are 256 x 256, so that a round of
+// tiles that is mostly empty or padding costs more, and the inputs are split first.  Device time of whole calls, this kernel / pairs (us):
+// three hidden layers of 768: 9345 rows 182 / 170, 30,011 525 / 495; 896: 8000 192 / 216, 12,000 257 / 245; 1024: 7000 206 / 225, 16,000
+// 405 / 394; one of 768 between 500 inputs and 3 outputs, 11,400 rows: 93 / 104.  The constants fit 361 calls (768 to 2048 features, 1500 to
+// 40,000 rows) within 11 %; of those that take pairs the slowest costs 1.02 of this kernel's time.
 bool f32tc_pair_wanted(const F32TcModel* m, long long nrows) {
   if (m->layers.size() < 2) return false;
+  if (g_tc_test.mlp_pair) return g_tc_test.mlp_pair == 1 && pair_available();
   long long narrow = 1 << 30;
   for (size_t l = 0; l + 1 < m->layers.size(); l++) narrow = m->layers[l].w.N_real < narrow ? m->layers[l].w.N_real : narrow;
-  return narrow >= 768 && narrow * nrows >= 7000000 && pair_available();
+  if (narrow < 768 || narrow * nrows < 7000000 || !pair_available()) return false;
+  // ns: launches and input first, then rounds of tiles, their steps of 32 k and their ends
+  const long long n_in = m->layers.front().w.K_real, n_out = m->layers.back().w.N_real, sms = sm_count(), pairs = sms / 2 > 0 ? sms / 2 : 1;
+  long long one = 4 * nrows * (n_in + n_out) / 2590, two = 5100 + 4 * nrows * (3 * n_in + n_out) / 3250;
+  for (size_t l = 0; l < m->layers.size(); l++) {
+    const SplitW& W = m->layers[l].w;
+    const long long steps = W.K_pad / kKt;
+    const int w = pick_tile(nrows, W.N_real, kStepLinear), nt = 32 << w, pt = pair_wide(nrows, W.N_real, false) ? 256 : 128;
+    const long long rounds = ((nrows + kM - 1) / kM * ((W.N_real + nt - 1) / nt) + sms - 1) / sms, prounds = ((nrows + 2 * kM - 1) / (2 * kM) * ((W.N_real + pt - 1) / pt) + pairs - 1) / pairs;
+    one += 6600 + rounds * (l == 0 && n_in % 4 ? steps * 1970 : w == 2 ? steps * 615 + 1000 : steps * 520);
+    two += 6100 + prounds * (pt == 256 ? steps * 885 + 5500 : steps * 440 + 2600);
+  }
+  return two < one;
 }
 
 size_t f32tc_pair_bytes(const F32TcModel* m, long long nrows) {

@@ -34,6 +34,7 @@ int fortis_debug_few_rows(const int* widths, int nlayers, int fp8w, long rows);
  *                             instead of staging whole tiles by bulk copies (same bits; for the comparison of the paths)
  *   "test_conv_route"  0 | 1 | 2  fp32 convolutions: by estimate (0), over split volumes wherever the layer's shape
  *                             allows it (1), never over split volumes (2)
+ *   "test_mlp_pair"    0 | 1 | 2  fp32 MLPs of two and more layers: by estimate (0), on pairs of CTAs (1), never (2)
  *   "test_volume_limit"  N    bytes: a device allocation for split volumes or their weights beyond it fails (0: no limit) */
 
 /* Launches of one kernel since the library was loaded ("conv_vol_kernel", "mlp_pair_kernel"; -1: no such counter), so that a
