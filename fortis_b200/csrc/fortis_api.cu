@@ -1917,6 +1917,8 @@ int fortis_debug_few_rows(const int* widths, int nlayers, int fp8w, long rows) {
   return tc_rows_layer_by_layer(widths, widths + 1, nlayers, fp8w != 0, rows) ? 1 : 0;
 }
 
+int fortis_debug_tile_width(long rows, int N, int K) { return f32tc_tile_width(rows, N, K); }
+
 long fortis_debug_launches(const char* kernel) {
   const std::string k = kernel ? kernel : "";
   return k == "conv_vol_kernel" ? g_launches.vol_conv : k == "mlp_pair_kernel" ? g_launches.mlp_pair : k == "volume_allocs" ? g_launches.volume_allocs : -1;

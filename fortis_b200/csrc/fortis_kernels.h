@@ -228,6 +228,7 @@ struct VolOut {
 // `early`: the launch may start (and read its weights) before the kernel in front of it in the stream has finished
 bool vol_conv(const VolW* w, const float* vol, int pitch, const VolGeom& g, const VolOut& o, const float* bias, int act, float slope, int* status,
               cudaStream_t s, bool early, std::string* err);
+int f32tc_tile_width(long long nrows, int N, int K);          // features of a tile of f32tc_gemm's
 // C[M][N] = A[M][K] . W[N][K]^T, row-major device operands (the memref entry fortis_gemm)
 bool f32tc_gemm(const float* A, const float* W, float* C, long long M, int N, int K, int* status, cudaStream_t s, std::string* err);
 

@@ -919,22 +919,30 @@ bool split_alloc(SplitW* w, int K, int N, std::string* err) {
   return true;
 }
 
-// The tile width (0, 1, 2: 32, 64, 128 features).  The launch lasts as many rounds of tiles as the SM that has the most, and a k step of a
-// tile, its share of the tile's end included, as many clocks as it measures: fortis_gemm, K = 768; rows off 16 bytes; inputs gathered from
-// host arrays; convolutions of K = 1728 (groups of eight channels) and of K = 405 (single channels).
-constexpr int kStepLinear[3] = {1140, 1200, 1520}, kStepLoads[3] = {2210, 2310, 2520}, kStepGather[3] = {1900, 2000, 2100}, kStepConv8[3] = {1240, 1280, 1430},
+// The tile width (0, 1, 2: 32, 64, 128 features).  The launch lasts as many rounds of tiles as the SM that has the most, and a round the k
+// steps of a tile and its end, ns, as fitted to 2700 timed calls (1 to 1000 features, 32 to 768 inputs, 512 to 60,000 rows; the width it
+// picks costs 1.004 of the fastest in the mean, at most 1.17): by operand (through the TMA, rows off 16 bytes, gathered from host arrays)
+// and by output (feature-major; rows; rows off 16 bytes, stored element by element; host arrays).  Without the ends, from steps at 768
+// inputs alone, products of few inputs took tiles too wide: 19,000 rows, 32 -> 129 features 35.7 us, now 22.8.
+// Convolutions: clocks a step with its share of the end (K = 1728, groups of eight channels; K = 405, single channels).
+constexpr int kStepTile[3] = {490, 505, 600}, kStepLoads[3] = {900, 915, 960}, kStepGather[3] = {690, 700, 740}, kStepConv8[3] = {1240, 1280, 1430},
               kStepConv1[3] = {1960, 2100, 2460};
-int pick_tile(long long nrows, int N, const int (&step)[3]) {
+constexpr int kEndFeatures[3] = {400, 850, 2000}, kEndRows[3] = {250, 900, 2100}, kEndRowsOff[3] = {1800, 4000, 8500}, kEndScatter[3] = {900, 2300, 5200},
+              kEndConv[3] = {0, 0, 0};
+int pick_tile(long long nrows, int N, int K_pad, const int (&step)[3], const int (&end)[3]) {
   const long long ntm = (nrows + kM - 1) / kM, sms = sm_count();
   long long best_cost = 0;
   int best = -1;
   for (int w = 2; w >= 0; w--) {
     const int nt = 32 << w;
     if (w > 0 && N <= nt / 2) continue;                     // more than half of the tile would be padding
-    const long long tiles = ntm * ((N + nt - 1) / nt), cost = ((tiles + sms - 1) / sms) * step[w];
+    const long long tiles = ntm * ((N + nt - 1) / nt), cost = ((tiles + sms - 1) / sms) * ((long long)(K_pad / kKt) * step[w] + end[w]);
     if (best < 0 || cost < best_cost) { best = w; best_cost = cost; }
   }
   return best;
+}
+const int (&tile_end(const F32Params& P))[3] {
+  return P.c_mode == C_CONV ? kEndConv : P.c_mode == C_SCATTER ? kEndScatter : P.c_mode == C_FEATURE_MAJOR ? kEndFeatures : P.c_vec ? kEndRows : kEndRowsOff;
 }
 
 template <int NT, int AMODE, int P16>
@@ -977,7 +985,7 @@ bool launch_as(F32Params& P, cudaStream_t s, bool early) {
 
 template <int AMODE>
 bool launch_tile(F32Params& P, const SplitW& W, const int (&step)[3], cudaStream_t s, bool early = true) {
-  const int w = pick_tile(P.nrows, W.N_real, step);
+  const int w = pick_tile(P.nrows, W.N_real, W.K_pad, step, tile_end(P));
   P.map_hi = W.map_hi[w]; P.map_lo = W.map_lo[w];
   P.K_pad = W.K_pad; P.K_real = W.K_real; P.N_real = W.N_real;
   P.chunk_kt = P.one_acc ? kChunkMlp : W.K_pad <= kShortK ? kChunkShort : kChunkLong;
@@ -987,7 +995,7 @@ bool launch_tile(F32Params& P, const SplitW& W, const int (&step)[3], cudaStream
 
 // a row-major operand: tiles through the TMA where rows start on 16-byte boundaries, else loads
 bool launch_rows(F32Params& P, const float* A, int K, const SplitW& W, cudaStream_t s, bool early) {
-  if (make_a_map(false, A, P.nrows, K, K, &P.map_a)) return launch_tile<A_TILE_R>(P, W, kStepLinear, s, early);
+  if (make_a_map(false, A, P.nrows, K, K, &P.map_a)) return launch_tile<A_TILE_R>(P, W, kStepTile, s, early);
   P.A = A; P.lda = K;
   return launch_tile<A_ROW_MAJOR>(P, W, kStepLoads, s, early);
 }
@@ -1074,7 +1082,7 @@ bool f32tc_pair_wanted(const F32TcModel* m, long long nrows) {
   for (size_t l = 0; l < m->layers.size(); l++) {
     const SplitW& W = m->layers[l].w;
     const long long steps = W.K_pad / kKt;
-    const int w = pick_tile(nrows, W.N_real, kStepLinear), nt = 32 << w, pt = pair_wide(nrows, W.N_real, false) ? 256 : 128;
+    const int w = pick_tile(nrows, W.N_real, W.K_pad, kStepTile, l + 1 < m->layers.size() ? kEndFeatures : kEndRows), nt = 32 << w, pt = pair_wide(nrows, W.N_real, false) ? 256 : 128;
     const long long rounds = ((nrows + kM - 1) / kM * ((W.N_real + nt - 1) / nt) + sms - 1) / sms, prounds = ((nrows + 2 * kM - 1) / (2 * kM) * ((W.N_real + pt - 1) / pt) + pairs - 1) / pairs;
     one += 6600 + rounds * (l == 0 && n_in % 4 ? steps * 1970 : w == 2 ? steps * 615 + 1000 : steps * 520);
     two += 6100 + prounds * (pt == 256 ? steps * 885 + 5500 : steps * 440 + 2600);
@@ -1157,7 +1165,7 @@ bool f32tc_forward(F32TcModel* m, const F32TcLaunch& L, cudaStream_t s, std::str
         if (err) *err = "split-TF32 step: activation rows must start on 16-byte boundaries";
         return false;
       }
-      ok = launch_tile<A_TILE_T>(P, T.w, kStepLinear, s);
+      ok = launch_tile<A_TILE_T>(P, T.w, kStepTile, s);
     }
     if (!launched(ok, err)) return false;
   }
@@ -1333,7 +1341,7 @@ bool f32tc_conv_supported(const ConvGeom& g) {
 // Estimated device time of a layer, ns: rounds of tiles times steps of 32 k, a step as it measures in one round of tiles and in many (groups of
 // eight channels 0.56 to 0.75 us, single channels 0.73 to 1.3 us).
 long long f32tc_conv_cost(const ConvGeom& g) {
-  const int G = conv_group(g.C), w = pick_tile((long long)g.N * g.Do * g.Ho * g.Wo, g.F, G == 8 ? kStepConv8 : kStepConv1), nt = 32 << w;
+  const int G = conv_group(g.C), w = pick_tile((long long)g.N * g.Do * g.Ho * g.Wo, g.F, kKt, G == 8 ? kStepConv8 : kStepConv1, kEndConv), nt = 32 << w;
   const long long steps = ((long long)g.KD * g.KH * g.KW * ((g.C + G - 1) / G * G) + kKt - 1) / kKt;
   const long long tiles = (((long long)g.N * g.Do * g.Ho * g.Wo + kM - 1) / kM) * ((g.F + nt - 1) / nt), sms = sm_count(), rounds = (tiles + sms - 1) / sms;
   static const int one[2] = {730, 560}, many[2][3] = {{1030, 1100, 1300}, {650, 670, 750}};
@@ -1341,6 +1349,10 @@ long long f32tc_conv_cost(const ConvGeom& g) {
   // channels innermost (a network's input): every load of a group of eight touches a line per row, 1.5 to 1.8 times the time (16 to 40
   // channels 3x3x3 and 5x5x5), and from where a tile's rows leave the L1 cache on (28 KB) 4 times (96 and 128 channels 5x5x5)
   return g.xs_w > 1 && G == 8 ? (g.C > 56 ? 4 * cost : cost + cost / 2) : cost;
+}
+
+int f32tc_tile_width(long long nrows, int N, int K) {
+  return 32 << pick_tile(nrows, N, round_up_f(K, kKt), K % 4 ? kStepLoads : kStepTile, N % 4 ? kEndRowsOff : kEndRows);
 }
 
 void f32tc_conv_free(F32ConvW* w) {

@@ -26,6 +26,9 @@ int fortis_debug_pack_layer(const float* W, const float* b, int cout, int cin, i
  * as one fused kernel (0)?  `fp8w`: FP8 weights. */
 int fortis_debug_few_rows(const int* widths, int nlayers, int fp8w, long rows);
 
+/* Host-only: features in a tile of fortis_gemm(B = rows, N, K) on the tensor cores (32, 64 or 128). */
+int fortis_debug_tile_width(long rows, int N, int K);
+
 /* Test-only keys of fortis_set_option (cleared by fortis_reset):
  *   "test_wait_limit"  N      polls before a bounded barrier wait of the tensor-core kernels gives up (0: the default)
  *   "test_skip_stage"  0 | 1  the first CTA's copy warp leaves out its first stage, so that a wait runs out: the
