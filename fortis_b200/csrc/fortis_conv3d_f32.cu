@@ -789,7 +789,12 @@ bool vol_supported(const ConvGeom& c) {
   const long long inside = (long long)(c.KD < c.D ? c.KD : c.D) * (c.KH < c.H ? c.KH : c.H) * (c.KW < c.W ? c.KW : c.W);
   if (inside * c.C < kF32TcConvMinProducts) return false;
   if ((long long)c.KD * c.KH * c.KW * ((c.C + 31) / 32) * ((c.F + 31) / 32) > (1 << 20)) return false;   // rows of the weight images in 32 bits
+  // channels are padded to 32, features to 32 or 64: no more memory than that is worth (1 -> 1 channel of 33^3 taps: 294 MB of weights for
+  // 144 KB; 1 channel on 512^3: 34 GB for 0.5)
+  const long long taps = (long long)c.KD * c.KH * c.KW, w_bytes = taps * ((c.C + 31) / 32) * (c.F <= 32 ? 32 : (c.F + 63) / 64 * 64) * kKt * 8;
+  if (w_bytes > (32LL << 20) && w_bytes > 4 * taps * c.C * c.F * 8) return false;
   const VolGeom g = vol_geom(c, c.pd, c.ph, vol_front_w(c));
+  if (vol_bytes(g, (c.C + 31) / 32 * 32) > (16ULL << 30)) return false;
   Sharing s;
   // rows, and the last ones a tile may ask for, in 32 bits
   return g.P * g.fd * g.fh * g.fw < (1LL << 30) && (long long)c.KD * g.Hq * g.Wq < (1LL << 29) && pick_sharing(g, vol_nt(c.F), g.line, &s) && vol_available();

@@ -111,6 +111,18 @@ def test_weights_are_kept_once_per_form_that_calls_take(host):
     assert rel(y, conv64(x, w, (1, 1, 1), (1, 1, 1))) < TOL
 
 
+def test_weights_and_volumes_are_not_padded_beyond_use(host):
+    """One channel, 33^3 taps: padded to 32 channels and features the weights would be 294 MB for 144 KB."""
+    from tests.test_gpu_f32tc import conv64, randn
+    x, w = randn((1, 1, 36, 37, 38), 1), randn((1, 1, 33, 33, 33), 2)
+    host.option("test_conv_route", 1)
+    allocs, launches = host.L.fortis_debug_launches(b"volume_allocs"), host.L.fortis_debug_launches(b"conv_vol_kernel")
+    y = layer(host, x, w, (0, 0, 0))
+    assert host.L.fortis_debug_launches(b"volume_allocs") == allocs and host.L.fortis_debug_launches(b"conv_vol_kernel") == launches
+    # 35,937 products on the FFMA kernel, one rounding each of up to 2^-24: at random 6.5e-6 of the 2-norm
+    assert rel(y, conv64(x, w, (1, 1, 1), (0, 0, 0))) < 35937 ** 0.5 * 2.0 ** -24
+
+
 def device_free():
     torch.cuda.synchronize()
     return torch.cuda.mem_get_info()[0]
