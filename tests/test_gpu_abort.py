@@ -79,7 +79,7 @@ def test_conv_pair_kernel_wait_gives_up_in_both_ctas_of_the_pair():
     h.reset()
 
 
-@pytest.mark.parametrize("case", ["fp32 step", "bf16 step of few rows", "fp32 conv network"])
+@pytest.mark.parametrize("case", ["fp32 step", "fp32 step on pairs of CTAs", "bf16 step of few rows", "fp32 conv network"])
 def test_layer_kernel_wait_gives_up_and_the_next_call_is_whole(case):
     """The kernel that runs layer by layer (fp32 layers and convolutions, 16-bit MLPs of few rows): every layer's first CTA
     misses its first weight stage, and the layers behind it run on what it left."""
@@ -93,16 +93,19 @@ def test_layer_kernel_wait_gives_up_and_the_next_call_is_whole(case):
         h.option("conv_shape", "%d,%d,%d,%d" % shape)
         call = lambda: h.forward(x, outs[0])
     else:
-        wl = W.column(1000)
+        wl = W.column(1000 if "pairs" not in case else 12000)
         h.configure(gather=wl["G"], scatter=wl["S"], loop=wl["Lp"])
         h.load_model(fortis_b200.write_blob(wl["layers"]))
         h.option("precision", case.split()[0])
         h.option("checksum", 1)
         d_in, outs = [dev(a) for a in wl["gin"]], [dev(a) for a in wl["sout"]]
         call = lambda: h.step(d_in, outs)
+    kernels = {k: h.L.fortis_debug_launches(k) for k in (b"mlp_pair_kernel", b"conv_vol_kernel")}
     call()
     h.sync()
     assert h.L.fortis_device_status() == 0
+    assert (h.L.fortis_debug_launches(b"mlp_pair_kernel") > kernels[b"mlp_pair_kernel"]) == ("pairs" in case)
+    assert (h.L.fortis_debug_launches(b"conv_vol_kernel") > kernels[b"conv_vol_kernel"]) == ("conv" in case)
     before = [t.clone() for t in outs]
     checksum = h.step_checksum()
     h.option("test_wait_limit", 4096)
