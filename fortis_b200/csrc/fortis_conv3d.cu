@@ -432,7 +432,7 @@ float* vol_workspace(size_t bytes, cudaStream_t s) {
 // Where a layer whose input is a plain array runs: over a split volume (packing, then no thread in the operand path), on the kernel whose
 // threads load the taps, or on the FFMA kernels (sums of few products: f32tc_conv_supported).  Small calls of few channels and many taps are
 // faster without packing (7 -> 47 channels 5x5x5 on 2 x 10x8x8 29 us, over a split volume 59; 10 -> 32 3x3x3 stride 2 15 and 28); large ones
-// over volumes (32 -> 64 on 40^3 73 and 53).
+// over volumes (32 -> 64 on 40^3 73 and 48).
 // `in_front`: what a kernel costs that packing makes unnecessary, ns.
 bool takes_volume(const ConvGeom& g, long long in_front = 0) {
   if (g_tc_test.conv_route) return g_tc_test.conv_route == 1 && vol_supported(g);

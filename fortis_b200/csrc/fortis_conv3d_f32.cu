@@ -166,7 +166,7 @@ template <int NT, bool LINE> struct Form {
   static constexpr int kTaps = LINE ? 3 : 1;
   static constexpr int kRowsOut = LINE ? kM - 2 : kM, kHalo = LINE ? 1 : 0;
   static constexpr int kWRows = LINE ? 3 * NT : NT;            // weight rows of a step held by one CTA, W_hi then W_lo
-  static constexpr int kWBytes = kWRows * kKt * 4, kWHalf = kWBytes / 2;
+  static constexpr int kWBytes = kWRows * kKt * 4;
   // tensor memory: two accumulators of kAcc columns, then the cross sums.  The accumulators take alternate steps, or where there is
   // no room for two (kHalves) 32 features each.
   static constexpr bool kHalves = LINE && NT == 64;
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
                 } else {
                   if (kt == 0 && !wait(cross_empty, (tile_it & 1) ^ 1, VST_ACC_EMPTY)) return false;   // the previous tile's cross sums have been read
                   tc_fence_after();
-                  if constexpr (LINE) mma_step32<idesc_tf32_pair(FM::kCross), kFull>(cross, row, wd + ((uint32_t)FM::kWHalf >> 4), (uint32_t)kt, nk8);
+                  if constexpr (LINE) mma_step32<idesc_tf32_pair(FM::kCross), kFull>(cross, row, wd + ((uint32_t)(FM::kWBytes / 2) >> 4), (uint32_t)kt, nk8);
                   mma_step32<idesc_tf32_pair(FM::kCross), kFull>(cross, row + (a_plane >> 4), wd, LINE ? 1u : (uint32_t)kt, nk8);
                 }
                 if constexpr (kFirst) {

@@ -24,7 +24,7 @@
 // k step read 12 KB per 128 clocks and the producers and the TMA write 96 KB per 1536, together 1.25 times what shared
 // memory moves; in this form only the weights (64 B/clk at any NT) and the fp32 tiles pass through it.
 // Measured, that form / this one: fortis_gemm 8192 x 768 x 768 756 / 62 us (a row-major operand was read by one dependent load
-// per row), column network 30,011 rows 991 / 750 us (on pairs of CTAs, fortis_mlp_pair.cu, 592); convolutions against the FFMA kernel: 32 -> 64 channels 3x3x3 on 40^3
+// per row), column network 30,011 rows 991 / 750 us (on pairs of CTAs, fortis_mlp_pair.cu, 680); convolutions against the FFMA kernel: 32 -> 64 channels 3x3x3 on 40^3
 // 297 / 73 us, 14-layer network 2 x 33^3 8.75 / 2.02 ms.
 //
 // The tensor core adds into its fp32 accumulator with truncation, not rounding, a bias per accumulation of half a unit in

@@ -16,7 +16,8 @@
 //     CTA; one MMA of N = 256 takes 128 clk and reads 8 KB of shared memory a CTA, the copies write 43 B/clk: bound by the tensor core.
 //   * one warp copies, one issues (12 MMAs a step), two accumulators of NT columns; eight epilogue warps (thread = row, half of the
 //     features) hold up to 128 sums a thread, so that the next tile's first two chunks (12,288 clk) run under a tile's end.
-// Measured: column network 244 -> 768 x4 -> 128, 30,011 rows 757 -> 592 us; a hidden layer 185 -> 151 (MMAs alone 97 at 1.9 GHz): what is left is
+// Measured: column network 244 -> 768 x4 -> 128, 30,011 rows, inputs that change from call to call 749 -> 680 us (the same inputs again 757 -> 592);
+// a hidden layer 316,000 -> 249,700 clk, 184,300 of them MMAs (151 us at the 1.65 GHz that the part runs at under this load): what is left is
 // the tiles' ends, 262 KB of split activations stored by every CTA at about the same time.
 #include <cuda.h>
 #include <cuda_runtime.h>
