@@ -28,11 +28,13 @@
 //    No multicast loads anywhere: every copy goes to the issuing CTA's own shared memory, its completion counted on
 //    the leader's barrier.
 //  * two accumulators (2 x 192 TMEM columns) so that the epilogue of a tile overlaps the MMAs of the next.
-//  * warp 0: TMA (both CTAs), warp 1: MMA (leader only), warps 2-9: epilogue, two warps per lane quadrant (thread =
-//    one voxel row x 32 channels): row neighbours by warp shuffle, the rows on either side of a warp boundary through
-//    shared memory; bias + residual row (prefetched one tile ahead) + LeakyReLU -> bf16 -> row store.  The
-//    accumulator is handed back with a RELAXED cluster-scope arrive: a release would first drain the thread's
-//    outstanding global stores (measured ~1700 cycles per tile).
+//  * warp 0: TMA (both CTAs), warp 1: MMA (leader only), then two groups of eight epilogue warps that take alternate tiles, group g
+//    the ones in accumulator g: a tile's epilogue is a chain of waits (accumulator, row exchange, residual, stores) longer than its
+//    MMAs, and two of them overlap.  In a group two warps share a lane quadrant (thread = one voxel row x 32 channels, 16 at a
+//    time): row neighbours by warp shuffle, the rows on either side of a warp boundary through shared memory; bias + residual row
+//    (prefetched one tile ahead) + LeakyReLU -> bf16 -> row store.  The accumulator is handed back with a RELAXED cluster-scope
+//    arrive: a release would first drain the thread's outstanding global stores (measured ~1700 cycles per tile).
+//    8 x 33^3, one layer of 64 channels without / with a residual: 62 / 74.5 us with one group, 58 / 70 with two.
 //
 // First layer: the fp32 NDHWC input is packed into its own padded bf16 volume with channels >= Cin zero, and the
 // weights are padded the same way, so the layer is the same GEMM with one k step per group instead of four.
@@ -59,30 +61,21 @@ using namespace tc;
 
 namespace {
 
-// How the kw taps are applied.  0 (default): one MMA of N = 3 NOUT per (kd, kh) group on unshifted rows, the shift
-// applied in the epilogue (three accumulator loads, 64 shuffles and a shared-memory exchange per row).  1: one MMA of
-// N = NOUT per tap, the kw shift taken on the A side (the descriptor's start address moves by kw rows, exactly as it
-// moves by kh (W+2) rows), so a tile's accumulator IS the output tile and the epilogue is one accumulator load per
-// row.  Bit-compatible tests pass for both; measured on the 8 x 33^3 network 1 is slower (0.895 vs 0.844 ms): three
-// N = 64 MMAs read the activation slice three times and the kernel becomes bound by shared-memory operand reads.
-#ifndef FORTIS_CONV_SHIFT_A
-#define FORTIS_CONV_SHIFT_A 0
-#endif
-constexpr bool kShiftA = FORTIS_CONV_SHIFT_A != 0;
 constexpr int kC = 64;                       // channels of the tensor-core layers
 constexpr int kTile = 128;                   // rows computed per tile (the MMA's M)
-constexpr int kTileOut = kShiftA ? kTile : kTile - 2;   // rows written per tile (epilogue-side shift: the first and last computed rows only feed their neighbours)
-constexpr int kHalo = kShiftA ? 1 : 0;       // rows in front of and behind a stage's 128 + 2 (W+2) rows, for the kw shift
+constexpr int kTileOut = kTile - 2;          // rows written per tile (the first and last computed rows only feed their neighbours)
 constexpr int kRingBytes = 108 * 1024;       // activation ring: nstages stages of (128 + 2 (W+2)) rows each
 constexpr int kMaxStages = 7;
-constexpr int kXchBytes = 2 * 2 * 4 * kC * 4; // rows exchanged between epilogue warps: [tile parity][up | down][quadrant][channel] floats
+constexpr int kXch = 2 * 4 * kC;             // floats exchanged between a group's warps: [up | down][quadrant][channel] ...
+constexpr int kXchBytes = 2 * 2 * kXch * 4;  // ... for [group][parity of its tiles]
 constexpr int kResW = 9 * 96 * kC * 2;       // 108 KB: this CTA's half of all 27 weight tiles, resident for the whole kernel
-constexpr int kConvThreads = 320;           // TMA warp, MMA warp, 8 epilogue warps (two per TMEM lane quadrant)
-constexpr int kConvSmem = kResW + kRingBytes + 256 + kXchBytes;
+constexpr int kConvThreads = 576;            // TMA warp, MMA warp, two groups of 8 epilogue warps (two per TMEM lane quadrant)
+constexpr int kConvSmem = kResW + kRingBytes + 256 + kXchBytes + kC * 4;
+static_assert(kConvSmem <= 227 * 1024, "shared memory");
 constexpr int kAccStride = 256;              // TMEM columns between the two accumulators (each 3 * NOUT wide)
 // the pair's M = 256; operand format code 1 = bf16, 0 = IEEE half (bits 7-9 for A, 10-12 for B)
 template <int NOUT, bool F16> struct ConvIdesc {
-  static constexpr uint32_t value = idesc_bf16(2 * kTile, kShiftA ? NOUT : 3 * NOUT) & ~(F16 ? ((1u << 7) | (1u << 10)) : 0u);
+  static constexpr uint32_t value = idesc_bf16(2 * kTile, 3 * NOUT) & ~(F16 ? ((1u << 7) | (1u << 10)) : 0u);
 };
 // the 16-bit storage format of activations and weights: bf16 (range of fp32, 8 significant bits) or IEEE half (11
 // significant bits, values beyond 65504 overflow)
@@ -117,9 +110,12 @@ struct ConvTcParams {
   long long* prof;             // optional cycle counters of CTA 0 (diagnostics; null in normal runs)
 };
 
-// cycle accounting for diagnostics: adds the time since *t to prof[slot] (CTA 0, one lane) and restarts the clock
+// cycle accounting for diagnostics (built with -DFORTIS_TC_PROF, printed when FORTIS_TC_PROF is set): adds the time since *t to
+// prof[slot] (CTA 0, one lane) and restarts the clock
 __device__ __forceinline__ void cprof_add(long long* prof, int slot, long long* t, bool who) {
+#ifdef FORTIS_TC_PROF
   if (prof && who) { const long long n = clock64(); atomicAdd((unsigned long long*)&prof[slot], (unsigned long long)(n - *t)); *t = n; }
+#endif
 }
 
 // KSTEPS: 16-wide k steps issued per (kd, kh) group (4 = all 64 input channels, 1 = only the first 16);  NOUT: output
@@ -127,10 +123,10 @@ __device__ __forceinline__ void cprof_add(long long* prof, int slot, long long* 
 // Launched as clusters of two CTAs (cta_group::2): the leader's MMA warp issues for both.
 template <int KSTEPS, int NOUT, bool LAST, bool F16>
 __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid_constant__ ConvTcParams P) {
-  constexpr uint32_t kIdescN = ConvIdesc<NOUT, F16>::value;            // M = 256 (128 rows per CTA), N = NOUT per tap (or 3 * NOUT per group)
-  constexpr int kWLoads = kShiftA ? 27 : 9;                       // weight tiles: one per tap, or one per (kd, kh) group
-  constexpr int kHalfRows = (kShiftA ? NOUT : 3 * NOUT) / 2;      // weight rows of one tile held by each CTA
-  constexpr int kHalfBytes = kHalfRows * kC * 2;                  // 4 KB per tap (12 KB per group)
+  constexpr uint32_t kIdescN = ConvIdesc<NOUT, F16>::value;            // M = 256 (128 rows per CTA), N = 3 * NOUT per group
+  constexpr int kWLoads = 9;                                      // weight tiles: one per (kd, kh) group
+  constexpr int kHalfRows = 3 * NOUT / 2;      // weight rows of one tile held by each CTA
+  constexpr int kHalfBytes = kHalfRows * kC * 2;                  // 12 KB per group
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t base = smem_u32(smem);                           // resident weights at offset 0
   if (base & 1023u) {                                             // same in both CTAs of a pair: both leave
@@ -146,6 +142,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
   uint32_t* tmem_slot = (uint32_t*)(barp + 160);
   volatile int* abort_flag = (volatile int*)(barp + 164);
   float* xch = (float*)(barp + 256);
+  float* bias_s = (float*)(barp + 256 + kXchBytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t crank = cluster_ctarank();
   const long long ntiles = (P.P + kTileOut - 1) / kTileOut;
@@ -155,11 +152,12 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMaxStages; s++) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); }
-    for (int b = 0; b < 2; b++) { mbar_init(bar_acc_full + 8 * b, 1); mbar_init(bar_acc_empty + 8 * b, 16); }   // 8 epilogue warps per CTA
+    for (int b = 0; b < 2; b++) { mbar_init(bar_acc_full + 8 * b, 1); mbar_init(bar_acc_empty + 8 * b, 16); }   // a group's 8 warps per CTA
     mbar_init(bar_w, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + kC) bias_s[threadIdx.x - 64] = __ldg(P.bias + threadIdx.x - 64);
   if (warp == 0 && lane < 2)
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(lane ? &P.wmap : &P.amap)) : "memory");
   if (warp == 1) {
@@ -190,13 +188,13 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
     uint32_t s = 0, ph = 0;
     bool stop = false;
     const bool pw = blockIdx.x == 0 && lane == 0;
-    long long pt = clock64();
+    long long pt = 0;
     for (long long tp = pair0; tp < npairs && !stop; tp += pair_step) {
-      const long long q0 = (2 * tp + crank) * kTileOut - (kShiftA ? 0 : 1);       // first computed row of this CTA's tile
+      const long long q0 = (2 * tp + crank) * kTileOut - 1;       // first computed row of this CTA's tile
       for (int kd = 0; kd < 3; kd++) {
         // rows q0 + (kd-1) Hp Wp - Wp ... + 127 + Wp serve the three kh taps of this kd.  The allocation carries zero
         // rows on both sides, so every coordinate is in bounds.
-        const int y0 = (int)(q0 + (long long)(kd - 1) * Hp * Wp - Wp - kHalo) + P.front;
+        const int y0 = (int)(q0 + (long long)(kd - 1) * Hp * Wp - Wp) + P.front;
         cprof_add(P.prof, 7, &pt, pw);
         if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, P.status, CST_EMPTY, P.wait_limit)) { stop = true; break; }
         cprof_add(P.prof, 6, &pt, pw);
@@ -214,7 +212,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
       uint32_t s = 0, ph = 0, acc_it = 0;
       const uint64_t desc_hi = make_kmajor_sw128_desc(0) & 0xFFFFFFFF00000000ull;
       const bool pw = blockIdx.x == 0 && lane == 0;
-      long long pt = clock64();
+      long long pt = 0;
       mbar_wait(bar_w, 0, abort_flag, P.status, CST_WEIGHTS, P.wait_limit);
       cprof_add(P.prof, 3, &pt, pw);
       for (long long tp = pair0; tp < npairs; tp += pair_step, acc_it++) {
@@ -234,23 +232,11 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
           for (int kh = 0; kh < 3; kh++) {
             // tap row kh reads the stage kh * Wp rows further down: the descriptor's start address moves; the 128-byte
             // swizzle is a function of the shared-memory address, so the shifted view matches what TMA wrote
-            if constexpr (kShiftA) {
+            const uint64_t ad = desc_hi | (uint64_t)(((sa + kh * Wp * (kC * 2)) >> 4) & 0x3FFF);
+            const uint64_t bd = desc_hi | (uint64_t)(((base + (kd * 3 + kh) * kHalfBytes) >> 4) & 0x3FFF);
 #pragma unroll
-              for (int kw = 0; kw < 3; kw++) {
-                // stage row 0 is input row q0 - (W+2) - 1 of this kd: output row r under tap (kh, kw) reads stage row r + kh (W+2) + kw
-                const uint64_t ad = desc_hi | (uint64_t)(((sa + (kh * Wp + kw) * (kC * 2)) >> 4) & 0x3FFF);
-                const uint64_t bd = desc_hi | (uint64_t)(((base + ((kd * 3 + kh) * 3 + kw) * kHalfBytes) >> 4) & 0x3FFF);
-#pragma unroll
-                for (int j = 0; j < KSTEPS; j++)
-                  tc_mma_ss_pair<kIdescN>(d_tmem, ad + (uint64_t)(j * 2), bd + (uint64_t)(j * 2), (uint32_t)(kd | kh | kw | j));
-              }
-            } else {
-              const uint64_t ad = desc_hi | (uint64_t)(((sa + kh * Wp * (kC * 2)) >> 4) & 0x3FFF);
-              const uint64_t bd = desc_hi | (uint64_t)(((base + (kd * 3 + kh) * kHalfBytes) >> 4) & 0x3FFF);
-#pragma unroll
-              for (int j = 0; j < KSTEPS; j++)
-                tc_mma_ss_pair<kIdescN>(d_tmem, ad + (uint64_t)(j * 2), bd + (uint64_t)(j * 2), (uint32_t)(kd | kh | j));
-            }
+            for (int j = 0; j < KSTEPS; j++)
+              tc_mma_ss_pair<kIdescN>(d_tmem, ad + (uint64_t)(j * 2), bd + (uint64_t)(j * 2), (uint32_t)(kd | kh | j));
           }
           tc_commit_pair(bar_empty + 8 * s);                      // frees this stage in both CTAs
           if (++s == (uint32_t)P.nstages) { s = 0; ph ^= 1; }
@@ -260,31 +246,23 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
     }
   } else {
     // ---- epilogue: thread = one computed row (voxel of the padded volume);
-    //      out[row] = acc_kw0[row - 1] + acc_kw1[row] + acc_kw2[row + 1], the neighbours by warp shuffle: each warp's 32
-    //      computed rows overlap the next warp's by two, so lanes 1..30 have both neighbours in their own warp
-    const int quad = warp & 3, half = (warp - 2) >> 2;            // TMEM lane quadrant; which half of the channels
+    //      out[row] = acc_kw0[row - 1] + acc_kw1[row] + acc_kw2[row + 1], the neighbours by warp shuffle.  Group g takes every other
+    //      tile, the ones in accumulator g, 16 channels of a row at a time.
+    const int quad = warp & 3, group = (warp - 2) >> 3, half = ((warp - 2) >> 2) & 1;   // TMEM lane quadrant; accumulator; half of the channels
     const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16);
     constexpr int CW = NOUT == kC ? kC / 2 : NOUT;                 // channels per warp: two warps share a row of 64
     const bool active = NOUT == kC || half == 0;                   // a 16-channel layer needs one warp per quadrant
     const int c0 = NOUT == kC ? CW * half : 0;
-    float bias[CW];
-#pragma unroll
-    for (int j = 0; j < CW / 4; j++) {
-      const float4 q = __ldg(reinterpret_cast<const float4*>(P.bias + c0) + j);
-      bias[4 * j] = q.x; bias[4 * j + 1] = q.y; bias[4 * j + 2] = q.z; bias[4 * j + 3] = q.w;
-    }
     asm volatile("griddepcontrol.wait;" ::: "memory");           // before the first read of the residual volume and the first store
-    const uint32_t arr_acc_empty = map_to_cta(bar_acc_empty, 0);   // the leader's barrier
+    const uint32_t acc_full = bar_acc_full + 8 * group, arr_acc_empty = map_to_cta(bar_acc_empty + 8 * group, 0);   // the latter the leader's
     const bool pw = blockIdx.x == 0 && threadIdx.x == 64;
-    long long pt = clock64();
+    long long pt = 0;
     const uint32_t uW = (uint32_t)Wp, uH = (uint32_t)Hp, uD = (uint32_t)Dp;
-    // row of this thread in tile pair tp_ and whether it is written / an interior voxel (P < 2^31: 32-bit arithmetic).
-    // (Advancing the coordinates from tile to tile by additions with carries instead of dividing was measured 6 %
-    // SLOWER over the whole kernel: the divisions sit in front of the accumulator wait, where the warp would idle.)
+    // row of this thread in tile pair tp_ and whether it is written / an interior voxel (P < 2^31: 32-bit arithmetic)
     auto locate = [&](long long tp_, uint32_t& p_, bool& writes_, bool& interior_, uint32_t& wp_, uint32_t& hp_, uint32_t& dp_, uint32_t& n_) {
-      const int r = quad * 32 + lane;                              // epilogue-side shift: rows 0 and 127 are computed for their neighbours only
-      const long long pl = (2 * tp_ + crank) * kTileOut + r - (kShiftA ? 0 : 1);
-      writes_ = active && tp_ < npairs && (kShiftA || (r >= 1 && r <= kTileOut)) && pl < P.P;
+      const int r = quad * 32 + lane;                              // rows 0 and 127 are computed for their neighbours only
+      const long long pl = (2 * tp_ + crank) * kTileOut + r - 1;
+      writes_ = active && tp_ < npairs && r >= 1 && r <= kTileOut && pl < P.P;
       p_ = writes_ ? (uint32_t)pl : 0u;
       const uint32_t t1 = p_ / uW, t2 = t1 / uH;
       wp_ = p_ - t1 * uW; hp_ = t1 - t2 * uH; n_ = t2 / uD; dp_ = t2 - n_ * uD;
@@ -292,102 +270,119 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
     };
     uint32_t p, wp, hp, dp, n_;
     bool writes, interior;
-    locate(pair0, p, writes, interior, wp, hp, dp, n_);
-    // this warp's half of the residual row of the thread's voxel, always fetched one tile ahead
+    locate(pair0 + group * pair_step, p, writes, interior, wp, hp, dp, n_);
+    // this warp's half of the residual row of the thread's voxel, always fetched one tile of the group ahead
     uint4 sk[CW / 8];
     bool use_skip = !LAST && P.skip != nullptr && interior;
     if (use_skip) {
 #pragma unroll
       for (int j = 0; j < CW / 8; j++) sk[j] = ld_global(reinterpret_cast<const uint4*>(P.skip + (size_t)p * kC + c0) + j);
     }
-    uint32_t acc_it = 0;
-    for (long long tp = pair0; tp < npairs; tp += pair_step, acc_it++) {
-      const uint32_t b = acc_it & 1, aph = (acc_it >> 1) & 1;
+    uint32_t it = 0;
+    for (long long tp = pair0 + group * pair_step; tp < npairs; tp += 2 * pair_step, it++) {
       uint32_t np, nwp, nhp, ndp, nn;
       bool nwrites, ninterior;
-      locate(tp + pair_step, np, nwrites, ninterior, nwp, nhp, ndp, nn);
+      locate(tp + 2 * pair_step, np, nwrites, ninterior, nwp, nhp, ndp, nn);
       const bool nuse_skip = !LAST && P.skip != nullptr && ninterior;
       cprof_add(P.prof, 10, &pt, pw);
-      mbar_wait(bar_acc_full + 8 * b, aph, abort_flag, P.status, CST_ACC_FULL, P.wait_limit);
+      mbar_wait(acc_full, it & 1, abort_flag, P.status, CST_ACC_FULL, P.wait_limit);
       cprof_add(P.prof, 8, &pt, pw);
       tc_fence_after();
-      const uint32_t accb = lane_addr + b * kAccStride + c0;
-      float v[CW];
-      if constexpr (kShiftA) {
-        uint32_t a1[CW];
-        if (active) { tmem_ldn(accb, a1); tmem_ld_wait(); }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster_relaxed(arr_acc_empty + 8 * b);   // one arrival per warp: the leader may refill this accumulator
-        if (!active) continue;
+      const uint32_t accb = lane_addr + group * kAccStride + c0;
+      float* xu = xch + (2 * group + (it & 1)) * kXch + c0;        // kw = 0 partials of each quadrant's last row
+      float* xd = xu + 4 * kC;                                     // kw = 2 partials of each quadrant's first row
 #pragma unroll
-        for (int i = 0; i < CW; i++) v[i] = __uint_as_float(a1[i]) + bias[i];
-      } else {
-        uint32_t a0[CW], a1[CW], a2[CW];
+      for (int c = 0; c < CW; c += 16) {
+        uint32_t a0[16], a1[16], a2[16];
         if (active) {
-          tmem_ldn(accb, a0);
-          tmem_ldn(accb + NOUT, a1);
-          tmem_ldn(accb + 2 * NOUT, a2);
+          tmem_ld16(accb + c, a0);
+          tmem_ld16(accb + NOUT + c, a1);
+          tmem_ld16(accb + 2 * NOUT + c, a2);
           tmem_ld_wait();
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster_relaxed(arr_acc_empty + 8 * b);   // one arrival per warp: the leader may refill this accumulator
+        if (c + 16 == CW) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster_relaxed(arr_acc_empty);   // one arrival per warp: the leader may refill this accumulator
+        }
         if (!active) continue;
-        // rows on either side of a warp boundary go through shared memory (the buffer alternates per tile, so one
-        // barrier per tile among the four warps that hold the same channels is enough)
-        float* xu = xch + (acc_it & 1) * (2 * 4 * kC);               // kw = 0 partials of each quadrant's last row
-        float* xd = xu + 4 * kC;                                     // kw = 2 partials of each quadrant's first row
+        // The rows on either side of a warp boundary go through shared memory: the last lane publishes its kw = 0 partials and
+        // takes the previous quadrant's in their place (the first lane likewise with kw = 2), so that a rotation by one lane
+        // brings every lane its neighbour's.  (The buffer alternates, so one barrier among the four warps that hold the same
+        // channels is enough.)
         if (lane == 31) {
 #pragma unroll
-          for (int i = 0; i < CW; i++) xu[quad * kC + c0 + i] = __uint_as_float(a0[i]);
+          for (int i = 0; i < 16; i += 4) *reinterpret_cast<uint4*>(xu + quad * kC + c + i) = make_uint4(a0[i], a0[i + 1], a0[i + 2], a0[i + 3]);
         }
         if (lane == 0) {
 #pragma unroll
-          for (int i = 0; i < CW; i++) xd[quad * kC + c0 + i] = __uint_as_float(a2[i]);
+          for (int i = 0; i < 16; i += 4) *reinterpret_cast<uint4*>(xd + quad * kC + c + i) = make_uint4(a2[i], a2[i + 1], a2[i + 2], a2[i + 3]);
         }
-        if (half == 0) asm volatile("bar.sync 1, 128;" ::: "memory"); else asm volatile("bar.sync 2, 128;" ::: "memory");
-#pragma unroll
-        for (int i = 0; i < CW; i++) {
-          float up = __shfl_up_sync(0xffffffffu, __uint_as_float(a0[i]), 1);
-          float dn = __shfl_down_sync(0xffffffffu, __uint_as_float(a2[i]), 1);
-          if (lane == 0 && quad > 0) up = xu[(quad - 1) * kC + c0 + i];
-          if (lane == 31 && quad < 3) dn = xd[(quad + 1) * kC + c0 + i];
-          v[i] = (__uint_as_float(a1[i]) + up) + (dn + bias[i]);
+        if (group == 0) {
+          if (half == 0) asm volatile("bar.sync 1, 128;" ::: "memory"); else asm volatile("bar.sync 2, 128;" ::: "memory");
+        } else {
+          if (half == 0) asm volatile("bar.sync 3, 128;" ::: "memory"); else asm volatile("bar.sync 4, 128;" ::: "memory");
         }
-      }
-      if (LAST) {
-        if (interior) {
-          float* dst = P.y + ((((size_t)n_ * P.D + dp - 1) * P.H + hp - 1) * P.W + wp - 1) * P.F;
+        if (lane == 31 && quad > 0) {
 #pragma unroll
-          for (int f = 0; f < CW; f++)
-            if (f < P.F) dst[f] = fmaxf(v[f], v[f] * P.slope);
-        }
-      } else {
-        if (use_skip) {
-#pragma unroll
-          for (int h = 0; h < CW / 8; h++) {
-            const uint32_t* s2 = reinterpret_cast<const uint32_t*>(&sk[h]);
-#pragma unroll
-            for (int e = 0; e < 4; e++) { const float2 f = cunpack16<F16>(s2[e]); v[8 * h + 2 * e] += f.x; v[8 * h + 2 * e + 1] += f.y; }
+          for (int i = 0; i < 16; i += 4) {
+            const uint4 q = *reinterpret_cast<const uint4*>(xu + (quad - 1) * kC + c + i);
+            a0[i] = q.x; a0[i + 1] = q.y; a0[i + 2] = q.z; a0[i + 3] = q.w;
           }
         }
-        if (nuse_skip) {                                           // these registers are free again: next tile's residual row
+        if (lane == 0 && quad < 3) {
 #pragma unroll
-          for (int h = 0; h < CW / 8; h++) sk[h] = ld_global(reinterpret_cast<const uint4*>(P.skip + (size_t)np * kC + c0) + h);
+          for (int i = 0; i < 16; i += 4) {
+            const uint4 q = *reinterpret_cast<const uint4*>(xd + (quad + 1) * kC + c + i);
+            a2[i] = q.x; a2[i + 1] = q.y; a2[i + 2] = q.z; a2[i + 3] = q.w;
+          }
         }
-        if (writes) {
-          uint4* dst = reinterpret_cast<uint4*>(P.out + (size_t)p * kC + c0);
+        __syncwarp();
+        float v[16];
 #pragma unroll
-          for (int h = 0; h < CW / 8; h++) {
-            uint32_t pk[4];
+        for (int i = 0; i < 16; i += 4) {
+          const float4 bq = *reinterpret_cast<const float4*>(bias_s + c0 + c + i);
+          const float bias[4] = {bq.x, bq.y, bq.z, bq.w};
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-              const float x0 = interior ? fmaxf(v[8 * h + 2 * e], v[8 * h + 2 * e] * P.slope) : 0.f;
-              const float x1 = interior ? fmaxf(v[8 * h + 2 * e + 1], v[8 * h + 2 * e + 1] * P.slope) : 0.f;
-              pk[e] = cpack16<F16>(x0, x1);
+          for (int j = 0; j < 4; j++) {
+            const float up = __uint_as_float(__shfl_sync(0xffffffffu, a0[i + j], lane - 1));    // the lane modulo 32
+            const float dn = __uint_as_float(__shfl_sync(0xffffffffu, a2[i + j], lane + 1));
+            v[i + j] = (__uint_as_float(a1[i + j]) + up) + (dn + bias[j]);
+          }
+        }
+        if (LAST) {
+          if (interior) {
+            float* dst = P.y + ((((size_t)n_ * P.D + dp - 1) * P.H + hp - 1) * P.W + wp - 1) * P.F;
+#pragma unroll
+            for (int f = 0; f < 16; f++)
+              if (f < P.F) dst[f] = fmaxf(v[f], v[f] * P.slope);
+          }
+        } else {
+          if (use_skip) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+              const uint32_t* s2 = reinterpret_cast<const uint32_t*>(&sk[c / 8 + h]);
+#pragma unroll
+              for (int e = 0; e < 4; e++) { const float2 f = cunpack16<F16>(s2[e]); v[8 * h + 2 * e] += f.x; v[8 * h + 2 * e + 1] += f.y; }
             }
-            dst[h] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+          }
+          if (nuse_skip) {                                         // these registers are free again: the next tile's residual row
+#pragma unroll
+            for (int h = 0; h < 2; h++) sk[c / 8 + h] = ld_global(reinterpret_cast<const uint4*>(P.skip + (size_t)np * kC + c0 + c) + h);
+          }
+          if (writes) {
+            uint4* dst = reinterpret_cast<uint4*>(P.out + (size_t)p * kC + c0 + c);
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+              uint32_t pk[4];
+#pragma unroll
+              for (int e = 0; e < 4; e++) {
+                const float x0 = interior ? fmaxf(v[8 * h + 2 * e], v[8 * h + 2 * e] * P.slope) : 0.f;
+                const float x1 = interior ? fmaxf(v[8 * h + 2 * e + 1], v[8 * h + 2 * e + 1] * P.slope) : 0.f;
+                pk[e] = cpack16<F16>(x0, x1);
+              }
+              dst[h] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            }
           }
         }
       }
@@ -457,7 +452,7 @@ bool make_map(CUtensorMap* m, void* base, long long rows, int box_rows) {
 // nbox boxes of box_rows (<= 256, multiple of 8) rows
 struct RingGeom { int stage_bytes, nstages, box_rows, nbox; };
 bool ring_geometry(int Wp, RingGeom* g) {
-  const int R = kTile + 2 * Wp + 2 * kHalo;
+  const int R = kTile + 2 * Wp;
   g->nbox = (R + 255) / 256;
   g->box_rows = (((R + g->nbox - 1) / g->nbox) + 7) / 8 * 8;
   g->stage_bytes = ((g->nbox * g->box_rows * kC * 2) + 1023) / 1024 * 1024;
@@ -553,7 +548,7 @@ ConvTcModel* conv_tc_create(const ModelHost& M, bool f16, std::string* err) {
     if (!dw || !db) return fail("out of device memory for conv weights");
     m->w.push_back(dw); m->b.push_back(db);
     CUtensorMap map;
-    if (!make_map(&map, dw, 27 * rows, (kShiftA ? rows : 3 * rows) / 2)) return fail("cuTensorMapEncodeTiled failed for conv weights");
+    if (!make_map(&map, dw, 27 * rows, 3 * rows / 2)) return fail("cuTensorMapEncodeTiled failed for conv weights");
     m->wmaps.push_back(map);
   }
   if (cudaMalloc(&m->status, sizeof(int)) != cudaSuccess) return fail("out of device memory");
