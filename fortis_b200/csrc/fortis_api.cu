@@ -755,11 +755,13 @@ bool stencil_operands(const StepArgs& A, const RowGeom& g, StencilLaunch* L) {
     L->in[f] = (const float*)A.TG.base[c.array] + c.off0;
   }
   const Access& o0 = Sc.stores[0].a;
+  L->in_order = 1;
   for (size_t q = 0; q < Sc.stores.size(); q++) {
     const Access& a = Sc.stores[q].a;
     if (a.elt != 0 || a.si != 1 || a.sj != o0.sj || a.sk != o0.sk || Sc.stores[q].slot > 3) return false;
     L->out[q] = (float*)A.TS.base[a.array] + a.off0;
     L->out_slot[q] = Sc.stores[q].slot;
+    if (Sc.stores[q].slot != (int)q) L->in_order = 0;
   }
   L->nstores = (int)Sc.stores.size();
   L->sj_in = c0.sj; L->sk_in = c0.sk; L->sj_out = o0.sj; L->sk_out = o0.sk;

@@ -58,6 +58,7 @@ void launch_small_mlp(int nlayers, const int* dims, const SmallMlpLaunch& L, cud
 struct StencilLaunch {
   const float* in[3];             // per field: the element the CENTRE tap of point (0, 0) of plane 0 reads
   float* out[4]; int out_slot[4]; int nstores;      // per store: the element point (0, 0, 0) writes, and which model output
+  int in_order;                   // store s writes output s
   long long sj_in, sk_in, sj_out, sk_out;           // element strides of the j index and of the plane (i has stride 1)
   int ni, nj, nk;                 // interior extent
   int has_in_div, has_out_mul;
