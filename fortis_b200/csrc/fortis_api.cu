@@ -722,6 +722,29 @@ bool small_fast_operands(const StepArgs& A, const RowGeom& g, SmallFast* F) {
   return true;
 }
 
+// Operands of the scatter that takes its plan as kernel parameters: a few stores, no lifted expressions, positions in 32 bits.
+// (Rows of more than 32 bytes are read coalesced by scatter_kernel.)
+bool scatter_rows_operands(const PlanDev& P, const ArrayTable& T, const RowGeom& g, const float* Y, ScatterRows* R) {
+  const long long nrows = g.count * g.nk;
+  if (P.h.prog.nops || !P.h.scalars.empty() || P.h.stores.empty() || (int)P.h.stores.size() > kScatterRowsStores || P.h.n > kScatterRowsWidth ||
+      nrows <= 0 || nrows >= (1LL << 30) || g.ni <= 0 || g.kk0 < 0)
+    return false;
+  std::memset(R, 0, sizeof *R);
+  const long long ci = g.ni - 1, cj = (g.count - 1) / g.ni, kk = g.kk0 + g.nk - 1;      // the largest positions
+  for (size_t s = 0; s < P.h.stores.size(); s++) {
+    const Access& a = P.h.stores[s].a;
+    const long long reach = ci * std::llabs(a.si) + cj * std::llabs(a.sj) + kk * std::llabs(a.sk);
+    if (std::llabs(a.si) >= (1LL << 31) || std::llabs(a.sj) >= (1LL << 31) || std::llabs(a.sk) >= (1LL << 31) || reach >= (1LL << 31)) return false;
+    R->ptr[s] = (char*)T.base[a.array] + a.off0 * (long long)elt_size(a.elt);
+    R->slot[s] = P.h.stores[s].slot; R->elt[s] = a.elt;
+    R->si[s] = (int)a.si; R->sj[s] = (int)a.sj; R->sk[s] = (int)a.sk;
+  }
+  R->nstores = (int)P.h.stores.size();
+  R->Y = Y; R->n = P.h.n;
+  R->nrows = (unsigned)nrows; R->count = (unsigned)g.count; R->ni = (unsigned)g.ni; R->kk0 = (unsigned)g.kk0;
+  return true;
+}
+
 // the standalone scatter of a step; with option "checksum" its stores are summed like those of the fused kernels
 void scatter_with_checksum(const StepArgs& A, const RowGeom& g) {
   Session& s = S();
@@ -729,6 +752,8 @@ void scatter_with_checksum(const StepArgs& A, const RowGeom& g) {
   double* partials = nullptr;
   const int grid = scatter_grid(g.count * g.nk);
   if (s.want_checksum) { ensure_aux(grid); partials = s.d_partials; }
+  ScatterRows R;
+  if (!partials && scatter_rows_operands(s.S, A.TS, g, s.dout, &R)) { launch_scatter_rows(R, st); return; }
   launch_scatter(s.S.hdr, (const StoreTarget*)s.S.items, s.S.h.n, A.TS, g, s.dout, st, partials);
   if (partials) launch_fold(s.d_partials, grid, s.d_sum, 1, st);
 }
@@ -1054,7 +1079,9 @@ void do_scatter(const int* iargs, int nint, void* const* ptrs, int narr) {
   const long long yoff = s.loop.kdist ? (long long)(args[0] - s.loop.klo) * count * s.model.n_out() : 0;
   if (s.loop.kdist && (args[0] < s.loop.klo || args[0] >= s.loop.klo + s.loop.nk))
     throw std::runtime_error("fortis_scatter: enclosing-loop index outside the distributed range");
-  launch_scatter(s.S.hdr, (const StoreTarget*)s.S.items, s.S.h.n, T, g, s.dout + yoff, st);
+  ScatterRows R;
+  if (scatter_rows_operands(s.S, T, g, s.dout + yoff, &R)) launch_scatter_rows(R, st);
+  else launch_scatter(s.S.hdr, (const StoreTarget*)s.S.items, s.S.h.n, T, g, s.dout + yoff, st);
   download_stores(s.S, args, nint, false);
   if (!s.async) cudaStreamSynchronize(st);
 }

@@ -21,6 +21,17 @@ void launch_gather(const IoPlanDev* P, const Access* slots, int n, const ArrayTa
 void launch_scatter(const IoPlanDev* P, const StoreTarget* stores, int nout, const ArrayTable& T, const RowGeom& g,
                     const float* Y, cudaStream_t s, double* partials = nullptr);
 int scatter_grid(long long nrows);
+// Operands of the scatter for plans of few stores without expressions (scatter_rows_kernel): the element that store s writes for a
+// row in (ci, cj, kk) is ptr[s] + ci si[s] + cj sj[s] + kk sk[s]
+constexpr int kScatterRowsStores = 8, kScatterRowsWidth = 8;
+struct ScatterRows {
+  const float* Y; int n;          // (rows, n) model output, n <= kScatterRowsWidth
+  void* ptr[kScatterRowsStores];
+  int slot[kScatterRowsStores], elt[kScatterRowsStores], si[kScatterRowsStores], sj[kScatterRowsStores], sk[kScatterRowsStores];
+  int nstores;
+  unsigned nrows, count, ni, kk0;
+};
+void launch_scatter_rows(const ScatterRows& R, cudaStream_t s);
 void launch_linear_f32(const float* A, const float* W, const float* bias, float* C, long long M, int N, int K, int act,
                        float slope, const float* in_div, const float* out_mul, const float* relu_mask, cudaStream_t s);
 
