@@ -528,6 +528,13 @@ bool is_device_ptr(const void* p) {
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+// which of a call's arrays lie in device memory: one query of the driver per array and call (0.15 us each), looked at by every path of the call
+std::vector<char> device_resident(const PlanDev& P, void* const* ptrs) {
+  std::vector<char> dev(P.h.arrays.size());
+  for (size_t ai = 0; ai < dev.size(); ai++) dev[ai] = is_device_ptr(ptrs[ai]);
+  return dev;
+}
+
 // pin once; an array whose address moves between calls is a temporary: unpin it and never pin it again
 void pin_policy(PlanDev& P, int ai, const void* H, size_t bytes) {
   if (P.reg[ai] == (const void*)1 || P.reg[ai] == H) return;
@@ -555,8 +562,8 @@ long long plane_off_args(const ArrayInfo& a, const int* args, int nargs) {
 }
 
 // Bind this call's arrays into an ArrayTable.  `multi_plane`: all planes klo..klo+nk-1 are addressed through kk
-// (k-distributed gather, fused step); otherwise the plane chosen by the integer arguments.
-void bind_arrays(PlanDev& P, void* const* ptrs, const int* args, int nargs, bool multi_plane, bool upload_readonly,
+// (k-distributed gather, fused step); otherwise the plane chosen by the integer arguments.  `dev`: device_resident of these arrays.
+void bind_arrays(PlanDev& P, void* const* ptrs, const std::vector<char>& dev, const int* args, int nargs, bool multi_plane, bool upload_readonly,
                  ArrayTable* T) {
   Session& s = S();
   cudaStream_t st = stream();
@@ -569,7 +576,7 @@ void bind_arrays(PlanDev& P, void* const* ptrs, const int* args, int nargs, bool
     P.cur[ai] = H;
     const bool planes = multi_plane && !a.vdims.empty();
     const long long first = planes ? (long long)(s.loop.klo - 1) * a.plane : (multi_plane ? 0 : plane_off_args(a, args, nargs));
-    P.on_dev[ai] = is_device_ptr(H);
+    P.on_dev[ai] = dev[ai];
     if (P.on_dev[ai]) { T->base[ai] = H + first * es; continue; }
     const long long need = planes ? a.plane * s.loop.nk : a.plane;
     pin_policy(P, (int)ai, H, (size_t)a.total * es);
@@ -997,7 +1004,7 @@ void do_gather(const int* iargs, int nint, void* const* ptrs, int narr) {
   for (int i = 0; i < 8; i++) s.gather_args[i] = i < nint ? iargs[i] : 1;
   // staging happens now (the host may change its arrays after this call returns); the gather itself is deferred
   ArrayTable T;
-  bind_arrays(s.G, ptrs, s.gather_args, nint, s.loop.kdist, true, &T);
+  bind_arrays(s.G, ptrs, device_resident(s.G, ptrs), s.gather_args, nint, s.loop.kdist, true, &T);
   s.gather_pending = true;
 }
 
@@ -1072,7 +1079,7 @@ void do_scatter(const int* iargs, int nint, void* const* ptrs, int narr) {
   int args[8];
   for (int i = 0; i < 8; i++) args[i] = i < nint ? iargs[i] : 1;
   ArrayTable T;
-  bind_arrays(s.S, ptrs, args, nint, false, true, &T);
+  bind_arrays(s.S, ptrs, device_resident(s.S, ptrs), args, nint, false, true, &T);
   RowGeom g = geom_all(rows);
   const long long count = g.count;
   g.nk = 1; g.kk0 = 0;
@@ -1098,7 +1105,7 @@ bool ranges_overlap(const void* a, size_t na, const void* b, size_t nb) {
 // chunks: chunk c's slices of the input arrays go up on the H2D stream, the step kernels run on chunk c as soon as they
 // have landed, and chunk c's slices of the stored arrays come back on the D2H stream while chunk c+1 computes and
 // chunk c+2 uploads.  Returns false when the call is not of that shape (the caller then takes the serial path).
-bool overlapped_step(void* const* gptrs, void* const* sptrs, long long rows) {
+bool overlapped_step(void* const* gptrs, const std::vector<char>& gdev, void* const* sptrs, const std::vector<char>& sdev, long long rows) {
   Session& s = S();
   if (s.loop.kdist || s.loop.has_outer || s.loop.nk != 1 || !s.fuse || rows < 4096 || std::getenv("FORTIS_NO_OVERLAP")) return false;
   const long long ncol = rows;
@@ -1108,7 +1115,7 @@ bool overlapped_step(void* const* gptrs, void* const* sptrs, long long rows) {
     const ArrayInfo& a = s.G.h.arrays[ai];
     if (!a.used) continue;
     if (!column_array(a)) return false;
-    if (!is_device_ptr(gptrs[ai]) && !maps_host(s.G)) any_host = true;
+    if (!gdev[ai] && !maps_host(s.G)) any_host = true;
   }
   for (auto& x : s.G.h.slots) if (x.si != 1) return false;
   for (auto& x : s.G.h.scalars) if (x.si != 1) return false;
@@ -1116,7 +1123,7 @@ bool overlapped_step(void* const* gptrs, void* const* sptrs, long long rows) {
     const ArrayInfo& a = s.S.h.arrays[ai];
     if (!a.used) continue;
     if (!column_array(a) || !s.S.h.written[ai]) return false;       // arrays a scatter only reads would need a whole upload
-    if (!is_device_ptr(sptrs[ai]) && !maps_host(s.S)) any_host = true;
+    if (!sdev[ai] && !maps_host(s.S)) any_host = true;
   }
   for (auto& t : s.S.h.stores) if (t.a.si != 1) return false;
   if (!any_host || !ensure_copy_streams()) return false;
@@ -1175,8 +1182,8 @@ bool overlapped_step(void* const* gptrs, void* const* sptrs, long long rows) {
   StepArgs A;
   A.use_gather = true; A.fuse_scatter = true;
   // pins the arrays, sizes the staging buffers; the copies themselves are issued per chunk below
-  bind_arrays(s.G, gptrs, args, 0, false, false, &A.TG);
-  bind_arrays(s.S, sptrs, args, 0, false, false, &A.TS);
+  bind_arrays(s.G, gptrs, gdev, args, 0, false, false, &A.TG);
+  bind_arrays(s.S, sptrs, sdev, args, 0, false, false, &A.TS);
   // Per-column vectors (one element per column) are not staged at all: a copy of a few hundred KB costs a copy's
   // latency (7-10 us each, and copies of one direction run one after another whatever their stream), which for a dozen
   // vectors is a tenth of the step.  The kernels load and store them through the pinned host pages instead; their
@@ -1258,7 +1265,7 @@ bool overlapped_step(void* const* gptrs, void* const* sptrs, long long rows) {
       if (threw) throw std::runtime_error(what);
       std::fprintf(stderr, "fortis: capture of the staging pipeline failed, running eagerly\n");
       s.ov_calls = 2;                                   // do not try again for this set of arrays
-      return overlapped_step(gptrs, sptrs, rows);
+      return overlapped_step(gptrs, gdev, sptrs, sdev, rows);
     }
   } else if (threw) throw std::runtime_error(what);
   if (!s.async) cudaStreamSynchronize(st);
@@ -1270,7 +1277,7 @@ bool overlapped_step(void* const* gptrs, void* const* sptrs, long long rows) {
 // back (driver/fortis_gather_emit.py:66-68, 91-96 moves all planes up, then computes, then copies back rectangle by
 // rectangle on one stream).  A plane is contiguous, so the uploads are plain 1-D copies; planes are independent (the
 // stencil is within a plane), so a plane is a step of its own with nk = 1.  Replayed as one graph from the second call.
-bool overlapped_planes_step(void* const* gptrs, void* const* sptrs) {
+bool overlapped_planes_step(void* const* gptrs, const std::vector<char>& gdev, void* const* sptrs, const std::vector<char>& sdev) {
   Session& s = S();
   if (!s.loop.kdist || s.loop.nk < 2 || s.loop.nk > kMaxChunks || !s.fuse || std::getenv("FORTIS_NO_OVERLAP")) return false;
   bool any_host = false;
@@ -1278,13 +1285,13 @@ bool overlapped_planes_step(void* const* gptrs, void* const* sptrs) {
     const ArrayInfo& a = s.G.h.arrays[ai];
     if (!a.used) continue;
     if (a.vdims.empty()) return false;
-    if (!is_device_ptr(gptrs[ai]) && !maps_host(s.G)) any_host = true;
+    if (!gdev[ai] && !maps_host(s.G)) any_host = true;
   }
   for (size_t ai = 0; ai < s.S.h.arrays.size(); ai++) {
     const ArrayInfo& a = s.S.h.arrays[ai];
     if (!a.used) continue;
     if (a.vdims.empty() || !s.S.h.written[ai]) return false;
-    if (!is_device_ptr(sptrs[ai]) && !maps_host(s.S)) any_host = true;
+    if (!sdev[ai] && !maps_host(s.S)) any_host = true;
   }
   if (!any_host || !ensure_copy_streams()) return false;
   cudaStream_t st = stream();
@@ -1305,8 +1312,8 @@ bool overlapped_planes_step(void* const* gptrs, void* const* sptrs) {
   int args[8] = {1, 1, 1, 1, 1, 1, 1, 1};
   StepArgs A;
   A.use_gather = true; A.fuse_scatter = true;
-  bind_arrays(s.G, gptrs, args, 0, true, false, &A.TG);          // pins, sizes the staging of all planes; no copies
-  bind_arrays(s.S, sptrs, args, 0, true, false, &A.TS);
+  bind_arrays(s.G, gptrs, gdev, args, 0, true, false, &A.TG);          // pins, sizes the staging of all planes; no copies
+  bind_arrays(s.S, sptrs, sdev, args, 0, true, false, &A.TS);
   const ArrayTable TG0 = A.TG, TS0 = A.TS;
   const LoopInfo saved = s.loop;
   bool capturing = (++s.ov_calls == 2) && !std::getenv("FORTIS_NO_STAGING_GRAPH");
@@ -1356,7 +1363,7 @@ bool overlapped_planes_step(void* const* gptrs, void* const* sptrs) {
       if (threw) throw std::runtime_error(what);
       std::fprintf(stderr, "fortis: capture of the staging pipeline failed, running eagerly\n");
       s.ov_calls = 2;
-      return overlapped_planes_step(gptrs, sptrs);
+      return overlapped_planes_step(gptrs, gdev, sptrs, sdev);
     }
   } else if (threw) throw std::runtime_error(what);
   if (!s.async) cudaStreamSynchronize(st);
@@ -1391,24 +1398,25 @@ void do_step(const int* iargs, int nint, void* const* gptrs, int ng, void* const
   }
   // a device-resident gather array that shares memory with a device-resident stored array forces the unfused sequence
   // below; the pipelined staging paths run fused kernels, so they are not taken then
+  const std::vector<char> gdev = device_resident(s.G, gptrs), sdev = device_resident(s.S, sptrs);
   bool dev_overlap = false;
   for (size_t gi = 0; gi < s.G.h.arrays.size() && !dev_overlap; gi++) {
-    if (!s.G.h.arrays[gi].used || !is_device_ptr(gptrs[gi])) continue;
+    if (!s.G.h.arrays[gi].used || !gdev[gi]) continue;
     const ArrayInfo& ga = s.G.h.arrays[gi];
     for (size_t si = 0; si < s.S.h.arrays.size(); si++) {
-      if (!s.S.h.written[si] || !is_device_ptr(sptrs[si])) continue;
+      if (!s.S.h.written[si] || !sdev[si]) continue;
       const ArrayInfo& sa = s.S.h.arrays[si];
       if (ranges_overlap(gptrs[gi], (size_t)ga.total * elt_size(ga.elt), sptrs[si], (size_t)sa.total * elt_size(sa.elt))) { dev_overlap = true; break; }
     }
   }
-  if (!dev_overlap && (overlapped_step(gptrs, sptrs, rows) || overlapped_planes_step(gptrs, sptrs))) return;
+  if (!dev_overlap && (overlapped_step(gptrs, gdev, sptrs, sdev, rows) || overlapped_planes_step(gptrs, gdev, sptrs, sdev))) return;
   cudaStream_t st = stream();
   int args[8];
   for (int i = 0; i < 8; i++) args[i] = i < nint ? iargs[i] : 1;
   StepArgs A;
   A.rows = rows; A.use_gather = true; A.fuse_scatter = true;
-  bind_arrays(s.G, gptrs, args, nint, multi, true, &A.TG);
-  bind_arrays(s.S, sptrs, args, nint, multi, true, &A.TS);
+  bind_arrays(s.G, gptrs, gdev, args, nint, multi, true, &A.TG);
+  bind_arrays(s.S, sptrs, sdev, args, nint, multi, true, &A.TS);
   // A fused kernel reads its inputs and writes its outputs in the same launch.  When a device-resident gather array
   // shares memory with a device-resident stored array, a stencil would read neighbours another thread is
   // overwriting; the reference is well-defined there because gather and scatter work on separate staging copies.
