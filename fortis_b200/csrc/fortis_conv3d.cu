@@ -174,7 +174,7 @@ __device__ __forceinline__ void voxel_at(const ConvGeom& g, unsigned v, int* n, 
 
 // FG: warps of a block that share their voxels and take FN channels each (1, 2 or 4, FG * FN <= 64)
 // vol.base: the output goes into a split volume (fortis_conv3d_f32.cu), for a network's next layer
-struct ShortVol { float* base; long long plane; int pitch, Dq, Hq, Wq, pd, ph, pw; };
+struct ShortVol { float* base; long long plane; int pitch; VolMap map; };
 template <int V, int FN>
 __global__ void __launch_bounds__(256, 2) conv_short_kernel(const float* __restrict__ x, const float* __restrict__ wt,   // wt [tap][C][F]
                                                             const float* __restrict__ bias, const float* __restrict__ residual,
@@ -265,7 +265,9 @@ __global__ void __launch_bounds__(256, 2) conv_short_kernel(const float* __restr
     int on, od, oh, ow;
     voxel_at(g, (unsigned)v, &on, &od, &oh, &ow);
     if (vol.base) {
-      float* op = vol.base + ((((long long)on * vol.Dq + od + vol.pd) * vol.Hq + oh + vol.ph) * vol.Wq + ow + vol.pw) * vol.pitch + ff;
+      const long long row = vol_row(vol.map, on, od, oh, ow);
+      if (row < 0) continue;
+      float* op = vol.base + row * vol.pitch + ff;
 #pragma unroll
       for (int j = 0; j < FN; j += 4) {
         if (ff + j >= vol.pitch) break;
@@ -522,6 +524,12 @@ struct OpNet {
   std::vector<F32ConvW*> split;
   float* buf[2] = {nullptr, nullptr};
   long long cap = 0;
+  // Split volumes that a layer writes for the next one (vols[l]: the input of layer l), for the network extents vol_shape; their padding is
+  // zero from the allocation on.  vol_refused: there was no memory for one, not asked for again.
+  std::vector<float*> vols;
+  size_t vol_total = 0;
+  int vol_shape[3] = {0, 0, 0};
+  bool vol_refused = false;
 };
 
 void opnet_destroy(OpNet* m) {
@@ -531,6 +539,7 @@ void opnet_destroy(OpNet* m) {
   for (VolW* p : m->vw) vol_weights_free(p);
   for (F32ConvW* p : m->split) f32tc_conv_free(p);
   for (float* p : m->buf) cudaFree(p);
+  for (float* p : m->vols) cudaFree(p);
   delete m;
 }
 
@@ -590,6 +599,35 @@ static ConvGeom opnet_geom(const LayerHost& L, int N, int h, int w, int h2, int 
   return g;
 }
 
+// The split volume that layer l reads where the layer in front of it writes one, or null: the layer then packs its input.  Nothing is
+// allocated or freed while the stream is captured (the eager call in front has the volumes), and a network keeps at most 4 GB of them.
+static float* opnet_volume(OpNet* m, int l, size_t bytes, int N, int H, int W, cudaStream_t s) {
+  const int shape[3] = {N, H, W};
+  if (std::memcmp(m->vol_shape, shape, sizeof shape) != 0) {
+    if (stream_capturing(s)) return nullptr;
+    for (float* p : m->vols) cudaFree(p);                        // waits for the kernels in flight
+    m->vols.assign(m->meta.size(), nullptr);
+    m->vol_total = 0;
+    std::memcpy(m->vol_shape, shape, sizeof shape);
+  }
+  if (m->vols[l]) return m->vols[l];
+  if (m->vol_refused || m->vol_total + bytes > (4ULL << 30) || stream_capturing(s)) return nullptr;
+  if (!vol_alloc((void**)&m->vols[l], bytes)) { m->vol_refused = true; return nullptr; }
+  cudaMemsetAsync(m->vols[l], 0, bytes, s);
+  m->vol_total += bytes;
+  return m->vols[l];
+}
+
+// Does a layer read a split volume that the layer in front of it writes?  Where it would pack its input anyway, and where it is faster over
+// a volume that needs no packing: the layer in front then writes more, at 2.5 TB/s.
+static bool takes_written_volume(const ConvGeom& g) {
+  if (!vol_supported(g) || g_tc_test.conv_route == 2) return false;
+  if (g_tc_test.conv_route == 1 || !f32tc_conv_supported(g)) return true;
+  const VolGeom vg = vol_geom(g, g.pd, g.ph, vol_front_w(g));
+  const long long more = (long long)vol_bytes(vg, (g.C + 31) / 32 * 32) - 4LL * g.N * g.D * g.H * g.W * g.C;
+  return vol_kernel_cost(vg, g.F) + (more > 0 ? more / 2500 : 0) < f32tc_conv_cost(g);
+}
+
 // x (N, Cin, H, W) -> y (N, Cout, Ho, Wo)
 bool opnet_forward(OpNet* m, const float* x, float* y, int N, int H, int W, int* status, cudaStream_t s, std::string* err) {
   if ((long long)N * H * W <= 0) { if (err) *err = "2-D network: set the input extent (option conv_shape = N,1,H,W)"; return false; }
@@ -614,6 +652,7 @@ bool opnet_forward(OpNet* m, const float* x, float* y, int N, int H, int W, int*
   const float* src = x;
   VolSource pending;                      // pooling or upsampling left to the next layer
   pending.op = VolSource::PLAIN;
+  const float* written = nullptr;         // the split volume that the layer in front has written instead of an array
   int h = H, w = W;
   const int nl = (int)m->meta.size();
   for (int l = 0; l < nl; l++) {
@@ -625,7 +664,37 @@ bool opnet_forward(OpNet* m, const float* x, float* y, int N, int H, int W, int*
     const unsigned blocks = (unsigned)((nout + 255) / 256 < 148 * 16 ? (nout + 255) / 256 : 148 * 16);
     if (L.kind == LAYER_CONV2D) {
       const ConvGeom g = opnet_geom(L, N, h, w, h2, w2);
-      if (!conv_layer(pending.op || takes_volume(g) ? m->vw[l] : nullptr, m->split[l], m->wt[l], m->bias[l], src, pending.op ? &pending : nullptr, nullptr, dst, g, L.act, L.slope, status, s, true, err)) return false;
+      const VolGeom vg = vol_geom(g, g.pd, g.ph, vol_front_w(g));
+      const int pitch = (g.C + 31) / 32 * 32;
+      const float* vol = written;                                  // the layer's input as a split volume ...
+      bool pack = false;
+      if (!vol && m->vw[l] && (pending.op || takes_volume(g))) { vol = vol_workspace(vol_bytes(vg, pitch), s); pack = vol != nullptr; }
+      if (!vol && pending.op) { if (err) *err = "out of device memory for a convolution's input"; return false; }
+      const bool threads = !vol && m->split[l] && f32tc_conv_supported(g), shorts = !vol && !threads && short_supported(g);
+      VolOut o;                                                    // ... and its output as the next layer's, where that is a convolution too
+      std::memset(&o, 0, sizeof o);
+      int h3, w3;
+      if ((vol || shorts) && l + 1 < nl && m->meta[l + 1].kind == LAYER_CONV2D && m->vw[l + 1] && opnet_layer_shape(m->meta[l + 1], h2, w2, &h3, &w3)) {
+        const ConvGeom gn = opnet_geom(m->meta[l + 1], N, h2, w2, h3, w3);
+        if (takes_written_volume(gn)) {
+          const VolGeom vn = vol_geom(gn, gn.pd, gn.ph, vol_front_w(gn));
+          o.pitch = (gn.C + 31) / 32 * 32;
+          o.vol = opnet_volume(m, l + 1, vol_bytes(vn, o.pitch), N, H, W, s);
+          o.remap = true; o.next = vol_map(vn);
+          o.plane = (long long)(vol_bytes(vn, o.pitch) / 8);
+        }
+      }
+      written = o.vol;
+      if (!o.vol) { o.remap = false; o.y = dst; o.ys_n = g.ys_n; o.ys_d = g.ys_d; o.ys_h = g.ys_h; o.ys_w = g.ys_w; o.ys_c = g.ys_c; }
+      if (vol) {
+        const VolSource plain = {VolSource::PLAIN, 1, 1, 1, 1, g.xs_n, g.xs_d, g.xs_h, g.xs_w, g.xs_c};
+        if (pack) vol_pack(src, const_cast<float*>(vol), pitch, vg, pending.op ? pending : plain, s);
+        if (!vol_conv(m->vw[l], vol, pitch, vg, o, m->bias[l], L.act, L.slope, status, s, true, err)) return false;
+      } else if (shorts) {
+        launch_short(src, m->wt[l], m->bias[l], nullptr, dst, g, L.act, L.slope, ShortVol{o.vol, o.plane, o.pitch, o.next}, s);
+      } else if (!conv_layer(nullptr, m->split[l], m->wt[l], m->bias[l], src, nullptr, nullptr, dst, g, L.act, L.slope, status, s, true, err)) {
+        return false;
+      }
       pending.op = VolSource::PLAIN;
     } else {
       const bool pool = L.kind == LAYER_MAXPOOL2D;
@@ -820,7 +889,7 @@ static bool conv_forward_volumes(ConvModel* m, const float* x, float* y, int N, 
     if (l < nl - 1) { o.vol = m->buf[dst]; o.pitch = pitch; o.skip = (L.flags & LFLAG_ADD_SKIP) ? m->buf[skip] : nullptr; }
     else { o.y = y; set_strides(&o.ys_n, &o.ys_d, &o.ys_h, &o.ys_w, &o.ys_c, true, L.cout, D, H, W); }
     if (l == 0 && first_short) {
-      const ShortVol sv = {o.vol, vg.P * pitch, pitch, vg.Dq, vg.Hq, vg.Wq, pad, pad, pad_w};
+      const ShortVol sv = {o.vol, vg.P * pitch, pitch, vol_map(vg)};
       launch_short(x, m->wt[0], m->bias[0], nullptr, nullptr, g, L.act, L.slope, sv, s);
     } else {
       const float* in = cur < 0 ? nullptr : m->buf[cur];

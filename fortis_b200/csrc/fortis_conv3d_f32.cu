@@ -74,6 +74,7 @@ struct VolParams {
   const float* bias; int act; float slope; int F;
   // output: a split volume of the same grid (pitch: channels of a row) ...
   float* out; long long out_plane; int out_pitch; long long out_shift;
+  int remap; VolMap next;                      // ... or one of another grid, the next layer's, whose padding is zero already
   const float* skip;                           // the residual, a split volume like `out`
   // ... or a plain array, with a plain residual
   float* y; long long ys_n, ys_d, ys_h, ys_w, ys_c;
@@ -386,12 +387,13 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
       const uint32_t q0 = (uint32_t)(in_rows ? p : 0), q1 = q0 / (uint32_t)G.Wq, q2 = q1 / (uint32_t)G.Hq, q3 = q2 / (uint32_t)G.Dq;
       const int ow = (int)(q0 - q1 * G.Wq), oh = (int)(q1 - q2 * G.Hq), od = (int)(q2 - q3 * G.Dq), on = (int)q3;
       const bool live = in_rows && ow < G.Wo && oh < G.Ho && od < G.Do;
-      const uint32_t rows_mask = __ballot_sync(0xffffffffu, in_rows), live_mask = __ballot_sync(0xffffffffu, live);
+      const uint32_t live_mask = __ballot_sync(0xffffffffu, live);
       if (!wait(stash_full, tile_it & 1, VST_STASH_FULL)) break;
       if (P.out) {
+        // this lane's row in the output volume (fewer than 2^30), or -1
+        const int row_out = P.remap ? (live ? (int)vol_row(P.next, on, od, oh, ow) : -1) : in_rows ? (int)(p + P.out_shift) : -1;
         // lanes along a row: whole lines of the split volume
         const int c = lane % LPR, f = n0 + 4 * c;
-        const long long o0 = (p - lane + P.out_shift) * P.out_pitch + f;
         const bool inside = f < P.out_pitch;
         float b[4];
 #pragma unroll
@@ -399,8 +401,9 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
 #pragma unroll 2
         for (int i = 0; i < 32; i += RPI) {
           const int rr = i + lane / LPR;
-          const bool mine = inside && ((rows_mask >> rr) & 1u), lv = (live_mask >> rr) & 1u;
-          const long long o = o0 + (long long)rr * P.out_pitch;
+          const int row = __shfl_sync(0xffffffffu, row_out, rr);
+          const bool mine = inside && row >= 0, lv = (live_mask >> rr) & 1u;
+          const long long o = (long long)row * P.out_pitch + f;
           float4 sh = make_float4(0.f, 0.f, 0.f, 0.f), sl = sh;
           if (P.skip && lv && inside) { sh = ld_plain4(P.skip + o); sl = ld_plain4(P.skip + P.out_plane + o); }
           const float4 q = *reinterpret_cast<const float4*>(stash + rr * NT + ((c ^ (rr & 7)) << 2));
@@ -754,6 +757,8 @@ VolGeom vol_geom(const ConvGeom& c, int front_d, int front_h, int front_w) {
   return g;
 }
 
+VolMap vol_map(const VolGeom& g) { return VolMap{g.Dq, g.Hq, g.Wq, g.pd, g.ph, g.pw, g.sd, g.sh, g.sw, g.fd, g.fh, g.fw, g.P}; }
+
 int vol_front_w(const ConvGeom& c) { return vol_line(c.KW, c.sw, c.pw) ? 0 : c.pw; }
 
 size_t vol_bytes(const VolGeom& g, int pitch) { return (size_t)g.P * g.fd * g.fh * g.fw * pitch * 8; }
@@ -889,7 +894,7 @@ bool vol_conv(const VolW* w, const float* vol, int pitch, const VolGeom& g, cons
   const Pieces pc = pick_pieces(g, w->ntn);
   P.pieces = pc.n; P.pairs_piece = pc.pairs; P.rows = pc.rows; P.piece_stride = pc.stride;
   P.bias = bias; P.act = act; P.slope = slope; P.F = w->F;
-  P.out = o.vol; P.out_plane = g.P * o.pitch; P.out_pitch = o.pitch; P.out_shift = ((long long)g.pd * g.Hq + g.ph) * g.Wq + g.pw;
+  P.out = o.vol; P.remap = o.remap; P.next = o.next; P.out_plane = o.remap ? o.plane : g.P * o.pitch; P.out_pitch = o.pitch; P.out_shift = ((long long)g.pd * g.Hq + g.ph) * g.Wq + g.pw;
   P.skip = o.skip; P.y = o.y; P.ys_n = o.ys_n; P.ys_d = o.ys_d; P.ys_h = o.ys_h; P.ys_w = o.ys_w; P.ys_c = o.ys_c;
   P.res = o.res; P.rs_n = o.rs_n; P.rs_d = o.rs_d; P.rs_h = o.rs_h; P.rs_w = o.rs_w; P.rs_c = o.rs_c;
   P.status = status;

@@ -7,6 +7,7 @@
 
 #include <cstdint>
 
+#include "fortis_kernels.h"
 #include "fortis_plan.h"
 
 namespace fortis {
@@ -25,6 +26,19 @@ __device__ __forceinline__ void vol_split(float x, float& hi, float& lo) {
   asm("cvt.rna.satfinite.tf32.f32 %0, %1;" : "=r"(h) : "f"(x));
   hi = __uint_as_float(h);
   lo = (x - hi) * 1024.f;
+}
+
+// the row of a split volume for position (n, d, h, w) of the array that it holds, -1 where no tap reads that position
+__device__ __forceinline__ long long vol_row(const VolMap& m, int n, int d, int h, int w) {
+  d += m.pd; h += m.ph; w += m.pw;
+  long long row = 0;
+  if ((m.sd | m.sh | m.sw) != 1) {
+    const int rd = d % m.sd, rh = h % m.sh, rw = w % m.sw;
+    if (rd >= m.fd || rh >= m.fh || rw >= m.fw) return -1;
+    row = ((rd * m.fh + rh) * m.fw + rw) * m.P;
+    d /= m.sd; h /= m.sh; w /= m.sw;
+  }
+  return row + (((long long)n * m.Dq + d) * m.Hq + h) * m.Wq + w;
 }
 
 struct IoPlanDev {

@@ -213,6 +213,9 @@ struct VolGeom {
   long long P;                                // rows of one phase
 };
 VolGeom vol_geom(const ConvGeom& c, int front_d, int front_h, int front_w);
+// where an output (n, d, h, w) of one layer lies in the split volume that the next layer reads (vol_row, fortis_device.cuh)
+struct VolMap { int Dq, Hq, Wq, pd, ph, pw, sd, sh, sw, fd, fh, fw; long long P; };
+VolMap vol_map(const VolGeom& g);
 int vol_front_w(const ConvGeom& c);                            // zero positions a layer needs in front of a line
 bool vol_supported(const ConvGeom& c);
 // estimated device times, ns: of a layer over a volume, of packing its input, and of both
@@ -233,7 +236,8 @@ struct VolSource {
 };
 void vol_pack(const float* x, float* vol, int pitch, const VolGeom& g, const VolSource& src, cudaStream_t s);
 struct VolOut {
-  float* vol; int pitch; const float* skip;                    // a split volume of the same grid, the residual likewise, or ...
+  float* vol; int pitch; const float* skip;                    // a split volume of the same grid, the residual likewise, or, with
+  bool remap; VolMap next; long long plane;                    // `remap`, one of another grid (whose planes are `plane` apart), or ...
   float* y; long long ys_n, ys_d, ys_h, ys_w, ys_c;            // ... a plain array ...
   const float* res; long long rs_n, rs_d, rs_h, rs_w, rs_c;    // ... with a plain residual
 };
