@@ -31,10 +31,15 @@
 //  * warp 0: TMA (both CTAs), warp 1: MMA (leader only), then two groups of eight epilogue warps that take alternate tiles, group g
 //    the ones in accumulator g: a tile's epilogue is a chain of waits (accumulator, row exchange, residual, stores) longer than its
 //    MMAs, and two of them overlap.  In a group two warps share a lane quadrant (thread = one voxel row x 32 channels, 16 at a
-//    time): row neighbours by warp shuffle, the rows on either side of a warp boundary through shared memory; bias + residual row
-//    (prefetched one tile ahead) + LeakyReLU -> bf16 -> row store.  The accumulator is handed back with a RELAXED cluster-scope
-//    arrive: a release would first drain the thread's outstanding global stores (measured ~1700 cycles per tile).
-//    8 x 33^3, one layer of 64 channels without / with a residual: 62 / 74.5 us with one group, 58 / 70 with two.
+//    time): row neighbours by warp shuffle, the rows on either side of a warp boundary through shared memory; bias + residual +
+//    LeakyReLU -> bf16.  The accumulator is handed back with a RELAXED cluster-scope arrive: a release would first drain the
+//    thread's outstanding global stores (measured ~1700 cycles per tile).
+//  * STAGED: the residual comes and the output goes by tile copies through 8 KB of shared memory per group and half of the
+//    channels.  As the threads' own loads and stores, 16 bytes of 32 rows each, they take the data path that shared memory and L1
+//    have in common 1024 clk a tile each, beside the MMAs' operands (2016 clk) and the copies (600).  The buffers cost a quarter of
+//    the activation ring; where that leaves fewer than a tile's three stages (W above 42), and in the last layer, threads store.
+//    8 x 33^3, one layer of 64 channels without / with a residual: 62 / 74.5 us with one group, 58 / 70 with two, 54 / 54 staged
+//    (its MMAs 35).
 //
 // First layer: the fp32 NDHWC input is packed into its own padded bf16 volume with channels >= Cin zero, and the
 // weights are padded the same way, so the layer is the same GEMM with one k step per group instead of four.
@@ -64,14 +69,19 @@ namespace {
 constexpr int kC = 64;                       // channels of the tensor-core layers
 constexpr int kTile = 128;                   // rows computed per tile (the MMA's M)
 constexpr int kTileOut = kTile - 2;          // rows written per tile (the first and last computed rows only feed their neighbours)
-constexpr int kRingBytes = 108 * 1024;       // activation ring: nstages stages of (128 + 2 (W+2)) rows each
+// activation ring: nstages stages of (128 + 2 (W+2)) rows each; less of it where outputs and residuals are staged
+constexpr int kRingBytes = 108 * 1024, kRingStaged = 82 * 1024;
+// Staged: a group's two halves have 126 rows of 32 channels each (64 bytes, 64-byte swizzle) in shared memory, through which the
+// residual comes and the output goes by tile copies
+constexpr int kOutRow = 64, kOutBytes = kTile * kOutRow, kOutAll = 4 * kOutBytes;
 constexpr int kMaxStages = 7;
 constexpr int kXch = 2 * 4 * kC;             // floats exchanged between a group's warps: [up | down][quadrant][channel] ...
-constexpr int kXchBytes = 2 * 2 * kXch * 4;  // ... for [group][parity of its tiles]
+constexpr int kXchBytes = 2 * 2 * kXch * 4;  // ... for [group][parity of its tiles]; staged: one buffer, a tile has two exchanges
 constexpr int kResW = 9 * 96 * kC * 2;       // 108 KB: this CTA's half of all 27 weight tiles, resident for the whole kernel
 constexpr int kConvThreads = 576;            // TMA warp, MMA warp, two groups of 8 epilogue warps (two per TMEM lane quadrant)
 constexpr int kConvSmem = kResW + kRingBytes + 256 + kXchBytes + kC * 4;
-static_assert(kConvSmem <= 227 * 1024, "shared memory");
+constexpr int kConvSmemStaged = kResW + kRingStaged + kOutAll + 256 + kXchBytes / 2 + kC * 4;
+static_assert(kConvSmem <= 227 * 1024 && kConvSmemStaged <= 227 * 1024, "shared memory");
 constexpr int kAccStride = 256;              // TMEM columns between the two accumulators (each 3 * NOUT wide)
 // the pair's M = 256; operand format code 1 = bf16, 0 = IEEE half (bits 7-9 for A, 10-12 for B)
 template <int NOUT, bool F16> struct ConvIdesc {
@@ -88,7 +98,17 @@ template <bool F16> __device__ __forceinline__ float2 cunpack16(uint32_t u) {
   else return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u));
 }
 constexpr int kEdgeC = 16;                   // first layer: input channels kept; last layer: output channels computed
-enum { CST_FULL = 11, CST_EMPTY = 12, CST_ACC_FULL = 13, CST_ACC_EMPTY = 14, CST_WEIGHTS = 15, CST_ALIGN = 16 };
+enum { CST_FULL = 11, CST_EMPTY = 12, CST_ACC_FULL = 13, CST_ACC_EMPTY = 14, CST_WEIGHTS = 15, CST_ALIGN = 16, CST_RESIDUAL = 17 };
+
+// the calling thread's tile copies (no election) and their completion
+__device__ __forceinline__ void tile_store_thread(const CUtensorMap* map, uint32_t src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];\n\tcp.async.bulk.commit_group;"
+               ::"l"(map), "r"(x), "r"(y), "r"(src) : "memory");
+}
+__device__ __forceinline__ void tile_load_thread(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+               ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
 
 struct ConvTcParams {
   CUtensorMap amap;            // the activation allocation [rows][64] bf16, box 64 x box_rows
@@ -96,6 +116,7 @@ struct ConvTcParams {
   int box_rows, nbox;          // a stage is loaded as nbox boxes of box_rows rows
   int front;                   // zero rows in front of row 0 of the volume inside the allocation
   CUtensorMap wmap;            // weights [27 * NOUT (tap, cout)][64 cin] bf16, box 64 x 3 NOUT
+  CUtensorMap omap, smap;      // staged: the output and the residual [rows][64], box 32 x 126
   const float* bias;           // [64] (zero beyond the layer's real outputs)
   const __nv_bfloat16* skip;   // [P][64] or null
   __nv_bfloat16* out;          // [P][64]
@@ -121,7 +142,7 @@ __device__ __forceinline__ void cprof_add(long long* prof, int slot, long long* 
 // KSTEPS: 16-wide k steps issued per (kd, kh) group (4 = all 64 input channels, 1 = only the first 16);  NOUT: output
 // channels (weight rows per tap);  LAST: write fp32 NDHWC instead of the padded bf16 volume.
 // Launched as clusters of two CTAs (cta_group::2): the leader's MMA warp issues for both.
-template <int KSTEPS, int NOUT, bool LAST, bool F16>
+template <int KSTEPS, int NOUT, bool LAST, bool F16, bool STAGED>
 __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid_constant__ ConvTcParams P) {
   constexpr uint32_t kIdescN = ConvIdesc<NOUT, F16>::value;            // M = 256 (128 rows per CTA), N = 3 * NOUT per group
   constexpr int kWLoads = 9;                                      // weight tiles: one per (kd, kh) group
@@ -134,15 +155,15 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
     return;
   }
   const uint32_t ring = base + kResW;
-  const uint32_t bars = ring + kRingBytes;
+  const uint32_t outs = ring + kRingStaged, bars = STAGED ? outs + kOutAll : ring + kRingBytes;
   // barrier block (256 B): full [0,56) empty [56,112) acc_full [112,128) acc_empty [128,144) weights [144,152)
-  // tmem base 160, abort flag 164
+  // tmem base 160, abort flag 164, residual [168,200)
   const uint32_t bar_full = bars, bar_empty = bars + 56, bar_acc_full = bars + 112, bar_acc_empty = bars + 128, bar_w = bars + 144;
-  uint8_t* barp = smem + kResW + kRingBytes;
+  uint8_t* barp = smem + (bars - base);
   uint32_t* tmem_slot = (uint32_t*)(barp + 160);
   volatile int* abort_flag = (volatile int*)(barp + 164);
   float* xch = (float*)(barp + 256);
-  float* bias_s = (float*)(barp + 256 + kXchBytes);
+  float* bias_s = (float*)(barp + 256 + (STAGED ? kXchBytes / 2 : kXchBytes));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t crank = cluster_ctarank();
   const long long ntiles = (P.P + kTileOut - 1) / kTileOut;
@@ -154,6 +175,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
     for (int s = 0; s < kMaxStages; s++) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); }
     for (int b = 0; b < 2; b++) { mbar_init(bar_acc_full + 8 * b, 1); mbar_init(bar_acc_empty + 8 * b, 16); }   // a group's 8 warps per CTA
     mbar_init(bar_w, 1);
+    for (int u = 0; u < 4; u++) mbar_init(bars + 168 + 8 * u, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -272,24 +294,47 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
     bool writes, interior;
     locate(pair0 + group * pair_step, p, writes, interior, wp, hp, dp, n_);
     // this warp's half of the residual row of the thread's voxel, always fetched one tile of the group ahead
-    uint4 sk[CW / 8];
-    bool use_skip = !LAST && P.skip != nullptr && interior;
-    if (use_skip) {
+    uint4 sk[STAGED ? 1 : CW / 8];
+    bool use_skip = !LAST && !STAGED && P.skip != nullptr && interior;
+    if constexpr (!STAGED) {
+      if (use_skip) {
 #pragma unroll
-      for (int j = 0; j < CW / 8; j++) sk[j] = ld_global(reinterpret_cast<const uint4*>(P.skip + (size_t)p * kC + c0) + j);
+        for (int j = 0; j < CW / 8; j++) sk[j] = ld_global(reinterpret_cast<const uint4*>(P.skip + (size_t)p * kC + c0) + j);
+      }
     }
+    // staged: this half's buffer, the thread's row there (rows 1 to 126 of the tile; 16-byte piece j at j ^ (row / 2 % 4)), and the
+    // thread that copies for the half's four warps
+    const int unit = 2 * group + half, orow = quad * 32 + lane - 1;
+    const uint32_t out_s = outs + unit * kOutBytes, res_bar = bars + 168 + 8 * unit;
+    uint8_t* out_row = smem + (out_s - base) + orow * kOutRow;
+    const bool copies = STAGED && quad == 0 && lane == 0;
+    auto unit_sync = [&]() {
+      if (group == 0) {
+        if (half == 0) asm volatile("bar.sync 1, 128;" ::: "memory"); else asm volatile("bar.sync 2, 128;" ::: "memory");
+      } else {
+        if (half == 0) asm volatile("bar.sync 3, 128;" ::: "memory"); else asm volatile("bar.sync 4, 128;" ::: "memory");
+      }
+    };
     uint32_t it = 0;
     for (long long tp = pair0 + group * pair_step; tp < npairs; tp += 2 * pair_step, it++) {
       uint32_t np, nwp, nhp, ndp, nn;
       bool nwrites, ninterior;
       locate(tp + 2 * pair_step, np, nwrites, ninterior, nwp, nhp, ndp, nn);
-      const bool nuse_skip = !LAST && P.skip != nullptr && ninterior;
+      const bool nuse_skip = !LAST && !STAGED && P.skip != nullptr && ninterior;
+      if (copies) {
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");        // the last tile's rows have left the buffer
+        if (P.skip) {
+          mbar_arrive_expect_tx_thread(res_bar, kTileOut * kOutRow);
+          tile_load_thread(out_s, &P.smap, c0, (int)((2 * tp + crank) * kTileOut) + P.front, res_bar);
+        }
+      }
+      __syncwarp();
       cprof_add(P.prof, 10, &pt, pw);
       mbar_wait(acc_full, it & 1, abort_flag, P.status, CST_ACC_FULL, P.wait_limit);
       cprof_add(P.prof, 8, &pt, pw);
       tc_fence_after();
       const uint32_t accb = lane_addr + group * kAccStride + c0;
-      float* xu = xch + (2 * group + (it & 1)) * kXch + c0;        // kw = 0 partials of each quadrant's last row
+      float* xu = xch + (STAGED ? group : 2 * group + (it & 1)) * kXch + c0;   // kw = 0 partials of each quadrant's last row
       float* xd = xu + 4 * kC;                                     // kw = 2 partials of each quadrant's first row
 #pragma unroll
       for (int c = 0; c < CW; c += 16) {
@@ -308,8 +353,8 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
         if (!active) continue;
         // The rows on either side of a warp boundary go through shared memory: the last lane publishes its kw = 0 partials and
         // takes the previous quadrant's in their place (the first lane likewise with kw = 2), so that a rotation by one lane
-        // brings every lane its neighbour's.  (The buffer alternates, so one barrier among the four warps that hold the same
-        // channels is enough.)
+        // brings every lane its neighbour's.  (The buffer alternates, or is read again only behind the tile's other exchange, so one
+        // barrier among the four warps that hold the same channels is enough.)
         if (lane == 31) {
 #pragma unroll
           for (int i = 0; i < 16; i += 4) *reinterpret_cast<uint4*>(xu + quad * kC + c + i) = make_uint4(a0[i], a0[i + 1], a0[i + 2], a0[i + 3]);
@@ -318,11 +363,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
 #pragma unroll
           for (int i = 0; i < 16; i += 4) *reinterpret_cast<uint4*>(xd + quad * kC + c + i) = make_uint4(a2[i], a2[i + 1], a2[i + 2], a2[i + 3]);
         }
-        if (group == 0) {
-          if (half == 0) asm volatile("bar.sync 1, 128;" ::: "memory"); else asm volatile("bar.sync 2, 128;" ::: "memory");
-        } else {
-          if (half == 0) asm volatile("bar.sync 3, 128;" ::: "memory"); else asm volatile("bar.sync 4, 128;" ::: "memory");
-        }
+        unit_sync();
         if (lane == 31 && quad > 0) {
 #pragma unroll
           for (int i = 0; i < 16; i += 4) {
@@ -357,6 +398,30 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
             for (int f = 0; f < 16; f++)
               if (f < P.F) dst[f] = fmaxf(v[f], v[f] * P.slope);
           }
+        } else if constexpr (STAGED) {
+          // (every row of the buffer but 126 and 127: rows behind the volume are zero, as what lies there is)
+          const bool mine = orow >= 0 && orow < kTileOut;
+          if (P.skip && c == 0) mbar_wait(res_bar, it & 1, abort_flag, P.status, CST_RESIDUAL, P.wait_limit);
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            uint4* piece = reinterpret_cast<uint4*>(out_row + (((c / 8 + h) ^ ((orow >> 1) & 3)) << 4));
+            uint32_t pk[4];
+            uint4 rv = make_uint4(0u, 0u, 0u, 0u);
+            if (P.skip && mine) rv = *piece;
+            const uint32_t r2[4] = {rv.x, rv.y, rv.z, rv.w};
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+              float x0 = v[8 * h + 2 * e], x1 = v[8 * h + 2 * e + 1];
+              if (P.skip) { const float2 f = cunpack16<F16>(r2[e]); x0 += f.x; x1 += f.y; }
+              pk[e] = interior ? cpack16<F16>(fmaxf(x0, x0 * P.slope), fmaxf(x1, x1 * P.slope)) : 0u;
+            }
+            if (mine) *piece = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+          }
+          if (c + 16 == CW) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the copy reads what these threads have written
+            unit_sync();
+            if (copies) tile_store_thread(&P.omap, out_s, c0, (int)((2 * tp + crank) * kTileOut) + P.front);
+          }
         } else {
           if (use_skip) {
 #pragma unroll
@@ -388,6 +453,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
       }
       p = np; writes = nwrites; interior = ninterior; wp = nwp; hp = nhp; dp = ndp; n_ = nn; use_skip = nuse_skip;
     }
+    if (copies) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");     // the rows are written before the grid's dependents go on
   }
   tc_fence_before();
   __syncthreads();
@@ -437,26 +503,26 @@ EncodeTiledFn conv_encode_fn() {
   return fn;
 }
 
-bool make_map(CUtensorMap* m, void* base, long long rows, int box_rows) {
+bool make_map(CUtensorMap* m, void* base, long long rows, int box_rows, bool half_rows = false) {
   EncodeTiledFn enc = conv_encode_fn();
   if (!enc) return false;
   const cuuint64_t dims[2] = {(cuuint64_t)kC, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)kC * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)kC, (cuuint32_t)box_rows};
+  const cuuint32_t box[2] = {(cuuint32_t)(half_rows ? kC / 2 : kC), (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+             half_rows ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // geometry of the activation ring for a volume whose padded W extent is Wp: a stage holds 128 + 2 Wp rows, loaded as
 // nbox boxes of box_rows (<= 256, multiple of 8) rows
 struct RingGeom { int stage_bytes, nstages, box_rows, nbox; };
-bool ring_geometry(int Wp, RingGeom* g) {
+bool ring_geometry(int Wp, RingGeom* g, int ring_bytes = kRingBytes) {
   const int R = kTile + 2 * Wp;
   g->nbox = (R + 255) / 256;
   g->box_rows = (((R + g->nbox - 1) / g->nbox) + 7) / 8 * 8;
   g->stage_bytes = ((g->nbox * g->box_rows * kC * 2) + 1023) / 1024 * 1024;
-  g->nstages = kRingBytes / g->stage_bytes;
+  g->nstages = ring_bytes / g->stage_bytes;
   if (g->nstages > kMaxStages) g->nstages = kMaxStages;
   return g->nstages >= 2;
 }
@@ -480,13 +546,21 @@ float slope_of(const LayerHost& L) { return L.act == ACT_NONE ? 1.f : L.act == A
 
 }  // namespace
 
+typedef void (*ConvTcKernel)(ConvTcParams);
+// [fp16][first, hidden, last layer, staged first, staged hidden layer]
+const ConvTcKernel kConvKernels[2][5] = {
+    {conv3d_tc_kernel<1, kC, false, false, false>, conv3d_tc_kernel<4, kC, false, false, false>, conv3d_tc_kernel<4, kEdgeC, true, false, false>,
+     conv3d_tc_kernel<1, kC, false, false, true>, conv3d_tc_kernel<4, kC, false, false, true>},
+    {conv3d_tc_kernel<1, kC, false, true, false>, conv3d_tc_kernel<4, kC, false, true, false>, conv3d_tc_kernel<4, kEdgeC, true, true, false>,
+     conv3d_tc_kernel<1, kC, false, true, true>, conv3d_tc_kernel<4, kC, false, true, true>}};
+
 struct ConvTcModel {
   std::vector<LayerHost> meta;
   std::vector<void*> w; std::vector<float*> b;             // per layer: bf16 [27 * rows][64] (rows = 64, last layer 16), fp32 bias [64]
   std::vector<CUtensorMap> wmaps;
   __nv_bfloat16* buf[4] = {nullptr, nullptr, nullptr, nullptr};   // three rotating activation volumes + the packed input (allocations)
   long long front = 0;                                            // zero rows in front of each volume inside its allocation
-  CUtensorMap amaps[4];
+  CUtensorMap amaps[4], omaps[4];                                 // operand tiles; output tiles
   long long P = 0;
   int shape[4] = {0, 0, 0, 0};
   int* status = nullptr;
@@ -554,13 +628,9 @@ ConvTcModel* conv_tc_create(const ModelHost& M, bool f16, std::string* err) {
   if (cudaMalloc(&m->status, sizeof(int)) != cudaSuccess) return fail("out of device memory");
   cudaMemset(m->status, 0, sizeof(int));
   const cudaFuncAttribute att = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  if (cudaFuncSetAttribute(conv3d_tc_kernel<4, kC, false, false>, att, kConvSmem) != cudaSuccess ||
-      cudaFuncSetAttribute(conv3d_tc_kernel<1, kC, false, false>, att, kConvSmem) != cudaSuccess ||
-      cudaFuncSetAttribute(conv3d_tc_kernel<4, kEdgeC, true, false>, att, kConvSmem) != cudaSuccess ||
-      cudaFuncSetAttribute(conv3d_tc_kernel<4, kC, false, true>, att, kConvSmem) != cudaSuccess ||
-      cudaFuncSetAttribute(conv3d_tc_kernel<1, kC, false, true>, att, kConvSmem) != cudaSuccess ||
-      cudaFuncSetAttribute(conv3d_tc_kernel<4, kEdgeC, true, true>, att, kConvSmem) != cudaSuccess)
-    return fail("cannot reserve shared memory for the tensor-core conv kernel");
+  for (const ConvTcKernel* k : {kConvKernels[0], kConvKernels[1]})
+    for (int i = 0; i < 5; i++)
+      if (cudaFuncSetAttribute(k[i], att, i < 3 ? kConvSmem : kConvSmemStaged) != cudaSuccess) return fail("cannot reserve shared memory for the tensor-core conv kernel");
   return m;
 }
 
@@ -580,12 +650,14 @@ bool conv_tc_forward(ConvTcModel* m, const float* x, float* y, int N, int D, int
       cudaMemsetAsync(m->buf[b], 0, (size_t)rows * kC * 2, s);     // padding and border must be zero before the first layer writes the interior
       RingGeom g;
       if (!ring_geometry(W + 2, &g)) { if (err) *err = "conv3d bf16 path: W too large for the shared-memory activation ring (use precision=fp32)"; return false; }
-      if (!make_map(&m->amaps[b], m->buf[b], rows, g.box_rows)) { if (err) *err = "cuTensorMapEncodeTiled failed for conv activations"; return false; }
+      if (!make_map(&m->amaps[b], m->buf[b], rows, g.box_rows) || !make_map(&m->omaps[b], m->buf[b], rows, kTileOut, true)) { if (err) *err = "cuTensorMapEncodeTiled failed for conv activations"; return false; }
     }
     m->P = P; m->shape[0] = N; m->shape[1] = D; m->shape[2] = H; m->shape[3] = W;
   }
-  RingGeom geom;
-  ring_geometry(W + 2, &geom);
+  // Outputs and residuals go through shared memory where that leaves the activations three stages, a tile's (W up to 42)
+  RingGeom geom, direct;
+  const bool staged = ring_geometry(W + 2, &geom, kRingStaged) && geom.nstages >= 3;
+  ring_geometry(W + 2, &direct);
   const int nl = (int)m->meta.size();
   int sms = 148, dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -599,7 +671,7 @@ bool conv_tc_forward(ConvTcModel* m, const float* x, float* y, int N, int D, int
   const int max_pairs = sms / 2 > 0 ? sms / 2 : 1;
   const int grid = 2 * (int)(npairs < max_pairs ? npairs : max_pairs);          // clusters of two CTAs
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(kConvThreads); cfg.dynamicSmemBytes = kConvSmem; cfg.stream = s;
+  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(kConvThreads); cfg.stream = s;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
@@ -622,16 +694,16 @@ bool conv_tc_forward(ConvTcModel* m, const float* x, float* y, int N, int D, int
     P_.amap = m->amaps[cur]; P_.wmap = m->wmaps[l]; P_.bias = m->b[l];
     P_.skip = (L.flags & LFLAG_ADD_SKIP) ? m->buf[skip] + m->front * kC : nullptr;
     P_.out = m->buf[dst] + m->front * kC; P_.y = y; P_.F = L.cout; P_.front = (int)m->front;
-    P_.stage_bytes = geom.stage_bytes; P_.nstages = geom.nstages; P_.box_rows = geom.box_rows; P_.nbox = geom.nbox;
+    const bool st = staged && l < nl - 1;
+    const RingGeom& rg = st ? geom : direct;
+    P_.stage_bytes = rg.stage_bytes; P_.nstages = rg.nstages; P_.box_rows = rg.box_rows; P_.nbox = rg.nbox;
+    P_.omap = m->omaps[dst];
+    if (L.flags & LFLAG_ADD_SKIP) P_.smap = m->omaps[skip];
+    cfg.dynamicSmemBytes = st ? kConvSmemStaged : kConvSmem;
     P_.wait_limit = g_tc_test.wait_limit ? g_tc_test.wait_limit : kWaitLimit;
     P_.test_skip_stage = g_tc_test.skip_stage;
     P_.D = D; P_.H = H; P_.W = W; P_.P = P; P_.slope = slope_of(L); P_.status = m->status; P_.prof = (want_prof && l == 2) ? dprof : nullptr;
-    const cudaError_t le = m->f16 ? (l == nl - 1 ? cudaLaunchKernelEx(&cfg, conv3d_tc_kernel<4, kEdgeC, true, true>, P_)
-                                     : l == 0    ? cudaLaunchKernelEx(&cfg, conv3d_tc_kernel<1, kC, false, true>, P_)
-                                                 : cudaLaunchKernelEx(&cfg, conv3d_tc_kernel<4, kC, false, true>, P_))
-                                  : (l == nl - 1 ? cudaLaunchKernelEx(&cfg, conv3d_tc_kernel<4, kEdgeC, true, false>, P_)
-                                     : l == 0    ? cudaLaunchKernelEx(&cfg, conv3d_tc_kernel<1, kC, false, false>, P_)
-                                                 : cudaLaunchKernelEx(&cfg, conv3d_tc_kernel<4, kC, false, false>, P_));
+    const cudaError_t le = cudaLaunchKernelEx(&cfg, kConvKernels[m->f16][l == nl - 1 ? 2 : (l == 0 ? 0 : 1) + (st ? 3 : 0)], P_);
     if (le != cudaSuccess) { if (err) *err = std::string("tensor-core conv launch: ") + cudaGetErrorString(le); return false; }
     if (L.flags & LFLAG_SAVE_SKIP) skip = dst;
     cur = dst;
