@@ -618,23 +618,27 @@ __global__ void __launch_bounds__(256) pack_volume_kernel(const float* __restric
 #pragma unroll
   for (int i = 0; i < 4; i++) o[i] = pos[i * 32 + lane];
   float v[4][4];
+  // one value of each of the thread's 16 outputs, all in flight together
+  auto load = [&](long long off, float (&t)[4][4]) {
 #pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int c = c0 + warp * 4 + k;
-    const float* p = x + (long long)c * src.xs_c;
+    for (int k = 0; k < 4; k++) {
+      const int c = c0 + warp * 4 + k;
+      const float* p = x + (long long)c * src.xs_c + off;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      v[k][i] = 0.f;
-      if (o[i] >= 0 && c < g.C) {
-        if constexpr (OP != VolSource::MAXPOOL) v[k][i] = __ldg(p + o[i]);
-        else {
-          float m = -INFINITY;
-          for (int a = 0; a < src.kh; a++)
-            for (int b = 0; b < src.kw; b++) m = max_nan(m, __ldg(p + o[i] + a * src.xs_h + b * src.xs_w));
-          v[k][i] = m;
-        }
-      }
+      for (int i = 0; i < 4; i++) t[k][i] = o[i] >= 0 && c < g.C ? __ldg(p + o[i]) : 0.f;
     }
+  };
+  load(0, v);
+  if constexpr (OP == VolSource::MAXPOOL) {
+    for (int a = 0; a < src.kh; a++)
+      for (int b = a == 0 ? 1 : 0; b < src.kw; b++) {
+        float t[4][4];
+        load(a * src.xs_h + b * src.xs_w, t);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+          for (int i = 0; i < 4; i++) v[k][i] = max_nan(v[k][i], t[k][i]);
+      }
   }
 #pragma unroll
   for (int k = 0; k < 4; k++)
