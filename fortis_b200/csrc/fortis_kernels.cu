@@ -31,13 +31,28 @@ __global__ void __launch_bounds__(256) gather_kernel(const IoPlanDev* __restrict
       row_to_pos(g, row, &ci, &cj, &kk);
       double sc[kMaxScalars];
       if (P->nscalars) load_scalars(*P, T, ci, cj, kk, sc);
-      for (int q = warp; q < n; q += 8) tile[lane * ld + q] = gather_value(*P, slots[q], T, q, ci, cj, kk, sc);
+      if (P->has_prog) {
+        for (int q = warp; q < n; q += 8) tile[lane * ld + q] = gather_value(*P, slots[q], T, q, ci, cj, kk, sc);
+      } else {
+        // eight slots at a time, their table entries and then their values in flight together: one after another, 244 slots of a
+        // few rows take 30 times both latencies
+        for (int q0 = warp; q0 < n; q0 += 64) {
+          Access a[8];
+          float v[8];
+#pragma unroll
+          for (int j = 0; j < 8; j++) a[j] = slots[q0 + 8 * j < n ? q0 + 8 * j : q0];
+#pragma unroll
+          for (int j = 0; j < 8; j++) v[j] = (float)load_elem(T, a[j], access_offset(a[j], ci, cj, kk));
+#pragma unroll
+          for (int j = 0; j < 8; j++)
+            if (q0 + 8 * j < n) tile[lane * ld + q0 + 8 * j] = v[j];
+        }
+      }
     }
     __syncthreads();
-    const long long rows_here = min((long long)32, nrows - r0);
-    const long long total = rows_here * n;
+    const unsigned total = (unsigned)min((long long)32, nrows - r0) * n;
     float* dst = X + r0 * n;
-    for (long long e = threadIdx.x; e < total; e += 256) dst[e] = tile[(e / n) * ld + (e % n)];
+    for (unsigned e = threadIdx.x; e < total; e += 256) { const unsigned r = e / n; dst[e] = tile[r * ld + (e - r * n)]; }
     __syncthreads();
   }
 }
@@ -55,10 +70,9 @@ __global__ void __launch_bounds__(256) scatter_kernel(const IoPlanDev* __restric
   const long long nrows = g.count * g.nk;
   double csum = 0.0;
   for (long long r0 = (long long)blockIdx.x * 32; r0 < nrows; r0 += (long long)gridDim.x * 32) {
-    const long long rows_here = min((long long)32, nrows - r0);
-    const long long total = rows_here * n;
+    const unsigned total = (unsigned)min((long long)32, nrows - r0) * n;
     const float* src = Y + r0 * n;
-    for (long long e = threadIdx.x; e < total; e += 256) tile[(e / n) * ld + (e % n)] = src[e];
+    for (unsigned e = threadIdx.x; e < total; e += 256) { const unsigned r = e / n; tile[r * ld + (e - r * n)] = src[e]; }
     __syncthreads();
     const long long row = r0 + lane;
     if (row < nrows) {
@@ -66,11 +80,17 @@ __global__ void __launch_bounds__(256) scatter_kernel(const IoPlanDev* __restric
       row_to_pos(g, row, &ci, &cj, &kk);
       double sc[kMaxScalars];
       if (P->nscalars) load_scalars(*P, T, ci, cj, kk, sc);
-      for (int s = warp; s < P->nstores; s += 8) {
-        const StoreTarget st = stores[s];
-        const double v = scatter_value(*P, T, st.slot, tile[lane * ld + st.slot], sc);
-        store_elem(T, st.a, access_offset(st.a, ci, cj, kk), v);
-        csum += st.a.elt == 0 ? (double)(float)v : v;
+      for (int s0 = warp; s0 < P->nstores; s0 += 32) {           // four table entries in flight, as in the gather
+        StoreTarget st[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) st[j] = stores[s0 + 8 * j < P->nstores ? s0 + 8 * j : s0];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          if (s0 + 8 * j >= P->nstores) break;
+          const double v = scatter_value(*P, T, st[j].slot, tile[lane * ld + st[j].slot], sc);
+          store_elem(T, st[j].a, access_offset(st[j].a, ci, cj, kk), v);
+          csum += st[j].a.elt == 0 ? (double)(float)v : v;
+        }
       }
     }
     __syncthreads();
@@ -240,9 +260,153 @@ __global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict
   }
 }
 
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {      // two IEEE multiply-adds
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
+      "l"(*reinterpret_cast<unsigned long long*>(&c)));
+  return *reinterpret_cast<float2*>(&d);
+}
+
+// The same layer for few rows (up to 511 of a program's fp32 calls) and small matrices, where the tiles above leave most SMs idle and
+// their warps wait for one load after another.  A block of eight warps owns 4 TM rows x 8 TN features and the warps split K: warp w
+// takes the chunks of KC inputs w, w + 8, ... through two stages of its own (asynchronous copies, no block barrier), every lane TM x TN
+// outputs with the even and the odd k in the two halves of a packed FMA, and the eight sums of an output are added in the order of the
+// warps.  Both operands keep k fastest in shared memory, rows KC + 4 floats apart: the sixteen-byte reads of the eight feature lanes and
+// the four row lanes meet no bank twice.  (Sixteen sums of K/16 products each instead of one of K: nearer to the exact sum.)
+// Bound: the latency of the loads and of the reduction for few tiles, FMA issue for many (linear_tile: both sides measured).
+template <int TM, int TN, int KC>
+__global__ void __launch_bounds__(256, 2) linear_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+                                                             float* __restrict__ C, long long M, int N, int K, int act, float slope,
+                                                             const float* __restrict__ in_div, const float* __restrict__ out_mul,
+                                                             const float* __restrict__ relu_mask, int vec) {
+  constexpr int BM = 4 * TM, BN = 8 * TN, LD = KC + 4, kStage = (BM + BN) * LD, kPieces = KC / 4;
+  static_assert((BM + BN) * kPieces % 32 == 0, "whole warps of pieces");
+  extern __shared__ __align__(16) float rows_smem[];         // [warp][2][BM + BN][LD], then the warps' sums [8][BM][BN + 1] in its place
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rg = lane >> 3, cg = lane & 7;
+  const long long m0 = (long long)blockIdx.x * BM;
+  const int n0 = blockIdx.y * BN;
+  float* mine = rows_smem + warp * 2 * kStage;
+  const uint32_t mine_s = (uint32_t)__cvta_generic_to_shared(mine);
+  const int nchunks = (K + KC - 1) / KC;
+  auto fetch = [&](int c, int buf) {
+    const int k0 = c * KC;
+#pragma unroll
+    for (int i = 0; i < (BM + BN) * kPieces / 32; i++) {
+      const int e = i * 32 + lane, r = e / kPieces, k = k0 + (e % kPieces) * 4;
+      const bool a = r < BM;
+      const bool live = a ? m0 + r < M : n0 + r - BM < N;
+      const float* src = a ? A + (m0 + r) * K + k : W + (long long)(n0 + r - BM) * K + k;
+      const uint32_t dst = mine_s + (buf * kStage + r * LD + (e % kPieces) * 4) * 4;
+      const int left = live ? K - k : 0;                       // inputs from here on; what lies behind them is filled with zeros
+      if (vec) {
+        const int n = left > 4 ? 16 : left > 0 ? 4 * left : 0;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(n ? src : A), "r"(n) : "memory");
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 4 * j), "l"(left > j ? src + j : A), "r"(left > j ? 4 : 0) : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float2 acc[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; i++)
+#pragma unroll
+    for (int j = 0; j < TN; j++) acc[i][j] = make_float2(0.f, 0.f);
+  int buf = 0;
+  if (warp < nchunks) fetch(warp, 0);
+  for (int c = warp; c < nchunks; c += 8, buf ^= 1) {
+    if (c + 8 < nchunks) {
+      fetch(c + 8, buf ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncwarp();
+    float* st = mine + buf * kStage;
+    if (in_div) {
+      for (int e = lane; e < BM * KC; e += 32) {
+        const int r = e / KC, k = e % KC;
+        if (c * KC + k < K) st[r * LD + k] = __fdiv_rn(st[r * LD + k], __ldg(in_div + c * KC + k));
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int q = 0; q < kPieces; q++) {
+      float4 w[TN];
+#pragma unroll
+      for (int j = 0; j < TN; j++) w[j] = *reinterpret_cast<const float4*>(st + (BM + cg + 8 * j) * LD + 4 * q);
+#pragma unroll
+      for (int i = 0; i < TM; i++) {
+        const float4 a = *reinterpret_cast<const float4*>(st + (rg + 4 * i) * LD + 4 * q);
+#pragma unroll
+        for (int j = 0; j < TN; j++) {
+          acc[i][j] = fma2(make_float2(a.x, a.y), make_float2(w[j].x, w[j].y), acc[i][j]);
+          acc[i][j] = fma2(make_float2(a.z, a.w), make_float2(w[j].z, w[j].w), acc[i][j]);
+        }
+      }
+    }
+    __syncwarp();                                              // every lane has read this stage before it is filled again
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < TM; i++)
+#pragma unroll
+    for (int j = 0; j < TN; j++) rows_smem[(warp * BM + rg + 4 * i) * (BN + 1) + cg + 8 * j] = acc[i][j].x + acc[i][j].y;
+  __syncthreads();
+  for (int e = threadIdx.x; e < BM * BN; e += 256) {
+    const int r = e / BN, n = e % BN, nn = n0 + n;
+    if (m0 + r >= M || nn >= N) continue;
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; w++) v += rows_smem[(w * BM + r) * (BN + 1) + n];
+    v += bias ? __ldg(bias + nn) : 0.f;
+    v = act_apply(v, act, slope);
+    if (out_mul) v = v * out_mul[nn];
+    if (relu_mask && relu_mask[nn] != 0.f) v = max_nan(v, 0.f);
+    C[(m0 + r) * N + nn] = v;
+  }
+}
+
+template <int TM, int TN, int KC>
+void launch_linear_rows(const float* A, const float* W, const float* bias, float* C, long long M, int N, int K, int act, float slope,
+                        const float* in_div, const float* out_mul, const float* relu_mask, int vec, cudaStream_t s) {
+  constexpr int BM = 4 * TM, BN = 8 * TN, stages = 8 * 2 * (BM + BN) * (KC + 4) * 4, sums = 8 * BM * (BN + 1) * 4, smem = stages > sums ? stages : sums;
+  static const bool set = cudaFuncSetAttribute(linear_rows_kernel<TM, TN, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+  (void)set;
+  const dim3 grid((unsigned)((M + BM - 1) / BM), (unsigned)((N + BN - 1) / BN));
+  linear_rows_kernel<TM, TN, KC><<<grid, 256, smem, s>>>(A, W, bias, C, M, N, K, act, slope, in_div, out_mul, relu_mask, vec);
+}
+
+// Which kernel and tile: 0, 1, 2 linear_rows_kernel with 8 x 8, 16 x 16, 32 x 32, 3 the tiles of 128 x 64.  Rounds of blocks over the SMs times
+// a round's time, 0.1 us, fitted to 108 shapes (1 to 30,000 rows, 8 to 2048 features and inputs): what a round costs at K = 0, what 768 inputs
+// add to it, and what they add where rows do not start on 16 bytes.  768 x 768, us, 8 x 8 / 16 x 16 / 32 x 32 / 128 x 64: 3 rows 4.8 / 6.3 /
+// 12.5 / 65.7, 50 rows 10.4 / 8.7 / 12.6 / 78, 300 rows 37 / 22.7 / 20.6 / 96.4, 6000 rows - / 330 / 243 / 320; 64 x 64 at 30,000 rows - / 45.9 /
+// 29.5 / 21.2; 768 x 8 at 1500 rows 62.8 / 26.7 / 16.5 / 8.3.
+int linear_tile(long long M, int N, int K, bool vec) {
+  static const int bm[4] = {8, 16, 32, LBM}, bn[4] = {8, 16, 32, LBN}, base[4] = {30, 35, 50, 50}, base_k[4] = {0, 0, 0, 190}, round0[4] = {5, 7, 15, 30},
+                   round_k[4] = {9, 20, 63, 668}, round_off[4] = {10, 18, 46, 0};
+  long long best_cost = 0;
+  int best = 3;
+  for (int t = 3; t >= 0; t--) {
+    const long long rows = (M + bm[t] - 1) / bm[t], cols = ((long long)N + bn[t] - 1) / bn[t], rounds = (rows * cols + 147) / 148;
+    if (t < 3 && cols > 65535) continue;                       // the grid's second extent
+    const long long cost = 768 * base[t] + (long long)K * base_k[t] + rounds * (768 * round0[t] + (long long)K * (round_k[t] + (vec ? 0 : round_off[t])));
+    if (t == 3 || cost < best_cost) { best = t; best_cost = cost; }
+  }
+  return best;
+}
+
 void launch_linear_f32(const float* A, const float* W, const float* bias, float* C, long long M, int N, int K, int act,
                        float slope, const float* in_div, const float* out_mul, const float* relu_mask, cudaStream_t s) {
   if (M <= 0) return;
+  const int vec = K % 4 == 0 && ((uintptr_t)A | (uintptr_t)W) % 16 == 0;
+  switch (linear_tile(M, N, K, vec)) {
+    case 0: return launch_linear_rows<2, 1, 32>(A, W, bias, C, M, N, K, act, slope, in_div, out_mul, relu_mask, vec, s);
+    case 1: return launch_linear_rows<4, 2, 32>(A, W, bias, C, M, N, K, act, slope, in_div, out_mul, relu_mask, vec, s);
+    case 2: return launch_linear_rows<8, 4, 16>(A, W, bias, C, M, N, K, act, slope, in_div, out_mul, relu_mask, vec, s);
+  }
   dim3 grid((unsigned)((M + LBM - 1) / LBM), (unsigned)((N + LBN - 1) / LBN));
   linear_f32_kernel<<<grid, 256, 0, s>>>(A, W, bias, C, M, N, K, act, slope, in_div, out_mul, relu_mask);
 }
