@@ -154,6 +154,7 @@ struct Session {
 
   long long buf_rows = 0;
   float *din = nullptr, *dout = nullptr, *act0 = nullptr, *act1 = nullptr;
+  void* x16 = nullptr; long long x16_bytes = 0;   // 16-bit steps of few rows: the gathered input
   long long act_bytes = 0, pair_refused = 0;      // of act0 and act1 each; bytes of split activations that there was no memory for (0: none)
   float *X_pinned = nullptr, *Y_pinned = nullptr;
   long long pinned_rows = 0;
@@ -467,7 +468,16 @@ bool runs_on_pairs(long long rows) {
 void ensure_activations(long long rows) {
   Session& s = S();
   if (!s.model.is_mlp() || s.model.layers.size() < 2) return;
-  int wmax = 1;
+  if (s.tc) {
+    const long long need = (long long)rows_mlp_input_bytes(s.model.n_in(), std::min(rows, kRowsMlpMaxRows));
+    if (s.x16_bytes < need) {
+      pool_free(s.x16);
+      s.x16 = pool_alloc(need);
+      s.x16_bytes = s.x16 ? need : 0;                // without it such steps run on the fused kernel
+      drop_graph();
+    }
+  }
+  int wmax = s.tc ? 4 : 1;                         // (16-bit rows begin on 16-byte boundaries: no row is shorter)
   for (auto& L : s.model.layers) wmax = L.cout > wmax ? L.cout : wmax;
   const long long plain = act_ld(rows) * wmax * 4, split = runs_on_pairs(rows) ? std::max<long long>((long long)f32tc_pair_bytes(s.f32, rows), plain) : 0;
   bool pair = split > 0 && (!s.pair_refused || split < s.pair_refused);
@@ -838,8 +848,8 @@ void run_step_kernels(const StepArgs& A) {
     if (fuse_out) { L.SP = s.S.hdr; L.stores = (const StoreTarget*)s.S.items; L.TS = A.TS; L.fast_out = 1;
                     L.store_by_slot = s.S.store_by_slot; std::memcpy(L.cout, s.S.cls, sizeof L.cout); }
     L.Y = fuse_out ? nullptr : s.dout;
-    L.read_once = fuse_in && s.G.mapped;
     L.act[0] = s.act0; L.act[1] = s.act1; L.act_ld = act_ld(rows);
+    L.x16 = s.x16_bytes >= (long long)rows_mlp_input_bytes(s.model.n_in(), rows) ? s.x16 : nullptr;
     L.g = g;
     ensure_aux(std::max(tc_grid(s.tc, rows), f32tc_grid(rows)));
     L.partials = (fuse_out && s.want_checksum) ? s.d_partials : nullptr;
@@ -1499,8 +1509,8 @@ int fortis_load_model_mem(const void* blob, long nbytes) {
   free_model_dev();
   s.model = std::move(M);
   s.have_model = true;
-  pool_free(s.din); pool_free(s.dout); pool_free(s.act0); pool_free(s.act1);
-  s.din = s.dout = s.act0 = s.act1 = nullptr; s.buf_rows = 0; s.act_bytes = s.pair_refused = 0;
+  pool_free(s.din); pool_free(s.dout); pool_free(s.act0); pool_free(s.act1); pool_free(s.x16);
+  s.din = s.dout = s.act0 = s.act1 = nullptr; s.x16 = nullptr; s.buf_rows = 0; s.act_bytes = s.pair_refused = s.x16_bytes = 0;
   g_err = 0;
   return 0;
   FORTIS_CATCH(return -1)
@@ -1563,7 +1573,7 @@ void fortis_reset(void) {
   if (g_stream) conv_workspace_release(g_stream);
   free_plan(s.G); free_plan(s.S);
   free_model_dev();
-  pool_free(s.din); pool_free(s.dout); pool_free(s.act0); pool_free(s.act1);
+  pool_free(s.din); pool_free(s.dout); pool_free(s.act0); pool_free(s.act1); pool_free(s.x16);
   pool_free(s.d_partials); pool_free(s.d_sum); pool_free(s.d_status); pool_free(s.d_done);
   if (s.X_pinned) cudaFreeHost(s.X_pinned);
   if (s.Y_pinned) cudaFreeHost(s.Y_pinned);

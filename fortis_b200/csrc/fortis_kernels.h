@@ -132,8 +132,8 @@ struct TcLaunch {
   RowGeom g;
   const float* X;                                    // (rows, n_in) when there is no gather plan
   float* Y;                                          // (rows, n_out) when there is no scatter plan (may be set with SP too)
-  float* act[2]; long long act_ld;                   // activation buffers of the layer-by-layer form, as F32TcLaunch
-  int read_once;                                     // gathered arrays lie in host memory: the form that loads them once
+  float* act[2]; long long act_ld;                   // activation buffers of the form for few rows, as F32TcLaunch ...
+  void* x16;                                         // ... and for its gathered input, rows_mlp_input_bytes()
   double* partials;                                  // per-CTA checksum partials (size >= tc_grid())
   double* sum; unsigned int* done;                   // optional: fold the partials into *sum inside the kernel (done: zeroed counter)
   int* status;                                       // device word: 0 ok, else the code of the wait that gave up
@@ -174,7 +174,7 @@ struct ConvGeom {
   long long ys_n, ys_d, ys_h, ys_w, ys_c;     // element strides of y
   long long rs_n, rs_d, rs_h, rs_w, rs_c;     // element strides of the residual, where there is one
 };
-// the 16-bit forms of the same kernel: MLPs of few rows, layer by layer
+// ---- 16-bit MLPs of few rows, one launch (fortis_mlp_rows.cu) ---------------------------------------------------------
 struct F16Layer {
   const void* w;                                       // [N_pad][K_pad] 16-bit, zero padded
   int K_pad, N_pad, k_real, n_real;
@@ -185,8 +185,10 @@ struct RowsMlp;
 RowsMlp* rows_mlp_create(const std::vector<F16Layer>& layers, bool f16, const float* in_div, const float* out_mul, const float* relu_mask,
                          std::string* err);
 void rows_mlp_destroy(RowsMlp* m);
-int rows_mlp_cost(const int* K, const int* N, int nlayers, long long nrows);     // estimated device time, 10 ns
-bool rows_mlp_forward(RowsMlp* m, const F32TcLaunch& L, cudaStream_t s, std::string* err);
+int rows_mlp_cost(const int* K, const int* N, int nlayers, long long nrows);     // estimated device time of launches layer by layer, 10 ns
+constexpr long long kRowsMlpMaxRows = 3072;
+size_t rows_mlp_input_bytes(int n_in, long long nrows);                          // of the buffer `x16`
+bool rows_mlp_forward(RowsMlp* m, const F32TcLaunch& L, void* x16, cudaStream_t s, std::string* err);
 // ---- fp32 convolutions on the tensor cores (fortis_conv3d_f32.cu): rows = positions of a grid that holds the padding ------
 // Shorter reductions stay on the FFMA kernel: the split keeps 21 bits of an operand, which sums of few products show, while
 // the FFMA kernel's roundings grow with their number.  Error against 64 bits, relative 2-norm, split / FFMA, inputs normal and

@@ -1,0 +1,574 @@
+// 16-bit MLP steps of few rows in ONE launch: gather -> all Linear layers -> scatter, a layer's tiles spread over the SMs and the
+// layers chained by counters in global memory instead of by launches (a cooperative launch: every CTA is resident).
+//
+// Replaces, for such calls, the reference's fortis_gather_k, one fortis_gemm plus epilogue kernel per layer and fortis_scatter_k
+// (driver/fortis_gather_emit.py:52-62, 75-83, compiler/FortisFuse.cpp:587-655); results are the fused kernel's (fortis_mlp_tc.cu) bit
+// for bit for finite values.
+//
+// Few rows leave a tile of 128 rows x 64 features nothing to spread, so the operands change places: a tile is 128 FEATURES (the MMA's
+// M, weights as the A operand) x `nr` rows (its N, 16 to 128), and `nr` is the least that gives every SM at most one tile of the widest
+// layer.  Per tile D[128 features x nr rows] = W[128 x K] . X[nr x K]^T in stages of 128 k, both operands through the TMA:
+//   * one warp streams weights through a ring that runs ahead of the layers: they wait for nobody, so the next tile's are in shared
+//     memory before its inputs are;
+//   * one warp polls the counter of its row tile (all feature tiles of the layer in front done), then streams the inputs, which lie
+//     16-bit and k-fastest in global memory ([row][feature], rows on 16-byte boundaries);
+//   * one warp issues the MMAs into two accumulators; eight epilogue warps (thread = feature, so bias, scale and slope are one register
+//     each) write the next layer's inputs and add to the counter, or scatter.
+// Inputs are gathered once, by all CTAs, into such rows (layer by layer every feature tile gathered them again).
+//
+// What bounds it: the chain from one layer to the next, not bytes or MMAs.  Clocks of a step of 244-768x4-128 at 30 and 3000 rows: set-up
+// and gather 8900 / 8500; a layer 13,200 / 21,500, of which seeing the count and the first inputs 3000, twelve chunks of MMAs 6300,
+// accumulator to stores 1200 / 8000, stores to the count 2500.  The call, bf16 (fp8 weights within 2 us), layer by layer in launches of
+// 128 x 64 tiles -> here: 1 row 65.4 -> 48.8 us, 300 66.0 -> 53.9, 1000 65.7 -> 56.6, 2000 72.0 -> 62.3, 3072 72.5 -> 66.6.  With
+// 3073 rows the fused kernel takes 78.8; below 3072 it is chosen where the estimates of rows_mlp_cost and of the caller cross.
+//
+// A count is released by the writing warp (stores, then a releasing add) and acquired by the polling lane (ld.acquire, then the fence
+// between what ordinary stores wrote and what copies read) in front of the copies.  The last CTA to finish sets the counters back to zero, so a captured launch can be replayed.
+// Every wait is bounded; a CTA whose wait gives up records which one, the CTAs behind it run into their own limits.
+#include <cuda.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include "fortis_device.cuh"
+#include "fortis_kernels.h"
+#include "fortis_tc.cuh"
+
+namespace fortis {
+
+namespace {
+
+using namespace tc;
+
+constexpr int kFt = 128, kKc = 64;              // features per tile, k per chunk (a 128-byte swizzle row)
+// chunks of a stage: waits, commits and counting take the issuing warp some 380 clk a stage, whose MMAs take 130 a chunk
+constexpr int kStageChunks = 2;
+constexpr int kMaxLayersR = 8, kMaxNr = 128;
+constexpr int kWChunkBytes = kFt * kKc * 2, kWSlotBytes = kStageChunks * kWChunkBytes;
+constexpr int kMaxW = 6, kMaxA = 8, kStagesOfK = 6;   // stages of 768 k
+constexpr int kEWarpsR = 8;                     // thread = feature; two warps share a lane quadrant and take alternate 32 rows
+constexpr int kRowThreads = (4 + kEWarpsR) * 32;   // warps: weights, inputs, MMA, none, epilogue; all but the first gather
+constexpr int kGatherWarps = 3 + kEWarpsR, kGatherRows = 16;
+constexpr int kTabRows = 256;                   // widest gathered input
+constexpr int kBarRows = 1024;
+constexpr int kSmemRowsMax = 227 * 1024;
+constexpr int kTailRows = kBarRows + kTabRows * 8 + kMaxNr * 16;
+// the wait codes of the layer-by-layer kernels
+enum { RST_A_FULL = 21, RST_A_EMPTY = 22, RST_ACC_FULL = 23, RST_ACC_EMPTY = 24, RST_ALIGN = 25, RST_W_FULL = 26, RST_W_EMPTY = 27, RST_COUNT = 28 };
+
+struct RowsLayer {
+  CUtensorMap wmap;                      // [features][K_pad] 16-bit, box 128 rows x 64
+  CUtensorMap amap;                      // the layer's input [rows][features], box nr x 64; what lies outside is zero
+  int kchunks, nft, n_real, pad;
+  const float *bias, *scale; float slope;
+  uint16_t* out; int out_pitch;          // hidden layers: the next layer's input, elements per row
+};
+struct RowsParams {
+  RowsLayer layer[kMaxLayersR];
+  int nlayers, nr, nrt;                  // rows per tile, row tiles
+  int nrows;
+  int w_slots, a_stages, a_bytes;
+  int n_in, x_pitch; uint16_t* x16;      // the gathered input
+  const float* in_div;
+  int fast_in; const Access* slots; ArrayTable TG; long long cin[2][3]; const float* X;
+  int fast_out; const Access* store_by_slot; ArrayTable TS; long long cout[2][3]; float* Y;
+  const float *out_mul, *relu_mask;
+  RowGeom g;
+  unsigned* count;                       // [nlayers][nrt]: parts of a layer's input that are there; then the CTAs that have finished
+  double* partials; double* sum;
+  int* status;
+  unsigned int wait_limit; int test_skip_stage;
+};
+
+// instruction descriptor without N: M = 128; bf16 is operand format code 1, fp16 0
+template <bool F16> struct IdescR { static constexpr uint32_t value = idesc_bf16(kFt, 0) & ~(F16 ? ((1u << 7) | (1u << 10)) : 0u); };
+template <bool F16> __device__ __forceinline__ uint32_t pack16(float lo, float hi) {
+  if constexpr (F16) { const __half2 v = __floats2half2_rn(lo, hi); return *reinterpret_cast<const uint32_t*>(&v); }
+  else return pack_bf16(lo, hi);
+}
+// D[tmem] (+)= A . B^T over a chunk of 64 k (four MMAs, 32 bytes of a row each); low words of the operands' shared-memory descriptors
+constexpr uint32_t kDescHiR = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ void mma_chunk(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred e, q;\n\t.reg .b64 a0, a1, a2, a3, b0, b1, b2, b3;\n\t"
+      "mov.b64 a0, {%1, %5};\n\tmov.b64 b0, {%2, %5};\n\t"
+      "add.s64 a1, a0, 2;\n\tadd.s64 b1, b0, 2;\n\tadd.s64 a2, a0, 4;\n\tadd.s64 b2, b0, 4;\n\tadd.s64 a3, a0, 6;\n\tadd.s64 b3, b0, 6;\n\t"
+      "setp.ne.b32 q, %4, 0;\n\telect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a0, b0, %3, q;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, 1;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, 1;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, 1;\n\t}"
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(kDescHiR) : "memory");
+}
+__device__ __forceinline__ float ld_once(const float* p, bool ok) {       // keeps its place, so that many are in flight
+  float v;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@p ld.global.f32 %0, [%1];\n\t}" : "=f"(v) : "l"(p), "r"((int)ok));
+  return v;
+}
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void add_release(unsigned* p) { asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory"); }
+__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async;" ::: "memory"); }
+__device__ __forceinline__ void drain_bar(uint32_t bar, uint32_t parity, uint32_t limit) {
+  for (uint32_t i = 0; i < limit; i++)
+    if (mbar_try_wait(bar, parity)) return;
+}
+
+template <bool F16>
+__global__ void __launch_bounds__(kRowThreads, 1) mlp_rows_kernel(const __grid_constant__ RowsParams P) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t base = smem_u32(smem);
+  if (base & 1023u) {                             // the same in every CTA: nobody waits for another one
+    if (threadIdx.x == 0) atomicCAS(P.status, 0, RST_ALIGN);
+    return;
+  }
+  const uint32_t a_ring = base + P.w_slots * kWSlotBytes, bars = a_ring + P.a_stages * P.a_bytes;
+  uint8_t* tail = smem + (bars - base);
+  // w_full [6] | w_empty [6] | a_full [8] | a_empty [8] | acc_full [2] | acc_empty [2] | drained; at 512 the tensor-memory base, at
+  // 516 the abort flag, at 520 "the last CTA", at 528 the checksum's warp sums; then the gather's table and the scatter's rows
+  const uint32_t w_full = bars, w_empty = bars + 48, a_full = bars + 96, a_empty = bars + 160, acc_full = bars + 224, acc_empty = bars + 240, drained = bars + 256;
+  uint32_t* tmem_slot = (uint32_t*)(tail + 512);
+  volatile int* abort_flag = (volatile int*)(tail + 516);
+  volatile int* last_cta = (volatile int*)(tail + 520);
+  double* wsum = (double*)(tail + 528);
+  unsigned long long* tab = (unsigned long long*)(tail + kBarRows);
+  long long* rowpos = (long long*)(tail + kBarRows + kTabRows * 8);          // [nr][2]: byte positions of the two stride classes
+  // through a shuffle, so that the compiler knows the roles' branches, loops and addresses to be the same in a whole warp
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  unsigned* finished = P.count + P.nlayers * P.nrt;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kMaxW; s++) { mbar_init(w_full + 8 * s, 1); mbar_init(w_empty + 8 * s, 1); }
+    for (int s = 0; s < kMaxA; s++) { mbar_init(a_full + 8 * s, 1); mbar_init(a_empty + 8 * s, 1); }
+    for (int s = 0; s < 2; s++) { mbar_init(acc_full + 8 * s, 1); mbar_init(acc_empty + 8 * s, kEWarpsR); }
+    mbar_init(drained, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (P.fast_in)
+    for (int q = threadIdx.x; q < P.n_in; q += kRowThreads) {
+      const Access a = P.slots[q];
+      const bool c0 = a.si == P.cin[0][0] && a.sj == P.cin[0][1] && a.sk == P.cin[0][2];
+      tab[q] = (unsigned long long)((const float*)P.TG.base[a.array] + a.off0) | (c0 ? 0ull : 1ull);
+    }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(256u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  auto wait = [&](uint32_t bar, uint32_t parity, int code) { return wait_polling(bar, parity, P.wait_limit, abort_flag, P.status, code); };
+  double csum = 0.0;
+
+  if (warp > 0) {
+    // ------------------------------------------------------------------ gather: 16 rows x 64 inputs a unit, half a row of it a thread
+    const int nkc = P.layer[0].kchunks, nsub = (P.nrows + kGatherRows - 1) / kGatherRows;
+    for (int u = blockIdx.x * kGatherWarps + warp - 1; u < nsub * nkc; u += gridDim.x * kGatherWarps) {
+      const int sub = u / nkc, k0 = (u - sub * nkc) * kKc + (lane >> 4) * 32, r0 = sub * kGatherRows;
+      const int row = r0 + (lane & 15), rl = row < P.nrows ? row : P.nrows - 1;
+      float v[32];
+      if (P.fast_in) {
+        long long ci, cj, kk;
+        row_to_pos(P.g, rl, &ci, &cj, &kk);
+        const long long p0 = 4 * (ci * P.cin[0][0] + cj * P.cin[0][1] + kk * P.cin[0][2]), p1 = 4 * (ci * P.cin[1][0] + cj * P.cin[1][1] + kk * P.cin[1][2]);
+#pragma unroll
+        for (int j = 0; j < 32; j++) {
+          const bool ok = k0 + j < P.n_in;
+          const unsigned long long e = ok ? tab[k0 + j] : 0ull;
+          v[j] = ld_once(reinterpret_cast<const float*>((e & ~1ull) + (unsigned long long)((e & 1ull) ? p1 : p0)), ok);
+        }
+      } else {
+        const float* x = P.X + (long long)rl * P.n_in + k0;
+#pragma unroll
+        for (int j = 0; j < 32; j++) v[j] = ld_once(x + j, k0 + j < P.n_in);
+      }
+      if (P.in_div) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) if (k0 + j < P.n_in) v[j] = __fdiv_rn(v[j], __ldg(P.in_div + k0 + j));
+      }
+      if (row < P.nrows) {
+        uint16_t* dst = P.x16 + (long long)row * P.x_pitch + k0;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          if (k0 + 8 * i < P.x_pitch)
+            *reinterpret_cast<uint4*>(dst + 8 * i) = make_uint4(pack16<F16>(v[8 * i], v[8 * i + 1]), pack16<F16>(v[8 * i + 2], v[8 * i + 3]),
+                                                                pack16<F16>(v[8 * i + 4], v[8 * i + 5]), pack16<F16>(v[8 * i + 6], v[8 * i + 7]));
+      }
+      __syncwarp();
+      if (lane == 0) add_release(P.count + r0 / P.nr);
+    }
+  }
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA: weights
+    uint32_t s = 0, ph = 0;
+    bool stop = false;
+    for (int l = 0; l < P.nlayers && !stop; l++) {
+      const RowsLayer& L = P.layer[l];
+      for (int t = blockIdx.x; t < L.nft * P.nrt && !stop; t += gridDim.x) {
+        const int f0 = (t % L.nft) * kFt;
+        for (int kc = 0; kc < L.kchunks; kc += kStageChunks) {
+          if (!wait(w_empty + 8 * s, ph ^ 1, RST_W_EMPTY)) { stop = true; break; }
+          const int n = L.kchunks - kc < kStageChunks ? L.kchunks - kc : kStageChunks;
+          const bool skip = P.test_skip_stage && blockIdx.x == 0 && l == 0 && t == 0 && kc == 0;     // test only: the stage never completes
+          if (!skip) {
+            mbar_expect_tx(w_full + 8 * s, n * kWChunkBytes);
+            for (int j = 0; j < n; j++) tma_load_2d(base + s * kWSlotBytes + j * kWChunkBytes, &L.wmap, (kc + j) * kKc, f0, w_full + 8 * s);
+          }
+          if (++s == (uint32_t)P.w_slots) { s = 0; ph ^= 1; }
+        }
+      }
+    }
+    if (!P.test_skip_stage || blockIdx.x != 0)
+      for (uint32_t q = 0; q < (uint32_t)P.w_slots; q++) drain_bar(w_full + 8 * q, q < s ? ph : ph ^ 1, P.wait_limit);
+    else
+      for (uint32_t q = 1; q < (uint32_t)P.w_slots; q++) drain_bar(w_full + 8 * q, q < s ? ph : ph ^ 1, P.wait_limit);
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ TMA: inputs, once their row tile is complete
+    uint32_t s = 0, ph = 0;
+    bool stop = false;
+    for (int l = 0; l < P.nlayers && !stop; l++) {
+      const RowsLayer& L = P.layer[l];
+      for (int t = blockIdx.x; t < L.nft * P.nrt && !stop; t += gridDim.x) {
+        const int rt = t / L.nft, left = P.nrows - rt * P.nr, rows_here = left < P.nr ? left : P.nr;
+        // layer 0: units of the gather; others: the epilogue warps of every feature tile of the layer in front
+        const unsigned want = l == 0 ? (unsigned)((rows_here + kGatherRows - 1) / kGatherRows * L.kchunks) : (unsigned)(kEWarpsR * P.layer[l - 1].nft);
+        const unsigned* c = P.count + l * P.nrt + rt;
+        int ok = 0;
+        if (lane == 0) {
+          for (unsigned i = 0; i < P.wait_limit; i++) {
+            if (ld_acquire(c) >= want) { ok = 1; break; }
+            if (*abort_flag) break;
+          }
+          if (!ok) { *abort_flag = 1; atomicCAS(P.status, 0, RST_COUNT); }
+        }
+        if (!__shfl_sync(0xffffffffu, ok, 0)) { stop = true; break; }
+        proxy_fence();
+        for (int kc = 0; kc < L.kchunks; kc += kStageChunks) {
+          if (!wait(a_empty + 8 * s, ph ^ 1, RST_A_EMPTY)) { stop = true; break; }
+          const int n = L.kchunks - kc < kStageChunks ? L.kchunks - kc : kStageChunks;
+          mbar_expect_tx(a_full + 8 * s, n * (P.a_bytes / kStageChunks));
+          for (int j = 0; j < n; j++) tma_load_2d(a_ring + s * P.a_bytes + j * (P.a_bytes / kStageChunks), &L.amap, (kc + j) * kKc, rt * P.nr, a_full + 8 * s);
+          if (++s == (uint32_t)P.a_stages) { s = 0; ph ^= 1; }
+        }
+      }
+    }
+    for (uint32_t q = 0; q < (uint32_t)P.a_stages; q++) drain_bar(a_full + 8 * q, q < s ? ph : ph ^ 1, P.wait_limit);
+  } else if (warp == 2) {
+    // ------------------------------------------------------------------ MMA issuer
+    uint32_t ws = 0, wph = 0, as = 0, aph = 0, it = 0;
+    const uint32_t idesc = __shfl_sync(0xffffffffu, IdescR<F16>::value | ((uint32_t)(P.nr >> 3) << 17), 0);
+    bool stop = false;
+    for (int l = 0; l < P.nlayers && !stop; l++) {
+      const RowsLayer& L = P.layer[l];
+      for (int t = blockIdx.x; t < L.nft * P.nrt && !stop; t += gridDim.x, it++) {
+        const uint32_t b = it & 1;
+        if (!wait(acc_empty + 8 * b, ((it >> 1) & 1) ^ 1, RST_ACC_EMPTY)) { stop = true; break; }
+        for (int kc = 0; kc < L.kchunks; kc += kStageChunks) {
+          if (!wait(w_full + 8 * ws, wph, RST_W_FULL) || !wait(a_full + 8 * as, aph, RST_A_FULL)) { stop = true; break; }
+          tc_fence_after();
+          // through shuffles: an MMA whose operands the compiler does not know to be the same in all lanes takes several times as long to issue
+          const uint32_t ad = __shfl_sync(0xffffffffu, ((base + ws * kWSlotBytes) >> 4) & 0x3FFFu, 0), bd = __shfl_sync(0xffffffffu, ((a_ring + as * P.a_bytes) >> 4) & 0x3FFFu, 0);
+#pragma unroll
+          for (int j = 0; j < kStageChunks; j++)
+            if (kc + j < L.kchunks)
+              mma_chunk(tmem + b * kMaxNr, ad + (uint32_t)(j * (kWChunkBytes >> 4)), bd + (uint32_t)j * (uint32_t)(P.a_bytes / kStageChunks >> 4), idesc, (uint32_t)(kc + j));
+          tc_commit(w_empty + 8 * ws);
+          tc_commit(a_empty + 8 * as);
+          if (++ws == (uint32_t)P.w_slots) { ws = 0; wph ^= 1; }
+          if (++as == (uint32_t)P.a_stages) { as = 0; aph ^= 1; }
+        }
+        if (!stop) tc_commit(acc_full + 8 * b);
+      }
+    }
+    tc_commit(drained);                             // nothing may still read shared or tensor memory when the CTA ends
+    drain_bar(drained, 0, P.wait_limit);
+  } else if (warp >= 4) {
+    // ------------------------------------------------------------------ epilogue: thread = feature, 32 rows at a time.  A wait that gives
+    // up ends no warp here: the others would wait for it at the scatter's barriers.  The waits behind it return at once.
+    const int quad = warp & 3, set = (warp - 4) >> 2;
+    const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16);
+    uint32_t it = 0;
+    for (int l = 0; l < P.nlayers; l++) {
+      const RowsLayer& L = P.layer[l];
+      const bool last = l == P.nlayers - 1;
+      for (int t = blockIdx.x; t < L.nft * P.nrt; t += gridDim.x, it++) {
+        const int rt = t / L.nft, f = (t - rt * L.nft) * kFt + quad * 32 + lane, row0 = rt * P.nr;
+        const int left = P.nrows - row0, rows_here = left < P.nr ? left : P.nr;
+        const uint32_t b = it & 1;
+        const bool real = f < L.n_real;
+        const float bias = real ? __ldg(L.bias + f) : 0.f, scale = L.scale && real ? __ldg(L.scale + f) : 1.f;
+        if (last && P.fast_out) {
+          asm volatile("bar.sync 1, 256;" ::: "memory");             // the previous tile's rows have been read
+          const int i = (int)threadIdx.x - 128;
+          if (i < P.nr) {
+            long long ci, cj, kk;
+            row_to_pos(P.g, row0 + i < P.nrows ? row0 + i : P.nrows - 1, &ci, &cj, &kk);
+            rowpos[2 * i] = 4 * (ci * P.cout[0][0] + cj * P.cout[0][1] + kk * P.cout[0][2]);
+            rowpos[2 * i + 1] = 4 * (ci * P.cout[1][0] + cj * P.cout[1][1] + kk * P.cout[1][2]);
+          }
+          asm volatile("bar.sync 1, 256;" ::: "memory");
+        }
+        float om = 1.f;
+        bool mask = false;
+        unsigned long long dst = 0ull;                               // scatter: the element of row position 0
+        int cls = 0;
+        if (last && real) {
+          if (P.out_mul) om = __ldg(P.out_mul + f);
+          mask = P.relu_mask && __ldg(P.relu_mask + f) != 0.f;
+          if (P.fast_out && P.store_by_slot[f].array >= 0) {
+            const Access a = P.store_by_slot[f];
+            cls = a.si == P.cout[0][0] && a.sj == P.cout[0][1] && a.sk == P.cout[0][2] ? 0 : 1;
+            dst = (unsigned long long)((float*)P.TS.base[a.array] + a.off0);
+          }
+        }
+        if (!wait(acc_full + 8 * b, (it >> 1) & 1, RST_ACC_FULL)) continue;
+        tc_fence_after();
+        for (int c0 = 32 * set; c0 < P.nr; c0 += 64) {             // (columns behind the tile's rows are read and not used)
+          uint32_t a[32];
+          tmem_ld32(lane_addr + b * kMaxNr + c0, a);
+          tmem_ld_wait();
+          float v[32];
+          // the fused kernel's expressions
+#pragma unroll
+          for (int j = 0; j < 32; j++) {
+            const float x = __uint_as_float(a[j]);
+            v[j] = !L.scale ? x + bias : fmaf(x, scale, bias);
+            v[j] = fmaxf(v[j], v[j] * L.slope);
+          }
+          if (!last) {
+            // two features a store: the even lane takes the even rows of its pair of features, the odd lane the odd ones
+            uint16_t* o = L.out + (long long)(row0 + c0 + (lane & 1)) * L.out_pitch + (f & ~1);
+            const bool mine = (f & ~1) < L.n_real;
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) {
+              const float got = __shfl_xor_sync(0xffffffffu, (lane & 1) ? v[j] : v[j + 1], 1);
+              const uint32_t p = (lane & 1) ? pack16<F16>(got, v[j + 1]) : pack16<F16>(v[j], got);
+              if (mine && c0 + j + (lane & 1) < rows_here) *reinterpret_cast<uint32_t*>(o + (long long)j * L.out_pitch) = p;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; j++) {
+              if (P.out_mul) v[j] *= om;
+              if (mask) v[j] = max_nan(v[j], 0.f);
+            }
+            if (!P.fast_out) {
+#pragma unroll
+              for (int j = 0; j < 32; j++)
+                if (real && c0 + j < rows_here) P.Y[(long long)(row0 + c0 + j) * L.n_real + f] = v[j];
+            } else if (dst) {
+#pragma unroll
+              for (int j = 0; j < 32; j += 4) {
+                const long long* rp = rowpos + 2 * (c0 + j) + cls;
+                if (c0 + j + 3 < rows_here && rp[2] == rp[0] + 4 && rp[4] == rp[0] + 8 && rp[6] == rp[0] + 12 && ((dst + (unsigned long long)rp[0]) & 15ull) == 0) {
+                  *reinterpret_cast<float4*>(dst + (unsigned long long)rp[0]) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                } else {
+#pragma unroll
+                  for (int e = 0; e < 4; e++)
+                    if (c0 + j + e < rows_here) *reinterpret_cast<float*>(dst + (unsigned long long)rp[2 * e]) = v[j + e];
+                }
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                  if (c0 + j + e < rows_here) csum += (double)v[j + e];
+              }
+            }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty + 8 * b);               // (an accumulator is filled again two tiles later)
+        if (!last) {
+          __syncwarp();
+          if (lane == 0) add_release(P.count + (l + 1) * P.nrt + rt);
+        }
+      }
+    }
+    if (P.partials) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) csum += __shfl_down_sync(0xffffffffu, csum, o);
+      if (lane == 0) wsum[warp - 4] = csum;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  // the CTA's part of the checksum, and the end of the launch: the last CTA adds the parts in a fixed order and clears the counters
+  if (threadIdx.x == 0) {
+    if (P.partials) P.partials[blockIdx.x] = ((wsum[0] + wsum[1]) + (wsum[2] + wsum[3])) + ((wsum[4] + wsum[5]) + (wsum[6] + wsum[7]));
+    __threadfence();
+    *last_cta = atomicAdd(finished, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (*last_cta) {
+    __threadfence();
+    for (int i = threadIdx.x; i < P.nlayers * P.nrt + 1; i += kRowThreads) P.count[i] = 0u;
+    if (threadIdx.x == 0 && P.partials && P.sum) {
+      double total = *P.sum;
+      for (unsigned i = 0; i < gridDim.x; i++) total += __ldcg(P.partials + i);
+      *P.sum = total;
+    }
+  }
+  if (warp == 2) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
+  }
+}
+
+typedef CUresult (*EncodeTiledFnR)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFnR encode_fn_r() {
+  static EncodeTiledFnR fn = nullptr;
+  if (fn) return fn;
+  void* p = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || !p) return nullptr;
+  return fn = (EncodeTiledFnR)p;
+}
+bool map16(CUtensorMap* m, const void* base, bool f16, long long cols, long long rows, long long pitch_bytes, int box_rows) {
+  EncodeTiledFnR enc = encode_fn_r();
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)pitch_bytes};
+  const cuuint32_t box[2] = {kKc, (cuuint32_t)box_rows}, estr[2] = {1, 1};
+  return enc && enc(m, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+int sms_r() {
+  static int sms = 0;
+  if (sms) return sms;
+  int n = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return sms = n;
+}
+int pitch16(int features) { return (features + 7) / 8 * 8; }
+
+// Rows of a tile: the least multiple of 16 that leaves every SM at most one tile of the widest layer.
+struct RowsTiling { int nr, nrt, w_slots, a_stages, a_bytes; };
+RowsTiling rows_tiling(long long nrows, int nft_max) {
+  RowsTiling T;
+  const long long tiles = sms_r() / nft_max > 0 ? sms_r() / nft_max : 1, per = (nrows + tiles - 1) / tiles;
+  T.nr = per >= kMaxNr ? kMaxNr : (int)((per + 15) / 16 * 16);
+  T.nrt = (int)((nrows + T.nr - 1) / T.nr);
+  T.a_bytes = T.nr * kKc * 2 * kStageChunks;
+  // both rings as far as possible into K = 768: what is behind a ring's end waits for its first MMAs
+  const int left = kSmemRowsMax - kTailRows;
+  T.w_slots = kMaxW; T.a_stages = 0;
+  for (int w = kMaxW; w >= 2; w--) {
+    const int a = (left - w * kWSlotBytes) / T.a_bytes;
+    T.w_slots = w; T.a_stages = a > kMaxA ? kMaxA : a;
+    if (T.a_stages >= w || T.a_stages >= kStagesOfK) break;
+  }
+  return T;
+}
+
+}  // namespace
+
+struct RowsMlp {
+  struct Layer { F16Layer d; CUtensorMap wmap; };
+  std::vector<Layer> layers;
+  const float *in_div = nullptr, *out_mul = nullptr, *relu_mask = nullptr;
+  bool f16 = false;
+  unsigned* count = nullptr;              // zero between launches
+};
+
+void rows_mlp_destroy(RowsMlp* m) {
+  if (!m) return;
+  cudaFree(m->count);
+  delete m;
+}
+
+RowsMlp* rows_mlp_create(const std::vector<F16Layer>& layers, bool f16, const float* in_div, const float* out_mul, const float* relu_mask, std::string* err) {
+  RowsMlp* m = new RowsMlp();
+  m->f16 = f16; m->in_div = in_div; m->out_mul = out_mul; m->relu_mask = relu_mask;
+  auto fail = [&](const char* why) { if (err) *err = why; rows_mlp_destroy(m); return (RowsMlp*)nullptr; };
+  for (auto& d : layers) {
+    m->layers.push_back(RowsMlp::Layer());
+    m->layers.back().d = d;
+    if (!map16(&m->layers.back().wmap, d.w, f16, d.K_pad, d.N_pad, (long long)d.K_pad * 2, kFt)) return fail("cuTensorMapEncodeTiled failed for 16-bit weights");
+  }
+  const size_t n = ((size_t)kRowsMlpMaxRows / 16 * kMaxLayersR + 1) * sizeof(unsigned);
+  if (cudaMalloc(&m->count, n) != cudaSuccess) { m->count = nullptr; cudaGetLastError(); return fail("out of device memory for the counters of 16-bit steps"); }
+  cudaMemset(m->count, 0, n);
+  if (cudaFuncSetAttribute(mlp_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemRowsMax) != cudaSuccess ||
+      cudaFuncSetAttribute(mlp_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemRowsMax) != cudaSuccess)
+    return fail("cannot reserve shared memory for 16-bit steps of few rows");
+  return m;
+}
+
+static bool wide_tiles16(int N, long long nrows, long long sms, long long* rounds) {
+  const long long ntm = (nrows + 127) / 128;
+  const long long r64 = (ntm * ((N + 63) / 64) + sms - 1) / sms, r128 = (ntm * ((N + 127) / 128) + sms - 1) / sms;
+  const bool wide = N > 64 && 3 * r128 < 2 * r64;                // a wide tile's step takes up to 1.5 times as long
+  *rounds = wide ? r128 : r64;
+  return wide;
+}
+
+// What a layer adds to a call, fitted to calls of 1 to 3072 rows and 2 to 8 layers of 16 to 768 features: its launch 2.6 us
+// (4.3 with wide tiles) and 0.3 us (0.27) per step of 64 inputs and round of tiles; the first layer's gather and the end 7 us.
+int rows_mlp_cost(const int* K, const int* N, int nlayers, long long nrows) {
+  int cost = 700;
+  for (int l = 0; l < nlayers; l++) {
+    long long rounds = 1;
+    const bool wide = wide_tiles16(N[l], nrows, 148, &rounds);
+    cost += (wide ? 430 : 260) + (wide ? 27 : 30) * ((K[l] + 63) / 64) * (int)rounds;
+  }
+  return cost;
+}
+
+size_t rows_mlp_input_bytes(int n_in, long long nrows) { return (size_t)nrows * pitch16(n_in) * 2; }
+
+bool rows_mlp_forward(RowsMlp* m, const F32TcLaunch& L, void* x16, cudaStream_t s, std::string* err) {
+  const long long nrows = L.g.count * L.g.nk;
+  if (nrows <= 0) return true;
+  auto fail = [&](const std::string& why) { if (err) *err = why; return false; };
+  const int nl = (int)m->layers.size();
+  if (nl > kMaxLayersR || nrows > kRowsMlpMaxRows) return fail("16-bit step of few rows: too many layers or rows");
+  int nft_max = 1;
+  for (auto& T : m->layers) nft_max = std::max(nft_max, (T.d.n_real + kFt - 1) / kFt);
+  const RowsTiling q = rows_tiling(nrows, nft_max);
+  RowsParams P;
+  std::memset(&P, 0, sizeof P);
+  P.nlayers = nl; P.nr = q.nr; P.nrt = q.nrt; P.nrows = (int)nrows; P.w_slots = q.w_slots; P.a_stages = q.a_stages; P.a_bytes = q.a_bytes;
+  P.n_in = m->layers[0].d.k_real; P.x_pitch = pitch16(P.n_in); P.x16 = (uint16_t*)x16;
+  P.in_div = m->in_div; P.out_mul = m->out_mul; P.relu_mask = m->relu_mask;
+  P.fast_in = L.fast_in; P.slots = L.slots; P.TG = L.TG; P.X = L.X;
+  P.fast_out = L.fast_out; P.store_by_slot = L.store_by_slot; P.TS = L.TS; P.Y = L.Y;
+  std::memcpy(P.cin, L.cin, sizeof P.cin); std::memcpy(P.cout, L.cout, sizeof P.cout);
+  P.g = L.g; P.count = m->count; P.status = L.status;
+  P.partials = L.fast_out ? L.partials : nullptr; P.sum = P.partials ? L.sum : nullptr;
+  P.wait_limit = g_tc_test.wait_limit ? g_tc_test.wait_limit : kWaitLimit;
+  P.test_skip_stage = g_tc_test.skip_stage;
+  const void* in = x16;
+  int in_pitch = P.x_pitch;
+  long long tiles = 1;
+  for (int l = 0; l < nl; l++) {
+    const RowsMlp::Layer& T = m->layers[l];
+    RowsLayer& R = P.layer[l];
+    R.wmap = T.wmap;
+    if (!map16(&R.amap, in, m->f16, T.d.k_real, nrows, (long long)in_pitch * 2, q.nr)) return fail("cuTensorMapEncodeTiled failed for 16-bit activations");
+    R.kchunks = (T.d.k_real + kKc - 1) / kKc; R.nft = (T.d.n_real + kFt - 1) / kFt; R.n_real = T.d.n_real;
+    R.bias = T.d.bias; R.scale = T.d.scale; R.slope = T.d.slope;
+    tiles = std::max<long long>(tiles, (long long)R.nft * q.nrt);
+    if (l < nl - 1) { R.out = (uint16_t*)L.act[l & 1]; R.out_pitch = pitch16(T.d.n_real); in = R.out; in_pitch = R.out_pitch; }
+  }
+  const long long gather = ((nrows + kGatherRows - 1) / kGatherRows * P.layer[0].kchunks + kGatherWarps - 1) / kGatherWarps;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)std::min<long long>(sms_r(), std::max(tiles, gather))); cfg.blockDim = dim3(kRowThreads);
+  cfg.dynamicSmemBytes = (size_t)q.w_slots * kWSlotBytes + (size_t)q.a_stages * q.a_bytes + kTailRows; cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  const cudaError_t e = m->f16 ? cudaLaunchKernelEx(&cfg, mlp_rows_kernel<true>, P) : cudaLaunchKernelEx(&cfg, mlp_rows_kernel<false>, P);
+  if (e != cudaSuccess) return fail(std::string("16-bit step of few rows: ") + cudaGetErrorString(e));
+  return true;
+}
+
+}  // namespace fortis

@@ -1206,9 +1206,8 @@ void tc_model_destroy(TcModel* m) {
 // 933 networks and row counts (2 to 8 layers of 16 to 768 features, alternating widths among them) the form it picks is at
 // most 7 % behind the other one.  Above 3072 rows neither
 // estimate holds (244-768x4-128: 4000 rows 61.8 / 61.9, 8192 62.1 / 75.9).
-constexpr long long kFewRows = 3072;
 bool tc_rows_layer_by_layer(const int* K, const int* N, int nlayers, bool fp8w, long long nrows) {
-  if (nlayers < 2 || nrows > kFewRows) return false;             // (one layer is one launch either way)
+  if (nlayers < 2 || nrows > kRowsMlpMaxRows) return false;             // (one layer is one launch either way)
   int fused = 1270;
   for (int l = 0; l < nlayers; l++) fused += (fp8w ? 245 : 165) + (fp8w ? 130 : 120) * ((K[l] + 255) / 256) * ((N[l] + 255) / 256);
   return rows_mlp_cost(K, N, nlayers, nrows) < fused;
@@ -1305,7 +1304,7 @@ TcModel* tc_model_create(const ModelHost& M, int precision, cudaStream_t s, std:
 bool tc_forward(TcModel* m, const TcLaunch& L, cudaStream_t s, std::string* err) {
   const long long nrows = L.g.count * L.g.nk;
   if (nrows <= 0) return true;
-  if (m->rows && !g_tc_test.no_stage && !L.read_once && L.act[0] && (m->nlayers < 3 || L.act[1]) &&
+  if (m->rows && !g_tc_test.no_stage && L.x16 && L.act[0] && (m->nlayers < 3 || L.act[1]) &&
       tc_rows_layer_by_layer(m->widths, m->widths + 1, m->nlayers, m->has_scale, nrows)) {
     F32TcLaunch R{};
     R.fast_in = L.fast_in; R.slots = L.slots; R.TG = L.TG; R.X = L.X;
@@ -1313,7 +1312,7 @@ bool tc_forward(TcModel* m, const TcLaunch& L, cudaStream_t s, std::string* err)
     std::memcpy(R.cin, L.cin, sizeof R.cin); std::memcpy(R.cout, L.cout, sizeof R.cout);
     R.g = L.g; R.act[0] = L.act[0]; R.act[1] = L.act[1]; R.act_ld = L.act_ld;
     R.partials = L.partials; R.sum = L.sum; R.done = L.done; R.status = L.status;
-    return rows_mlp_forward(m->rows, R, s, err);
+    return rows_mlp_forward(m->rows, R, L.x16, s, err);
   }
   TcParams P;
   std::memset(&P, 0, sizeof P);

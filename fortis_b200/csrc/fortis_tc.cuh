@@ -77,6 +77,30 @@ __device__ __forceinline__ bool mbar_wait_inline(uint32_t bar, uint32_t parity, 
   return false;
 }
 
+// A bounded wait without a function call, which would empty the uniform registers and fix one register budget for all warps.  Every
+// lane of a warp goes on or gives up together; a CTA in which a wait has given up polls no more.
+__device__ __forceinline__ bool wait_polling(uint32_t bar, uint32_t parity, uint32_t limit, volatile int* abort_flag, int* status, int code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .u32 i;\n\tmov.u32 i, 0;\n"
+      "WAIT_LOOP_%=:\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "@p bra WAIT_DONE_%=;\n\t"
+      "add.u32 i, i, 1;\n\t"
+      "setp.lt.u32 q, i, %3;\n\t"
+      "@q bra WAIT_LOOP_%=;\n"
+      "WAIT_DONE_%=:\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok) : "r"(bar), "r"(parity), "r"(*abort_flag ? 1u : limit) : "memory");
+  if (__all_sync(0xffffffffu, ok)) return true;
+  if ((threadIdx.x & 31) == 0) {
+    *abort_flag = 1;
+    atomicCAS(status, 0, code);
+  }
+  return false;
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile(
       "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\t"

@@ -1,0 +1,68 @@
+"""16-bit MLP steps of few rows in one launch (mlp_rows_kernel) at the edges of its tiles (16 to 128 rows x 128 features), with inputs
+gathered from host layouts and read as rows, captured and replayed: the fused kernel's results bit for bit."""
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import fortis_b200
+from fortis_b200 import descriptors as D
+
+
+def randn(shape, seed):
+    return torch.randn(shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(seed))
+
+
+@pytest.mark.parametrize("precision", ["bf16", "fp16", "fp8w"])
+@pytest.mark.parametrize("dims,rows", [([244, 768, 768, 128], 15), ([244, 768, 768, 128], 17), ([244, 768, 768, 128], 385), ([244, 768, 768, 128], 2049),
+                                       ([300, 129, 65, 7], 47), ([8, 16, 1], 49), ([1, 127, 128], 3071), ([256, 640, 257, 128], 1537), ([500, 520, 511, 100], 130), ([5, 1, 3, 2], 3072)])
+def test_edges(precision, dims, rows):
+    layers = fortis_b200.mlp_layers(dims, seed=3, act="leaky", slope=0.15, bias="uniform", scale=0.1)
+    x = randn((rows, dims[0]), 10)
+    got = []
+    h = fortis_b200.Host()
+    for pair in ("1", "default"):
+        h.reset()
+        h.option("tc_pair", pair)
+        h.option("precision", precision)
+        h.load_model(fortis_b200.write_blob(layers))
+        h.L.fortis_begin(rows)
+        y = torch.full((rows, dims[-1]), float("nan"), device="cuda")
+        h.forward_batched(x, y)
+        h.sync()
+        assert h.L.fortis_device_status() == 0
+        got.append(y)
+    assert torch.equal(got[0], got[1])
+    h.reset()
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+@pytest.mark.parametrize("rows", [33, 1000, 2500])
+def test_column_layout_called_again_and_again(rows, graph):
+    """Counters are back at zero behind every launch; tiles of four rows are stored together where they lie together."""
+    layers = fortis_b200.mlp_layers([64, 300, 200, 30], seed=5, act="leaky", slope=0.1, bias="uniform")
+    h = fortis_b200.Host()
+    want = None
+    for pair in ("1", "default"):
+        h.reset()
+        G, S, Lp, K = D.column(rows, 15, nfields=4, nscal=4, nout_fields=2, nout_scal=0)
+        h.configure(gather=G, scatter=S, loop=Lp, kdist=K)
+        h.option("tc_pair", pair)
+        h.option("graph", graph)
+        h.option("precision", "bf16")
+        h.option("checksum", 1)
+        h.load_model(fortis_b200.write_blob(layers))
+        gin = [randn((15, rows), q) for q in range(4)] + [randn(rows, 10 + q) for q in range(4)]
+        out = [torch.zeros((15, rows), device="cuda") for _ in range(2)]
+        for call in range(5):
+            for a in out:
+                a.fill_(float("nan"))
+            h.step(gin, out)
+            h.sync()
+            assert h.L.fortis_device_status() == 0
+            if want is None:
+                want = [a.clone() for a in out]
+            assert all(torch.equal(a, b) for a, b in zip(out, want))
+        total = 5 * sum(float(a.double().sum()) for a in want)
+        assert abs(h.step_checksum() - total) <= 1e-9 * sum(float(a.double().abs().sum()) for a in want)
+    h.reset()
