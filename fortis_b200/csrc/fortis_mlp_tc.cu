@@ -14,7 +14,8 @@
 //     bandwidth is spent on the weights only.
 //   * W streams from L2 through a ring of 32 KB TMA stages (64 features x 256 k, 128-byte swizzle, one 3-D tile
 //     load per stage, no multicast).
-//   * D: two 64-column fp32 accumulators in TMEM; the epilogue of chunk c overlaps the MMAs of chunk c+1.
+//   * D: two 64-column fp32 accumulators in TMEM; the epilogue of chunk c overlaps the MMAs of chunk c+1.  A layer of one K-block has
+//     six: its MMAs are a third of a wide layer's and would wait for the epilogue at every chunk.
 //   * The epilogue (8 warps; thread = one row x 32 features) adds bias, applies the activation, rounds to bf16 and
 //     parks the chunk: chunks 0-9 in shared memory, chunks 10-11 in registers (0-7 and 8-11 with one CTA per SM; A
 //     is still being read by later chunks, so the output cannot overwrite it).  When the layer's last MMA has retired, the parked chunks are
@@ -25,7 +26,7 @@
 //     in the park), any other tile element by element (thread = row, so every access is coalesced).  This fusion is
 //     table-driven and covers fp32 arrays without lifted expressions; any other descriptor is served by the
 //     standalone gather / scatter kernels writing X / reading Y around this kernel.
-// TMEM: 384 (A) + 2 x 64 (D) = 512 columns.  Shared memory: 128 KB parked chunks + 3 x 32 KB weight ring (one CTA per
+// TMEM: 384 (A) + 2 x 64 (D) = 512 columns; layers of one K-block 128 (A) + 6 x 64 (D).  Shared memory: 128 KB parked chunks + 3 x 32 KB weight ring (one CTA per
 // SM), 160 KB parked chunks + 4 x 16 KB ring (CTA of a pair).
 //
 // Every wait on an mbarrier is bounded; a wait that gives up records a code in the status word, raises a CTA-wide
@@ -103,12 +104,20 @@ constexpr int kRingBytes = kStages * kStageBytes;                   // 96 KB
 constexpr int kPairParkChunks = FORTIS_TC_PAIR_PARK;                // two-CTA form: parked chunks in shared memory (8 or 10) ...
 constexpr int kPairStages = (kParkBytes + kRingBytes) / (kStageBytes / 2) - kPairParkChunks;   // ... and the 16 KB stages that fit beside them (6 or 4)
 static_assert(kPairStages >= 3 && kPairStages <= 6 && kPairParkChunks <= 12, "two-CTA form: ring depth");
-constexpr int kBarBytes = 384;             // barriers in the first 256 bytes, then the tensor-memory base, the abort flag and the checksum scratch
+constexpr int kBarBytes = 448;             // barriers in the first 320 bytes and at 328, the tensor-memory base, the abort flag and the checksum scratch
 constexpr int kFastIn = 256, kFastOut = 128;          // widest model input / output the fast I/O tables hold
 constexpr int kTabBytes = kFastIn * 5 + kFastOut * 5 + 2 * kMaxArrays * 8;   // uint32 offset + uint8 code per slot / store, array bases
 constexpr int kSmemBytes = kParkBytes + kRingBytes + kBarBytes + kTabBytes;   // the base must be 1024-byte aligned
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kAccCol0 = 384;
+// Accumulators (64 columns each): two behind A's 384 columns, and in layers of one K-block, whose A takes 128, four more in the
+// columns that are free there.  A chunk's accumulator is the issuer's of its parity, and the pairs of chunks take them in turn.
+// Such a layer's MMAs end before the epilogue of the chunk in front: with two accumulators its issuers wait at every chunk, with six they
+// run half a layer of twelve chunks ahead.  Together with the issue of mma_sub4: 49,152 columns of 244-768x4-128 215.9 -> 199.8 us
+// (bf16), 12,000 columns 99.2 -> 88.4, 262,144 columns with fp8 weights 912 -> 846.
+constexpr int kSlots = 6;
+__device__ __forceinline__ uint32_t acc_slot(int c, uint32_t parity, bool many) { return many ? 2u * ((uint32_t)(c >> 1) % 3u) + parity : parity; }
+__device__ __forceinline__ uint32_t acc_col(uint32_t slot) { return slot < 2 ? kAccCol0 + slot * 64u : 128u + (slot - 2) * 64u; }
 
 // status codes (which wait gave up)
 enum { ST_OK = 0, ST_FULL = 1, ST_EMPTY = 2, ST_ACC_FULL = 3, ST_ACC_EMPTY = 4, ST_A_READY = 5, ST_SMEM_ALIGN = 6, ST_A_DEAD = 7, ST_IN = 8 };
@@ -163,23 +172,30 @@ struct TcParams {
 
 using namespace tc;
 
-// shared-memory matrix descriptor: K-major, 128-byte swizzle, rows 128 B apart, 8-row groups 1024 B apart
-__device__ __forceinline__ uint64_t make_b_desc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFF);            // start address
-  d |= (uint64_t)0 << 16;                            // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;                  // stride byte offset
-  d |= (uint64_t)1 << 46;                            // descriptor version (sm_100)
-  d |= (uint64_t)2 << 61;                            // SWIZZLE_128B
-  return d;
-}
-
 // instruction descriptor: D = f32, A and B both bf16 (format code 1) or both IEEE half (code 0), both K-major,
 // N = 64, M = 128
 template <bool F16, bool PAIR = false> struct MlpIdesc {
   static constexpr uint32_t value = (1u << 4) | (F16 ? 0u : ((1u << 7) | (1u << 10))) | ((uint32_t)(kChunkN >> 3) << 17) |
                                     ((uint32_t)((PAIR ? 2 * kTileM : kTileM) >> 4) << 24);
 };
+// D[tmem] (+)= A[tmem] . B[smem]^T over 64 k: four MMAs, one elected lane issues
+constexpr uint32_t kBDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);      // high word of the descriptor of a K-major, 128-byte-swizzled tile
+template <uint32_t IDESC, bool PAIR>
+__device__ __forceinline__ void mma_sub4(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t accumulate) {
+#define FORTIS_MMA_SUB4(CG)                                                                                            \
+  asm volatile(                                                                                                        \
+      "{\n\t.reg .pred e, q;\n\t.reg .b64 b0, b1, b2, b3;\n\t.reg .b32 a1, a2, a3;\n\t"                                   \
+      "mov.b64 b0, {%2, %4};\n\tadd.s64 b1, b0, 2;\n\tadd.s64 b2, b0, 4;\n\tadd.s64 b3, b0, 6;\n\t"                       \
+      "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"                                            \
+      "setp.ne.b32 q, %5, 0;\n\telect.sync _|e, 0xffffffff;\n\t"                                                       \
+      "@e tcgen05.mma.cta_group::" CG ".kind::f16 [%0], [%1], b0, %3, q;\n\t"                                           \
+      "@e tcgen05.mma.cta_group::" CG ".kind::f16 [%0], [a1], b1, %3, 1;\n\t"                                           \
+      "@e tcgen05.mma.cta_group::" CG ".kind::f16 [%0], [a2], b2, %3, 1;\n\t"                                           \
+      "@e tcgen05.mma.cta_group::" CG ".kind::f16 [%0], [a3], b3, %3, 1;\n\t}"                                          \
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "n"(IDESC), "n"(kBDescHi), "r"(accumulate) : "memory")
+  if constexpr (PAIR) FORTIS_MMA_SUB4("2"); else FORTIS_MMA_SUB4("1");
+#undef FORTIS_MMA_SUB4
+}
 // two consecutive k values as one 32-bit tensor-memory column, in the kernel's 16-bit operand format
 template <bool F16> __device__ __forceinline__ uint32_t pack16(float lo, float hi) {
   if constexpr (F16) { const __half2 v = __floats2half2_rn(lo, hi); return *reinterpret_cast<const uint32_t*>(&v); }
@@ -249,19 +265,20 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
   }
   const uint32_t ring = base + kParkB;                      // kStages x 32 KB
   const uint32_t bars = ring + kRingB;
-  // barrier block: full [kIssuers][kStages] | empty [kStages] | acc_full [2] | acc_empty [2] | a_ready [3] | a_dead [2]
-  // within the first 256 bytes; tmem base 256, abort flag 260, checksum scratch [272,336).
+  // barrier block: full [kIssuers][kStages] | empty [kStages] | acc_full [6] | acc_empty [6] | a_ready [3] | a_dead [2] | retired
+  // within the first 320 bytes; tmem base 320, abort flag 324, two more barriers [328,344), checksum scratch [344,408).
   // Every stage has one "full" barrier PER ISSUER: a parity wait can only tell a barrier's current phase from the
   // previous one, so each barrier needs a single waiter that sees every one of its phases; the TMA warp arms the
   // barrier of the issuer that will consume the stage.
-  static_assert(8 * ((kIssuers + 1) * kStg + 9) <= 256, "the barriers must fit the first 256 bytes of the barrier block");
+  static_assert(8 * ((kIssuers + 1) * kStg + 2 * kSlots + 6) <= 320, "the barriers must fit the first 320 bytes of the barrier block");
   const uint32_t bar_full = bars, bar_empty = bars + 8 * kIssuers * kStg;
-  const uint32_t bar_acc_full = bar_empty + 8 * kStg, bar_acc_empty = bar_acc_full + 16;
-  const uint32_t bar_a_ready = bar_acc_empty + 16, bar_a_dead = bar_a_ready + 24;
-  const uint32_t bar_park = bars + 240;                           // every row thread has read its parked chunks 0-7 of the last hidden layer
-  const uint32_t bar_in = bars + 248;                             // the staged inputs of the next tile have landed (one phase per staged tile)
-  uint32_t* tmem_slot = (uint32_t*)(smem + kParkB + kRingB + 256);
-  volatile int* abort_flag = (volatile int*)(smem + kParkB + kRingB + 260);
+  const uint32_t bar_acc_full = bar_empty + 8 * kStg, bar_acc_empty = bar_acc_full + 8 * kSlots;
+  const uint32_t bar_a_ready = bar_acc_empty + 8 * kSlots, bar_a_dead = bar_a_ready + 24;
+  const uint32_t bar_retired = bar_a_dead + 16;                   // all MMAs of a layer have retired (one phase per layer, seen by the issuers)
+  const uint32_t bar_park = bars + 328;                           // every row thread has read its parked chunks 0-7 of the last hidden layer
+  const uint32_t bar_in = bars + 336;                             // the staged inputs of the next tile have landed (one phase per staged tile)
+  uint32_t* tmem_slot = (uint32_t*)(smem + kParkB + kRingB + 320);
+  volatile int* abort_flag = (volatile int*)(smem + kParkB + kRingB + 324);
   uint32_t* s_off = (uint32_t*)(smem + kParkB + kRingB + kBarBytes);          // [kFastIn] input slot offsets
   uint32_t* o_off = s_off + kFastIn;                                                  // [kFastOut] store offsets
   uint8_t* s_code = (uint8_t*)(o_off + kFastOut);                                     // array | class << 7, 0xFF: none
@@ -271,7 +288,8 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
   const float** s_base_in = (const float**)(o_code + kFastOut);
   float** s_base_out = (float**)(s_base_in + kMaxArrays);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // through a shuffle, so that the compiler knows the roles' branches and addresses to be the same in a whole warp
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const long long ntiles = (P.nrows + kTileM - 1) / kTileM;
   // work units: tiles, or (PAIR) pairs of tiles 2 u and 2 u + 1, one per CTA of the cluster
   uint32_t crank = 0;
@@ -283,7 +301,8 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
   if (threadIdx.x == 0) {
     for (int s = 0; s < kIssuers * kStg; s++) mbar_init(bar_full + 8 * s, 1);
     for (int s = 0; s < kStg; s++) mbar_init(bar_empty + 8 * s, 1);
-    for (int b = 0; b < 2; b++) { mbar_init(bar_acc_full + 8 * b, 1); mbar_init(bar_acc_empty + 8 * b, kRowArrivals); }
+    for (int b = 0; b < kSlots; b++) { mbar_init(bar_acc_full + 8 * b, 1); mbar_init(bar_acc_empty + 8 * b, kRowArrivals); }
+    mbar_init(bar_retired, kIssuers);
     for (int k = 0; k < kMaxKBlocks; k++) mbar_init(bar_a_ready + 8 * k, kRowArrivals);
     for (int k = 0; k < kMaxKBlocks - 1; k++) mbar_init(bar_a_dead + 8 * k, kIssuers);
     mbar_init(bar_in, kEpiThreads);
@@ -340,7 +359,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
   const bool can_stage_out = (__syncthreads_or(stage_out_bad) == 0) && P.fast_out && !P.no_stage_outputs && !P.Y;
   if constexpr (PAIR) cluster_sync_all();      // both CTAs' barriers exist before either signals the other's
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp >= 8) {
     // Register re-allocation between warpgroups (deep-ring build): the producer warpgroup (TMA warp, MMA warp, two idle
@@ -406,7 +425,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
       const uint32_t me = (uint32_t)(warp - 9);
       const uint32_t my_full = bar_full + 8 * kStg * me;
       uint32_t s = 0, full_par = 0, acc_it = 0, lay_it = 0;     // full_par: bit s = parity of this issuer's next phase of stage s
-      const uint64_t desc_hi = make_b_desc(0) & 0xFFFFFFFF00000000ull;
+      uint32_t empty_par = (1u << kSlots) - 1u;                 // bit q: parity of the next phase of accumulator q's "empty"
       PROF_DECL(blockIdx.x == 0 && lane == 0 && me == 0);
       // commits arrive on this CTA's barrier or (PAIR) on the barrier at the same offset in both CTAs
       auto commit = [&](uint32_t bar) { if constexpr (PAIR) tc_commit_pair(bar); else tc_commit(bar); };
@@ -414,9 +433,10 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
         for (int l = 0; l < P.nlayers; l++, lay_it++) {
           const int nchunks = P.layer[l].N / kChunkN, nkb = P.layer[l].K / kBlockK;
           const uint32_t lph = lay_it & 1;
-          bool first = true, any = false;
+          const bool many = nkb == 1;
+          bool first = true, any = false, free_cols = !many || lay_it == 0;
           for (int c = 0; c < nchunks; c++, acc_it++) {
-            const uint32_t b = acc_it & 1, aph = (acc_it >> 1) & 1;
+            const uint32_t b = acc_it & 1;
             if (b != me) {                                    // the other issuer's chunk: step over its stages
               s = (s + (uint32_t)(nkb * kSubStages)) % kStg;
               continue;
@@ -425,10 +445,16 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
             // this issuer's last chunk of the layer: no later chunk lands in accumulator `me`
             const bool mine_last = c + kIssuers >= nchunks;
             PROF_ADDL(0, l);
-            wait_bar(bar_acc_empty + 8 * b, aph ^ 1, abort_flag, P.status, ST_ACC_EMPTY, P.wait_limit);
+            const uint32_t slot = acc_slot(c, b, many);
+            if (!free_cols && slot >= 2) {                    // the layer in front may have read these columns as its A
+              wait_bar(bar_retired, lph ^ 1, abort_flag, P.status, ST_A_DEAD, P.wait_limit);
+              free_cols = true;
+            }
+            wait_bar(bar_acc_empty + 8 * slot, (empty_par >> slot) & 1u, abort_flag, P.status, ST_ACC_EMPTY, P.wait_limit);
+            empty_par ^= 1u << slot;
             PROF_ADDL(2, l);
             tc_fence_after();
-            const uint32_t d_tmem = tmem + kAccCol0 + b * kChunkN;
+            const uint32_t d_tmem = __shfl_sync(0xffffffffu, tmem + acc_col(slot), 0);
             for (int kb = 0; kb < nkb; kb++) {
               if (first) {                                    // K-block kb of this layer's A is in tensor memory
                 PROF_ADDL(0, l);
@@ -442,22 +468,14 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
                 full_par ^= 1u << s;
                 PROF_ADDL(3, l);
                 tc_fence_after();
-                // descriptor of the stage's first 64-wide k sub-tile; the next sub-tile starts kSubBytes further, and
-                // stepping k by 16 inside a 128-byte swizzle row adds 32 bytes (the address field is in 16-byte units)
-                const uint32_t sb = ring + s * kStgBytes;
-                const uint64_t bd0 = desc_hi | (uint64_t)((sb >> 4) & 0x3FFF);
-                const uint32_t a0 = tmem + kb * (kBlockK / 2) + sub * (kStageK / 2);
-                if constexpr (PAIR) {
-                  tc_mma_ts_first_pair<kIdesc>(d_tmem, a0, bd0, (uint32_t)(kb | sub));
+                // A sub-tile's four MMAs at a time: the next sub-tile starts kSubB further, stepping k by 16 inside a 128-byte swizzle
+                // row adds 32 bytes (the address field is in 16-byte units).  Through shuffles: an MMA whose operands the compiler
+                // does not know to be the same in all lanes takes several times as long to issue.
+                const uint32_t bd = __shfl_sync(0xffffffffu, ((ring + s * kStgBytes) >> 4) & 0x3FFFu, 0);
+                const uint32_t a0 = __shfl_sync(0xffffffffu, tmem + kb * (kBlockK / 2) + sub * (kStageK / 2), 0);
 #pragma unroll
-                  for (int j = 1; j < kStageK / 16; j++)
-                    tc_mma_ts_acc_pair<kIdesc>(d_tmem, a0 + j * 8, bd0 + (uint64_t)((j >> 2) * (kSubB >> 4) + (j & 3) * 2));
-                } else {
-                  tc_mma_ts_first<kIdesc>(d_tmem, a0, bd0, (uint32_t)(kb | sub));
-#pragma unroll
-                  for (int j = 1; j < kStageK / 16; j++)
-                    tc_mma_ts_acc<kIdesc>(d_tmem, a0 + j * 8, bd0 + (uint64_t)((j >> 2) * (kSubBytes >> 4) + (j & 3) * 2));
-                }
+                for (int j = 0; j < kStageK / 64; j++)
+                  mma_sub4<kIdesc, PAIR>(d_tmem, a0 + j * 32, bd + (uint32_t)(j * (kSubB >> 4)), j == 0 ? (uint32_t)(kb | sub) : 1u);
                 commit(bar_empty + 8 * s);                    // stage reusable once these MMAs have read it
                 if (++s == kStg) s = 0;
               }
@@ -474,7 +492,9 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
               }
             }
             first = false;
-            commit(bar_acc_full + 8 * b);                     // accumulator complete
+            commit(bar_acc_full + 8 * slot);                  // accumulator complete
+            if (mine_last)
+              for (int rep = 0; rep < (nchunks < kIssuers ? kIssuers : 1); rep++) commit(bar_retired);
           }
           if (!any)                                           // a one-chunk layer: the idle issuer still sees the layer's phases complete
             for (int kb = 0; kb < nkb; kb++) wait_bar(bar_a_ready + 8 * kb, lph, abort_flag, P.status, ST_A_READY, P.wait_limit);
@@ -486,7 +506,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
     const int quad = warp & 3, half = warp >> 2;              // TMEM lane quadrant, which 32 of a chunk's 64 features
     const int r = quad * 32 + lane;                           // row of the tile = TMEM lane
     const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16);
-    uint32_t acc_it = 0, lay_it = 0;
+    uint32_t acc_it = 0, lay_it = 0, acc_par = 0;             // acc_par: bit q = parity of the next phase of accumulator q's "full"
     double csum = 0.0;
     PROF_DECL(blockIdx.x == 0 && threadIdx.x == 0);
     const int per0 = P.layer[0].K / 2;                        // model inputs per half row (padded)
@@ -658,14 +678,14 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
       for (int l = 0; l < P.nlayers; l++, lay_it++) {
         const TcLayer& L = P.layer[l];
         const int nchunks = L.N / kChunkN, nkb = L.K / kBlockK;
-        const bool last = l == P.nlayers - 1;
+        const bool last = l == P.nlayers - 1, many = nkb == 1;
         const float slope = L.slope;
         const uint32_t lph = lay_it & 1;
         if (!last) {
           uint32_t kept[(kMaxChunks - kPark) * 16];     // this thread's parked chunks beyond those in shared memory (16-bit pairs)
           // epilogue of one chunk: accumulator -> (x scale) + bias -> activation -> 16 packed 16-bit pairs
           auto chunk_epilogue = [&](int c, uint32_t (&pk)[16]) {
-            const uint32_t b = acc_it & 1, aph = (acc_it >> 1) & 1;
+            const uint32_t slot = acc_slot(c, acc_it & 1, many);
             acc_it++;
             const int n0 = c * kChunkN + half * 32;
             // the 32 biases of this thread's features: warp-uniform 16-byte loads issued before the wait
@@ -673,14 +693,15 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
 #pragma unroll
             for (int j = 0; j < 8; j++) bq[j] = __ldg(reinterpret_cast<const float4*>(L.bias + n0) + j);
             PROF_ADD(11);
-            wait_bar(bar_acc_full + 8 * b, aph, abort_flag, P.status, ST_ACC_FULL, P.wait_limit);
+            wait_bar(bar_acc_full + 8 * slot, (acc_par >> slot) & 1u, abort_flag, P.status, ST_ACC_FULL, P.wait_limit);
+            acc_par ^= 1u << slot;
             PROF_ADD(10);
             tc_fence_after();
             uint32_t a[32];
-            tmem_ld32(lane_addr + kAccCol0 + b * kChunkN + half * 32, a);
+            tmem_ld32(lane_addr + acc_col(slot) + half * 32, a);
             tmem_ld_wait();
             tc_fence_before();
-            signal(bar_acc_empty + 8 * b);                    // the MMA warp may refill this accumulator
+            signal(bar_acc_empty + 8 * slot);                 // the MMA warp may refill this accumulator
 #pragma unroll
             for (int j = 0; j < 8; j++) {
               // FP8 weights: acc * scale + bias as one fused multiply-add (the last layer's epilogue does the same)
@@ -769,6 +790,8 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
                 }
             }
           }
+          // the next layer's A may go where accumulators lay that the row's other half has yet to read
+          if (many) asm volatile("bar.sync 1, %0;" ::"r"(kEpiThreads) : "memory");
           if (wall <= 0 && 0 < nkb2) move_block(std::integral_constant<int, 0>{}); else if (nkb2 <= 0) signal(bar_a_ready + 0);
           if (wall <= 1 && 1 < nkb2) move_block(std::integral_constant<int, 1>{}); else if (nkb2 <= 1) signal(bar_a_ready + 8);
           // Chunks 0-7 have left the park (what block 2 still reads lies behind them): the first 128 KB may take the next
@@ -868,30 +891,31 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
               prefetched = true;
               PROF_ADD(21);
             }
-            const uint32_t b = acc_it & 1, aph = (acc_it >> 1) & 1;
+            const uint32_t slot = acc_slot(c, acc_it & 1, many);
             acc_it++;
             const int n0 = c * kChunkN + half * 32;
             float4 bq[8];
 #pragma unroll
             for (int j = 0; j < 8; j++) bq[j] = __ldg(reinterpret_cast<const float4*>(L.bias + n0) + j);
             PROF_ADD(13);
-            wait_bar(bar_acc_full + 8 * b, aph, abort_flag, P.status, ST_ACC_FULL, P.wait_limit);
+            wait_bar(bar_acc_full + 8 * slot, (acc_par >> slot) & 1u, abort_flag, P.status, ST_ACC_FULL, P.wait_limit);
+            acc_par ^= 1u << slot;
             PROF_ADD(14);
             tc_fence_after();
             uint32_t a[32];
-            tmem_ld32(lane_addr + kAccCol0 + b * kChunkN + half * 32, a);
+            tmem_ld32(lane_addr + acc_col(slot) + half * 32, a);
             tmem_ld_wait();
             tc_fence_before();
-            signal(bar_acc_empty + 8 * b);
+            signal(bar_acc_empty + 8 * slot);
             float v[32];
 #pragma unroll
             for (int j = 0; j < 8; j++) {
               float4 sq = make_float4(1.f, 1.f, 1.f, 1.f);
               if (HAS_SCALE) sq = __ldg(reinterpret_cast<const float4*>(L.scale + n0) + j);
-              v[4 * j] = act_f(__uint_as_float(a[4 * j]) * sq.x + bq[j].x, slope);
-              v[4 * j + 1] = act_f(__uint_as_float(a[4 * j + 1]) * sq.y + bq[j].y, slope);
-              v[4 * j + 2] = act_f(__uint_as_float(a[4 * j + 2]) * sq.z + bq[j].z, slope);
-              v[4 * j + 3] = act_f(__uint_as_float(a[4 * j + 3]) * sq.w + bq[j].w, slope);
+              v[4 * j] = act_f(HAS_SCALE ? fmaf(__uint_as_float(a[4 * j]), sq.x, bq[j].x) : __uint_as_float(a[4 * j]) + bq[j].x, slope);
+              v[4 * j + 1] = act_f(HAS_SCALE ? fmaf(__uint_as_float(a[4 * j + 1]), sq.y, bq[j].y) : __uint_as_float(a[4 * j + 1]) + bq[j].y, slope);
+              v[4 * j + 2] = act_f(HAS_SCALE ? fmaf(__uint_as_float(a[4 * j + 2]), sq.z, bq[j].z) : __uint_as_float(a[4 * j + 2]) + bq[j].z, slope);
+              v[4 * j + 3] = act_f(HAS_SCALE ? fmaf(__uint_as_float(a[4 * j + 3]), sq.w, bq[j].w) : __uint_as_float(a[4 * j + 3]) + bq[j].w, slope);
             }
             if (P.out_mul || P.relu_mask) {
 #pragma unroll
@@ -914,7 +938,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
                   const uint32_t code = (n0 + j < kFastOut) ? o_code[n0 + j] : 0xFFu;
                   if (code != 0xFF) {
                     *reinterpret_cast<float*>(smem + kOutStage + (n0 + j) * (kTileM * 4) + r * 4) = v[j];
-                    csum += (double)v[j];
+                    if (P.partials) csum += (double)v[j];
                   }
                 }
               } else if (P.fast_out) {
@@ -923,12 +947,14 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
                   const uint32_t code = (n0 + j < kFastOut) ? o_code[n0 + j] : 0xFFu;
                   if (code != 0xFF) {
                     s_base_out[code & 0x7F][(long long)o_off[n0 + j] + ((code & 0x80) ? opos1 : opos0)] = v[j];
-                    csum += (double)v[j];
+                    if (P.partials) csum += (double)v[j];
                   }
                 }
               }
             }
           }
+          // the next tile's A, where it is gathered into more than one K-block, may go where accumulators lay (as above)
+          if (many && !can_prefetch) asm volatile("bar.sync 1, %0;" ::"r"(kEpiThreads) : "memory");
           if (out_staged) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");          // this thread's values, for the copy engine
             asm volatile("bar.sync 1, %0;" ::"r"(kEpiThreads) : "memory");        // every row of every output is there
@@ -949,7 +975,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_tc_fused_kernel(const __grid_
     if (out_pending) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");     // the last tile's output stores are complete
     if (P.partials) {
       // per-CTA checksum partial in a fixed order: shuffle tree per warp, then warp results in index order
-      double* wsum = (double*)(smem + kParkB + kRingB + 272);
+      double* wsum = (double*)(smem + kParkB + kRingB + 344);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) csum += __shfl_down_sync(0xffffffffu, csum, o);
       if (lane == 0) wsum[warp] = csum;
