@@ -38,6 +38,7 @@
 //    channels.  As the threads' own loads and stores, 16 bytes of 32 rows each, they take the data path that shared memory and L1
 //    have in common 1024 clk a tile each, beside the MMAs' operands (2016 clk) and the copies (600).  The buffers cost a quarter of
 //    the activation ring; where that leaves fewer than a tile's three stages (W above 42), and in the last layer, threads store.
+//    Launches of one tile a pair (SOLO) have one group of epilogue warps, 32 channels at a time, and store directly.
 //    8 x 33^3, one layer of 64 channels without / with a residual: 62 / 74.5 us with one group, 58 / 70 with two, 54 / 54 staged
 //    (its MMAs 35).
 //
@@ -79,6 +80,7 @@ constexpr int kXch = 2 * 4 * kC;             // floats exchanged between a group
 constexpr int kXchBytes = 2 * 2 * kXch * 4;  // ... for [group][parity of its tiles]; staged: one buffer, a tile has two exchanges
 constexpr int kResW = 9 * 96 * kC * 2;       // 108 KB: this CTA's half of all 27 weight tiles, resident for the whole kernel
 constexpr int kConvThreads = 576;            // TMA warp, MMA warp, two groups of 8 epilogue warps (two per TMEM lane quadrant)
+constexpr int kSoloThreads = 320;            // ... or one group
 constexpr int kConvSmem = kResW + kRingBytes + 256 + kXchBytes + kC * 4;
 constexpr int kConvSmemStaged = kResW + kRingStaged + kOutAll + 256 + kXchBytes / 2 + kC * 4;
 static_assert(kConvSmem <= 227 * 1024 && kConvSmemStaged <= 227 * 1024, "shared memory");
@@ -142,8 +144,8 @@ __device__ __forceinline__ void cprof_add(long long* prof, int slot, long long* 
 // KSTEPS: 16-wide k steps issued per (kd, kh) group (4 = all 64 input channels, 1 = only the first 16);  NOUT: output
 // channels (weight rows per tap);  LAST: write fp32 NDHWC instead of the padded bf16 volume.
 // Launched as clusters of two CTAs (cta_group::2): the leader's MMA warp issues for both.
-template <int KSTEPS, int NOUT, bool LAST, bool F16, bool STAGED>
-__global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid_constant__ ConvTcParams P) {
+template <int KSTEPS, int NOUT, bool LAST, bool F16, bool STAGED, bool SOLO>
+__global__ void __launch_bounds__(SOLO ? kSoloThreads : kConvThreads, 1) conv3d_tc_kernel(const __grid_constant__ ConvTcParams P) {
   constexpr uint32_t kIdescN = ConvIdesc<NOUT, F16>::value;            // M = 256 (128 rows per CTA), N = 3 * NOUT per group
   constexpr int kWLoads = 9;                                      // weight tiles: one per (kd, kh) group
   constexpr int kHalfRows = 3 * NOUT / 2;      // weight rows of one tile held by each CTA
@@ -275,6 +277,8 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
     constexpr int CW = NOUT == kC ? kC / 2 : NOUT;                 // channels per warp: two warps share a row of 64
     const bool active = NOUT == kC || half == 0;                   // a 16-channel layer needs one warp per quadrant
     const int c0 = NOUT == kC ? CW * half : 0;
+    constexpr int CH = SOLO ? CW : 16;                             // channels at a time: a SOLO block's threads have the registers for all of them
+    static_assert(!SOLO || !STAGED, "SOLO stores directly");
     asm volatile("griddepcontrol.wait;" ::: "memory");           // before the first read of the residual volume and the first store
     const uint32_t acc_full = bar_acc_full + 8 * group, arr_acc_empty = map_to_cta(bar_acc_empty + 8 * group, 0);   // the latter the leader's
     const bool pw = blockIdx.x == 0 && threadIdx.x == 64;
@@ -337,15 +341,15 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
       float* xu = xch + (STAGED ? group : 2 * group + (it & 1)) * kXch + c0;   // kw = 0 partials of each quadrant's last row
       float* xd = xu + 4 * kC;                                     // kw = 2 partials of each quadrant's first row
 #pragma unroll
-      for (int c = 0; c < CW; c += 16) {
-        uint32_t a0[16], a1[16], a2[16];
+      for (int c = 0; c < CW; c += CH) {
+        uint32_t a0[CH], a1[CH], a2[CH];
         if (active) {
-          tmem_ld16(accb + c, a0);
-          tmem_ld16(accb + NOUT + c, a1);
-          tmem_ld16(accb + 2 * NOUT + c, a2);
+          tmem_ldn(accb + c, a0);
+          tmem_ldn(accb + NOUT + c, a1);
+          tmem_ldn(accb + 2 * NOUT + c, a2);
           tmem_ld_wait();
         }
-        if (c + 16 == CW) {
+        if (c + CH == CW) {
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster_relaxed(arr_acc_empty);   // one arrival per warp: the leader may refill this accumulator
@@ -357,31 +361,31 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
         // barrier among the four warps that hold the same channels is enough.)
         if (lane == 31) {
 #pragma unroll
-          for (int i = 0; i < 16; i += 4) *reinterpret_cast<uint4*>(xu + quad * kC + c + i) = make_uint4(a0[i], a0[i + 1], a0[i + 2], a0[i + 3]);
+          for (int i = 0; i < CH; i += 4) *reinterpret_cast<uint4*>(xu + quad * kC + c + i) = make_uint4(a0[i], a0[i + 1], a0[i + 2], a0[i + 3]);
         }
         if (lane == 0) {
 #pragma unroll
-          for (int i = 0; i < 16; i += 4) *reinterpret_cast<uint4*>(xd + quad * kC + c + i) = make_uint4(a2[i], a2[i + 1], a2[i + 2], a2[i + 3]);
+          for (int i = 0; i < CH; i += 4) *reinterpret_cast<uint4*>(xd + quad * kC + c + i) = make_uint4(a2[i], a2[i + 1], a2[i + 2], a2[i + 3]);
         }
         unit_sync();
         if (lane == 31 && quad > 0) {
 #pragma unroll
-          for (int i = 0; i < 16; i += 4) {
+          for (int i = 0; i < CH; i += 4) {
             const uint4 q = *reinterpret_cast<const uint4*>(xu + (quad - 1) * kC + c + i);
             a0[i] = q.x; a0[i + 1] = q.y; a0[i + 2] = q.z; a0[i + 3] = q.w;
           }
         }
         if (lane == 0 && quad < 3) {
 #pragma unroll
-          for (int i = 0; i < 16; i += 4) {
+          for (int i = 0; i < CH; i += 4) {
             const uint4 q = *reinterpret_cast<const uint4*>(xd + (quad + 1) * kC + c + i);
             a2[i] = q.x; a2[i + 1] = q.y; a2[i + 2] = q.z; a2[i + 3] = q.w;
           }
         }
         __syncwarp();
-        float v[16];
+        float v[CH];
 #pragma unroll
-        for (int i = 0; i < 16; i += 4) {
+        for (int i = 0; i < CH; i += 4) {
           const float4 bq = *reinterpret_cast<const float4*>(bias_s + c0 + c + i);
           const float bias[4] = {bq.x, bq.y, bq.z, bq.w};
 #pragma unroll
@@ -425,7 +429,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
         } else {
           if (use_skip) {
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
+            for (int h = 0; h < CH / 8; h++) {
               const uint32_t* s2 = reinterpret_cast<const uint32_t*>(&sk[c / 8 + h]);
 #pragma unroll
               for (int e = 0; e < 4; e++) { const float2 f = cunpack16<F16>(s2[e]); v[8 * h + 2 * e] += f.x; v[8 * h + 2 * e + 1] += f.y; }
@@ -433,12 +437,12 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3d_tc_kernel(const __grid
           }
           if (nuse_skip) {                                         // these registers are free again: the next tile's residual row
 #pragma unroll
-            for (int h = 0; h < 2; h++) sk[c / 8 + h] = ld_global(reinterpret_cast<const uint4*>(P.skip + (size_t)np * kC + c0 + c) + h);
+            for (int h = 0; h < CH / 8; h++) sk[c / 8 + h] = ld_global(reinterpret_cast<const uint4*>(P.skip + (size_t)np * kC + c0 + c) + h);
           }
           if (writes) {
             uint4* dst = reinterpret_cast<uint4*>(P.out + (size_t)p * kC + c0 + c);
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
+            for (int h = 0; h < CH / 8; h++) {
               uint32_t pk[4];
 #pragma unroll
               for (int e = 0; e < 4; e++) {
@@ -547,12 +551,14 @@ float slope_of(const LayerHost& L) { return L.act == ACT_NONE ? 1.f : L.act == A
 }  // namespace
 
 typedef void (*ConvTcKernel)(ConvTcParams);
-// [fp16][first, hidden, last layer, staged first, staged hidden layer]
-const ConvTcKernel kConvKernels[2][5] = {
-    {conv3d_tc_kernel<1, kC, false, false, false>, conv3d_tc_kernel<4, kC, false, false, false>, conv3d_tc_kernel<4, kEdgeC, true, false, false>,
-     conv3d_tc_kernel<1, kC, false, false, true>, conv3d_tc_kernel<4, kC, false, false, true>},
-    {conv3d_tc_kernel<1, kC, false, true, false>, conv3d_tc_kernel<4, kC, false, true, false>, conv3d_tc_kernel<4, kEdgeC, true, true, false>,
-     conv3d_tc_kernel<1, kC, false, true, true>, conv3d_tc_kernel<4, kC, false, true, true>}};
+// [fp16][first, hidden, last layer; the same of one tile a pair of CTAs; staged first, staged hidden layer]
+const ConvTcKernel kConvKernels[2][8] = {
+    {conv3d_tc_kernel<1, kC, false, false, false, false>, conv3d_tc_kernel<4, kC, false, false, false, false>, conv3d_tc_kernel<4, kEdgeC, true, false, false, false>,
+     conv3d_tc_kernel<1, kC, false, false, false, true>, conv3d_tc_kernel<4, kC, false, false, false, true>, conv3d_tc_kernel<4, kEdgeC, true, false, false, true>,
+     conv3d_tc_kernel<1, kC, false, false, true, false>, conv3d_tc_kernel<4, kC, false, false, true, false>},
+    {conv3d_tc_kernel<1, kC, false, true, false, false>, conv3d_tc_kernel<4, kC, false, true, false, false>, conv3d_tc_kernel<4, kEdgeC, true, true, false, false>,
+     conv3d_tc_kernel<1, kC, false, true, false, true>, conv3d_tc_kernel<4, kC, false, true, false, true>, conv3d_tc_kernel<4, kEdgeC, true, true, false, true>,
+     conv3d_tc_kernel<1, kC, false, true, true, false>, conv3d_tc_kernel<4, kC, false, true, true, false>}};
 
 struct ConvTcModel {
   std::vector<LayerHost> meta;
@@ -629,8 +635,8 @@ ConvTcModel* conv_tc_create(const ModelHost& M, bool f16, std::string* err) {
   cudaMemset(m->status, 0, sizeof(int));
   const cudaFuncAttribute att = cudaFuncAttributeMaxDynamicSharedMemorySize;
   for (const ConvTcKernel* k : {kConvKernels[0], kConvKernels[1]})
-    for (int i = 0; i < 5; i++)
-      if (cudaFuncSetAttribute(k[i], att, i < 3 ? kConvSmem : kConvSmemStaged) != cudaSuccess) return fail("cannot reserve shared memory for the tensor-core conv kernel");
+    for (int i = 0; i < 8; i++)
+      if (cudaFuncSetAttribute(k[i], att, i < 6 ? kConvSmem : kConvSmemStaged) != cudaSuccess) return fail("cannot reserve shared memory for the tensor-core conv kernel");
   return m;
 }
 
@@ -671,7 +677,11 @@ bool conv_tc_forward(ConvTcModel* m, const float* x, float* y, int N, int D, int
   const int max_pairs = sms / 2 > 0 ? sms / 2 : 1;
   const int grid = 2 * (int)(npairs < max_pairs ? npairs : max_pairs);          // clusters of two CTAs
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(kConvThreads); cfg.stream = s;
+  // One tile a pair of CTAs: a layer is as long as that tile's chain, a second group would only wait, and one group has the registers for
+  // all of a thread's channels at once.  14 layers in bf16, 3 x 16x24x6 120.7 us (two groups 132.4, staged 129.9), 1 x 5^3 108.3 (121.5,
+  // 120.2); from two tiles on the staged form is faster: 2 x 20^3, 1.15 tiles a pair, 145.5 (one group, before: 153.5).
+  const bool solo = npairs <= max_pairs;
+  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(solo ? kSoloThreads : kConvThreads); cfg.stream = s;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
@@ -694,7 +704,7 @@ bool conv_tc_forward(ConvTcModel* m, const float* x, float* y, int N, int D, int
     P_.amap = m->amaps[cur]; P_.wmap = m->wmaps[l]; P_.bias = m->b[l];
     P_.skip = (L.flags & LFLAG_ADD_SKIP) ? m->buf[skip] + m->front * kC : nullptr;
     P_.out = m->buf[dst] + m->front * kC; P_.y = y; P_.F = L.cout; P_.front = (int)m->front;
-    const bool st = staged && l < nl - 1;
+    const bool st = staged && !solo && l < nl - 1;
     const RingGeom& rg = st ? geom : direct;
     P_.stage_bytes = rg.stage_bytes; P_.nstages = rg.nstages; P_.box_rows = rg.box_rows; P_.nbox = rg.nbox;
     P_.omap = m->omaps[dst];
@@ -703,7 +713,7 @@ bool conv_tc_forward(ConvTcModel* m, const float* x, float* y, int N, int D, int
     P_.wait_limit = g_tc_test.wait_limit ? g_tc_test.wait_limit : kWaitLimit;
     P_.test_skip_stage = g_tc_test.skip_stage;
     P_.D = D; P_.H = H; P_.W = W; P_.P = P; P_.slope = slope_of(L); P_.status = m->status; P_.prof = (want_prof && l == 2) ? dprof : nullptr;
-    const cudaError_t le = cudaLaunchKernelEx(&cfg, kConvKernels[m->f16][l == nl - 1 ? 2 : (l == 0 ? 0 : 1) + (st ? 3 : 0)], P_);
+    const cudaError_t le = cudaLaunchKernelEx(&cfg, kConvKernels[m->f16][(l == nl - 1 ? 2 : l == 0 ? 0 : 1) + (solo ? 3 : st ? 6 : 0)], P_);
     if (le != cudaSuccess) { if (err) *err = std::string("tensor-core conv launch: ") + cudaGetErrorString(le); return false; }
     if (L.flags & LFLAG_SAVE_SKIP) skip = dst;
     cur = dst;
