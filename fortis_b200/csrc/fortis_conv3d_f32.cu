@@ -56,6 +56,10 @@ constexpr float kLoScale = 1024.f;
 // warps: 0 activations, 1 weights (TMA), 2 and 3 MMA issuers, then the epilogue and the storers
 constexpr int kEWarps = 8, kWarpE0 = 4, kWarpS0 = kWarpE0 + kEWarps, kThreads = (kWarpS0 + 4) * 32;
 constexpr int kMaxStages = 8;
+// A turn barrier is used again a weight ring later, which the first issuer cannot reach before the second has issued the step and let go
+// of its weights.  Where the weights stay it is kTurns steps, and the first can be ahead by the tile's steps and the next tile's first two
+// (two accumulators, and the epilogue ends a tile with the second issuer's sums).
+constexpr int kTurns = 8, kMaxResident = kTurns - 2;
 constexpr int kBarBytes = 512;
 constexpr int kSmemMax = 227 * 1024;
 enum { VST_A_FULL = 21, VST_A_EMPTY = 22, VST_ACC_FULL = 23, VST_ACC_EMPTY = 24, VST_ALIGN = 25, VST_W_FULL = 26, VST_W_EMPTY = 27, VST_STASH_FULL = 28,
@@ -189,7 +193,8 @@ __device__ __forceinline__ long long stage_shift(const VolParams& P, int g_) {
   return phase * g.P + ((long long)(g.od0 + kd / g.sd) * g.Hq + g.oh0 + kh / g.sh) * g.Wq + g.ow0 + (LINE ? 1 : kw / g.sw);
 }
 
-template <int NT, bool LINE>
+// RESIDENT: the weight ring holds all steps of a tile and is loaded once
+template <int NT, bool LINE, bool RESIDENT>
 __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vol_kernel(const __grid_constant__ VolParams P) {
   using FM = Form<NT, LINE>;
   constexpr int kWBytes = FM::kWBytes;
@@ -288,6 +293,7 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
               tma_load_2d_pair(w_ring + s * kWBytes, &P.wmap, 0, ((((g * P.tpg + tp) * P.nchb + cb) * P.ntn + nt) * 2 + (int)crank) * FM::kWRows, full0 + 8 * s);
               if (++s == (uint32_t)P.w_stages) { s = 0; ph ^= 1; }
             }
+        if constexpr (RESIDENT) break;
       }
       if (crank == 0)
         for (uint32_t q = 0; q < (uint32_t)P.w_stages; q++) drain_wait(w_full + 8 * q, q < s ? ph : ph ^ 1, P.wait_limit);
@@ -312,7 +318,8 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
             uint32_t row_ = desc_lo(base + as * a_bytes);        // the stage's row of the tile's first row under the present step
             for (int tp = P.tpg; tp > 0; tp--, kt++) {
               // the second follows the first: what the first has waited for is there
-              if (!wait((kFirst ? w_full : turn) + 8 * ws, wph, VST_W_FULL)) return;
+              const uint32_t turn_bar = turn + 8 * (RESIDENT ? chunk_it % kTurns : ws);
+              if (!wait(kFirst ? w_full + 8 * ws : turn_bar, !RESIDENT ? wph : kFirst ? 0 : chunk_it / kTurns & 1, VST_W_FULL)) return;
               // through shuffles: an MMA whose operands the compiler does not know to be the same in all lanes costs 18 clk and more
               // to issue (7 otherwise)
               const uint32_t row = __shfl_sync(0xffffffffu, row_, 0), wd = __shfl_sync(0xffffffffu, desc_lo(w_ring + ws * kWBytes), 0);
@@ -340,13 +347,13 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1) conv_vo
                 }
                 if constexpr (kFirst) {
                   __syncwarp();
-                  if (lane == 0) mbar_arrive(turn + 8 * ws);
+                  if (lane == 0) mbar_arrive(turn_bar);
                 }
                 return true;
               };
               if (!(nk8 == 4 ? groups(std::true_type{}) : groups(std::false_type{}))) return;
               chunk_it++;
-              tc_commit_pair(w_empty + 8 * ws);
+              if constexpr (!RESIDENT) tc_commit_pair(w_empty + 8 * ws);
               if (++ws == (uint32_t)P.w_stages) { ws = 0; wph ^= 1; }
               if (++dw == P.sub_w) { dw = 0; row_ += line; } else row_ += 8;
             }
@@ -689,11 +696,16 @@ EncodeFn encode_fn() {
   return fn = (EncodeFn)p;
 }
 
+int vol_nt(int F) { return F <= 32 ? 32 : 64; }
+
 // How a stage serves steps: those of a kd, of a line, or one; the widest sharing whose rows fit a box and leave two stages.  What
-// shared memory is left goes to the ring that reaches less far ahead, in steps.
-struct Sharing { int ng, tpg, sub_w, box_rows, a_stages, w_stages; size_t smem; };
-bool pick_sharing(const VolGeom& g, int NT, bool line, Sharing* o) {
-  const int nw = line ? 1 : g.KW, w_bytes = (line ? 3 : 1) * NT * kKt * 4;
+// shared memory is left goes to the ring that reaches less far ahead, in steps.  Where a tile's steps are so few that all their weights
+// fit, and two steps' activations beside the present one's, the weights stay (2-D network 4 x 180^2, a line's
+// rows a stage: a quarter of what a step brings in; its layers 29.4 -> 28.4, 38.9 -> 37.4 and 39.5 -> 38.0 us, a call 173.6 -> 169.7).
+struct Sharing { int ng, tpg, sub_w, box_rows, a_stages, w_stages; bool resident; size_t smem; };
+bool pick_sharing(const VolGeom& g, int F, Sharing* o) {
+  const bool line = g.line;
+  const int NT = vol_nt(F), nw = line ? 1 : g.KW, w_bytes = (line ? 3 : 1) * NT * kKt * 4;
   const int fixed = kBarBytes + (line ? Form<32, true>::kXchBytes / 32 * NT : 0) + kM * NT * 4;
   for (int level = 0; level < 3; level++) {
     long long span;
@@ -714,6 +726,16 @@ bool pick_sharing(const VolGeom& g, int NT, bool line, Sharing* o) {
     const int a_bytes = 2 * o->box_rows * kKt * 4;
     int left = kSmemMax - fixed - 2 * a_bytes - 2 * w_bytes;
     if (left < 0) continue;
+    const long long steps = (long long)o->ng * o->tpg * ((g.C + kKt - 1) / kKt);
+    o->resident = false;
+    if (F <= NT && steps <= kMaxResident) {
+      const int n = (kSmemMax - fixed - (int)steps * w_bytes) / a_bytes, a_stages = n < kMaxStages ? n : kMaxStages;
+      if (a_stages >= 2 && (a_stages - 1) * o->tpg >= 2) {
+        o->resident = true; o->a_stages = a_stages; o->w_stages = (int)steps;
+        o->smem = fixed + (size_t)a_stages * a_bytes + (size_t)steps * w_bytes;
+        return true;
+      }
+    }
     o->a_stages = o->w_stages = 2;
     for (;;) {
       const bool a_ok = o->a_stages < kMaxStages && left >= a_bytes, w_ok = o->w_stages < kMaxStages && left >= w_bytes;
@@ -735,7 +757,6 @@ int sm_count() {
   return sms = n;
 }
 
-int vol_nt(int F) { return F <= 32 ? 32 : 64; }
 bool vol_line(int kw, int sw, int pw) { return kw == 3 && sw == 1 && pw <= 1; }       // the taps of a line in one step
 
 }  // namespace
@@ -768,7 +789,8 @@ int vol_front_w(const ConvGeom& c) { return vol_line(c.KW, c.sw, c.pw) ? 0 : c.p
 size_t vol_bytes(const VolGeom& g, int pitch) { return (size_t)g.P * g.fd * g.fh * g.fw * pitch * 8; }
 
 typedef void (*VolKernel)(VolParams);
-const VolKernel kVolKernels[4] = {conv_vol_kernel<32, false>, conv_vol_kernel<64, false>, conv_vol_kernel<32, true>, conv_vol_kernel<64, true>};
+const VolKernel kVolKernels[8] = {conv_vol_kernel<32, false, false>, conv_vol_kernel<64, false, false>, conv_vol_kernel<32, true, false>, conv_vol_kernel<64, true, false>,
+                                  conv_vol_kernel<32, false, true>, conv_vol_kernel<64, false, true>, conv_vol_kernel<32, true, true>, conv_vol_kernel<64, true, true>};
 
 // The widest form (the one that moves registers between its warps) needs the number the compiler gave it (128 a thread); with another
 // compiler's the layers stay on the other kernels.
@@ -777,9 +799,9 @@ bool vol_available() {
     cudaFuncAttributes fa;
     for (VolKernel k : kVolKernels)
       if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess) { cudaGetLastError(); return false; }
-    if (cudaFuncGetAttributes(&fa, kVolKernels[3]) == cudaSuccess && fa.numRegs == 128) return true;
-    cudaGetLastError();
-    return false;
+    for (int k : {3, 7})
+      if (cudaFuncGetAttributes(&fa, kVolKernels[k]) != cudaSuccess || fa.numRegs != 128) { cudaGetLastError(); return false; }
+    return true;
   }();
   return ok;
 }
@@ -806,7 +828,7 @@ bool vol_supported(const ConvGeom& c) {
   if (vol_bytes(g, (c.C + 31) / 32 * 32) > (16ULL << 30)) return false;
   Sharing s;
   // rows, and the last ones a tile may ask for, in 32 bits
-  return g.P * g.fd * g.fh * g.fw < (1LL << 30) && (long long)c.KD * g.Hq * g.Wq < (1LL << 29) && pick_sharing(g, vol_nt(c.F), g.line, &s) && vol_available();
+  return g.P * g.fd * g.fh * g.fw < (1LL << 30) && (long long)c.KD * g.Hq * g.Wq < (1LL << 29) && pick_sharing(g, c.F, &s) && vol_available();
 }
 
 // The rows as one piece, or image by image (which leaves the padding planes between them out) where that takes fewer rounds of tiles:
@@ -828,7 +850,7 @@ Pieces pick_pieces(const VolGeom& g, int ntn) {
 long long vol_kernel_cost(const VolGeom& g, int F) {
   const int NT = vol_nt(F), blocks = (g.C + 31) / 32, last = g.C % 32;
   Sharing s;
-  if (!pick_sharing(g, NT, g.line, &s)) return 1LL << 60;
+  if (!pick_sharing(g, F, &s)) return 1LL << 60;
   const Pieces pc = pick_pieces(g, (F + NT - 1) / NT);
   const long long pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1, tiles = (long long)pc.n * pc.pairs * ((F + NT - 1) / NT), rounds = (tiles + pairs - 1) / pairs;
   const long long taps = s.ng * s.tpg, step = g.line ? (NT == 64 ? 680 : 500) : s.tpg > 1 ? 380 : 570, end = g.line ? (NT == 64 ? 2600 : 2000) : 1500;
@@ -883,7 +905,7 @@ bool vol_conv(const VolW* w, const float* vol, int pitch, const VolGeom& g, cons
               cudaStream_t s, bool early, std::string* err) {
   auto fail = [&](const char* why) { if (err) *err = why; return false; };
   Sharing sh;
-  if (!pick_sharing(g, w->NT, g.line, &sh)) return fail("convolution: no stage layout");
+  if (!pick_sharing(g, w->F, &sh)) return fail("convolution: no stage layout");
   VolParams P;
   std::memset(&P, 0, sizeof P);
   const long long R = g.P * g.fd * g.fh * g.fw;
@@ -913,7 +935,7 @@ bool vol_conv(const VolW* w, const float* vol, int pitch, const VolGeom& g, cons
   at[0].val.programmaticStreamSerializationAllowed = 1;
   static const bool pdl = std::getenv("FORTIS_NO_PDL") == nullptr;
   cfg.attrs = at; cfg.numAttrs = (pdl && early) ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kVolKernels[2 * g.line + (w->NT == 64)], P);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kVolKernels[4 * sh.resident + 2 * g.line + (w->NT == 64)], P);
   if (e != cudaSuccess) { if (err) *err = std::string("convolution launch: ") + cudaGetErrorString(e); return false; }
   g_launches.vol_conv++;
   return true;
