@@ -14,8 +14,8 @@
 //     tile ahead (two buffers, one barrier a tile), so a point's 27 inputs are shared-memory reads at immediate offsets (no
 //     address arithmetic), each input is read from L2 once, and no warp waits for a load;
 //   * a tile's coordinates advance by additions with carries, outputs in the model's order are stored without indexed registers,
-//     and the checksum is added up only where it is asked for.  (1440 x 1080 x 4 points, 27-20-20-3: 310 -> 268 us with the last
-//     two points; the multiply-adds alone take 170 at 128 a clock and SM.)
+//     and the checksum is added up only where it is asked for.  (1440 x 1080 x 4 points, 27-20-20-3, a call: 329 -> 271 us with
+//     the last two points; the multiply-adds alone take 170 at 128 a clock and SM.)
 //   * accumulators start at the bias; ReLU is one instruction per value; outputs are stored coalesced along i.
 // Widths are template parameters (that is what makes every weight an immediate-address operand): hidden widths are
 // padded to 16, 20 or 32, outputs to 4.  Other stencil nets take the generic small-MLP kernel.
