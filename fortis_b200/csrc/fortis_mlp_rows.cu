@@ -16,10 +16,10 @@
 //     each) write the next layer's inputs and add to the counter, or scatter.
 // Inputs are gathered once, by all CTAs, into such rows (layer by layer every feature tile gathered them again).
 //
-// What bounds it: the chain from one layer to the next, not bytes or MMAs.  Clocks of a step of 244-768x4-128 at 30 and 3000 rows: set-up
-// and gather 8900 / 8500; a layer 13,200 / 21,500, of which seeing the count and the first inputs 3000, twelve chunks of MMAs 6300,
-// accumulator to stores 1200 / 8000, stores to the count 2500.  The call, bf16 (fp8 weights within 2 us), layer by layer in launches of
-// 128 x 64 tiles -> here: 1 row 65.4 -> 48.8 us, 300 66.0 -> 53.9, 1000 65.7 -> 56.6, 2000 72.0 -> 62.3, 3072 72.5 -> 66.6.  With
+// What bounds it: the chain from one layer to the next, not bytes or MMAs.  Clocks of a step of 244-768x4-128 at 30 / 3000 rows: set-up
+// and gather 7500 / 8200; a layer 8900 / 13,900, of which seeing the count and the first inputs 1400 / 1500, twelve chunks of MMAs 4600 /
+// 5000, accumulator to stores 1000 / 3700, stores to the count 1600 / 3100.  The call, bf16 (fp8 weights within 2 us), layer by layer in
+// launches of 128 x 64 tiles -> here: 1 row 65.4 -> 48.8 us, 300 66.0 -> 53.9, 1000 65.7 -> 56.6, 2000 72.0 -> 62.3, 3072 72.5 -> 66.6.  With
 // 3073 rows the fused kernel takes 78.8; below 3072 it is chosen where the estimates of rows_mlp_cost and of the caller cross.
 //
 // A count is released by the writing warp (stores, then a releasing add) and acquired by the polling lane (ld.acquire, then the fence
