@@ -800,7 +800,7 @@ bool vol_available() {
     for (VolKernel k : kVolKernels)
       if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess) { cudaGetLastError(); return false; }
     for (int k : {3, 7})
-      if (cudaFuncGetAttributes(&fa, kVolKernels[k]) != cudaSuccess || fa.numRegs != 128) { cudaGetLastError(); return false; }
+      if (!(cudaFuncGetAttributes(&fa, kVolKernels[k]) == cudaSuccess && fa.numRegs == 128)) { cudaGetLastError(); return false; }
     return true;
   }();
   return ok;
