@@ -46,11 +46,14 @@ namespace {
 using namespace tc;
 
 constexpr int kFt = 128, kKc = 64;              // features per tile, k per chunk (a 128-byte swizzle row)
-// chunks of a stage: waits, commits and counting take the issuing warp some 380 clk a stage, whose MMAs take 130 a chunk
-constexpr int kStageChunks = 2;
+// chunks of a stage: waits, commits and counting take the issuing warp some 380 clk a stage, whose MMAs take 130 a chunk.  Calls of 1, 300,
+// 1000, 2000, 3072 rows, us: two chunks 56.3 / 53.5 / 56.0 / 62.2 / 66.6, three 54.9 / 52.6 / 54.9 / 62.3 / 67.1, four 54.8 / 51.8 / 55.1 /
+// 68.2 / 79.5 (only two stages beside the weights).
+constexpr int kStageChunks = 3;
 constexpr int kMaxLayersR = 8, kMaxNr = 128;
 constexpr int kWChunkBytes = kFt * kKc * 2, kWSlotBytes = kStageChunks * kWChunkBytes;
-constexpr int kMaxW = 6, kMaxA = 8, kStagesOfK = 6;   // stages of 768 k
+constexpr int kStagesOfK = 12 / kStageChunks, kMaxW = kStagesOfK, kMaxA = 8;   // stages of 768 k
+static_assert(kMaxW <= 6 && kMaxA <= 8, "room for the barriers");
 constexpr int kEWarpsR = 8;                     // thread = feature; two warps share a lane quadrant and take alternate 32 rows
 constexpr int kRowThreads = (4 + kEWarpsR) * 32;   // warps: weights, inputs, MMA, none, epilogue; all but the first gather
 constexpr int kGatherWarps = 3 + kEWarpsR, kGatherRows = 16;
