@@ -260,140 +260,128 @@ __global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict
   }
 }
 
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {      // two IEEE multiply-adds
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
-      "l"(*reinterpret_cast<unsigned long long*>(&c)));
-  return *reinterpret_cast<float2*>(&d);
-}
-
 // The same layer for few rows (up to 511 of a program's fp32 calls) and small matrices, where the tiles above leave most SMs idle and
-// their warps wait for one load after another.  A block of eight warps owns 4 TM rows x 8 TN features and the warps split K: warp w
-// takes the chunks of KC inputs w, w + 8, ... through two stages of its own (asynchronous copies, no block barrier), every lane TM x TN
-// outputs with the even and the odd k in the two halves of a packed FMA, and the eight sums of an output are added in the order of the
-// warps.  Both operands keep k fastest in shared memory, rows KC + 4 floats apart: the sixteen-byte reads of the eight feature lanes and
-// the four row lanes meet no bank twice.  (Sixteen sums of K/16 products each instead of one of K: nearer to the exact sum.)
-// Bound: the latency of the loads and of the reduction for few tiles, FMA issue for many (linear_tile: both sides measured).
-template <int TM, int TN, int KC>
-__global__ void __launch_bounds__(256, 2) linear_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+// their warps wait for one load after another.  A block of WR x WC warps owns a tile of 4 WR TM rows x 8 WC TN features and streams chunks of
+// kRowsK inputs through S stages of asynchronous copies; a thread owns TM x TN outputs and adds their products in the order of the
+// inputs, as the kernel above does: the same bits.  Both operands keep k fastest in shared memory, rows kRowsK + 4 floats apart: the
+// sixteen-byte reads of the eight feature lanes and the four row lanes meet no bank twice.
+// Bound: the chain of a sum's multiply-adds and the first loads' latency for few tiles, FMA issue and shared-memory reads for many
+// (linear_tile: both sides measured).
+constexpr int kRowsK = 64;
+template <int TM, int TN, int WR, int WC, int S>
+__global__ void __launch_bounds__(WR * WC * 32, 2) linear_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
                                                              float* __restrict__ C, long long M, int N, int K, int act, float slope,
                                                              const float* __restrict__ in_div, const float* __restrict__ out_mul,
                                                              const float* __restrict__ relu_mask, int vec) {
-  constexpr int BM = 4 * TM, BN = 8 * TN, LD = KC + 4, kStage = (BM + BN) * LD, kPieces = KC / 4;
-  static_assert((BM + BN) * kPieces % 32 == 0, "whole warps of pieces");
-  extern __shared__ __align__(16) float rows_smem[];         // [warp][2][BM + BN][LD], then the warps' sums [8][BM][BN + 1] in its place
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rg = lane >> 3, cg = lane & 7;
+  constexpr int BM = 4 * WR * TM, BN = 8 * WC * TN, LD = kRowsK + 4, kStage = (BM + BN) * LD, kPieces = kRowsK / 4, T = WR * WC * 32;
+  static_assert((BM + BN) * kPieces % T == 0, "whole blocks of pieces");
+  extern __shared__ __align__(16) float rows_smem[];         // [S][BM + BN][LD]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r0 = (warp / WC) * 4 * TM + (lane >> 3), c0 = (warp % WC) * 8 * TN + (lane & 7);
   const long long m0 = (long long)blockIdx.x * BM;
   const int n0 = blockIdx.y * BN;
-  float* mine = rows_smem + warp * 2 * kStage;
-  const uint32_t mine_s = (uint32_t)__cvta_generic_to_shared(mine);
-  const int nchunks = (K + KC - 1) / KC;
+  const uint32_t smem_s = (uint32_t)__cvta_generic_to_shared(rows_smem);
+  const int nchunks = (K + kRowsK - 1) / kRowsK;
   auto fetch = [&](int c, int buf) {
-    const int k0 = c * KC;
+    if (c < nchunks) {
+      const int k0 = c * kRowsK;
 #pragma unroll
-    for (int i = 0; i < (BM + BN) * kPieces / 32; i++) {
-      const int e = i * 32 + lane, r = e / kPieces, k = k0 + (e % kPieces) * 4;
-      const bool a = r < BM;
-      const bool live = a ? m0 + r < M : n0 + r - BM < N;
-      const float* src = a ? A + (m0 + r) * K + k : W + (long long)(n0 + r - BM) * K + k;
-      const uint32_t dst = mine_s + (buf * kStage + r * LD + (e % kPieces) * 4) * 4;
-      const int left = live ? K - k : 0;                       // inputs from here on; what lies behind them is filled with zeros
-      if (vec) {
-        const int n = left > 4 ? 16 : left > 0 ? 4 * left : 0;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(n ? src : A), "r"(n) : "memory");
-      } else {
+      for (int i = 0; i < (BM + BN) * kPieces / T; i++) {
+        const int e = i * T + threadIdx.x, r = e / kPieces, k = k0 + (e % kPieces) * 4;
+        const bool a = r < BM;
+        const bool live = a ? m0 + r < M : n0 + r - BM < N;
+        const float* src = a ? A + (m0 + r) * K + k : W + (long long)(n0 + r - BM) * K + k;
+        const uint32_t dst = smem_s + (buf * kStage + r * LD + (e % kPieces) * 4) * 4;
+        const int left = live ? K - k : 0;                     // inputs from here on; what lies behind them is filled with zeros
+        if (vec) {
+          const int n = left > 4 ? 16 : left > 0 ? 4 * left : 0;
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(n ? src : A), "r"(n) : "memory");
+        } else {
 #pragma unroll
-        for (int j = 0; j < 4; j++)
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 4 * j), "l"(left > j ? src + j : A), "r"(left > j ? 4 : 0) : "memory");
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  float2 acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; i++)
-#pragma unroll
-    for (int j = 0; j < TN; j++) acc[i][j] = make_float2(0.f, 0.f);
-  int buf = 0;
-  if (warp < nchunks) fetch(warp, 0);
-  for (int c = warp; c < nchunks; c += 8, buf ^= 1) {
-    if (c + 8 < nchunks) {
-      fetch(c + 8, buf ^ 1);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
-    __syncwarp();
-    float* st = mine + buf * kStage;
-    if (in_div) {
-      for (int e = lane; e < BM * KC; e += 32) {
-        const int r = e / KC, k = e % KC;
-        if (c * KC + k < K) st[r * LD + k] = __fdiv_rn(st[r * LD + k], __ldg(in_div + c * KC + k));
-      }
-      __syncwarp();
-    }
-#pragma unroll
-    for (int q = 0; q < kPieces; q++) {
-      float4 w[TN];
-#pragma unroll
-      for (int j = 0; j < TN; j++) w[j] = *reinterpret_cast<const float4*>(st + (BM + cg + 8 * j) * LD + 4 * q);
-#pragma unroll
-      for (int i = 0; i < TM; i++) {
-        const float4 a = *reinterpret_cast<const float4*>(st + (rg + 4 * i) * LD + 4 * q);
-#pragma unroll
-        for (int j = 0; j < TN; j++) {
-          acc[i][j] = fma2(make_float2(a.x, a.y), make_float2(w[j].x, w[j].y), acc[i][j]);
-          acc[i][j] = fma2(make_float2(a.z, a.w), make_float2(w[j].z, w[j].w), acc[i][j]);
+          for (int j = 0; j < 4; j++)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 4 * j), "l"(left > j ? src + j : A), "r"(left > j ? 4 : 0) : "memory");
         }
       }
     }
-    __syncwarp();                                              // every lane has read this stage before it is filled again
-  }
-  __syncthreads();
+    asm volatile("cp.async.commit_group;" ::: "memory");       // (empty behind the last chunk, so that the count below holds)
+  };
+  float acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; i++)
 #pragma unroll
-    for (int j = 0; j < TN; j++) rows_smem[(warp * BM + rg + 4 * i) * (BN + 1) + cg + 8 * j] = acc[i][j].x + acc[i][j].y;
-  __syncthreads();
-  for (int e = threadIdx.x; e < BM * BN; e += 256) {
-    const int r = e / BN, n = e % BN, nn = n0 + n;
-    if (m0 + r >= M || nn >= N) continue;
-    float v = 0.f;
+    for (int j = 0; j < TN; j++) acc[i][j] = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; w++) v += rows_smem[(w * BM + r) * (BN + 1) + n];
-    v += bias ? __ldg(bias + nn) : 0.f;
-    v = act_apply(v, act, slope);
-    if (out_mul) v = v * out_mul[nn];
-    if (relu_mask && relu_mask[nn] != 0.f) v = max_nan(v, 0.f);
-    C[(m0 + r) * N + nn] = v;
+  for (int c = 0; c < S - 1; c++) fetch(c, c);
+  int buf = 0, next = S - 1;
+  for (int c = 0; c < nchunks; c++) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
+    __syncthreads();                                           // chunk c has landed, and every thread has read the one in front of it
+    fetch(c + S - 1, next);
+    if (++next == S) next = 0;
+    float* st = rows_smem + buf * kStage;
+    if (++buf == S) buf = 0;
+    if (in_div) {
+      for (int e = threadIdx.x; e < BM * kRowsK; e += T) {
+        const int r = e / kRowsK, k = e % kRowsK;
+        if (c * kRowsK + k < K) st[r * LD + k] = __fdiv_rn(st[r * LD + k], __ldg(in_div + c * kRowsK + k));
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int q = 0; q < kPieces; q++) {
+      float4 a[TM], w[TN];
+#pragma unroll
+      for (int j = 0; j < TN; j++) w[j] = *reinterpret_cast<const float4*>(st + (BM + c0 + 8 * j) * LD + 4 * q);
+#pragma unroll
+      for (int i = 0; i < TM; i++) a[i] = *reinterpret_cast<const float4*>(st + (r0 + 4 * i) * LD + 4 * q);
+#pragma unroll
+      for (int i = 0; i < TM; i++)
+#pragma unroll
+        for (int j = 0; j < TN; j++)
+          acc[i][j] = fmaf(a[i].w, w[j].w, fmaf(a[i].z, w[j].z, fmaf(a[i].y, w[j].y, fmaf(a[i].x, w[j].x, acc[i][j]))));
+    }
   }
+#pragma unroll
+  for (int i = 0; i < TM; i++)
+#pragma unroll
+    for (int j = 0; j < TN; j++) {
+      const int nn = n0 + c0 + 8 * j;
+      if (m0 + r0 + 4 * i >= M || nn >= N) continue;
+      float v = acc[i][j] + (bias ? __ldg(bias + nn) : 0.f);
+      v = act_apply(v, act, slope);
+      if (out_mul) v = v * out_mul[nn];
+      if (relu_mask && relu_mask[nn] != 0.f) v = max_nan(v, 0.f);
+      C[(m0 + r0 + 4 * i) * N + nn] = v;
+    }
 }
 
-template <int TM, int TN, int KC>
+template <int TM, int TN, int WR, int WC, int S>
 void launch_linear_rows(const float* A, const float* W, const float* bias, float* C, long long M, int N, int K, int act, float slope,
                         const float* in_div, const float* out_mul, const float* relu_mask, int vec, cudaStream_t s) {
-  constexpr int BM = 4 * TM, BN = 8 * TN, stages = 8 * 2 * (BM + BN) * (KC + 4) * 4, sums = 8 * BM * (BN + 1) * 4, smem = stages > sums ? stages : sums;
-  static const bool set = cudaFuncSetAttribute(linear_rows_kernel<TM, TN, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+  constexpr int BM = 4 * WR * TM, BN = 8 * WC * TN, smem = S * (BM + BN) * (kRowsK + 4) * 4;
+  static const bool set = cudaFuncSetAttribute(linear_rows_kernel<TM, TN, WR, WC, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
   (void)set;
   const dim3 grid((unsigned)((M + BM - 1) / BM), (unsigned)((N + BN - 1) / BN));
-  linear_rows_kernel<TM, TN, KC><<<grid, 256, smem, s>>>(A, W, bias, C, M, N, K, act, slope, in_div, out_mul, relu_mask, vec);
+  linear_rows_kernel<TM, TN, WR, WC, S><<<grid, WR * WC * 32, smem, s>>>(A, W, bias, C, M, N, K, act, slope, in_div, out_mul, relu_mask, vec);
 }
 
-// Which kernel and tile: 0, 1, 2 linear_rows_kernel with 8 x 8, 16 x 16, 32 x 32, 3 the tiles of 128 x 64.  Rounds of blocks over the SMs times
-// a round's time, 0.1 us, fitted to 108 shapes (1 to 30,000 rows, 8 to 2048 features and inputs): what a round costs at K = 0, what 768 inputs
-// add to it, and what they add where rows do not start on 16 bytes.  768 x 768, us, 8 x 8 / 16 x 16 / 32 x 32 / 128 x 64: 3 rows 4.8 / 6.3 /
-// 12.5 / 65.7, 50 rows 10.4 / 8.7 / 12.6 / 78, 300 rows 37 / 22.7 / 20.6 / 96.4, 6000 rows - / 330 / 243 / 320; 64 x 64 at 30,000 rows - / 45.9 /
-// 29.5 / 21.2; 768 x 8 at 1500 rows 62.8 / 26.7 / 16.5 / 8.3.
+// Which kernel and tile: 0 to 3 linear_rows_kernel with 8 x 8, 16 x 16, 32 x 32, 64 x 64, 4 the tiles of 128 x 64.  Rounds of blocks over the
+// SMs times a round's time, 0.1 us, fitted to 108 shapes (1 to 30,000 rows, 8 to 2048 features and inputs): what a call and a round cost at
+// K = 0, what 768 inputs add to them, and what they add to a round where rows do not start on 16 bytes.  Over these shapes the choice
+// costs 1.02 of the fastest in the mean and never more than 128 x 64.  768 x 768, us, 8 x 8 / 16 x 16 / 32 x 32 / 64 x 64 / 128 x 64:
+// 3 rows 8.3 / 10.4 / 18.6 / 32.9 / 65.7, 50 rows 12.4 / 14.5 / 18.6 / 32.9 / 78, 300 rows 43 / 31 / 24.7 / 33 / 96.4, 6000 rows 705 / 461 /
+// 284 / 212 / 319; 768 x 8 at 6000 rows 126 / 58 / 40 / 29.4 / 23.3.
 int linear_tile(long long M, int N, int K, bool vec) {
-  static const int bm[4] = {8, 16, 32, LBM}, bn[4] = {8, 16, 32, LBN}, base[4] = {30, 35, 50, 50}, base_k[4] = {0, 0, 0, 190}, round0[4] = {5, 7, 15, 30},
-                   round_k[4] = {9, 20, 63, 668}, round_off[4] = {10, 18, 46, 0};
+  static const int bm[5] = {8, 16, 32, 64, LBM}, bn[5] = {8, 16, 32, 64, LBN}, base[5] = {36, 36, 29, 28, 31}, base_k[5] = {27, 30, 65, 50, 93},
+                   round0[5] = {2, 4, 11, 28, 29}, round_k[5] = {12, 33, 75, 219, 612}, round_off[5] = {9, 15, 28, 90, 0};
   long long best_cost = 0;
-  int best = 3;
-  for (int t = 3; t >= 0; t--) {
+  int best = 4;
+  for (int t = 4; t >= 0; t--) {
     const long long rows = (M + bm[t] - 1) / bm[t], cols = ((long long)N + bn[t] - 1) / bn[t], rounds = (rows * cols + 147) / 148;
-    if (t < 3 && cols > 65535) continue;                       // the grid's second extent
-    const long long cost = 768 * base[t] + (long long)K * base_k[t] + rounds * (768 * round0[t] + (long long)K * (round_k[t] + (vec ? 0 : round_off[t])));
-    if (t == 3 || cost < best_cost) { best = t; best_cost = cost; }
+    if (t < 4 && cols > 65535) continue;                       // the grid's second extent
+    if (t == 0 && rounds > 16) continue;                       // (there the fit is too low)
+    long long cost = 768 * base[t] + (long long)K * base_k[t] + rounds * (768 * round0[t] + (long long)K * (round_k[t] + (vec ? 0 : round_off[t])));
+    if (t == 4 && M >= 512) cost = cost * 100 / 115;           // many rows: only where the fit's error cannot turn it round
+    if (t == 4 || cost < best_cost) { best = t; best_cost = cost; }
   }
   return best;
 }
@@ -403,9 +391,10 @@ void launch_linear_f32(const float* A, const float* W, const float* bias, float*
   if (M <= 0) return;
   const int vec = K % 4 == 0 && ((uintptr_t)A | (uintptr_t)W) % 16 == 0;
   switch (linear_tile(M, N, K, vec)) {
-    case 0: return launch_linear_rows<2, 1, 32>(A, W, bias, C, M, N, K, act, slope, in_div, out_mul, relu_mask, vec, s);
-    case 1: return launch_linear_rows<4, 2, 32>(A, W, bias, C, M, N, K, act, slope, in_div, out_mul, relu_mask, vec, s);
-    case 2: return launch_linear_rows<8, 4, 16>(A, W, bias, C, M, N, K, act, slope, in_div, out_mul, relu_mask, vec, s);
+    case 0: return launch_linear_rows<1, 1, 2, 1, 6>(A, W, bias, C, M, N, K, act, slope, in_div, out_mul, relu_mask, vec, s);
+    case 1: return launch_linear_rows<2, 1, 2, 2, 5>(A, W, bias, C, M, N, K, act, slope, in_div, out_mul, relu_mask, vec, s);
+    case 2: return launch_linear_rows<4, 2, 2, 2, 4>(A, W, bias, C, M, N, K, act, slope, in_div, out_mul, relu_mask, vec, s);
+    case 3: return launch_linear_rows<4, 4, 4, 2, 3>(A, W, bias, C, M, N, K, act, slope, in_div, out_mul, relu_mask, vec, s);
   }
   dim3 grid((unsigned)((M + LBM - 1) / LBM), (unsigned)((N + LBN - 1) / LBN));
   linear_f32_kernel<<<grid, 256, 0, s>>>(A, W, bias, C, M, N, K, act, slope, in_div, out_mul, relu_mask);
